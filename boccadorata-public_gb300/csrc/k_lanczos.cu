@@ -1190,7 +1190,7 @@ namespace bd {
 //                sums on one SM would take tens of microseconds);
 //   k_lz_groups  a CTA per chain: one-pole groups, the small groups (a warp each), the
 //                sums of the pieces, the eliminations and the cumulative counts.
-constexpr int kGrpThreads = 256;
+constexpr int kGrpThreads = 512;
 constexpr int kGstartThreads = 512;
 constexpr int kGramThreads = 128;
 constexpr int kGramCtas = 608;   // four per SM
@@ -1431,30 +1431,22 @@ __device__ int warp_rank(const double *tri, double *H, int lane) {
 
 // Directions of group q that no coupling reaches, m - rank(M_q), written to gE[N + q].
 // One-pole groups: rank 1 exactly when a coupling is non-zero (the elimination's second
-// pivot is rounding), one thread each over the whole CTA.  Larger groups a warp each,
-// round robin: up to kGrpSmall poles the Gram entries are summed here (lanes over the
-// entries, one FP64 instruction per pole for all of them, when they fit in a warp),
-// beyond that from the pieces' partial sums in piece order; then warp_rank.
+// pivot is rounding), a thread each, kGrpPer of them in flight.  Larger groups a warp each,
+// taken from the warp's ballots (group q belongs to warp q mod the warps, so a few large
+// groups spread over all of them): up to kGrpSmall poles the Gram entries are summed here
+// (lanes over the entries, one FP64 instruction per pole for all of them, when they fit in
+// a warp), beyond that from the pieces' partial sums in piece order; then warp_rank.
+// A dressed propagator's chain has one group per pole, tens of thousands: with each warp
+// walking over its groups one after another to skip the one-pole ones the kernel took
+// 2.47 ms at 2.1 M poles in 52 chains (0.82 ms at 0.9 M in 68).
 template <int D>
 __device__ void group_counts(const LzChain &C, int Q, double *gE, const int *gInfo, const GrpScratch &S, int warp,
                              int lane, double *tri, double *H) {
     constexpr int P = D * (D + 1) / 2;
+    constexpr int kGrpPer = 4, kWarps = kGrpThreads / 32;
     const int N = C.N;
-    for (int q = warp * 32 + lane; q < Q; q += kGrpThreads) {
-        const int h0 = gInfo[1 + q];
-        const int mm = ((q + 1 < Q) ? gInfo[2 + q] : N) - h0;
-        if (mm == 1) {
-            bool any = false;
-#pragma unroll
-            for (int a = 0; a < D; ++a) any |= (C.M[(size_t)a * N + h0] != 0.0);
-            gE[N + q] = any ? 0.0 : 1.0;
-        }
-    }
-    for (int q = warp; q < Q; q += kGrpThreads / 32) {
-        const int g0 = gInfo[1 + q];
-        const int g1 = (q + 1 < Q) ? gInfo[2 + q] : N;
-        const int m = g1 - g0;
-        if (m <= 1) continue;
+    auto large_group = [&](int q, int g0, int m) {
+        const int g1 = g0 + m;
         if (m > kGrpSmall) {
             const double *pp = S.part + (size_t)S.first[q] * kGramEntries;
             const int np = (m + kGrpPiece - 1) / kGrpPiece;
@@ -1498,6 +1490,32 @@ __device__ void group_counts(const LzChain &C, int Q, double *gE, const int *gIn
         __syncwarp();
         const int rank = warp_rank<D>(tri, H, lane);
         if (lane == 0) gE[N + q] = (double)max(0, m - rank);
+    };
+    for (int b = 0; b < Q; b += kGrpPer * kGrpThreads) {
+        int g0[kGrpPer], m[kGrpPer];
+        bool any[kGrpPer];
+#pragma unroll
+        for (int u = 0; u < kGrpPer; ++u) {
+            const int q = b + u * kGrpThreads + lane * kWarps + warp;
+            g0[u] = (q < Q) ? gInfo[1 + q] : 0;
+            m[u] = (q < Q) ? ((q + 1 < Q) ? gInfo[2 + q] : N) - g0[u] : 0;
+            any[u] = false;
+        }
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+#pragma unroll
+            for (int u = 0; u < kGrpPer; ++u)
+                if (m[u] == 1) any[u] |= (C.M[(size_t)a * N + g0[u]] != 0.0);
+#pragma unroll
+        for (int u = 0; u < kGrpPer; ++u)
+            if (m[u] == 1) gE[N + b + u * kGrpThreads + lane * kWarps + warp] = any[u] ? 0.0 : 1.0;
+#pragma unroll
+        for (int u = 0; u < kGrpPer; ++u)
+            for (unsigned big = __ballot_sync(0xffffffffu, m[u] > 1); big; big &= big - 1) {
+                const int src = __ffs(big) - 1;
+                large_group(b + u * kGrpThreads + src * kWarps + warp, __shfl_sync(0xffffffffu, g0[u], src),
+                            __shfl_sync(0xffffffffu, m[u], src));
+            }
     }
 }
 
@@ -1526,14 +1544,26 @@ __global__ void __launch_bounds__(kGrpThreads) k_lz_groups(const LzChain *chains
     }
     __syncthreads();
     // inclusive cumulative counts: gInfo[1 + q] = directions of groups 0..q, so a
-    // direction index finds its group by binary search
+    // direction index finds its group by binary search; eight groups a thread and pass
+    constexpr int kPer = 8;
     int base = 0;
-    for (int b = 0; b < Q; b += kGrpThreads) {
-        const int q = b + tid;
-        const int x = (q < Q) ? (int)gE[N + q] : 0;
+    for (int b = 0; b < Q; b += kPer * kGrpThreads) {
+        int x[kPer], sum = 0;
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+            const int q = b + kPer * tid + u;
+            x[u] = (q < Q) ? (int)gE[N + q] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) sum += x[u];
         int tot;
-        const int ex = block_excl_scan<kGrpThreads>(x, tot, ws);
-        if (q < Q) gInfo[1 + q] = base + ex + x;
+        int ex = base + block_excl_scan<kGrpThreads>(sum, tot, ws);
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+            const int q = b + kPer * tid + u;
+            ex += x[u];
+            if (q < Q) gInfo[1 + q] = ex;
+        }
         base += tot;
     }
 }
