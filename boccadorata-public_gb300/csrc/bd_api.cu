@@ -332,6 +332,7 @@ struct bd_ctx {
     char *d_lzslice = nullptr;
     char *d_lzgrp = nullptr;     // per chain: energy groups and their Gram pieces (lz_group_bytes)
     int *d_lzslot = nullptr;     // per chain: vector slot of every row
+    char *d_lzcp = nullptr;      // per chain (2 I + dir): the reduction in the couplings' space (kCpBytes each)
     LzChain *d_chains = nullptr;
     int lz_two_pass = 0;
     // Dyson
@@ -915,6 +916,10 @@ int dy_cluster_for(const bd_ctx *ctx, int nch) { return nch == 1 ? std::max(ctx-
 // Lanczos chains of channels [ch_lo, ch_hi), both directions.
 int launch_lanczos_range(bd_ctx *ctx, int ch_lo, int ch_hi, bool fp32) {
     const int CL = lz_cluster_for(ctx, ch_hi - ch_lo);
+    // FP64 vectors: chains of few distinct energies are reduced in the space their couplings
+    // span, unless the caller chose where k_lanczos keeps its slices.  (With FP32 vectors the
+    // rounding of the stored vectors is part of the result.)
+    const bool compact = !fp32 && ctx->lz_slices == 0;
     std::vector<LzChain> ch;
     int Smax = 1, rmax = 1;
     for (int I = ch_lo; I < ch_hi; ++I) {
@@ -940,6 +945,8 @@ int launch_lanczos_range(bd_ctx *ctx, int ch_lo, int ch_hi, bool fp32) {
                 z.gE = reinterpret_cast<const double *>(g);
                 z.gInfo = reinterpret_cast<const int *>(g + (size_t)16 * P.N);
                 z.rowslot = ctx->d_lzslot + ctx->lz_slot_off[dir][I];
+                z.cp = ctx->d_lzcp + (size_t)(2 * I + dir) * kCpBytes;
+                z.cp_on = compact;
             }
             z.slice = ctx->d_lzslice + ctx->lz_slice_off[dir][I];
             z.slice_stride = ((long long)z.S * kLzSliceBytesPerPole + 255) / 256 * 256;
@@ -971,6 +978,10 @@ int launch_lanczos_range(bd_ctx *ctx, int ch_lo, int ch_hi, bool fp32) {
     CU(launch_lz_groups(d_ch, (int)ch.size(), gram_cap, ctx->st));   // energy groups for the deflated tails
     ctx->launches += 3;
     CU(record(ctx, ctx->ev_lz[0]));
+    if (compact) {
+        CU(launch_lz_compact(d_ch, (int)ch.size(), ctx->eta, ctx->st));
+        ctx->launches += 1;
+    }
     // chains whose slices do not fit next to the scalars keep them in global memory
     const bool gslices = ctx->lz_slices == 2 || (ctx->lz_slices == 0 && lanczos_smem_bytes(Smax, rmax) > kLanczosSmemSliceCap);
     if (!gslices && lanczos_smem_bytes(Smax, rmax) > (size_t)227 * 1024)
@@ -1157,6 +1168,8 @@ int alloc_lanczos(bd_ctx *ctx) {
     if ((rc = dalloc(ctx, &ctx->d_lzslice, (size_t)slices))) return rc;
     if ((rc = dalloc(ctx, &ctx->d_lzgrp, (size_t)groups))) return rc;
     if ((rc = dalloc(ctx, &ctx->d_lzslot, (size_t)slots))) return rc;
+    if ((rc = dalloc(ctx, &ctx->d_lzcp, (size_t)2 * ctx->nsubsh * (size_t)kCpBytes))) return rc;
+    CU(cudaMemset2DAsync(ctx->d_lzcp, (size_t)kCpBytes, 0, sizeof(CompactInfo), (size_t)2 * ctx->nsubsh, ctx->st));
     return BD_OK;
 }
 
@@ -1664,6 +1677,7 @@ int bd_create(bd_ctx **out, int device) {
     eig_smem_init();
     sigma2_smem_init();
     lanczos_smem_init();
+    compact_smem_init();
     *out = ctx;
     return BD_OK;
 }
@@ -2103,8 +2117,22 @@ int bd_lanczos_vectors(bd_ctx *ctx, int ish, int dir, int fp32, double *out, lon
     const long long need = (long long)P.L * P.N;
     if (!out || cap < need) return fail(ctx, BD_ERR_CAPACITY, "need %lld doubles", need);
     const int ld = lz_ld(P.N);
-    const char *base = ctx->d_lzV + ctx->lz_v_off[dir][ish];
+    char *base = ctx->d_lzV + ctx->lz_v_off[dir][ish];
     CU(cudaStreamSynchronize(ctx->st));
+    if (!fp32 && P.L > 0) {   // a chain reduced in its couplings' space: its vectors over the poles, formed here
+        char *cp = ctx->d_lzcp + (size_t)(2 * ish + dir) * kCpBytes;
+        CompactInfo info;
+        CU(cudaMemcpy(&info, cp, sizeof info, cudaMemcpyDeviceToHost));
+        if (info.handled) {
+            const Chan &C = ctx->chans[ish];
+            LzChain z{};
+            z.N = P.N; z.D = C.D; z.ld = ld; z.V = base; z.cp = cp;
+            z.M = (dir == 0 ? ctx->d_Mfw_s : ctx->d_Mbk_s) + (dir == 0 ? C.mfw_off : C.mbk_off);
+            CU(launch_lz_expand(z, ctx->st));
+            ctx->launches += 1;
+            CU(cudaStreamSynchronize(ctx->st));
+        }
+    }
     // rows of a deflated tail have no stored vector: zero rows
     std::vector<int> slot(std::max(P.L, 0));
     if (P.L > 0)

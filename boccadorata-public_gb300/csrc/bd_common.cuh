@@ -108,6 +108,10 @@ struct LzChain {
     const double *gE;
     const int *gInfo;
     int *rowslot;           // [L] vector slot of every row, -1 for a deflated row (written at the end)
+    // Scratch of the reduction in the space the couplings span (k_compact.cu), nullptr: none;
+    // cp_on: whether this launch may take it (FP64 vectors).
+    char *cp;
+    int cp_on;
 };
 
 // Energy-group scratch of a chain of N poles, behind gE [2N doubles] and gInfo [N + 1
@@ -137,6 +141,39 @@ __host__ __device__ inline GrpScratch lz_grp_scratch(const double *gE, long long
     char *g = reinterpret_cast<char *>(const_cast<double *>(gE));
     return GrpScratch{reinterpret_cast<int *>(g + lz_grp_first_off(N)), reinterpret_cast<int4 *>(g + lz_grp_list_off(N)),
                       reinterpret_cast<double *>(g + lz_grp_part_off(N)), reinterpret_cast<int *>(g + lz_grp_count_off(N))};
+}
+
+// The same chain in the space its couplings span (k_compact.cu): at most kCpGroups distinct
+// energies, kCpMerged groups of them and kCpDim rotated poles.
+constexpr int kCpGroups = 256, kCpMerged = 160, kCpDim = 160;
+struct CompactInfo {
+    int handled;    // 1: k_lz_compact reduced the chain; 0: k_lanczos does
+    int q;          // distinct energies, 0 when there are more than kCpGroups
+    int np, ng;     // rotated poles, groups
+    int nvec;       // vectors stored in V
+};
+struct CompactGroup {
+    int p0, m;      // first pole and poles of the group
+    int c, off;     // its rotated poles, the first one's index
+    int kept;       // 1: the poles themselves, 0: the columns of L
+};
+struct CompactScratch {
+    CompactInfo *info;
+    int *start;          // [kCpGroups + 1] first pole of every energy, then N
+    CompactGroup *grp;   // [kCpMerged]
+    double *gram;        // [kCpGroups][kGramEntries] M M^T of every energy's poles, lower triangle
+    double *L;           // [kCpMerged][64] Cholesky factors, D x D row-major
+    double *V;           // [kCpDim][np] stored vectors
+};
+constexpr long long kCpStartOff = 256, kCpGrpOff = kCpStartOff + 4 * (kCpGroups + 4),
+                    kCpGramOff = (kCpGrpOff + 20 * kCpMerged + 255) / 256 * 256,
+                    kCpLOff = kCpGramOff + 8LL * kCpGroups * kGramEntries, kCpVOff = kCpLOff + 8LL * 64 * kCpMerged,
+                    kCpBytes = (kCpVOff + 8LL * kCpDim * kCpDim + 255) / 256 * 256;
+static_assert(sizeof(CompactInfo) <= kCpStartOff && sizeof(CompactGroup) == 20, "compact scratch layout");
+__host__ __device__ inline CompactScratch lz_compact(char *b) {
+    return CompactScratch{reinterpret_cast<CompactInfo *>(b), reinterpret_cast<int *>(b + kCpStartOff),
+                          reinterpret_cast<CompactGroup *>(b + kCpGrpOff), reinterpret_cast<double *>(b + kCpGramOff),
+                          reinterpret_cast<double *>(b + kCpLOff), reinterpret_cast<double *>(b + kCpVOff)};
 }
 
 // Global scratch of one chain's slices: enough for any cluster size up to 16 with FP64

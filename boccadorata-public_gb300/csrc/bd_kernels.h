@@ -81,6 +81,13 @@ constexpr size_t kLanczosSmemSliceCap = 100 * 1024;   // above this the slices g
 cudaError_t launch_to_float(const double *in, float *out, long long n, cudaStream_t st);
 cudaError_t launch_lz_groups(const LzChain *d_chains, int nchains, long long gram_cap, cudaStream_t st);
 
+// The reduction in the space the couplings span (k_compact.cu): chains with cp_on, after
+// launch_lz_groups and before launch_lanczos, which leaves out the chains it handled; and
+// the stored vectors of such a chain in the poles' space.
+cudaError_t launch_lz_compact(const LzChain *d_chains, int nchains, double eta, cudaStream_t st);
+cudaError_t launch_lz_expand(const LzChain &chain, cudaStream_t st);
+void compact_smem_init();
+
 int dyson_launch_count(int nmax);
 cudaError_t launch_dyson(const DyJob *d_jobs, int njobs, const long long *d_row_first, long long total_rows,
                          int nmax, int Dmax, int cluster, double *work, const long long *d_work_first, cudaStream_t st);

@@ -1,0 +1,459 @@
+// k_compact.cu -- pole sets with few distinct energies, reduced in the space their
+// couplings span.
+//
+// E is diagonal, so inside a group of poles of one energy every rotation leaves the
+// problem unchanged: with M_g (D x m) the group's couplings and G_g = M_g M_g^T = L L^T,
+// the poles M_g^T = Q L^T act through L alone -- D couplings of at most D rotated poles of
+// that energy -- and the other m - D directions couple to nothing.  The unperturbed
+// propagator's spectra have about a dozen distinct energies a channel (the oscillator
+// shells) however many thousand poles they hold, so a chain of N poles is a chain of
+// N' = sum_g rank(M_g) <= 12 D rotated ones: 54 instead of 4 863 for the largest channel
+// at N_max = 10.  alpha, beta, g and m are inner products, the same in both.
+//
+//   k_lz_compact   the multi-pivot Lanczos reduction (k_lanczos's steps, FP64 vectors) of
+//                  a chain in that space, one CTA with the whole basis in shared memory.
+//                  A chain it cannot take is left to k_lanczos (CompactInfo::handled).
+//   k_lz_expand    its stored vectors in the poles' space, v = sum_g M_g^T L^-T v'_g.
+//
+// Energies that differ by rounding only (e1 + e2 - e3 of orbits of the same shells added
+// in another order, a few ulp) count as one group: kMergeUlp ulp of the largest energy, a
+// relative change of E below its own rounding.  The Gram matrices come from k_lz_groups
+// (sums of FP64 products in a fixed order).  A group keeps its poles as they are when it
+// has at most kKeep, or at most kGrpSmall and a pivot that loses digits (below kPivot of
+// its diagonal entry); a larger group with such a pivot leaves the whole chain to
+// k_lanczos.  The reduction depends on a group through G_g only, so the Cholesky factor's
+// backward error, a few eps of G's diagonal, is the rounding of the result.
+#include <cfloat>
+#include "bd_common.cuh"
+#include "bd_kernels.h"
+
+namespace bd {
+
+namespace {
+
+constexpr int kCpThreads = 256;
+constexpr int kCpWarps = kCpThreads / 32;
+constexpr int kKeep = 12;
+constexpr double kMergeUlp = 16.0;
+constexpr double kPivot = 1e-6;
+constexpr int kCpSmem = 200 * 1024;
+
+// Lower-triangular factor of a D x D Gram matrix (lower triangle in tri), a warp; L (D x D,
+// row-major, zero above the diagonal) to out.  A row without couplings (zero diagonal
+// entry) gives a zero column.  False when a pivot falls below kPivot of its diagonal entry
+// or anything is not finite; then out is not to be used.
+__device__ bool warp_cholesky(const double *tri, int D, double *out, int lane) {
+    bool ok = true;
+    for (int e = lane; e < D * D; e += 32) {
+        const int a = e / D, b = e % D;
+        out[e] = (b <= a) ? tri[a * (a + 1) / 2 + b] : 0.0;
+    }
+    __syncwarp();
+    for (int s = 0; s < D; ++s) {
+        const double p = out[s * D + s], g = tri[s * (s + 1) / 2 + s];
+        const bool zero = (g == 0.0);
+        if (!zero && !(p > kPivot * g && p <= DBL_MAX)) ok = false;
+        if (!ok) break;   // the same in every lane
+        const double r = zero ? 0.0 : sqrt(p), ri = zero ? 0.0 : 1.0 / r;
+        __syncwarp();
+        if (lane >= s && lane < D) out[lane * D + s] = (lane == s) ? r : out[lane * D + s] * ri;
+        __syncwarp();
+        for (int e = lane; e < D * D; e += 32) {
+            const int a = e / D, b = e % D;
+            if (a > s && b > s && b <= a) out[e] = fma(-out[a * D + s], out[b * D + s], out[e]);
+        }
+        __syncwarp();
+    }
+    return ok;
+}
+
+// Exclusive scan over one int per thread of the CTA.
+__device__ __forceinline__ int scan_ints(int x, int &total, int *ws) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int v = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += y;
+    }
+    if (lane == 31) ws[warp] = v;
+    __syncthreads();
+    int off = 0;
+    total = 0;
+#pragma unroll
+    for (int w = 0; w < kCpWarps; ++w) {
+        if (w < warp) off += ws[w];
+        total += ws[w];
+    }
+    __syncthreads();
+    return off + v - x;
+}
+
+// The merged groups of a chain (first exact group of each, s_first[0 .. n], s_first[n] = Q)
+// from the exact groups' energies; returns their number.  One thread per exact group.
+__device__ int merge_groups(const double *gE, int Q, int *s_first, int *ws) {
+    const int tid = threadIdx.x;
+    const double tol = kMergeUlp * DBL_EPSILON * fmax(fabs(gE[0]), fabs(gE[Q - 1]));
+    const int brk = (tid < Q) ? (tid == 0 || fabs(gE[tid] - gE[tid - 1]) > tol) : 0;
+    int n;
+    const int pos = scan_ints(brk, n, ws);
+    if (brk) s_first[pos] = tid;
+    if (tid == 0) s_first[n] = Q;
+    __syncthreads();
+    return n;
+}
+
+static_assert(kCpThreads >= kCpGroups, "a thread per exact group");
+
+// A warp's sums of NV values at once (see warp_sums in k_lanczos.cu): lane L ends with the
+// total of value L >> (5 - log2 NV).
+template <int NV>
+__device__ __forceinline__ double warp_sums_d(double *v, int lane) {
+#pragma unroll
+    for (int lev = 0; lev < 5; ++lev) {
+        const int o = 16 >> lev;
+        const int n = NV >> (lev + 1);
+        if (n >= 1) {
+            const bool up = (lane & o) != 0;
+#pragma unroll
+            for (int i = 0; i < (NV >> 1); ++i)
+                if (i < n) {
+                    const double send = up ? v[i] : v[i + n];
+                    const double keep = up ? v[i + n] : v[i];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+    return v[0];
+}
+
+}  // namespace
+
+// ------------------------------------------------------------------ Lanczos
+// One CTA per chain.  The steps, decisions and rows are k_lanczos's with FP64 vectors; a
+// chain that would need what only the full space has (a restart vector, a direction no
+// group has left) is left to k_lanczos as a whole.
+//
+// A step is bound by the FP64 unit (a warp instruction holds an SM sub-partition's for ~64
+// cycles) and by its barriers, so: every vector of the basis in shared memory, a warp per
+// group of four dot products, four barriers a step; and the sweep's update, whose
+// coefficients are rounding-sized after the three-term recurrence, in FP32 from an FP32
+// copy of the basis where |c| <= 1e-9 |w| (its error is below 2^-24 1e-9 |w| < eps |w|).
+// Measured (N_max = 10, 100 iterations per pivot): the reduction of all 84 chains takes
+// 0.49 ms against 3.59 ms in the poles' space (N_max = 12: 0.73 against 12.2).
+__global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains, int nchains, double eta2) {
+    const int cid = blockIdx.x;
+    if (cid >= nchains) return;
+    const LzChain C = chains[cid];
+    if (!C.cp || !C.cp_on) return;
+    const CompactScratch S = lz_compact(C.cp);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int N = C.N, D = C.D, L = C.L, NT = C.nden_out + C.D;
+    const int Q = S.info->q;
+    if (Q < 1) return;   // too many distinct energies (k_lz_groups cleared S.info->handled)
+    __shared__ int ws[kCpWarps];
+    __shared__ int s_first[kCpGroups + 1], s_off[kCpGroups + 1];
+    __shared__ int s_bad;
+    __shared__ double s_tri[kCpWarps][kGramEntries], s_l[kCpWarps][64];
+    extern __shared__ double sm[];
+    if (tid == 0) s_bad = 0;
+    const int ng = merge_groups(C.gE, Q, s_first, ws);
+    if (ng > kCpMerged) return;
+    // 1. every merged group's coordinates: its own poles (kept), or the columns of L
+    for (int g = warp; g < ng; g += kCpWarps) {
+        const int q0 = s_first[g], q1 = s_first[g + 1];
+        const int p0 = S.start[q0], m = S.start[q1] - p0;
+        CompactGroup G;
+        G.p0 = p0; G.m = m; G.kept = 1; G.c = m;
+        if (m > kKeep) {
+            for (int e = lane; e < D * (D + 1) / 2; e += 32) {
+                double s = 0.0;
+                for (int q = q0; q < q1; ++q) s += S.gram[(size_t)q * kGramEntries + e];
+                s_tri[warp][e] = s;
+            }
+            __syncwarp();
+            const bool ok = warp_cholesky(s_tri[warp], D, s_l[warp], lane);
+            if (ok) {
+                G.kept = 0;
+                G.c = D;
+                for (int e = lane; e < D * D; e += 32) S.L[(size_t)g * 64 + e] = s_l[warp][e];
+            } else if (m > kGrpSmall) {
+                if (lane == 0) s_bad = 1;
+            }
+            __syncwarp();
+        }
+        if (lane == 0) { S.grp[g] = G; s_off[g] = G.c; }
+    }
+    __syncthreads();
+    int np;
+    {
+        const int x = (tid < ng) ? s_off[tid] : 0;
+        const int off = scan_ints(x, np, ws);
+        if (tid < ng) s_off[tid] = off;
+        if (tid == 0) s_off[ng] = np;
+        __syncthreads();
+    }
+    const int R = min(L, np);               // vectors, at most
+    const int rq = (R + 4) & ~3;
+    // shared layout (doubles): E[np] | M[D][np] | w[np] | ew[np] | c[rq + 4] | sc[20] | V[R][np],
+    // then floats cf[rq] | Vf[R][np], ints rowslot[L]
+    const size_t need = sizeof(double) * ((size_t)(D + 3) * np + rq + 4 + 20 + (size_t)R * np) +
+                        sizeof(float) * (rq + (size_t)R * np) + sizeof(int) * (size_t)L;
+    if (s_bad || np > kCpDim || need > (size_t)kCpSmem) return;
+    double *E = sm, *M = E + np, *w = M + (size_t)D * np, *ew = w + np, *c = ew + np, *sc = c + rq + 4, *V = sc + 20;
+    float *cf = reinterpret_cast<float *>(V + (size_t)R * np), *Vf = cf + rq;
+    int *rowslot = reinterpret_cast<int *>(Vf + (size_t)R * np);
+    for (int g = warp; g < ng; g += kCpWarps) {
+        const CompactGroup G = S.grp[g];
+        const double e0 = C.E[G.p0], eg = 0.5 * (e0 + C.E[G.p0 + G.m - 1]);
+        for (int i = lane; i < G.c; i += 32) {
+            E[s_off[g] + i] = G.kept ? C.E[G.p0 + i] : eg;
+            for (int d = 0; d < D; ++d)
+                M[(size_t)d * np + s_off[g] + i] = G.kept ? C.M[(size_t)d * N + G.p0 + i] : S.L[(size_t)g * 64 + d * D + i];
+        }
+    }
+    __shared__ int s_start[10], s_last[10], lslot[8], lt[16];
+    __shared__ double lc[16], s_row[32];
+    if (tid <= C.n_used && tid < 10) s_start[tid] = C.start[tid];
+    if (tid < C.n_used && tid < 10) s_last[tid] = C.last[tid];
+    const int Qg = C.gInfo[0];
+    const int dtot = Qg > 0 ? C.gInfo[Qg] : 0;
+    auto group_of = [&](int d) {
+        int lo = 0, hi = Qg - 1;
+        while (lo < hi) { const int mid = (lo + hi) >> 1; if (C.gInfo[1 + mid] > d) hi = mid; else lo = mid + 1; }
+        return lo;
+    };
+    constexpr double tau = 1e-48, thr_exh = 1e-20;   // k_lanczos's, FP64 vectors
+    int dcur = 0, ndefl = 0, nvec = 0, extra = 0, k = -1;
+    double e2v = 0.0;            // |E v|^2 of the last built vector
+    int nl0 = 0;                 // vectors of the next recurrence (lt, lc)
+    // <a_u, b_u> of a warp's four items at once (lane 8 u holds item u's sum)
+    auto dots4 = [&](const double *const *a, const double *const *b, int nu) {
+        double acc[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[u] = 0.0;
+        for (int i = lane; i < np; i += 32)
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (u < nu) acc[u] = fma(a[u][i], b[u][i], acc[u]);
+        return warp_sums_d<4>(acc, lane);
+    };
+    __syncthreads();
+    for (int j = 0; j < L; ++j) {
+        const bool newv = (k + 1 < C.n_used) && (j == s_start[k + 1]);
+        if (newv) ++k;
+        const int nq = k;
+        if (tid < nq) lslot[tid] = rowslot[s_last[tid]];
+        // w = M p, or E v_{j-1} less its known components
+        for (int i = tid; i < np; i += kCpThreads) {
+            double x = 0.0;
+            if (newv) {
+                const double *p = C.piv + (size_t)k * D;
+                for (int d = 0; d < D; ++d) x = fma(M[(size_t)d * np + i], p[d], x);
+            } else {
+                x = V[(size_t)lt[0] * np + i] * E[i];
+                for (int t = 0; t < nl0; ++t) x = fma(-lc[t], V[(size_t)lt[t] * np + i], x);
+            }
+            w[i] = x;
+        }
+        __syncthreads();
+        int fl, nfull = 0;
+        double wn2_first = e2v, x2 = 0.0, ixb = 0.0;
+        for (;;) {
+            // c_t = <v_t, w> for every stored vector, and |w|^2 as item nvec
+            for (int t0 = 4 * warp; t0 <= nvec; t0 += 4 * kCpWarps) {
+                const double *a[4], *b[4];
+                const int nu = min(4, nvec + 1 - t0);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    a[u] = (t0 + u < nvec) ? V + (size_t)(t0 + u) * np : w;
+                    b[u] = w;
+                }
+                const double r = dots4(a, b, nu);
+                if ((lane & 7) == 0 && (lane >> 3) < nu) {
+                    c[t0 + (lane >> 3)] = r;
+                    if (t0 + (lane >> 3) < nvec) cf[t0 + (lane >> 3)] = (float)r;
+                }
+            }
+            __syncthreads();
+            const double wn2 = c[nvec];
+            if (newv && nfull == 0) wn2_first = wn2;
+            // the sweep's size in FP32 (only the choice of the update's arithmetic), then the update
+            float c2 = 0.0f;
+            for (int t = lane; t < nvec; t += 32) c2 = fmaxf(c2, fabsf(cf[t]));
+            for (int o = 16; o > 0; o >>= 1) c2 = fmaxf(c2, __shfl_xor_sync(0xffffffffu, c2, o));
+            const float wf = (float)wn2;
+            const bool small = (c2 * 1e9f) * (c2 * 1e9f) * (float)max(nvec, 1) <= wf && wf > 1e-30f;
+            for (int i = tid; i < np; i += kCpThreads) {
+                double x = w[i];
+                if (small) {
+                    float s0 = 0.0f, s1 = 0.0f;
+                    int t = 0;
+                    for (; t + 1 < nvec; t += 2) {
+                        s0 = fmaf(cf[t], Vf[(size_t)t * np + i], s0);
+                        s1 = fmaf(cf[t + 1], Vf[(size_t)(t + 1) * np + i], s1);
+                    }
+                    if (t < nvec) s0 = fmaf(cf[t], Vf[(size_t)t * np + i], s0);
+                    x -= (double)(s0 + s1);
+                } else {
+                    double s = 0.0;
+                    for (int t = 0; t < nvec; ++t) s = fma(c[t], V[(size_t)t * np + i], s);
+                    x -= s;
+                }
+                w[i] = x;
+                ew[i] = E[i] * x;
+            }
+            __syncthreads();
+            // the scalars of the updated w: |w|^2, <w|E|w>, |E w|^2, <M_d|w>, <v_last(q)|E|w>
+            const int nsc = 3 + D + nq;
+            for (int t0 = 4 * warp; t0 < nsc; t0 += 4 * kCpWarps) {
+                const double *a[4], *b[4];
+                const int nu = min(4, nsc - t0);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int t = t0 + u;
+                    a[u] = w;
+                    b[u] = w;
+                    if (t == 1) b[u] = ew;
+                    else if (t == 2) { a[u] = ew; b[u] = ew; }
+                    else if (t >= 3 && t < 3 + D) a[u] = M + (size_t)(t - 3) * np;
+                    else if (t >= 3 + D && t < nsc && lslot[t - 3 - D] >= 0) { a[u] = V + (size_t)lslot[t - 3 - D] * np; b[u] = ew; }
+                }
+                const double r = dots4(a, b, nu);
+                const int t = t0 + (lane >> 3);
+                if ((lane & 7) == 0 && t < nsc) sc[t] = (t >= 3 + D && lslot[t - 3 - D] < 0) ? 0.0 : r;
+            }
+            __syncthreads();
+            // k_lanczos's decision, by every thread alike
+            x2 = sc[0];
+            if (nvec > 0 && nfull + 1 < 4 && x2 < eta2 * wn2) fl = 1;
+            else if (x2 <= thr_exh * wn2_first || x2 == 0.0) fl = (dcur < dtot) ? 2 : 3;
+            else if (!(x2 <= tau * wn2_first) && x2 <= DBL_MAX) fl = 0;
+            else fl = 3;   // (not finite)
+            if (nfull++ > 0) ++extra;
+            if (fl != 1) break;
+        }
+        if (fl == 3) return;   // the full space's (handled stays 0)
+        if (fl == 2) {
+            // exhausted: the rest of this pivot chain takes unreached directions
+            const int jend = (k + 1 < C.n_used) ? min(L, s_start[k + 1]) : L;
+            const int nr = jend - j;
+            for (int r = tid; r < nr; r += kCpThreads) {
+                const int d = dcur + r;
+                const double a = (d < dtot) ? C.gE[group_of(d)] : C.gE[Qg - 1];
+                double *row = C.out + (size_t)(j + r) * NT;
+                for (int e = 0; e < NT; ++e) row[e] = 0.0;
+                row[0] = a;
+                rowslot[j + r] = -1;
+            }
+            dcur = min(dcur + nr, dtot);
+            ndefl += nr;
+            j = jend - 1;
+            __syncthreads();
+            continue;
+        }
+        if (nvec >= R) return;   // (beyond the space's dimension: not reached with exact arithmetic)
+        // normalise and store; the row
+        ixb = rsqrt_newton(x2);
+        for (int i = tid; i < np; i += kCpThreads) {
+            const double v = w[i] * ixb;
+            V[(size_t)nvec * np + i] = v;
+            Vf[(size_t)nvec * np + i] = (float)v;
+            S.V[(size_t)nvec * np + i] = v;
+        }
+        e2v = sc[2] * ixb * ixb;
+        if (tid < NT) {
+            double x = 0.0;
+            if (tid == 0) x = sc[1] * ixb * ixb;
+            else if (tid == 1) x = (newv && k >= 1) ? sc[3 + D + (k - 1)] * ixb : x2 * ixb;
+            else if (tid < 2 + k) x = sc[3 + D + (tid - 2)] * ixb;
+            else if (tid >= C.nden_out && tid < C.nden_out + D) x = sc[3 + (tid - C.nden_out)] * ixb;
+            s_row[tid] = x;
+            C.out[(size_t)j * NT + tid] = x;
+        }
+        // the next step's recurrence, listed by the warp that holds the row
+        if (warp == 0) {
+            __syncwarp();
+            if (lane == 0) {
+                rowslot[j] = nvec;
+                int n = 0;
+                lt[n] = nvec; lc[n++] = s_row[0];
+                if (j >= 1 && rowslot[j - 1] >= 0) { lt[n] = rowslot[j - 1]; lc[n++] = s_row[1]; }
+                for (int q = 0; q < k; ++q)
+                    if (s_last[q] < j - 1 && rowslot[s_last[q]] >= 0) { lt[n] = rowslot[s_last[q]]; lc[n++] = s_row[2 + q]; }
+                lt[15] = n;
+            }
+        }
+        ++nvec;
+        __syncthreads();
+        nl0 = lt[15];
+    }
+    for (int q = tid; q < L; q += kCpThreads) C.rowslot[q] = rowslot[q];
+    if (tid == 0) {
+        atomicAdd(&C.stat[0], extra);
+        atomicAdd(&C.stat[2], ndefl);
+        S.info->np = np;
+        S.info->ng = ng;
+        S.info->nvec = nvec;
+        S.info->handled = 1;
+    }
+    for (int g = tid; g < ng; g += kCpThreads) S.grp[g].off = s_off[g];
+}
+
+// The stored vectors of a compact chain in the poles' space, into C.V (slot-major, stride
+// ld): a thread per pole, its group's L^-T v' formed by the D-term back substitution
+// against the pole's own couplings (y = L^-1 M_p, then v_p = sum_c y_c v'_c).
+__global__ void k_lz_expand(const LzChain C) {
+    const CompactScratch S = lz_compact(C.cp);
+    const int np = S.info->np, ng = S.info->ng, nvec = S.info->nvec, D = C.D;
+    double *V = reinterpret_cast<double *>(C.V);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < C.N; i += gridDim.x * blockDim.x) {
+        int lo = 0, hi = ng - 1;   // the last group starting at or before pole i
+        while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (S.grp[mid].p0 <= i) lo = mid; else hi = mid - 1; }
+        const CompactGroup G = S.grp[lo];
+        double y[8];
+        if (!G.kept) {
+            const double *Lg = S.L + (size_t)lo * 64;
+#pragma unroll
+            for (int a = 0; a < 8; ++a) {
+                y[a] = 0.0;
+                if (a < D) {
+                    double s = C.M[(size_t)a * C.N + i];
+#pragma unroll
+                    for (int b = 0; b < a; ++b) s = fma(-Lg[a * D + b], y[b], s);
+                    y[a] = (Lg[a * D + a] != 0.0) ? s / Lg[a * D + a] : 0.0;
+                }
+            }
+        }
+        for (int t = 0; t < nvec; ++t) {
+            const double *vt = S.V + (size_t)t * np + G.off;
+            double s = 0.0;
+            if (G.kept) {
+                s = vt[i - G.p0];
+            } else {
+#pragma unroll
+                for (int a = 0; a < 8; ++a) if (a < D) s = fma(y[a], vt[a], s);
+            }
+            V[(size_t)t * C.ld + i] = s;
+        }
+    }
+}
+
+cudaError_t launch_lz_compact(const LzChain *d_chains, int nchains, double eta, cudaStream_t st) {
+    if (nchains <= 0) return cudaSuccess;
+    cudaError_t e = allow_dynamic_smem((const void *)k_lz_compact);
+    if (e != cudaSuccess) return e;
+    k_lz_compact<<<nchains, kCpThreads, kCpSmem, st>>>(d_chains, nchains, eta * eta);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_lz_expand(const LzChain &chain, cudaStream_t st) {
+    k_lz_expand<<<(chain.N + 127) / 128, 128, 0, st>>>(chain);
+    return cudaGetLastError();
+}
+
+void compact_smem_init() { allow_dynamic_smem((const void *)k_lz_compact); }
+
+}  // namespace bd

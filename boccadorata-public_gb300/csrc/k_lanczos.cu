@@ -245,6 +245,7 @@ __global__ void __launch_bounds__(kLzThreads, 2) k_lanczos(const LzChain *chains
     const int cid = blockIdx.x / CL;
     if (cid >= nchains) return;  // whole clusters only: every CTA of a cluster has the same cid
     const LzChain C = chains[cid];
+    if (sizeof(VT) == 8 && C.cp && lz_compact(C.cp).info->handled) return;   // done by k_lz_compact (the whole cluster leaves)
     const int N = C.N, D = C.D, L = C.L, NT = C.nden_out + C.D;
     const int S = C.S;                       // multiple of 4
     const int i0 = rank * S;
@@ -1441,7 +1442,7 @@ __device__ int warp_rank(const double *tri, double *H, int lane) {
 // 2.47 ms at 2.1 M poles in 52 chains (0.82 ms at 0.9 M in 68).
 template <int D>
 __device__ void group_counts(const LzChain &C, int Q, double *gE, const int *gInfo, const GrpScratch &S, int warp,
-                             int lane, double *tri, double *H) {
+                             int lane, double *tri, double *H, double *gram) {
     constexpr int P = D * (D + 1) / 2;
     constexpr int kGrpPer = 4, kWarps = kGrpThreads / 32;
     const int N = C.N;
@@ -1488,6 +1489,8 @@ __device__ void group_counts(const LzChain &C, int Q, double *gE, const int *gIn
                 for (int u = 0; u < P; ++u) tri[u] = G[u];
         }
         __syncwarp();
+        if (gram)   // for the reduction in the couplings' space
+            for (int e = lane; e < P; e += 32) gram[(size_t)q * kGramEntries + e] = tri[e];
         const int rank = warp_rank<D>(tri, H, lane);
         if (lane == 0) gE[N + q] = (double)max(0, m - rank);
     };
@@ -1517,6 +1520,16 @@ __device__ void group_counts(const LzChain &C, int Q, double *gE, const int *gIn
                             __shfl_sync(0xffffffffu, m[u], src));
             }
     }
+    if (gram)   // the one-pole groups' Gram matrices
+        for (int q = warp * 32 + lane; q < Q; q += kGrpThreads) {
+            const int p = gInfo[1 + q];
+            if (((q + 1 < Q) ? gInfo[2 + q] : N) - p != 1) continue;
+            double *G = gram + (size_t)q * kGramEntries;
+#pragma unroll 1
+            for (int a = 0; a < D; ++a)
+#pragma unroll 1
+                for (int b = 0; b <= a; ++b) *G++ = C.M[(size_t)a * N + p] * C.M[(size_t)b * N + p];
+        }
 }
 
 __global__ void __launch_bounds__(kGrpThreads) k_lz_groups(const LzChain *chains, int nchains) {
@@ -1532,15 +1545,26 @@ __global__ void __launch_bounds__(kGrpThreads) k_lz_groups(const LzChain *chains
     __shared__ double s_tri[kGrpThreads / 32][kGramEntries];
     __shared__ double s_h[kGrpThreads / 32][64];
     const int Q = gInfo[0];
+    // the group starts (gInfo's are replaced below) and Gram matrices the reduction in the
+    // couplings' space takes over, when there are few enough
+    double *gram = nullptr;
+    if (C.cp) {
+        const CompactScratch cp = lz_compact(C.cp);
+        const bool on = C.cp_on && Q <= kCpGroups;
+        if (on) gram = cp.gram;
+        if (tid == 0) { cp.info->handled = 0; cp.info->q = on ? Q : 0; }
+        if (on)
+            for (int q = tid; q <= Q; q += kGrpThreads) cp.start[q] = q < Q ? gInfo[1 + q] : N;
+    }
     switch (D) {
-        case 1: group_counts<1>(C, Q, gE, gInfo, S, warp, lane, s_tri[warp], s_h[warp]); break;
-        case 2: group_counts<2>(C, Q, gE, gInfo, S, warp, lane, s_tri[warp], s_h[warp]); break;
-        case 3: group_counts<3>(C, Q, gE, gInfo, S, warp, lane, s_tri[warp], s_h[warp]); break;
-        case 4: group_counts<4>(C, Q, gE, gInfo, S, warp, lane, s_tri[warp], s_h[warp]); break;
-        case 5: group_counts<5>(C, Q, gE, gInfo, S, warp, lane, s_tri[warp], s_h[warp]); break;
-        case 6: group_counts<6>(C, Q, gE, gInfo, S, warp, lane, s_tri[warp], s_h[warp]); break;
-        case 7: group_counts<7>(C, Q, gE, gInfo, S, warp, lane, s_tri[warp], s_h[warp]); break;
-        default: group_counts<8>(C, Q, gE, gInfo, S, warp, lane, s_tri[warp], s_h[warp]); break;
+        case 1: group_counts<1>(C, Q, gE, gInfo, S, warp, lane, s_tri[warp], s_h[warp], gram); break;
+        case 2: group_counts<2>(C, Q, gE, gInfo, S, warp, lane, s_tri[warp], s_h[warp], gram); break;
+        case 3: group_counts<3>(C, Q, gE, gInfo, S, warp, lane, s_tri[warp], s_h[warp], gram); break;
+        case 4: group_counts<4>(C, Q, gE, gInfo, S, warp, lane, s_tri[warp], s_h[warp], gram); break;
+        case 5: group_counts<5>(C, Q, gE, gInfo, S, warp, lane, s_tri[warp], s_h[warp], gram); break;
+        case 6: group_counts<6>(C, Q, gE, gInfo, S, warp, lane, s_tri[warp], s_h[warp], gram); break;
+        case 7: group_counts<7>(C, Q, gE, gInfo, S, warp, lane, s_tri[warp], s_h[warp], gram); break;
+        default: group_counts<8>(C, Q, gE, gInfo, S, warp, lane, s_tri[warp], s_h[warp], gram); break;
     }
     __syncthreads();
     // inclusive cumulative counts: gInfo[1 + q] = directions of groups 0..q, so a

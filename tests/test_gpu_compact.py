@@ -1,0 +1,60 @@
+"""The Lanczos reduction in the space the couplings span (chains of few distinct energies)
+against the reduction over all poles, which bd_set_lanczos_slices(1) keeps."""
+import numpy as np
+import pytest
+
+from helpers import strong_diffs
+
+pytestmark = pytest.mark.gpu
+
+
+# h-bar omega values whose shell energies round to one and to several doubles; groups smaller
+# and larger than a rotation keeps; one step a pivot, truncated and exhausted chains; L = N
+# (every backward chain at N_max = 2, where some need a restart vector and are left to the
+# full space); odd N_max
+@pytest.mark.parametrize("nmax,hw,nit", [(2, 20.0, 10), (3, 13.7, 7), (4, 27.3, 3), (5, 20.0, 1), (6, 11.9, 50),
+                                         (7, 23.1, 30)])
+def test_compact_reduction_equals_full(bdmod, problems, nmax, hw, nit):
+    p = problems(nmax, hw, 3, nit)
+    ctx = bdmod.Context().upload(p)
+    pv = p.piv
+    built = 0
+    for ish in range(p.ms.nsubsh):
+        D = int(p.ms.no[ish])
+        s1 = np.diag(p.ms.orb_xe[p.ms.orb_start[ish]:p.ms.orb_start[ish] + D])
+        got = []
+        for mode in (0, 1):
+            ctx.set_lanczos_slices(mode)
+            ctx.sigma2_build(ish, copy=False)
+            lz = ctx.lanczos_reduce(ish, pv.vec[ish], pv.n_fw[ish], pv.n_bk[ish])
+            got.append((lz, ctx.lanczos_stored()[ish].copy(), ctx.dyson_solve(ish, s1)))
+            if mode == 0:
+                # the stored vectors, formed over the poles: orthonormal, and T = V E V^T on the rows
+                fw, bk = ctx.sigma2_build(ish)
+                for d, sig, tag in ((0, fw, "lz_fw"), (1, bk, "lz_bk")):
+                    L, N = len(lz[tag]), len(sig)
+                    if L == 0:
+                        continue
+                    V = ctx.lanczos_vectors(ish, d, L, N)
+                    on = np.abs(V).max(1) > 0
+                    Vs = V[on]
+                    # a factor's error grows with its pivots' loss, at most 1e3 eps (kPivot)
+                    assert np.abs(Vs @ Vs.T - np.eye(len(Vs))).max() < 1e-12
+                    E = sig[np.argsort(sig[:, 0] if d == 0 else -sig[:, 0], kind="stable"), 0]
+                    alpha = np.einsum("ti,i,ti->t", Vs, E, Vs)
+                    assert np.abs(alpha - lz[tag][on, 0]).max() < 1e-10 * np.abs(E).max()
+                    built += len(Vs)
+        (la, sa, ra), (lb, sb, rb) = got
+        assert np.array_equal(sa, sb), ish                      # as many vectors built
+        for tag in ("lz_fw", "lz_bk"):
+            assert la[tag].shape == lb[tag].shape
+            na = np.abs(la[tag][:, 1:]).max(1) == 0              # the same deflated rows
+            nb = np.abs(lb[tag][:, 1:]).max(1) == 0
+            assert np.array_equal(na, nb) and np.array_equal(la[tag][na], lb[tag][nb]), (ish, tag)
+        for tag in ("qp", "qh"):
+            assert len(ra[tag]) == len(rb[tag])
+            e, z = strong_diffs(rb[tag], ra[tag])
+            assert e < 1e-10 and z < 1e-10, (ish, tag, e, z)
+        np.testing.assert_allclose(ra["koltun"], rb["koltun"], rtol=1e-10, atol=1e-11)
+    assert built > 0
+    ctx.close()
