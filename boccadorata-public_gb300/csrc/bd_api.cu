@@ -337,6 +337,13 @@ struct bd_ctx {
     int lz_two_pass = 0;
     // Dyson
     std::vector<long long> dy_A_off, dy_vec_off, dy_sol_off, dy_R_off, dy_work_off;
+    // full (un-reduced) Dyson: the plain rows with equal energies rotated (launch_plain),
+    // laid out like d_Efw / d_Mfw / d_Ebk / d_Mbk one after another
+    double *d_dyplain = nullptr;
+    char *d_dygrp = nullptr, *d_dycp = nullptr;   // their energy groups (dy_grp_off), Gram matrices and factors
+    LzChain *d_dychains = nullptr;
+    PlainIO *d_dyio = nullptr;
+    std::vector<long long> dy_grp_off[2];
     double *d_dyA = nullptr, *d_dyvec = nullptr, *d_dysol = nullptr, *d_dykol = nullptr, *d_dyR = nullptr,
            *d_dywork = nullptr;
     long long *d_work_first = nullptr;
@@ -503,7 +510,10 @@ void release(bd_ctx *ctx, std::vector<DevBuf> &list) {
     list.clear();
 }
 
-void free_all(bd_ctx *ctx) { release(ctx, ctx->bufs); }
+void free_all(bd_ctx *ctx) {
+    release(ctx, ctx->bufs);
+    ctx->d_dyplain = nullptr;   // ensure_dyson lays the plain rows out again
+}
 void free_static(bd_ctx *ctx) { release(ctx, ctx->sbufs); }
 
 // Allocations made while one of these is alive go to the given list.
@@ -1013,6 +1023,22 @@ int ensure_dyson(bd_ctx *ctx, bool lanczos) {
         ctx->dy_work_off[I] = (long long)w; w += 5 * n * n;
     }
     if (a > (size_t)2 << 30) return fail(ctx, BD_ERR_CAPACITY, "Dyson matrices need %.1f GB", a * 8.0 / 1e9);
+    if (!lanczos && !ctx->d_dyplain) {   // (with the propagator's buffers: the layout follows its pole counts)
+        long long g = 0;
+        for (int dir = 0; dir < 2; ++dir) {
+            ctx->dy_grp_off[dir].assign(ns, 0);
+            for (int I = 0; I < ns; ++I) {
+                ctx->dy_grp_off[dir][I] = g;
+                g += lz_group_bytes(dir == 0 ? ctx->chans[I].nfw : ctx->chans[I].nbk);
+            }
+        }
+        int rc;
+        if ((rc = dalloc(ctx, &ctx->d_dygrp, (size_t)g))) return rc;
+        if ((rc = dalloc(ctx, &ctx->d_dycp, (size_t)2 * ns * (size_t)kCpBytes))) return rc;
+        if ((rc = dalloc(ctx, &ctx->d_dychains, (size_t)2 * ns))) return rc;
+        if ((rc = dalloc(ctx, &ctx->d_dyio, (size_t)2 * ns))) return rc;
+        if ((rc = dalloc(ctx, &ctx->d_dyplain, (size_t)(ctx->tot_fw + ctx->tot_mfw + ctx->tot_bk + ctx->tot_mbk)))) return rc;
+    }
     if (a > ctx->dyA_cap || v > ctx->dyvec_cap || s > ctx->dysol_cap || r > ctx->dyR_cap || w > ctx->dywork_cap) {
         graph_invalidate(ctx);
         CU(cudaStreamSynchronize(ctx->st));
@@ -1050,6 +1076,56 @@ int ensure_dyson(bd_ctx *ctx, bool lanczos) {
     return BD_OK;
 }
 
+// The plain rows of channels [ch_lo, ch_hi) for the full Dyson matrix: the poles sorted,
+// their energy groups and Gram matrices, and every group of equal energies rotated so that
+// only D of its rows couple (k_plain_rotate).  ensure_dyson(ctx, false) must have run.
+double *plain_rows(bd_ctx *ctx, int I, int dir, double **M) {
+    const Chan &C = ctx->chans[I];
+    double *e = ctx->d_dyplain + (dir == 0 ? 0 : ctx->tot_fw + ctx->tot_mfw);
+    *M = e + (dir == 0 ? ctx->tot_fw + C.mfw_off : ctx->tot_bk + C.mbk_off);
+    return e + (dir == 0 ? C.fw_off : C.bk_off);
+}
+
+int launch_plain(bd_ctx *ctx, int ch_lo, int ch_hi) {
+    std::vector<LzChain> ch;
+    std::vector<PlainIO> io;
+    long long gram_cap = 0;
+    for (int I = ch_lo; I < ch_hi; ++I)
+        for (int dir = 0; dir < 2; ++dir) {
+            const Chan &C = ctx->chans[I];
+            const int N = dir == 0 ? C.nfw : C.nbk;
+            if (N <= 0) continue;
+            const long long off = dir == 0 ? C.fw_off : C.bk_off, moff = dir == 0 ? C.mfw_off : C.mbk_off;
+            LzChain z{};
+            z.N = N; z.D = C.D;
+            z.E = (dir == 0 ? ctx->d_Efw_s : ctx->d_Ebk_s) + off;
+            z.M = (dir == 0 ? ctx->d_Mfw_s : ctx->d_Mbk_s) + moff;
+            char *g = ctx->d_dygrp + ctx->dy_grp_off[dir][I];
+            z.gE = reinterpret_cast<const double *>(g);
+            z.gInfo = reinterpret_cast<const int *>(g + (size_t)16 * N);
+            z.cp = ctx->d_dycp + (size_t)(2 * I + dir) * kCpBytes;
+            z.cp_on = 1;
+            PlainIO p{};
+            p.E0 = (dir == 0 ? ctx->d_Efw : ctx->d_Ebk) + off;
+            p.M0 = (dir == 0 ? ctx->d_Mfw : ctx->d_Mbk) + moff;
+            p.E = plain_rows(ctx, I, dir, &p.M);
+            ch.push_back(z);
+            io.push_back(p);
+            gram_cap += lz_gram_cap(N);
+        }
+    if (ch.empty()) return BD_OK;
+    int rc;
+    if ((rc = launch_sort(ctx, ch_lo, ch_hi, false))) return rc;
+    LzChain *d_ch = ctx->d_dychains + 2 * ch_lo;   // this range's own slots
+    PlainIO *d_io = ctx->d_dyio + 2 * ch_lo;
+    if ((rc = h2d_table(ctx, d_ch, ch.data(), sizeof(LzChain) * ch.size()))) return rc;
+    if ((rc = h2d_table(ctx, d_io, io.data(), sizeof(PlainIO) * io.size()))) return rc;
+    CU(launch_lz_groups(d_ch, (int)ch.size(), gram_cap, ctx->st));
+    CU(launch_plain_rotate(d_ch, d_io, (int)ch.size(), ctx->st));
+    ctx->launches += 4;
+    return BD_OK;
+}
+
 // Dyson jobs of channels [ch_lo, ch_hi); ensure_dyson must have run for this mode.
 int launch_dyson_range(bd_ctx *ctx, int ch_lo, int ch_hi, bool lanczos) {
     std::vector<DyJob> jobs;
@@ -1070,8 +1146,9 @@ int launch_dyson_range(bd_ctx *ctx, int ch_lo, int ch_hi, bool lanczos) {
             J.ipiv_bk = ctx->d_lzint + ctx->lz_int_off[1][I] + 2 * (B.n_used + 1);
         } else {
             J.nfw = C.nfw; J.nbk = C.nbk; J.nden = 2;
-            J.E_fw = ctx->d_Efw + C.fw_off; J.M_fw = ctx->d_Mfw + C.mfw_off;
-            J.E_bk = ctx->d_Ebk + C.bk_off; J.M_bk = ctx->d_Mbk + C.mbk_off;
+            double *mf, *mb;   // from launch_plain
+            J.E_fw = plain_rows(ctx, I, 0, &mf); J.M_fw = mf;
+            J.E_bk = plain_rows(ctx, I, 1, &mb); J.M_bk = mb;
         }
         J.n = C.D + J.nfw + J.nbk;
         J.nc = J.n;   // k_dyson_deflate sets the order after deflation
@@ -1993,6 +2070,7 @@ int bd_dyson_solve(bd_ctx *ctx, int ish, const double *sig1b, const double *sig_
     const double saved_ef = C.efermi;
     if (!std::isnan(e_fermi)) { C.efermi = e_fermi; ctx->ef_override = true; }
     rc = ensure_dyson(ctx, C.state == ST_LANCZOS);
+    if (!rc && C.state != ST_LANCZOS) rc = launch_plain(ctx, ish, ish + 1);
     if (!rc) rc = launch_dyson_range(ctx, ish, ish + 1, C.state == ST_LANCZOS);
     C.efermi = saved_ef;
     ctx->ef_override = false;
@@ -2175,6 +2253,7 @@ int enqueue_step(bd_ctx *ctx, int flags) {
         CU(record(ctx, ctx->ev[2]));
         if (lanczos) for (int I = 0; I < ns; ++I) if ((rc = launch_lanczos_range(ctx, I, I + 1, fp32))) return rc;
         CU(record(ctx, ctx->ev[3]));
+        if (!lanczos) for (int I = 0; I < ns; ++I) if ((rc = launch_plain(ctx, I, I + 1))) return rc;
         for (int I = 0; I < ns; ++I) if ((rc = launch_dyson_range(ctx, I, I + 1, lanczos))) return rc;
     } else {
         // The static self-energy (EHF) depends only on the propagator and is read only by
@@ -2195,6 +2274,7 @@ int enqueue_step(bd_ctx *ctx, int flags) {
         CU(record(ctx, ctx->ev[2]));
         if (lanczos && (rc = launch_lanczos_range(ctx, 0, ns, fp32))) return rc;
         CU(record(ctx, ctx->ev[3]));
+        if (!lanczos && (rc = launch_plain(ctx, 0, ns))) return rc;
         CU(cudaStreamWaitEvent(ctx->st, ctx->ev_join, 0));
         if ((rc = launch_dyson_range(ctx, 0, ns, lanczos))) return rc;
     }

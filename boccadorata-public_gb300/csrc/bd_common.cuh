@@ -176,6 +176,12 @@ __host__ __device__ inline CompactScratch lz_compact(char *b) {
                           reinterpret_cast<double *>(b + kCpLOff), reinterpret_cast<double *>(b + kCpVOff)};
 }
 
+// Rows of a plain Sigma(2) for the full Dyson matrix (k_plain_rotate): as built, and rotated.
+struct PlainIO {
+    const double *E0, *M0;
+    double *E, *M;
+};
+
 // Global scratch of one chain's slices: enough for any cluster size up to 16 with FP64
 // slices (E, w and E w as doubles and a touched byte: 25 bytes per pole, each CTA's share
 // rounded up to 256 bytes); a multiple of 256 bytes, so consecutive chains' slices stay

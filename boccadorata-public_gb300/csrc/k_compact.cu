@@ -14,6 +14,11 @@
 //                  a chain in that space, one CTA with the whole basis in shared memory.
 //                  A chain it cannot take is left to k_lanczos (CompactInfo::handled).
 //   k_lz_expand    its stored vectors in the poles' space, v = sum_g M_g^T L^-T v'_g.
+//   k_plain_rotate the plain Sigma(2) rows of the full Dyson matrix with every group of
+//                  more than kKeep poles rotated the same way: its first D rows couple by L, the
+//                  others not at all, and k_dyson_deflate takes those out of the matrix
+//                  (N_max = 4 without Lanczos: a step of 152 ms, 111 of them spent on
+//                  orthonormalising clusters of a hundred equal eigenvalues, takes 0.92).
 //
 // Energies that differ by rounding only (e1 + e2 - e3 of orbits of the same shells added
 // in another order, a few ulp) count as one group: kMergeUlp ulp of the largest energy, a
@@ -439,6 +444,63 @@ __global__ void k_lz_expand(const LzChain C) {
             V[(size_t)t * C.ld + i] = s;
         }
     }
+}
+
+// ------------------------------------------------------------------ full Dyson
+// One CTA per pole set (C.E, C.M sorted; C.cp from k_lz_groups): its rows for the Dyson
+// matrix to io.E [N] and io.M [D][N].  A set in which no group is rotated keeps the order it
+// was built in (io.E0, io.M0).
+__global__ void __launch_bounds__(kCpThreads) k_plain_rotate(const LzChain *chains, const PlainIO *ios, int nchains) {
+    const int cid = blockIdx.x;
+    if (cid >= nchains) return;
+    const LzChain C = chains[cid];
+    const PlainIO io = ios[cid];
+    const CompactScratch S = lz_compact(C.cp);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, N = C.N, D = C.D;
+    __shared__ int ws[kCpWarps];
+    __shared__ int s_first[kCpGroups + 1];
+    __shared__ int s_any;
+    __shared__ double s_tri[kCpWarps][kGramEntries], s_l[kCpWarps][64];
+    const int Q = S.info->q;
+    if (tid == 0) s_any = 0;
+    __syncthreads();
+    const int ng = Q > 0 ? merge_groups(C.gE, Q, s_first, ws) : 0;
+    for (int g = warp; g < ng; g += kCpWarps)
+        if (S.start[s_first[g + 1]] - S.start[s_first[g]] > kKeep && lane == 0) s_any = 1;
+    __syncthreads();
+    if (!s_any) {
+        for (int i = tid; i < N; i += kCpThreads) io.E[i] = io.E0[i];
+        for (size_t i = tid; i < (size_t)D * N; i += kCpThreads) io.M[i] = io.M0[i];
+        return;
+    }
+    for (int g = warp; g < ng; g += kCpWarps) {
+        const int q0 = s_first[g], q1 = s_first[g + 1];
+        const int p0 = S.start[q0], m = S.start[q1] - p0;
+        bool rot = false;
+        if (m > kKeep) {
+            for (int e = lane; e < D * (D + 1) / 2; e += 32) {
+                double s = 0.0;
+                for (int q = q0; q < q1; ++q) s += S.gram[(size_t)q * kGramEntries + e];
+                s_tri[warp][e] = s;
+            }
+            __syncwarp();
+            rot = warp_cholesky(s_tri[warp], D, s_l[warp], lane);
+            __syncwarp();
+        }
+        const double eg = 0.5 * (C.E[p0] + C.E[p0 + m - 1]);
+        for (int i = lane; i < m; i += 32) {
+            io.E[p0 + i] = (rot && i < D) ? eg : C.E[p0 + i];
+            for (int d = 0; d < D; ++d)
+                io.M[(size_t)d * N + p0 + i] = !rot ? C.M[(size_t)d * N + p0 + i] : i < D ? s_l[warp][d * D + i] : 0.0;
+        }
+        __syncwarp();
+    }
+}
+
+cudaError_t launch_plain_rotate(const LzChain *d_chains, const PlainIO *d_ios, int nchains, cudaStream_t st) {
+    if (nchains <= 0) return cudaSuccess;
+    k_plain_rotate<<<nchains, kCpThreads, 0, st>>>(d_chains, d_ios, nchains);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_lz_compact(const LzChain *d_chains, int nchains, double eta, cudaStream_t st) {

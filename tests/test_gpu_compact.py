@@ -58,3 +58,37 @@ def test_compact_reduction_equals_full(bdmod, problems, nmax, hw, nit):
         np.testing.assert_allclose(ra["koltun"], rb["koltun"], rtol=1e-10, atol=1e-11)
     assert built > 0
     ctx.close()
+
+
+@pytest.mark.parametrize("nmax,hw,kind", [(2, 20.0, "batched"), (3, 13.7, "channel"), (4, 27.3, "batched"),
+                                          (4, 20.0, "channel"), (4, 20.0, "dressed")])
+def test_rotated_full_dyson_equals_plain_rows(bdmod, problems, nmax, hw, kind):
+    """The un-reduced solve, its equal energies rotated, against the same rows handed in by the
+    caller (bd_dyson_rows solves them as they are)."""
+    p = problems(nmax, hw, 3, 1)
+    ctx = bdmod.Context().upload(p)
+    if kind == "dressed":                       # distinct energies: nothing to rotate
+        ctx.run_all(lanczos=False)
+        ctx.dressed_propagator(0.5, 1)
+    ctx.run_all(lanczos=False, graph=(kind == "batched"))
+    for ish in range(0, p.ms.nsubsh, 3):
+        D = int(p.ms.no[ish])
+        s1 = np.diag(p.ms.orb_xe[p.ms.orb_start[ish]:p.ms.orb_start[ish] + D])
+        a = ctx.result(ish)
+        hf = ctx.ehf(ish)
+        fw, bk = ctx.sigma2_build(ish)
+        if kind == "channel":
+            a = ctx.dyson_solve(ish, s1, hf)
+        ctx2 = bdmod.Context().upload(p)
+        ef = float((a["qp"][-1, 0] + a["qh"][0, 0]) / 2) if len(a["qh"]) else float(a["qp"][-1, 0]) - 1.0
+        b = ctx2.dyson_rows(ish, 2, fw, bk, sig1b=s1, sighf=hf, efermi=ef)
+        ctx2.close()
+        for tag in ("qp", "qh"):
+            assert len(a[tag]) == len(b[tag])
+            assert np.all(np.diff(a[tag][:, 0]) <= 0)
+            # every energy, the unreached directions' among them
+            np.testing.assert_allclose(a[tag][:, 0], b[tag][:, 0], rtol=1e-10, atol=1e-10)
+            e, z = strong_diffs(b[tag], a[tag])
+            assert e < 1e-10 and z < 1e-10, (ish, tag, e, z)
+        np.testing.assert_allclose(a["koltun"], b["koltun"], rtol=1e-10, atol=1e-11)
+    ctx.close()
