@@ -1180,7 +1180,7 @@ int launch_dyson_range(bd_ctx *ctx, int ch_lo, int ch_hi, bool lanczos) {
         return rct;
     CU(launch_dyson(ctx->d_jobs + ch_lo, (int)jobs.size(), ctx->d_row_first + ch_lo, rows, nmax, Dmax,
                     dy_cluster_for(ctx, ch_hi - ch_lo), ctx->d_dywork, ctx->d_work_first + ch_lo, ctx->st));
-    ctx->launches += dyson_launch_count(nmax);
+    ctx->launches += dyson_launch_count(nmax, Dmax, dy_cluster_for(ctx, ch_hi - ch_lo));
     return BD_OK;
 }
 
@@ -2155,7 +2155,7 @@ int bd_dyson_rows(bd_ctx *ctx, int ish, int nden, int n_fw, const double *fw_row
     CU(cudaMemcpyAsync(dwf, zero, sizeof zero, cudaMemcpyHostToDevice, ctx->st));
     CU(cudaMemcpyAsync(drf, zero, sizeof zero, cudaMemcpyHostToDevice, ctx->st));
     CU(launch_dyson(dj, 1, drf, n, n, D, dy_cluster_for(ctx, 1), dwork, dwf, ctx->st));
-    ctx->launches += dyson_launch_count(n);
+    ctx->launches += dyson_launch_count(n, D, dy_cluster_for(ctx, 1));
     int nq[2] = {0, 0}, dst = 0;
     double kol[3];
     CU(cudaMemcpyAsync(nq, ctx->d_dynq + 2 * ish, sizeof nq, cudaMemcpyDeviceToHost, ctx->st));

@@ -90,11 +90,13 @@ cudaError_t launch_lz_expand(const LzChain &chain, cudaStream_t st);
 cudaError_t launch_plain_rotate(const LzChain *d_chains, const PlainIO *d_ios, int nchains, cudaStream_t st);
 void compact_smem_init();
 
-int dyson_launch_count(int nmax);
+int dyson_launch_count(int nmax, int Dmax, int cluster);
 cudaError_t launch_dyson(const DyJob *d_jobs, int njobs, const long long *d_row_first, long long total_rows,
                          int nmax, int Dmax, int cluster, double *work, const long long *d_work_first, cudaStream_t st);
-cudaError_t launch_eig(const DyJob *d_jobs, int njobs, const long long *d_row_first, long long total_rows,
-                       double *work, const long long *d_work_first, cudaStream_t st);
+// nmax bounds the orders; those beyond nlim come from k_tridiag (reflectors in A), whose first
+// rows of Q k_qrows forms
+cudaError_t launch_eig(const DyJob *d_jobs, int njobs, const long long *d_row_first, long long total_rows, int nmax,
+                       int nlim, double *work, const long long *d_work_first, cudaStream_t st);
 size_t tridiag_smem_bytes(int nmax, int cluster);
 int tridiag_fit_order(int cluster);   // the largest order the cluster reduction's layout holds
 void tridiag_fit_warm();              // fills tridiag_fit_order's cache (cluster sizes 1..16) and

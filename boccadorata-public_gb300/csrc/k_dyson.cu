@@ -7,8 +7,10 @@
 //   K3 k_dyson_assemble   fills the dense matrix row by row (:269-390),
 //   K4a k_tridiag_small   Householder reduction A = Q T Q^T of a matrix of order
 //                         <= 160 in one CTA's shared memory, with the first D rows of Q,
-//       k_tridiag         the same for larger orders, one thread-block cluster per
-//                         matrix (rows split across the CTAs, Q's rows by k_qrows),
+//       k_tridiag_df      the same for larger orders, one thread-block cluster per
+//                         matrix (rows split across the CTAs),
+//       k_tridiag         in FP64 for orders beyond that kernel's shared memory (Q's rows
+//                         by k_qrows),
 //   K4b..K5 (k_eig.cu)    eigenvalues and the first D eigenvector components of T,
 //                         back-transformed, split by E_F, Koltun sums.
 #include <algorithm>
@@ -238,7 +240,7 @@ __device__ inline void tridiag_beyond_layout(const DyJob &J, int rank) {
     if (threadIdx.x == 0) *J.stat = kDyStatCapacity;
 }
 
-__global__ void __launch_bounds__(kTdThreads) k_tridiag(const DyJob *jobs, int njobs, int nmax, int npriv) {
+__global__ void __launch_bounds__(kTdThreads) k_tridiag(const DyJob *jobs, int njobs, int nmax, int npriv, int nlim) {
     cg::cluster_group cluster = cg::this_cluster();
     const int CL = (int)cluster.num_blocks();
     const int rank = (int)cluster.block_rank();
@@ -246,7 +248,7 @@ __global__ void __launch_bounds__(kTdThreads) k_tridiag(const DyJob *jobs, int n
     if (jid >= njobs) return;
     const DyJob J = jobs[jid];
     const int n = J.nc;   // order after deflation
-    if (n <= kTsMax) return;   // k_tridiag_small's (the whole cluster leaves together)
+    if (n <= nlim) return;   // k_tridiag_small's or k_tridiag_df's (the whole cluster leaves together)
     if (n > nmax) { tridiag_beyond_layout(J, rank); return; }
     extern __shared__ double sm[];
     double *v = sm;
@@ -364,21 +366,28 @@ __global__ void __launch_bounds__(kTdThreads) k_tridiag(const DyJob *jobs, int n
     cluster.sync();
 }
 
-// ---------------------------------------------------------------- K4a'' double-float clusters
-// The cluster reduction above in double-float (df64.cuh) where every warp keeps its own
-// partial vector (npriv = 8): k_tridiag's steps, rows and sums unchanged, the matrix's
-// lower triangle turned into (hi, lo) FP32 pairs in place first (each CTA its own rows,
-// from the doubles' bits), the reflector's scalars from the column scaled by a power of
-// two (as k_tridiag_small forms them), and the reflectors stored for k_qrows in FP64 as
-// before.  An FP64 multiply-add holds an SM sub-partition's FP64 unit for ~64 cycles;
-// the double-float one is ~14 FP32 instructions.
+// ---------------------------------------------------------------- K4a'' clusters, one pass a column
+// Orders beyond kTsMax: a cluster per matrix, row i with CTA (i mod CL), both triangles of a
+// row (so a row's product needs no other CTA's partial sums), in double-float (df64.cuh).
+// Rows live in shared memory, the last ones first (they stay longest); those that do not fit
+// in the job's work area.  Step k (trailing rows and columns > k) takes one pass over the
+// matrix instead of a product and an update: the pass applies step k-1's rank-2 update and
+// multiplies by step k's column as it goes.  The column is used unscaled, as in
+// k_tridiag_small, so the reflector's scalars are formed by one warp beside the pass:
+//   pass      a_ij -= v'_i w'_j + w'_i v'_j (v', w' of step k-1), S_i = sum_{j>k+1} a_ij x_j, two
+//             rows a warp; the same product for this CTA's rows of R; warp kTdScal: |x|^2 from
+//             the CTAs' partial sums, then tau and s
+//   own rows  y_i = a_i,k+1 + s S_i = (A v)_i to every CTA, with the warps' partials of v^T A v;
+//             cluster barrier
+//   all rows  v = s x, w = tau y - (tau^2 / 2) (v^T A v) v; R -= tau (R v) v^T
+//   own rows  column k+1 of the updated matrix to every CTA (x of the next step, d_{k+1} from
+//             the diagonal), with the partials of its square; cluster barrier
+// Bound by these two cluster barriers and the chains between them (about 4 000 cycles a
+// column) up to orders of a few hundred, by the FP32 pipe (41 instructions an element)
+// beyond.  Against the two passes from L2 with eight warps that this replaced, and k_qrows
+// for R (one CTA, FP64, a pass of its own): order 1 000 alone on 16 CTAs 34.4 + 6.4 -> 12.8 ms,
+// a batch of orders up to 205 on 8 CTAs each 1.99 + 0.96 -> 0.68 ms.
 namespace {
-
-__device__ inline dfm::df ld_df(const double *p) {
-    const float2 f = __ldcg(reinterpret_cast<const float2 *>(p));
-    return dfm::df{f.x, f.y};
-}
-__device__ inline void st_df(double *p, dfm::df x) { *reinterpret_cast<float2 *>(p) = make_float2(x.h, x.l); }
 
 // x as hi + lo from its bits: hi the double truncated to FP32, lo the next bits of the
 // significand (rounded to FP32), then renormalised; no FP64 instruction (values inside
@@ -401,156 +410,278 @@ __device__ inline dfm::df df_from_bits(double x) {
     return dfm::renorm(hi, lo);
 }
 
-__device__ inline dfm::df block_sum_df(dfm::df v, dfm::df *scratch) {
-    v = dfm::warp_sum(v);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) scratch[warp] = v;
-    __syncthreads();
-    dfm::df s{0.0f, 0.0f};
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) s = dfm::add(s, scratch[q]);
-    return s;
-}
-
 __device__ inline int f32_exponent(float x) { return (int)((__float_as_uint(x) >> 23) & 255u) - 127; }
 __device__ inline float pow2_f32(int e) { return __uint_as_float((unsigned)(e + 127) << 23); }
 
+constexpr int kTdfThreads = 512, kTdfWarps = kTdfThreads / 32, kTdScal = kTdfWarps - 1;
+
+// 8-byte slots before the resident rows: V[2], W[2], the partials kb and sb, R rows, S and
+// a_{i,k+1} of own rows
+__host__ __device__ inline size_t tdf_fixed(int n, int CL, int D) {
+    const int nrm = (n + CL - 1) / CL;
+    return (size_t)(4 + (D + CL - 1) / CL) * n + 2 * (size_t)nrm + 2 * (size_t)CL * kTdfWarps + 32;
+}
+
+// a - (vi wj + wi vj): both products exact to ~2^-48, summed before they meet a; the same bits
+// with i and j exchanged, so the two triangles stay equal
+__device__ __forceinline__ dfm::df rank2(dfm::df a, dfm::df vi, dfm::df wj, dfm::df wi, dfm::df vj) {
+    const float p = dfm::fmul(vi.h, wj.h), q = dfm::fmul(wi.h, vj.h);
+    float e = dfm::ffma(vi.h, wj.h, -p);
+    e = dfm::ffma(vi.h, wj.l, e);
+    e = dfm::ffma(vi.l, wj.h, e);
+    float f = dfm::ffma(wi.h, vj.h, -q);
+    f = dfm::ffma(wi.l, vj.h, f);
+    f = dfm::ffma(wi.h, vj.l, f);
+    float s, r, t, u;
+    dfm::two_sum(p, q, s, r);
+    dfm::two_sum(a.h, -s, t, u);
+    return dfm::renorm(t, dfm::fadd(dfm::fadd(u, a.l), -dfm::fadd(r, dfm::fadd(e, f))));
+}
+
 }  // namespace
 
-__global__ void __launch_bounds__(kTdThreads) k_tridiag_df(const DyJob *jobs, int njobs, int nmax, int npriv) {
+template <int CL>
+__global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_df(const DyJob *jobs, int njobs, int nlim, int smem_df,
+                                                               double *work, const long long *work_first) {
     using dfm::df;
     cg::cluster_group cluster = cg::this_cluster();
-    const int CL = (int)cluster.num_blocks();
     const int rank = (int)cluster.block_rank();
     const int jid = blockIdx.x / CL;
     if (jid >= njobs) return;
     const DyJob J = jobs[jid];
-    const int n = J.nc;
-    if (n <= kTsMax) return;   // k_tridiag_small's (the whole cluster leaves together)
-    if (n > nmax) { tridiag_beyond_layout(J, rank); return; }
-    extern __shared__ double sm[];
-    df *v = reinterpret_cast<df *>(sm);
-    df *p = v + nmax;
-    df *pc = p + nmax;
-    df *pt = pc + nmax;
-    df *pr = pt + (size_t)npriv * nmax;
-    df *scratch = pr + (nmax / CL + 1);
-    double *A = J.A;
+    const int n = J.nc, D = J.D;
+    if (n <= kTsMax || n > nlim) return;   // another kernel's (the whole cluster leaves together)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int kWarps = kTdThreads / 32;
-    df *ptw = pt + (size_t)warp * nmax;   // npriv == kWarps: a partial vector per warp
-    const df zero{0.0f, 0.0f};
-    // this CTA's rows (i = rank, rank + CL, ...), lower triangle, to double-float in place
-    for (int i = rank; i < n; i += CL)
-        for (int j = tid; j <= i; j += kTdThreads) {
-            double *a = A + (size_t)i * n + j;
-            st_df(a, df_from_bits(__ldcg(a)));
-        }
-    cluster.sync();
-    for (int k = 0; k + 2 < n; ++k) {
-        const int b0 = k + 1, m = n - b0;
-        // 1. reflector from column k (rows > k), every CTA alike: alpha, |x_1:|^2, the
-        //    power of two that scales them into [1, 2), then beta, tau and 1/(alpha - beta)
-        df s2 = zero;
-        for (int t = 1 + tid; t < m; t += kTdThreads) { const df x = ld_df(A + (size_t)(b0 + t) * n + k); s2 = dfm::fma(x, x, s2); }
-        s2 = block_sum_df(s2, scratch);
-        const df al = ld_df(A + (size_t)b0 * n + k);
-        const bool nz = (s2.h != 0.0f || s2.l != 0.0f);
-        df tau = zero, scal = zero, beta = al;
-        if (nz) {
-            const int ea = (al.h != 0.0f) ? f32_exponent(al.h) : -1000;
-            int e = max(ea, f32_exponent(s2.h) >> 1);
-            e = min(max(e, -126), 126);
-            const float sg = pow2_f32(-e);
-            const df alt{al.h * sg, al.l * sg}, s2t{(s2.h * sg) * sg, (s2.l * sg) * sg};
-            const df x2 = dfm::fma(alt, alt, s2t);   // in [1, 12)
-            const df r = dfm::rsqrt(x2, 2), nx = dfm::mul(x2, r);
-            const bool ng = signbit(alt.h);
-            const df aa = ng ? dfm::neg(alt) : alt;
-            tau = dfm::fma(aa, r, df{1.0f, 0.0f});
-            df st = dfm::rcp(dfm::add(aa, nx), 2);   // 1 / (alpha~ - beta~)
-            if (ng) st = dfm::neg(st);
-            scal = df{st.h * sg, st.l * sg};         // 1 / (alpha - beta)
-            const df bt = ng ? nx : dfm::neg(nx);
-            const float un = pow2_f32(e);
-            beta = df{bt.h * un, bt.l * un};
-            for (int t = tid; t < m; t += kTdThreads) v[t] = (t == 0) ? df{1.0f, 0.0f} : dfm::mul(ld_df(A + (size_t)(b0 + t) * n + k), scal);
-        }
-        if (rank == 0 && tid == 0) { J.e[k] = dfm::to_double(beta); J.tau[k] = dfm::to_double(tau); J.d[k] = dfm::to_double(ld_df(A + (size_t)k * n + k)); }
-        if (nz) {
-            for (int t = tid; t < kWarps * m; t += kTdThreads) pt[(size_t)(t / m) * nmax + t % m] = zero;
-            __syncthreads();
-            // 2. own rows: row part and transposed part of A v (two chains per lane)
-            const int first = b0 + ((rank - b0 % CL) % CL + CL) % CL;
-            for (int i = first + warp * CL; i < n; i += CL * kWarps) {
-                const double *Ai = A + (size_t)i * n;
-                const df vi = v[i - b0];
-                df rs0 = zero, rs1 = zero;
-                int j = b0 + lane;
-                for (; j + 32 < i; j += 64) {
-                    const int t = j - b0;
-                    const df a0 = ld_df(Ai + j), a1 = ld_df(Ai + j + 32);
-                    rs0 = dfm::fma(a0, v[t], rs0);
-                    rs1 = dfm::fma(a1, v[t + 32], rs1);
-                    ptw[t] = dfm::fma(a0, vi, ptw[t]);
-                    ptw[t + 32] = dfm::fma(a1, vi, ptw[t + 32]);
-                }
-                for (; j <= i; j += 32) {
-                    const df a = ld_df(Ai + j);
-                    rs0 = dfm::fma(a, v[j - b0], rs0);
-                    if (j < i) ptw[j - b0] = dfm::fma(a, vi, ptw[j - b0]);
-                }
-                const df rs = dfm::warp_sum(dfm::add(rs0, rs1));
-                if (lane == 0) pr[(i - first) / CL] = rs;
+    const int nrm = (n + CL - 1) / CL, nr = (n - rank + CL - 1) / CL;   // own rows i = rank + q CL, q < nr
+    const int NRR = (D - rank + CL - 1) / CL;                            // own rows of R: d = rank + u CL (<= 0: none)
+    constexpr int RW = 32 / CL;                  // own rows per warp in the own-rows phases, a lane per (row, CTA)
+    extern __shared__ double sm[];
+    df *V = reinterpret_cast<df *>(sm);          // [2][n]
+    df *W = V + 2 * (size_t)n;                   // [2][n]
+    df *kb = W + 2 * (size_t)n;                  // [kTdfWarps][CL] partials of v . y
+    df *sb = kb + (size_t)CL * kTdfWarps;        // [kTdfWarps][CL] partials of |x_1:|^2
+    df *R = sb + (size_t)CL * kTdfWarps;         // [NRR][n]
+    df *rs = R + (size_t)((D + CL - 1) / CL) * n;   // [nrm] S of own rows
+    df *ra = rs + nrm;                           // [nrm] a_{i,k+1}
+    df *rows = reinterpret_cast<df *>(sm) + tdf_fixed(n, CL, D);
+    const int room = max(0, (smem_df - (int)tdf_fixed(n, CL, D)) / n);
+    const int qs = max(0, nr - room);            // own rows q >= qs in shared memory
+    df *spill = reinterpret_cast<df *>(work + work_first[jid]);
+    auto row = [&](int q) -> df * { return q >= qs ? rows + (size_t)(q - qs) * n : spill + (size_t)(rank + q * CL) * n; };
+    __shared__ df s_sc[2];      // tau, s of the step
+    __shared__ df s_rd[8];      // R_d . v of own R rows
+    const df zero{0.0f, 0.0f}, one{1.0f, 0.0f};
+    // d, e and tau stay double-float pairs in their FP64 slots until the end: a conversion is
+    // two FP64 instructions on a chain that other warps wait for
+    auto put = [](double *p, df x) { *reinterpret_cast<float2 *>(p) = make_float2(x.h, x.l); };
+    // the sum of cnt values by a warp, the same in every lane
+    auto sum_of = [&](const df *p, int cnt) {
+        df t = lane < cnt ? p[lane] : zero;
+        for (int e = lane + 32; e < cnt; e += 32) t = dfm::add(t, p[e]);
+        return dfm::warp_sum(t);
+    };
+    // this CTA's rows, both triangles, from the assembled lower one
+    for (int q = warp; q < nr; q += kTdfWarps) {
+        const int i = rank + q * CL;
+        df *a = row(q);
+        for (int j = lane; j < n; j += 32) a[j] = df_from_bits(__ldcg(J.A + (j <= i ? (size_t)i * n + j : (size_t)j * n + i)));
+    }
+    df sq0 = zero;
+    for (int j = tid; j < n; j += kTdfThreads) {
+        const df xj = df_from_bits(__ldcg(J.A + (size_t)j * n));   // x of step 0
+        V[j] = xj;
+        V[n + j] = zero;
+        W[n + j] = zero;
+        for (int u = 0; u < NRR; ++u) R[(size_t)u * n + j] = (j == rank + u * CL) ? one : zero;
+        if (j >= 2) sq0 = dfm::fma(xj, xj, sq0);
+    }
+    // the squares of column 0, summed by every CTA for itself
+    sq0 = dfm::warp_sum(sq0);
+    if (lane == 0) sb[warp] = sq0;
+    int nsb = kTdfWarps;        // partials of |x_1:|^2
+    if (rank == 0 && tid == 0) put(J.d, V[0]);
+    cluster.sync();   // every CTA runs, and this CTA's arrays are set
+    int cur = 0;
+    for (int k = 0; k + 2 < n; ++k, cur ^= 1) {
+        df *x = V + (size_t)cur * n, *vp = V + (size_t)(cur ^ 1) * n;
+        df *y = W + (size_t)cur * n, *wp = W + (size_t)(cur ^ 1) * n;
+        const int b0 = k + 1;
+        const int q0 = (unsigned)(b0 - rank + CL - 1) / CL;   // first own row >= b0 (b0 - rank + CL - 1 >= 1)
+        // pass
+        if (warp == kTdScal) {
+            const df s2 = sum_of(sb, nsb);
+            const df al = x[b0];
+            df tau = zero, scal = zero, beta = al;
+            if (s2.h != 0.0f || s2.l != 0.0f) {
+                const int ea = (al.h != 0.0f) ? f32_exponent(al.h) : -1000;
+                int e = max(ea, f32_exponent(s2.h) >> 1);
+                e = min(max(e, -126), 126);
+                const float sg = pow2_f32(-e);
+                const df alt{al.h * sg, al.l * sg}, s2t{(s2.h * sg) * sg, (s2.l * sg) * sg};
+                const df x2 = dfm::fma(alt, alt, s2t);   // in [1, 12)
+                const df r = dfm::rsqrt(x2, 2), nx = dfm::mul(x2, r);
+                const bool ng = signbit(alt.h);
+                const df aa = ng ? dfm::neg(alt) : alt;
+                tau = dfm::fma(aa, r, one);
+                df st = dfm::rcp(dfm::add(aa, nx), 2);   // 1 / (alpha~ - beta~)
+                if (ng) st = dfm::neg(st);
+                scal = df{st.h * sg, st.l * sg};         // 1 / (alpha - beta)
+                const df bt = ng ? nx : dfm::neg(nx);
+                const float un = pow2_f32(e);
+                beta = df{bt.h * un, bt.l * un};
             }
-            __syncthreads();
-            for (int t = tid; t < m; t += kTdThreads) {
-                df s = zero;
-                for (int q = 0; q < kWarps; ++q) s = dfm::add(s, pt[(size_t)q * nmax + t]);
-                const int i = b0 + t;
-                if (i >= first && (i - first) % CL == 0) s = dfm::add(s, pr[(i - first) / CL]);
-                pc[t] = s;
+            if (lane == 0) {
+                s_sc[0] = tau;
+                s_sc[1] = scal;
+                if (rank == 0) { put(J.e + k, beta); put(J.tau + k, tau); }
             }
-            cluster.sync();
-            // 3. p = tau A v over the cluster in rank order; w = p - (tau/2)(p.v) v
+        }
+        {   // the active own rows in runs of consecutive ones, one run a warp (the scalars' warp
+            // after them, the first to go without); two rows at a time share the vectors' loads,
+            // and the next columns' entries are loaded before this one's are used
+            const int na = nr - q0;
+            const int per = na / kTdfWarps, ext = na - per * kTdfWarps;
+            int q = q0 + warp * per + min(warp, ext);
+            const int q1 = q + per + (warp < ext ? 1 : 0);
+            for (; q < q1; q += 2) {
+                const bool two = q + 1 < q1;
+                df *a0 = row(q);
+                const int i0 = rank + q * CL;
+                const df v0 = vp[i0], w0 = wp[i0];
+                if (two) {
+                    df *a1 = row(q + 1);
+                    const df v1 = vp[i0 + CL], w1 = wp[i0 + CL];
+                    df s0 = zero, s1 = zero;
+                    int j = b0 + lane;
+                    df p0 = j < n ? a0[j] : zero, p1 = j < n ? a1[j] : zero;
+                    for (; j < n; j += 32) {
+                        const int jn = min(j + 32, n - 1);
+                        const df n0 = a0[jn], n1 = a1[jn];
+                        const df vj = vp[j], wj = wp[j], xj = (j == b0) ? zero : x[j];
+                        const df t0 = rank2(p0, v0, wj, w0, vj), t1 = rank2(p1, v1, wj, w1, vj);
+                        a0[j] = t0;
+                        a1[j] = t1;
+                        s0 = dfm::fma(t0, xj, s0);
+                        s1 = dfm::fma(t1, xj, s1);
+                        if (j == b0) { ra[q] = t0; ra[q + 1] = t1; }
+                        p0 = n0;
+                        p1 = n1;
+                    }
+                    s0 = dfm::warp_sum(s0);
+                    s1 = dfm::warp_sum(s1);
+                    if (lane == 0) { rs[q] = s0; rs[q + 1] = s1; }
+                } else {
+                    df s0 = zero, s1 = zero;   // two columns at a time
+                    for (int j = b0 + lane; j < n; j += 64) {
+                        const bool in = j + 32 < n;
+                        const int j2 = in ? j + 32 : j;
+                        const df p0 = a0[j], p1 = a0[j2];
+                        const df t0 = rank2(p0, v0, wp[j], w0, vp[j]), t1 = rank2(p1, v0, wp[j2], w0, vp[j2]);
+                        a0[j] = t0;
+                        if (in) a0[j2] = t1;
+                        s0 = dfm::fma(t0, (j == b0) ? zero : x[j], s0);
+                        s1 = dfm::fma(t1, in ? x[j2] : zero, s1);
+                        if (j == b0) ra[q] = t0;
+                    }
+                    s0 = dfm::warp_sum(dfm::add(s0, s1));
+                    if (lane == 0) rs[q] = s0;
+                }
+            }
+            // R_d . x_{1:} of own R rows, from the warps before the scalars' one
+            if (warp < kTdScal && kTdScal - 1 - warp < NRR) {
+                const int u = kTdScal - 1 - warp;
+                const df *r = R + (size_t)u * n;
+                df s0 = zero, s1 = zero;
+                int j = b0 + 1 + lane;
+                for (; j + 32 < n; j += 64) { s0 = dfm::fma(r[j], x[j], s0); s1 = dfm::fma(r[j + 32], x[j + 32], s1); }
+                if (j < n) s0 = dfm::fma(r[j], x[j], s0);
+                s0 = dfm::warp_sum(dfm::add(s0, s1));
+                if (lane == 0) s_rd[u] = s0;
+            }
+        }
+        __syncthreads();
+        const df tau = s_sc[0], s = s_sc[1];
+        const bool nz = (tau.h != 0.0f);
+        // own rows, a lane per (row, receiving CTA): y to every CTA, partials of v . y (of the
+        // warp's RW rows, the same count of warps in every CTA)
+        const int wpk = min(kTdfWarps, (int)((unsigned)((n - b0 + CL - 1) / CL + RW - 1) / RW));
+        const int to = lane % CL, q_ = q0 + warp * RW + lane / CL;
+        if (warp < wpk) {
             df kv = zero;
-            for (int t = tid; t < m; t += kTdThreads) {
-                df s = zero;
-                for (int r = 0; r < CL; ++r) s = dfm::add(s, cluster.map_shared_rank(pc, r)[t]);
-                s = dfm::mul(s, tau);
-                p[t] = s;
-                kv = dfm::fma(s, v[t], kv);
+            df *yr = cluster.map_shared_rank(y, to);
+            for (int q = q_; q < nr; q += kTdfWarps * RW) {
+                const int i = rank + q * CL;
+                const df yi = nz ? dfm::fma(s, rs[q], ra[q]) : zero;
+                yr[i] = yi;
+                kv = (i == b0) ? dfm::add(kv, yi) : dfm::fma(dfm::mul(s, x[i]), yi, kv);
             }
-            const df K = block_sum_df(kv, scratch);
-            const df nK = dfm::neg(dfm::mul(df{0.5f * tau.h, 0.5f * tau.l}, K));
-            for (int t = tid; t < m; t += kTdThreads) p[t] = dfm::fma(nK, v[t], p[t]);
-            __syncthreads();
-            // 4. A_ij -= v_i w_j + w_i v_j on the own rows, j <= i
-            for (int i = first + warp * CL; i < n; i += CL * kWarps) {
-                double *Ai = A + (size_t)i * n;
-                const df vi = v[i - b0], wi = p[i - b0];
-                for (int j = b0 + lane; j <= i; j += 32) {
-                    const int t = j - b0;
-                    const df t2 = dfm::fma(vi, p[t], dfm::mul(wi, v[t]));
-                    st_df(Ai + j, dfm::add(ld_df(Ai + j), dfm::neg(t2)));
-                }
-            }
-            if (rank == 0)   // the reflector for k_qrows, in FP64, in row k right of the diagonal
-                for (int t = tid; t < m; t += kTdThreads) A[(size_t)k * n + b0 + t] = dfm::to_double(v[t]);
+#pragma unroll
+            for (int o = 16; o >= CL; o >>= 1) kv = dfm::add(kv, dfm::shfl_xor(kv, o));
+            if (lane < CL) cluster.map_shared_rank(kb, to)[warp * CL + rank] = kv;
         }
         cluster.sync();
-    }
-    if (rank == 0 && tid == 0) {
-        if (n >= 2) {
-            J.d[n - 2] = dfm::to_double(ld_df(A + (size_t)(n - 2) * n + (n - 2)));
-            J.e[n - 2] = dfm::to_double(ld_df(A + (size_t)(n - 1) * n + (n - 2)));
-            J.tau[n - 2] = 0.0;
+        // all rows: v, w; R
+        {
+            const df K = sum_of(kb, wpk * CL);
+            const df tk = dfm::mul(tau, tau);
+            const df nK = dfm::neg(dfm::mul(df{0.5f * tk.h, 0.5f * tk.l}, K));
+            for (int j = b0 + tid; j < n; j += kTdfThreads) {
+                const df vj = !nz ? zero : (j == b0) ? one : dfm::mul(s, x[j]);
+                y[j] = dfm::fma(nK, vj, dfm::mul(tau, y[j]));
+                x[j] = vj;
+                for (int u = 0; u < NRR; ++u) {
+                    df &r = R[(size_t)u * n + j];
+                    const df c = dfm::neg(dfm::mul(tau, dfm::fma(s, s_rd[u], R[(size_t)u * n + b0])));
+                    if (j != b0) r = dfm::fma(c, vj, r);
+                }
+            }
         }
-        J.d[n - 1] = dfm::to_double(ld_df(A + (size_t)(n - 1) * n + (n - 1)));
-        J.e[n - 1] = 0.0;
-        J.tau[n - 1] = 0.0;
+        __syncthreads();
+        if (tid < NRR && nz) {   // R_d[b0], read by every thread above
+            df &r = R[(size_t)tid * n + b0];
+            r = dfm::fma(dfm::neg(dfm::mul(tau, dfm::fma(s, s_rd[tid], r))), one, r);
+        }
+        // own rows: column k+1 of the updated matrix
+        if (warp < wpk) {
+            const df vb = x[b0], wb = y[b0];
+            df *xr = cluster.map_shared_rank(vp, to);
+            df sq = zero;
+            for (int q = q_; q < nr; q += kTdfWarps * RW) {
+                const int i = rank + q * CL;
+                const df t = rank2(row(q)[b0], x[i], wb, y[i], vb);
+                if (i == b0) {
+                    if (to == 0) put(J.d + b0, t);
+                } else {
+                    xr[i] = t;
+                    if (i > b0 + 1) sq = dfm::fma(t, t, sq);
+                    if (k + 3 == n && to == 0) {   // the last step: e_{n-2}, and the last diagonal entry
+                        put(J.e + n - 2, t);
+                        put(J.d + n - 1, rank2(row(q)[n - 1], x[i], y[i], y[i], x[i]));
+                    }
+                }
+            }
+#pragma unroll
+            for (int o = 16; o >= CL; o >>= 1) sq = dfm::add(sq, dfm::shfl_xor(sq, o));
+            if (lane < CL) cluster.map_shared_rank(sb, to)[warp * CL + rank] = sq;
+        }
+        nsb = wpk * CL;
+        cluster.sync();
     }
-    cluster.sync();
+    if (rank == 0)   // every CTA's entries are visible since the last barrier
+        for (int j = tid; j < n; j += kTdfThreads) {
+            auto conv = [](double *p) { const float2 f = __ldcg(reinterpret_cast<const float2 *>(p)); *p = dfm::to_double(df{f.x, f.y}); };
+            conv(J.d + j);
+            if (j + 1 < n) conv(J.e + j); else J.e[j] = 0.0;
+            if (j + 2 < n) conv(J.tau + j); else J.tau[j] = 0.0;
+        }
+    for (int u = 0; u < NRR; ++u)
+        for (int j = tid; j < n; j += kTdfThreads) J.R[(size_t)(rank + u * CL) * n + j] = dfm::to_double(R[(size_t)u * n + j]);
+}
+
+// the kernel for a cluster size (1, 2, 4, 8 or 16)
+static auto tridiag_df_kernel(int cluster) {
+    return cluster == 16 ? k_tridiag_df<16> : cluster == 8 ? k_tridiag_df<8> : cluster == 4 ? k_tridiag_df<4>
+           : cluster == 2 ? k_tridiag_df<2> : k_tridiag_df<1>;
 }
 
 // ---------------------------------------------------------------- K4a' small matrices
@@ -842,12 +973,12 @@ int tridiag_fit_order(int cluster) {
         if (v) return v;
     }
     int dev = 0, optin = 0;
-    cudaFuncAttributes a{}, b{};
+    cudaFuncAttributes a{};
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-        cudaFuncGetAttributes(&a, k_tridiag) != cudaSuccess || cudaFuncGetAttributes(&b, k_tridiag_df) != cudaSuccess)
+        cudaFuncGetAttributes(&a, k_tridiag) != cudaSuccess)
         return kTsMax + 1;   // the launch that follows reports the error
-    const size_t limit = (size_t)optin - std::max(a.sharedSizeBytes, b.sharedSizeBytes);
+    const size_t limit = (size_t)optin - a.sharedSizeBytes;
     int lo = kTsMax + 1, hi = 1 << 22;
     while (lo < hi) {
         const int mid = lo + (hi - lo + 1) / 2;
@@ -861,12 +992,28 @@ void tridiag_fit_warm() {
     for (int c = 1; c <= 16; c <<= 1) tridiag_fit_order(c);
     allow_dynamic_smem((const void *)k_tridiag_small);
     allow_dynamic_smem((const void *)k_tridiag);
-    allow_dynamic_smem((const void *)k_tridiag_df);
+    for (int c = 1; c <= 16; c <<= 1) allow_dynamic_smem((const void *)tridiag_df_kernel(c));
+}
+
+// Shared memory of k_tridiag_df (8-byte slots, at most kTdfSlots: 224 KB) and the largest
+// order whose vectors fit in it (the rows may spill).
+constexpr int kTdfSlots = 224 * 1024 / 8;
+int tridiag_df_limit(int cluster, int D) {
+    int lo = kTsMax, hi = 1 << 16;
+    while (lo < hi) {
+        const int mid = lo + (hi - lo + 1) / 2;
+        if (tdf_fixed(mid, cluster, D) <= (size_t)kTdfSlots) lo = mid; else hi = mid - 1;
+    }
+    return lo;
 }
 
 // Kernels launch_dyson starts for matrices of order up to nmax: deflate, assemble, the
-// small-matrix reduction (and the cluster one beyond kTsMax), then launch_eig's nine.
-int dyson_launch_count(int nmax) { return (nmax <= kTsMax ? 3 : 4) + 9; }
+// small-matrix reduction (the cluster one beyond kTsMax, the FP64 one and k_qrows beyond
+// its limit), then launch_eig's.
+int dyson_launch_count(int nmax, int Dmax, int cluster) {
+    const int nlim = tridiag_df_limit(cluster, Dmax);
+    return 3 + (nmax > kTsMax ? 1 : 0) + (nmax > nlim ? 2 : 0) + (nmax > kTsMax ? 8 : 7);
+}
 
 cudaError_t launch_dyson(const DyJob *d_jobs, int njobs, const long long *d_row_first, long long total_rows,
                          int nmax, int Dmax, int cluster, double *work, const long long *d_work_first, cudaStream_t st) {
@@ -882,15 +1029,9 @@ cudaError_t launch_dyson(const DyJob *d_jobs, int njobs, const long long *d_row_
     k_tridiag_small<<<njobs, kTsThreads, ssmem, st>>>(d_jobs, njobs);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    if (nmax <= kTsMax) return launch_eig(d_jobs, njobs, d_row_first, total_rows, work, d_work_first, st);
-    // the full orders bound the deflated ones; the layout is sized for at most the
-    // largest order shared memory holds, and larger deflated orders report it
-    nmax = std::min(nmax, tridiag_fit_order(cluster));
-    size_t smem = tridiag_smem_bytes(nmax, cluster);
+    if (nmax <= kTsMax) return launch_eig(d_jobs, njobs, d_row_first, total_rows, nmax, nmax, work, d_work_first, st);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(njobs * cluster, 1, 1);
-    cfg.blockDim = dim3(kTdThreads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -899,14 +1040,35 @@ cudaError_t launch_dyson(const DyJob *d_jobs, int njobs, const long long *d_row_
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const int npriv = tridiag_npriv(nmax, cluster);
-    auto kern = (npriv == kTdThreads / 32) ? k_tridiag_df : k_tridiag;   // double-float with a partial per warp
-    e = allow_dynamic_smem((const void *)kern);
-    if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-    e = cudaLaunchKernelEx(&cfg, kern, d_jobs, njobs, nmax, npriv);
-    if (e != cudaSuccess) return e;
-    return launch_eig(d_jobs, njobs, d_row_first, total_rows, work, d_work_first, st);
+    auto prepare = [&](const void *kern) {
+        e = allow_dynamic_smem(kern);
+        if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        return e == cudaSuccess;
+    };
+    const int nlim = tridiag_df_limit(cluster, Dmax);
+    {
+        // as many slots as the largest order (the full orders bound the deflated ones) needs
+        // to keep all its rows, at most kTdfSlots
+        const int nb = std::min(nmax, nlim);
+        const size_t slots = std::min((size_t)kTdfSlots, tdf_fixed(nb, cluster, Dmax) + (size_t)((nb + cluster - 1) / cluster) * nb);
+        cfg.blockDim = dim3(kTdfThreads, 1, 1);
+        cfg.dynamicSmemBytes = slots * 8;
+        const auto kern = tridiag_df_kernel(cluster);
+        if (!prepare((const void *)kern)) return e;
+        e = cudaLaunchKernelEx(&cfg, kern, d_jobs, njobs, nb, (int)slots, work, d_work_first);
+        if (e != cudaSuccess) return e;
+    }
+    if (nmax > nlim) {
+        // the layout is sized for at most the largest order shared memory holds, and larger
+        // deflated orders report it
+        const int nb = std::min(nmax, tridiag_fit_order(cluster));
+        cfg.blockDim = dim3(kTdThreads, 1, 1);
+        cfg.dynamicSmemBytes = tridiag_smem_bytes(nb, cluster);
+        if (!prepare((const void *)k_tridiag)) return e;
+        e = cudaLaunchKernelEx(&cfg, k_tridiag, d_jobs, njobs, nb, tridiag_npriv(nb, cluster), nlim);
+        if (e != cudaSuccess) return e;
+    }
+    return launch_eig(d_jobs, njobs, d_row_first, total_rows, nmax, nlim, work, d_work_first, st);
 }
 
 }  // namespace bd

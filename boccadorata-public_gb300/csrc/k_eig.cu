@@ -3,8 +3,8 @@
 // (source/BcDor-DysonMatrix.cpp:442-488): every eigenvalue W_k and the first D
 // components x_k[0:D] of the corresponding eigenvector of A.
 //
-//   k_qrows   R = first D rows of Q = H_0 H_1 ... H_{n-3} (reflectors kept in A's rows;
-//             matrices of order <= kTsMax get R from k_tridiag_small)
+//   k_qrows   R = first D rows of Q = H_0 H_1 ... H_{n-3} from the reflectors k_tridiag
+//             keeps in A's rows (the other reductions form R themselves)
 //   k_bisect_prep  splits T into unreduced blocks at negligible off-diagonals
 //   k_bisect  W_k by bisection on Sturm counts over its block, four threads per
 //             eigenvalue (eig_sturm.cuh): an FP32 bracket, checked and finished in
@@ -31,12 +31,12 @@ namespace bd {
 constexpr int kEigThreads = 256;
 
 // ------------------------------------------------------------------ K4b
-__global__ void __launch_bounds__(kEigThreads) k_qrows(const DyJob *jobs, int njobs) {
+__global__ void __launch_bounds__(kEigThreads) k_qrows(const DyJob *jobs, int njobs, int nlim) {
     const int jid = blockIdx.x;
     if (jid >= njobs) return;
     const DyJob J = jobs[jid];
     const int n = J.nc, D = J.D, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;   // order after deflation
-    if (n <= kTsMax) return;   // k_tridiag_small formed R
+    if (n <= nlim) return;   // k_tridiag_small or k_tridiag_df formed R
     __shared__ double red[kEigThreads / 32][8];
     __shared__ double sums[8];
     double *R = J.R;
@@ -225,106 +225,14 @@ __device__ inline EigTol eig_tol(double onenrm) {
     return t;
 }
 
-// Storage of one eigenvector's LU factors (first and second superdiagonal, pivots as
-// reciprocals, multipliers, interchanges) and of its iterate, element i of each.
-struct InvitGlobal {   // the job's work area and matrix region, column k at stride n
-    double *U1, *U2, *DD, *LL, *PV, *Y;
-    int n, k;
-    __device__ double &u1(int i) { return U1[(size_t)i * n + k]; }
-    __device__ double &u2(int i) { return U2[(size_t)i * n + k]; }
-    __device__ double &dd(int i) { return DD[(size_t)i * n + k]; }
-    __device__ double &ll(int i) { return LL[(size_t)i * n + k]; }
-    __device__ double &y(int i) { return Y[(size_t)i * n + k]; }
-    __device__ bool pv(int i) { return PV[(size_t)i * n + k] != 0.0; }
-    __device__ void set_pv(int i, bool b) { PV[(size_t)i * n + k] = b ? 1.0 : 0.0; }
-};
-
 constexpr int kIvThreads = 16;   // eigenvectors per CTA of the shared-memory variant
 
-// Eigenvector k of block [b0, b1] (b1 > b0) into a.y(b0 .. b1).
-template <class S>
-__device__ void invit_vector(const DyJob &J, int k, int b0, int b1, S &a) {
-    const int NS = 2 + J.D;
-    const double *d = J.d, *e = J.e;
-    const EigTol tl = eig_tol(J.tau[k]);
-    auto W = [&](int q) { return J.sol[(size_t)q * NS]; };
-    // shift: walk to the start of the cluster inside the block, then apply the separation rule forward
-    int k0 = k;
-    while (k0 > b0 && W(k0) - W(k0 - 1) <= tl.ortol) --k0;
-    double x = W(k0);
-    for (int q = k0 + 1; q <= k; ++q) x = fmax(W(q), x + tl.pertol);
-    // LU with partial pivoting of T_b - x I; rows i and i+1 may swap
-    for (int i = b0; i <= b1; ++i) {
-        a.dd(i) = d[i] - x;
-        a.u1(i) = (i < b1) ? e[i] : 0.0;
-        a.ll(i) = (i < b1) ? e[i] : 0.0;
-        a.u2(i) = 0.0;
-    }
-    for (int i = b0; i < b1; ++i) {
-        const double di = a.dd(i), li = a.ll(i);
-        if (fabs(di) >= fabs(li)) {
-            a.set_pv(i, false);
-            const double f = (di != 0.0) ? li * rcp_newton(di) : 0.0;
-            a.ll(i) = f;
-            a.dd(i + 1) -= f * a.u1(i);
-        } else {
-            a.set_pv(i, true);
-            const double f = di * rcp_newton(li);
-            a.dd(i) = li;
-            a.ll(i) = f;
-            const double tt = a.u1(i);
-            a.u1(i) = a.dd(i + 1);
-            a.dd(i + 1) = tt - f * a.dd(i + 1);
-            if (i + 1 < b1) {
-                a.u2(i) = a.u1(i + 1);
-                a.u1(i + 1) = -f * a.u1(i + 1);
-            }
-        }
-    }
-    // pivots no smaller than pertol, kept as reciprocals for the solves
-    for (int i = b0; i <= b1; ++i) {
-        double p = a.dd(i);
-        if (fabs(p) < tl.pertol) p = (p < 0 ? -tl.pertol : tl.pertol);
-        a.dd(i) = rcp_newton(p);
-    }
-    for (int i = b0; i <= b1; ++i)
-        a.y(i) = 0.5 + (double)(hash32((unsigned)(i * 2654435761u) ^ (unsigned)(k * 97 + 13)) & 0xffff) / 65536.0;
-    // two sweeps: the shift is within 1e-13 |T_b| of W_k and eigenvalues of a block
-    // closer than 1e-6 |T_b| are clustered (orthonormalised together), so each sweep
-    // scales the other eigenvectors' share by at most 1e-7 against this one's
-    for (int it = 0; it < 2; ++it) {
-        for (int i = b0; i < b1; ++i) {   // L^-1 with the interchanges
-            double bi = a.y(i), bi1 = a.y(i + 1);
-            const double f = a.ll(i);
-            if (!a.pv(i)) bi1 -= f * bi;
-            else { const double tt = bi; bi = bi1; bi1 = tt - f * bi1; }
-            a.y(i) = bi; a.y(i + 1) = bi1;
-        }
-        double y1 = 0.0, y2 = 0.0, nrm = 0.0;
-        for (int i = b1; i >= b0; --i) {   // U y = b, two superdiagonals
-            double v = a.y(i);
-            if (i + 1 <= b1) v -= a.u1(i) * y1;
-            if (i + 2 <= b1) v -= a.u2(i) * y2;
-            v *= a.dd(i);
-            a.y(i) = v;
-            y2 = y1; y1 = v;
-            nrm = fmax(nrm, fabs(v));
-        }
-        const double sc = (nrm > 0.0) ? rcp_newton(nrm) : 1.0;
-        double s2 = 0.0;
-        for (int i = b0; i <= b1; ++i) { const double v = a.y(i) * sc; a.y(i) = v; s2 += v * v; }
-        const double inv = (s2 > 0.0) ? 1.0 / sqrt(s2) : 0.0;
-        for (int i = b0; i <= b1; ++i) a.y(i) *= inv;
-    }
-}
-
-// The same in double-float (df64.cuh: FP32 hi + lo pairs, ~48 bits) for the shared-memory
-// variant: every step of the factorisation and of the solves is a dependent chain, and
+// Orders <= kTsMax: eigenvector k of block [b0, b1] (b1 > b0), in double-float (df64.cuh:
+// FP32 hi + lo pairs, ~48 bits): every step of the factorisation and of the solves is a dependent chain, and
 // an FP64 instruction holds an SM sub-partition's FP64 unit for ~64 cycles on this GPU
 // (a reciprocal by Newton's iteration is four of them), while the double-float forms
-// run on the FP32 pipe at a few cycles per operation.  The shifts, the tolerances and
-// the start vectors are those of invit_vector; the pivot choice compares the high parts
-// (any choice that keeps the multipliers bounded serves), and the result goes to y in
+// run on the FP32 pipe at a few cycles per operation.  The pivot choice compares the high
+// parts (any choice that keeps the multipliers bounded serves), and the result goes to y in
 // FP64.  The tridiagonal is converted to double-float once per CTA, into shared memory.
 struct InvitSharedDF {   // shared memory, element i of this thread at i * kIvThreads + lane
     dfm::df *U1, *U2, *DD, *LL, *Y;
@@ -444,22 +352,161 @@ __device__ void invit_vector_df(const DyJob &J, int k, int b0, int b1, const dfm
     }
 }
 
-// Matrices of order > kTsMax: one thread per position, factors in the job's work area.
-__global__ void k_invit(const DyJob *jobs, int njobs, const long long *row_first, long long total, double *work,
-                        const long long *work_first) {
-    const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (g >= total) return;
-    const int lo = job_of(row_first, njobs, g);
+// Matrices of order > kTsMax: one thread per position, the same steps in FP64 with the factors
+// in the job's work area (columns at stride n, so a warp's accesses are contiguous).  A
+// position is one dependent chain of rows.  The running entries of the factorisation and of
+// the solves stay in registers, the first solve's forward half runs along with the
+// factorisation, and nothing read back depends on the chain, so the solves load kIvAhead
+// rows' factors before they use them: the L2 round trips overlap instead of adding one to
+// every row.  The pivoting is by selects (a warp's lanes disagree about it row by row).  What
+// is left is the FP64 unit, about twenty instructions a row at ~64 cycles each; 1 000
+// positions are 32 warps, one an SM.  Order 1 000: 4.06 -> 1.43 ms.
+constexpr int kIvAhead = 8;
+constexpr int kIvLarge = 32;   // positions per CTA
+constexpr int kIvTri = 6144;   // rows of the tridiagonal kept in shared memory
+
+__global__ void __launch_bounds__(kIvLarge) k_invit(const DyJob *jobs, int njobs, const long long *row_first,
+                                                    long long total, double *work, const long long *work_first) {
+    const long long g = blockIdx.x * (long long)kIvLarge + threadIdx.x;
+    extern __shared__ double smi[];
+    // the CTA's positions usually belong to one matrix: its tridiagonal in shared memory
+    const int j0 = job_of(row_first, njobs, min(blockIdx.x * (long long)kIvLarge, total - 1));
+    const int j1 = job_of(row_first, njobs, min(blockIdx.x * (long long)kIvLarge + kIvLarge - 1, total - 1));
+    const double *d = jobs[j0].d, *e = jobs[j0].e;
+    const int nj = jobs[j0].nc;
+    const bool one_job = j0 == j1;
+    const int lo = one_job ? j0 : job_of(row_first, njobs, min(g, total - 1));
     const DyJob J = jobs[lo];
+    if (one_job && (nj <= kTsMax || blockIdx.x * (long long)kIvLarge - row_first[j0] >= nj)) return;
+    if (one_job && nj <= kIvTri) {
+        for (int i = threadIdx.x; i < nj; i += kIvLarge) { smi[i] = d[i]; smi[nj + i] = e[i]; }
+        __syncwarp();
+        d = smi;
+        e = smi + nj;
+    } else {
+        d = J.d;
+        e = J.e;
+    }
     const int k = (int)(g - row_first[lo]), n = J.nc;
-    if (k >= n || n <= kTsMax) return;
+    if (g >= total || k >= n || n <= kTsMax) return;
     const int b0 = J.blk[k], b1 = J.blk[n + k];
-    double *Y = J.A;
-    if (b0 == b1) { Y[(size_t)b0 * n + k] = 1.0; return; }
-    double *wk = work + work_first[lo];   // 5 arrays of n*n
-    InvitGlobal a{wk, wk + (size_t)n * n, wk + 2 * (size_t)n * n, wk + 3 * (size_t)n * n, wk + 4 * (size_t)n * n, Y,
-                  n, k};
-    invit_vector(J, k, b0, b1, a);
+    double *Y = J.A + k;
+    if (b0 == b1) { Y[(size_t)b0 * n] = 1.0; return; }
+    const size_t nn = (size_t)n * n;
+    double *wk = work + work_first[lo] + k;   // five arrays of n x n, this column
+    double *U1 = wk, *U2 = wk + nn, *DD = wk + 2 * nn, *LL = wk + 3 * nn;
+    unsigned *PV = reinterpret_cast<unsigned *>(work + work_first[lo] + 4 * nn) + k;   // bits of row i in word i / 32
+    const int NS = 2 + J.D;
+    const EigTol tl = eig_tol(J.tau[k]);
+    auto W = [&](int q) { return J.sol[(size_t)q * NS]; };
+    // shift: walk to the start of the cluster inside the block, then apply the separation rule forward
+    int k0 = k;
+    while (k0 > b0 && W(k0) - W(k0 - 1) <= tl.ortol) --k0;
+    double x = W(k0);
+    for (int q = k0 + 1; q <= k; ++q) x = fmax(W(q), x + tl.pertol);
+    // magnitudes as integers: an FP64 comparison takes the FP64 unit too
+    auto mag = [](double v) { return __double_as_longlong(v) & 0x7fffffffffffffffLL; };
+    const long long pmag = mag(tl.pertol);
+    auto clamp_piv = [&](double p) { return mag(p) < pmag ? (p < 0.0 ? -tl.pertol : tl.pertol) : p; };
+    auto start = [&](int i) { return 0.5 + (double)(hash32((unsigned)(i * 2654435761u) ^ (unsigned)(k * 97 + 13)) & 0xffff) / 65536.0; };
+    // LU with partial pivoting of T_b - x I (rows i and i+1 may swap); pivots no smaller than
+    // pertol, kept as reciprocals
+    double cur_d = d[b0] - x, cur_u = e[b0], cur_y = start(b0);
+    unsigned bits = 0;
+    for (int i = b0; i < b1; ++i) {
+        const double li = e[i], nd = d[i + 1] - x, nu = (i + 1 < b1) ? e[i + 1] : 0.0, yn = start(i + 1);
+        const bool sw = mag(cur_d) < mag(li);
+        const double piv = sw ? li : cur_d, oth = sw ? cur_d : li, cp = clamp_piv(piv);
+        const double r = rcp_newton(cp);
+        // (a pivot below pertol: the multiplier from the pivot itself, zero for a zero pivot)
+        const double f = (__double_as_longlong(cp) == __double_as_longlong(piv)) ? oth * r : (mag(piv) != 0 ? oth * rcp_newton(piv) : 0.0);
+        const double ui = sw ? nd : cur_u, uo = sw ? cur_u : nd;
+        const double yi = sw ? yn : cur_y, yo = sw ? cur_y : yn;
+        const size_t o = (size_t)i * n;
+        LL[o] = f;
+        U1[o] = ui;
+        U2[o] = sw ? nu : 0.0;
+        DD[o] = r;
+        Y[o] = yi;
+        cur_y = fma(-f, yi, yo);
+        cur_d = fma(-f, ui, uo);
+        cur_u = sw ? -f * nu : nu;
+        bits |= (unsigned)sw << (i & 31);
+        if ((i & 31) == 31 || i + 1 == b1) { PV[(size_t)(i >> 5) * n] = bits; bits = 0; }
+    }
+    U1[(size_t)b1 * n] = 0.0;
+    U2[(size_t)b1 * n] = 0.0;
+    DD[(size_t)b1 * n] = rcp_newton(clamp_piv(cur_d));
+    Y[(size_t)b1 * n] = cur_y;
+    // two sweeps: the shift is within 1e-13 |T_b| of W_k and eigenvalues of a block
+    // closer than 1e-6 |T_b| are clustered (orthonormalised together), so each sweep
+    // scales the other eigenvectors' share by at most 1e-7 against this one's
+    long long nmag = 0;
+    auto back = [&]() {   // U y = b, two superdiagonals, from the last row up
+        double y1 = 0.0, y2 = 0.0;
+        nmag = 0;
+        for (int t = b1; t >= b0; t -= kIvAhead) {
+            double u1[kIvAhead], u2[kIvAhead], dd[kIvAhead], yy[kIvAhead];
+#pragma unroll
+            for (int u = 0; u < kIvAhead; ++u) {
+                const size_t o = (size_t)max(t - u, b0) * n;
+                u1[u] = U1[o]; u2[u] = U2[o]; dd[u] = DD[o]; yy[u] = Y[o];
+            }
+#pragma unroll
+            for (int u = 0; u < kIvAhead; ++u)
+                if (t - u >= b0) {
+                    const double v = fma(-u1[u], y1, fma(-u2[u], y2, yy[u])) * dd[u];
+                    Y[(size_t)(t - u) * n] = v;
+                    y2 = y1; y1 = v;
+                    nmag = max(nmag, mag(v));
+                }
+        }
+    };
+    back();
+    double sc = nmag > 0 ? rcp_newton(__longlong_as_double(nmag)) : 1.0;
+    double cur = Y[(size_t)b0 * n] * sc;
+    for (int t = b0; t < b1; t += kIvAhead) {   // L^-1 with the interchanges, on the scaled iterate
+        double ll[kIvAhead], yn[kIvAhead];
+        unsigned pw[kIvAhead];
+#pragma unroll
+        for (int u = 0; u < kIvAhead; ++u) {
+            const int i = min(t + u, b1 - 1);
+            ll[u] = LL[(size_t)i * n]; yn[u] = Y[(size_t)(i + 1) * n]; pw[u] = PV[(size_t)(i >> 5) * n];
+        }
+#pragma unroll
+        for (int u = 0; u < kIvAhead; ++u)
+            if (t + u < b1) {
+                const bool sw = pw[u] >> ((t + u) & 31) & 1u;
+                const double nx = yn[u] * sc;
+                const double bi = sw ? nx : cur, o = sw ? cur : nx;
+                Y[(size_t)(t + u) * n] = bi;
+                cur = fma(-ll[u], bi, o);
+            }
+    }
+    Y[(size_t)b1 * n] = cur;
+    back();
+    sc = nmag > 0 ? rcp_newton(__longlong_as_double(nmag)) : 1.0;
+    double s2a = 0.0, s2b = 0.0;   // two chains
+    for (int t = b0; t <= b1; t += kIvAhead) {
+        double yy[kIvAhead];
+#pragma unroll
+        for (int u = 0; u < kIvAhead; ++u) yy[u] = Y[(size_t)min(t + u, b1) * n];
+#pragma unroll
+        for (int u = 0; u < kIvAhead; ++u)
+            if (t + u <= b1) {
+                const double v = yy[u] * sc;
+                if (u & 1) s2b = fma(v, v, s2b); else s2a = fma(v, v, s2a);
+            }
+    }
+    const double s2 = s2a + s2b, inv = (s2 > 0.0) ? sc / sqrt(s2) : 0.0;
+    for (int t = b0; t <= b1; t += kIvAhead) {
+        double yy[kIvAhead];
+#pragma unroll
+        for (int u = 0; u < kIvAhead; ++u) yy[u] = Y[(size_t)min(t + u, b1) * n];
+#pragma unroll
+        for (int u = 0; u < kIvAhead; ++u)
+            if (t + u <= b1) Y[(size_t)(t + u) * n] = yy[u] * inv;
+    }
 }
 
 // Orders <= kTsMax: CTA (job, chunk of kIvThreads positions), each thread's factors and
@@ -790,15 +837,20 @@ __global__ void __launch_bounds__(kPlaceThreads) k_koltun(const DyJob *jobs, int
     }
 }
 
-cudaError_t launch_eig(const DyJob *d_jobs, int njobs, const long long *d_row_first, long long total_rows,
-                       double *work, const long long *d_work_first, cudaStream_t st) {
-    k_qrows<<<njobs, kEigThreads, 0, st>>>(d_jobs, njobs);
+cudaError_t launch_eig(const DyJob *d_jobs, int njobs, const long long *d_row_first, long long total_rows, int nmax,
+                       int nlim, double *work, const long long *d_work_first, cudaStream_t st) {
+    if (nmax > nlim) k_qrows<<<njobs, kEigThreads, 0, st>>>(d_jobs, njobs, nlim);
     k_bisect_prep<<<njobs, 256, 0, st>>>(d_jobs, njobs, work, d_work_first);
     // four lanes per eigenvalue; a matrix's few hundred eigenvalues spread over many SMs
     k_bisect<<<(unsigned)((total_rows * 4 + kBisectThreads - 1) / kBisectThreads), kBisectThreads, 0, st>>>(
         d_jobs, njobs, d_row_first, total_rows, work, d_work_first);
-    k_invit<<<(unsigned)((total_rows + 31) / 32), 32, 0, st>>>(d_jobs, njobs, d_row_first, total_rows, work,
-                                                               d_work_first);
+    if (nmax > kTsMax) {
+        const size_t smem = sizeof(double) * 2 * (size_t)(nmax < kIvTri ? nmax : kIvTri);
+        cudaError_t e = allow_dynamic_smem((const void *)k_invit);
+        if (e != cudaSuccess) return e;
+        k_invit<<<(unsigned)((total_rows + kIvLarge - 1) / kIvLarge), kIvLarge, smem, st>>>(d_jobs, njobs, d_row_first,
+                                                                                             total_rows, work, d_work_first);
+    }
     {
         const int smem = (int)(sizeof(double) * 5 * kTsMax * kIvThreads + kTsMax * kIvThreads + sizeof(double) * 2 * kTsMax);
         cudaError_t e = allow_dynamic_smem((const void *)k_invit_small);
@@ -812,6 +864,9 @@ cudaError_t launch_eig(const DyJob *d_jobs, int njobs, const long long *d_row_fi
     return cudaGetLastError();
 }
 
-void eig_smem_init() { allow_dynamic_smem((const void *)k_invit_small); }
+void eig_smem_init() {
+    allow_dynamic_smem((const void *)k_invit_small);
+    allow_dynamic_smem((const void *)k_invit);
+}
 
 }  // namespace bd
