@@ -16,7 +16,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libbd_gb300.so")
 BUILD = os.path.join(HERE, "_build")
 SOURCES = ["bd_api.cu", "k_sigma2.cu", "k_lanczos.cu", "k_dyson.cu", "k_eig.cu", "k_sort.cu", "bd_files.cu",
-           "k_coupling_tc.cu", "k_compact.cu"]
+           "k_coupling_tc.cu", "k_compact.cu", "k_lanczos_long.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 

@@ -931,7 +931,7 @@ int launch_lanczos_range(bd_ctx *ctx, int ch_lo, int ch_hi, bool fp32) {
     // rounding of the stored vectors is part of the result.)
     const bool compact = !fp32 && ctx->lz_slices == 0;
     std::vector<LzChain> ch;
-    int Smax = 1, rmax = 1;
+    int Smax = 1, rmax = 1, long_rmax = 0;
     for (int I = ch_lo; I < ch_hi; ++I) {
         Chan &C = ctx->chans[I];
         for (int dir = 0; dir < 2; ++dir) {
@@ -957,6 +957,7 @@ int launch_lanczos_range(bd_ctx *ctx, int ch_lo, int ch_hi, bool fp32) {
                 z.rowslot = ctx->d_lzslot + ctx->lz_slot_off[dir][I];
                 z.cp = ctx->d_lzcp + (size_t)(2 * I + dir) * kCpBytes;
                 z.cp_on = compact;
+                z.done = &lz_compact(z.cp).info->handled;
             }
             z.slice = ctx->d_lzslice + ctx->lz_slice_off[dir][I];
             z.slice_stride = ((long long)z.S * kLzSliceBytesPerPole + 255) / 256 * 256;
@@ -966,6 +967,7 @@ int launch_lanczos_range(bd_ctx *ctx, int ch_lo, int ch_hi, bool fp32) {
             ch.push_back(z);
             Smax = std::max(Smax, z.S);
             rmax = std::max(rmax, P.L + 1);
+            if (z.N >= kLzLong) long_rmax = std::max(long_rmax, P.L + 1);
         }
     }
     if (ch.empty()) return BD_OK;
@@ -991,6 +993,11 @@ int launch_lanczos_range(bd_ctx *ctx, int ch_lo, int ch_hi, bool fp32) {
     if (compact) {
         CU(launch_lz_compact(d_ch, (int)ch.size(), ctx->eta, ctx->st));
         ctx->launches += 1;
+        const size_t smem = long_rmax > 0 ? lanczos_long_smem(Smax, rmax, true) : 0;
+        if (smem > 0) {
+            CU(launch_lanczos_long(d_ch, (int)ch.size(), rmax, CL, ctx->eta, smem, ctx->st));
+            ctx->launches += 1;
+        }
     }
     // chains whose slices do not fit next to the scalars keep them in global memory
     const bool gslices = ctx->lz_slices == 2 || (ctx->lz_slices == 0 && lanczos_smem_bytes(Smax, rmax) > kLanczosSmemSliceCap);
@@ -1755,6 +1762,7 @@ int bd_create(bd_ctx **out, int device) {
     sigma2_smem_init();
     lanczos_smem_init();
     compact_smem_init();
+    lanczos_long_smem_init();
     *out = ctx;
     return BD_OK;
 }
@@ -2197,11 +2205,13 @@ int bd_lanczos_vectors(bd_ctx *ctx, int ish, int dir, int fp32, double *out, lon
     const int ld = lz_ld(P.N);
     char *base = ctx->d_lzV + ctx->lz_v_off[dir][ish];
     CU(cudaStreamSynchronize(ctx->st));
+    int handled = 0;
     if (!fp32 && P.L > 0) {   // a chain reduced in its couplings' space: its vectors over the poles, formed here
         char *cp = ctx->d_lzcp + (size_t)(2 * ish + dir) * kCpBytes;
         CompactInfo info;
         CU(cudaMemcpy(&info, cp, sizeof info, cudaMemcpyDeviceToHost));
-        if (info.handled) {
+        handled = info.handled;
+        if (handled == 1) {
             const Chan &C = ctx->chans[ish];
             LzChain z{};
             z.N = P.N; z.D = C.D; z.ld = ld; z.V = base; z.cp = cp;
@@ -2223,6 +2233,15 @@ int bd_lanczos_vectors(bd_ctx *ctx, int ish, int dir, int fp32, double *out, lon
     } else {
         std::vector<double> tmp((size_t)P.L * ld);
         CU(cudaMemcpy(tmp.data(), base, sizeof(double) * tmp.size(), cudaMemcpyDeviceToHost));
+        if (handled == 2) {   // two planes of integers a slot: (a 2^27 + b) 2^-57
+            std::vector<double> row(P.N);
+            for (int j = 0; j < P.L; ++j) {
+                double *r = tmp.data() + (size_t)j * ld;
+                const int *a = reinterpret_cast<const int *>(r), *b = a + ld;
+                for (int i = 0; i < P.N; ++i) row[i] = (double)((long long)a[i] * (1LL << 27) + b[i]) * 0x1p-57;
+                std::memcpy(r, row.data(), sizeof(double) * P.N);
+            }
+        }
         for (int j = 0; j < P.L; ++j)
             for (int i = 0; i < P.N; ++i) out[(size_t)j * P.N + i] = slot[j] < 0 ? 0.0 : tmp[(size_t)slot[j] * ld + i];
     }
@@ -2791,6 +2810,7 @@ extern "C" int bd_lanczos_chain_noalloc(const double *d_E, const double *d_M, in
     z.V = base + kNoallocVectors;
     z.out = d_rows;
     z.stat = reinterpret_cast<int *>(base + kNoallocCounters);
+    z.done = z.stat + 3;   // zeroed with the counters
     std::memcpy(stage, &z, sizeof(z));
 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -2800,6 +2820,9 @@ extern "C" int bd_lanczos_chain_noalloc(const double *d_E, const double *d_M, in
     if (e == cudaSuccess && fp32)
         e = launch_to_float(d_M, reinterpret_cast<float *>(base + mf_off), (long long)D * N, st);
     if (e == cudaSuccess) e = launch_lz_groups(reinterpret_cast<const LzChain *>(base), 1, lz_gram_cap(N), st);
+    if (e == cudaSuccess && !fp32 && N >= kLzLong)
+        e = launch_lanczos_long(reinterpret_cast<const LzChain *>(base), 1, P.L + 1, kNoallocCluster, kNoallocEta,
+                                lanczos_long_smem(S, P.L + 1, false), st);
     if (e == cudaSuccess)
         e = launch_lanczos(reinterpret_cast<const LzChain *>(base), 1, S, P.L + 1, fp32, kNoallocCluster, kNoallocEta,
                            false, st);

@@ -112,7 +112,10 @@ struct LzChain {
     // cp_on: whether this launch may take it (FP64 vectors).
     char *cp;
     int cp_on;
+    int *done;              // set by the kernel that reduced the chain ahead of k_lanczos (k_lz_compact's
+                            // CompactInfo::handled in a context); nullptr: k_lanczos alone
 };
+constexpr int kLzLong = 2048;   // poles from which k_lz_long takes a chain with FP64 vectors
 
 // Energy-group scratch of a chain of N poles, behind gE [2N doubles] and gInfo [N + 1
 // ints]: the Gram pieces of the groups of more than kGrpSmall poles (a piece is at most
@@ -147,7 +150,7 @@ __host__ __device__ inline GrpScratch lz_grp_scratch(const double *gE, long long
 // energies, kCpMerged groups of them and kCpDim rotated poles.
 constexpr int kCpGroups = 256, kCpMerged = 160, kCpDim = 160;
 struct CompactInfo {
-    int handled;    // 1: k_lz_compact reduced the chain; 0: k_lanczos does
+    int handled;    // 1: k_lz_compact reduced the chain, 2: k_lz_long did, 0: k_lanczos does
     int q;          // distinct energies, 0 when there are more than kCpGroups
     int np, ng;     // rotated poles, groups
     int nvec;       // vectors stored in V
@@ -183,10 +186,10 @@ struct PlainIO {
 };
 
 // Global scratch of one chain's slices: enough for any cluster size up to 16 with FP64
-// slices (E, w and E w as doubles and a touched byte: 25 bytes per pole, each CTA's share
-// rounded up to 256 bytes); a multiple of 256 bytes, so consecutive chains' slices stay
+// slices (E, w and E w as doubles and a touched byte in k_lanczos, four doubles in k_lz_long: 33
+// bytes per pole, each CTA's share rounded up to 256 bytes); a multiple of 256 bytes, so consecutive chains' slices stay
 // aligned.
-constexpr int kLzSliceBytesPerPole = 25;
+constexpr int kLzSliceBytesPerPole = 33;
 __host__ __device__ inline long long lz_slice_bytes(long long N) {
     return (kLzSliceBytesPerPole * N + 16 * (kLzSliceBytesPerPole * 4 + 256) + 255) / 256 * 256;
 }

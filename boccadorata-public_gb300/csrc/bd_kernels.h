@@ -89,6 +89,14 @@ cudaError_t launch_lz_expand(const LzChain &chain, cudaStream_t st);
 // The plain Sigma(2) rows of the full Dyson matrix, equal energies rotated (k_compact.cu).
 cudaError_t launch_plain_rotate(const LzChain *d_chains, const PlainIO *d_ios, int nchains, cudaStream_t st);
 void compact_smem_init();
+// FP64 vectors, long chains (k_lanczos_long.cu): chains with done set and at least kLzLong
+// poles, before launch_lanczos.  lanczos_long_smem: its shared memory, 0 when it cannot run
+// (rows beyond shared memory, or slices that fit neither there nor, without have_slices,
+// anywhere).  Their stored vectors are two planes of integers (k_lanczos_long.cu) per slot.
+size_t lanczos_long_smem(int S, int rmax, bool have_slices);
+cudaError_t launch_lanczos_long(const LzChain *d_chains, int nchains, int rmax, int cluster, double eta, size_t smem,
+                                cudaStream_t st);
+void lanczos_long_smem_init();
 
 int dyson_launch_count(int nmax, int Dmax, int cluster);
 cudaError_t launch_dyson(const DyJob *d_jobs, int njobs, const long long *d_row_first, long long total_rows,

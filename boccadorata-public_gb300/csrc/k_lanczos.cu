@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kLzThreads, 2) k_lanczos(const LzChain *chains
     const int cid = blockIdx.x / CL;
     if (cid >= nchains) return;  // whole clusters only: every CTA of a cluster has the same cid
     const LzChain C = chains[cid];
-    if (sizeof(VT) == 8 && C.cp && lz_compact(C.cp).info->handled) return;   // done by k_lz_compact (the whole cluster leaves)
+    if (sizeof(VT) == 8 && C.done && *C.done) return;   // done by k_lz_compact or k_lz_long (the whole cluster leaves)
     const int N = C.N, D = C.D, L = C.L, NT = C.nden_out + C.D;
     const int S = C.S;                       // multiple of 4
     const int i0 = rank * S;

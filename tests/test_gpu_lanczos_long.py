@@ -1,0 +1,119 @@
+"""The FP64 Lanczos reduction of long chains (fixed-point sweeps) against numpy and against
+the kernel of shorter chains."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from helpers import strong_diffs
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+def _reference(E, M, nit):
+    """Rows of the multi-pivot reduction with unit pivots, three Gram-Schmidt sweeps a step."""
+    D = len(M)
+    V, rows, last = [], [], []
+    for p in range(D):
+        for k in range(nit):
+            w = M[p].copy() if k == 0 else E * V[-1]
+            for _ in range(3):
+                if V:
+                    B = np.array(V)
+                    w = w - (B @ w) @ B
+            beta = np.linalg.norm(w)
+            u = w / beta
+            g = [float(np.dot(V[t], E * u)) for t in last]
+            row = np.zeros(2 * D + 1)
+            row[0], row[1] = np.dot(u, E * u), g[-1] if k == 0 and g else beta
+            row[2:2 + len(g)] = g
+            row[D + 1:] = M @ u
+            V.append(u)
+            rows.append(row)
+        last.append(len(V) - 1)
+    return np.array(rows)
+
+
+def _run(bdmod, E, M, nit):
+    D, N = M.shape
+    tE, tM = torch.from_numpy(E).cuda(), torch.from_numpy(M).cuda()
+    out = torch.full((min(N, D * nit), 2 * D + 1), float("nan"), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    L, ipiv, piv, nits = bdmod.lanczos_chain_noalloc(tE.data_ptr(), tM.data_ptr(), N, D, np.eye(D),
+                                                     np.full(D, nit, np.int32), out.data_ptr(), len(out))
+    return out.cpu().numpy()[:L]
+
+
+# the shortest chain it takes and one less; remainders of the 16 slices and of the four poles a
+# thread; more vectors than the 64 a round of warps takes; D = 1 and 8
+@pytest.mark.parametrize("N,D,nit", [(2047, 2, 9), (2048, 2, 9), (2049, 1, 30), (4099, 8, 9), (20011, 4, 17)])
+def test_rows_against_numpy(bdmod, N, D, nit):
+    rng = np.random.default_rng(N)
+    E = np.sort(rng.uniform(20.0, 300.0, N))
+    M = rng.standard_normal((D, N)) * np.exp(-E / 100.0)
+    got, ref = _run(bdmod, E, M, nit), _reference(E, M, nit)
+    scale = np.maximum(np.abs(ref).max(0), 1e-300)
+    # FP64 rounding of E v (a few hundred eps of a coupling) over the steps
+    assert (np.abs(got - ref) / scale).max() < 1e-11
+
+
+@pytest.mark.parametrize("kind", ["zeros", "huge", "tiny", "few"])
+def test_unusual_chains(bdmod, kind):
+    """Poles no vector reaches; energies and couplings outside the fixed-point range (left to
+    the other kernel); a space of fewer directions than rows (its restart vectors too)."""
+    rng = np.random.default_rng(5)
+    N, D, nit = 3001, 2, 10
+    E = np.sort(rng.uniform(20.0, 300.0, N))
+    M = rng.standard_normal((D, N))
+    scale = 1.0
+    if kind == "zeros":
+        M[:, 1::3] = 0.0
+    elif kind == "huge":
+        scale = 1e14
+        E = E * scale
+    elif kind == "tiny":
+        M = M * 1e-14
+    else:
+        M[:, 12:] = 0.0                # twelve reachable poles: both chains end early
+        nit = 40
+    got = _run(bdmod, E, M, nit)
+    assert np.isfinite(got).all() and len(got) == D * nit
+    if kind == "few":
+        # the twelve poles the couplings reach and rows that couple to nothing: sum of m m^T kept
+        G = got[:, D + 1:].T @ got[:, D + 1:]
+        np.testing.assert_allclose(G, M @ M.T, rtol=1e-10)
+        return
+    ref = _reference(E, M, nit)
+    s = np.maximum(np.abs(ref).max(0), 1e-300)
+    assert (np.abs(got - ref) / s).max() < 1e-11
+
+
+def test_dressed_chains_vectors_and_slices(bdmod, problems):
+    """A context's long chains: the stored basis read back (two integer planes a vector), and
+    clusters of 2 CTAs, whose slices do not fit in shared memory, against 8."""
+    p = problems(6, 20.0, 1, 12)
+    ctx = bdmod.Context().upload(p)
+    ctx.run_all(lanczos=True)
+    ctx.dressed_propagator(1e-3, 2)
+    ish = max(range(p.ms.nsubsh), key=lambda i: ctx.count_poles(i)[0])
+    n = ctx.count_poles(ish)
+    assert n[0] > 20000
+    ctx.run_all(lanczos=True)
+    a = ctx.result(ish)
+    pv = p.piv
+    fw, _ = ctx.sigma2_build(ish)
+    lz = ctx.lanczos_reduce(ish, pv.vec[ish], pv.n_fw[ish], pv.n_bk[ish])
+    V = ctx.lanczos_vectors(ish, 0, len(lz["lz_fw"]), n[0])
+    assert np.abs(V @ V.T - np.eye(len(V))).max() < 1e-13
+    E = np.sort(fw[:, 0])
+    alpha = np.einsum("ti,i,ti->t", V, E, V)
+    assert np.abs(alpha - lz["lz_fw"][:, 0]).max() < 1e-12 * np.abs(E).max()
+    ctx.set_tuning(lz_cluster=2)
+    ctx.run_all(lanczos=True)
+    b = ctx.result(ish)
+    for tag in ("qp", "qh"):
+        e, z = strong_diffs(a[tag], b[tag])
+        assert e < 1e-10 and z < 1e-9
+    ctx.close()
