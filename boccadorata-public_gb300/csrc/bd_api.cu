@@ -1249,10 +1249,12 @@ int alloc_lanczos(bd_ctx *ctx) {
     if ((rc = dalloc(ctx, &ctx->d_lzstat, 4))) return rc;
     CU(cudaMemsetAsync(ctx->d_lzstat, 0, sizeof(int) * 4, ctx->st));
     if ((rc = dalloc(ctx, &ctx->d_chains, (size_t)2 * ctx->nsubsh))) return rc;
-    if ((rc = dalloc(ctx, &ctx->d_lzslice, (size_t)slices))) return rc;
-    if ((rc = dalloc(ctx, &ctx->d_lzgrp, (size_t)groups))) return rc;
-    if ((rc = dalloc(ctx, &ctx->d_lzslot, (size_t)slots))) return rc;
-    if ((rc = dalloc(ctx, &ctx->d_lzcp, (size_t)2 * ctx->nsubsh * (size_t)kCpBytes))) return rc;
+    // the chains' scratch in one allocation (slices, groups and kCpBytes are multiples of 256)
+    const size_t cpb = (size_t)2 * ctx->nsubsh * (size_t)kCpBytes;
+    if ((rc = dalloc(ctx, &ctx->d_lzslice, (size_t)slices + (size_t)groups + cpb + sizeof(int) * (size_t)slots))) return rc;
+    ctx->d_lzgrp = ctx->d_lzslice + slices;
+    ctx->d_lzcp = ctx->d_lzgrp + groups;
+    ctx->d_lzslot = reinterpret_cast<int *>(ctx->d_lzcp + cpb);
     CU(cudaMemset2DAsync(ctx->d_lzcp, (size_t)kCpBytes, 0, sizeof(CompactInfo), (size_t)2 * ctx->nsubsh, ctx->st));
     return BD_OK;
 }
@@ -2203,9 +2205,10 @@ int bd_lanczos_vectors(bd_ctx *ctx, int ish, int dir, int fp32, double *out, lon
     const long long need = (long long)P.L * P.N;
     if (!out || cap < need) return fail(ctx, BD_ERR_CAPACITY, "need %lld doubles", need);
     const int ld = lz_ld(P.N);
-    char *base = ctx->d_lzV + ctx->lz_v_off[dir][ish];
+    const char *base = ctx->d_lzV + ctx->lz_v_off[dir][ish];
     CU(cudaStreamSynchronize(ctx->st));
     int handled = 0;
+    double *expanded = nullptr;
     if (!fp32 && P.L > 0) {   // a chain reduced in its couplings' space: its vectors over the poles, formed here
         char *cp = ctx->d_lzcp + (size_t)(2 * ish + dir) * kCpBytes;
         CompactInfo info;
@@ -2213,12 +2216,14 @@ int bd_lanczos_vectors(bd_ctx *ctx, int ish, int dir, int fp32, double *out, lon
         handled = info.handled;
         if (handled == 1) {
             const Chan &C = ctx->chans[ish];
+            CU(cudaMallocAsync(&expanded, sizeof(double) * (size_t)P.L * ld, ctx->st));
             LzChain z{};
-            z.N = P.N; z.D = C.D; z.ld = ld; z.V = base; z.cp = cp;
+            z.N = P.N; z.D = C.D; z.ld = ld; z.V = ctx->d_lzV + ctx->lz_v_off[dir][ish]; z.cp = cp;
             z.M = (dir == 0 ? ctx->d_Mfw_s : ctx->d_Mbk_s) + (dir == 0 ? C.mfw_off : C.mbk_off);
-            CU(launch_lz_expand(z, ctx->st));
+            CU(launch_lz_expand(z, expanded, ctx->st));
             ctx->launches += 1;
             CU(cudaStreamSynchronize(ctx->st));
+            base = reinterpret_cast<const char *>(expanded);
         }
     }
     // rows of a deflated tail have no stored vector: zero rows
@@ -2245,6 +2250,7 @@ int bd_lanczos_vectors(bd_ctx *ctx, int ish, int dir, int fp32, double *out, lon
         for (int j = 0; j < P.L; ++j)
             for (int i = 0; i < P.N; ++i) out[(size_t)j * P.N + i] = slot[j] < 0 ? 0.0 : tmp[(size_t)slot[j] * ld + i];
     }
+    if (expanded) CU(cudaFreeAsync(expanded, ctx->st));
     return BD_OK;
 }
 

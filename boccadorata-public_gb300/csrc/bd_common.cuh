@@ -148,12 +148,12 @@ __host__ __device__ inline GrpScratch lz_grp_scratch(const double *gE, long long
 
 // The same chain in the space its couplings span (k_compact.cu): at most kCpGroups distinct
 // energies, kCpMerged groups of them and kCpDim rotated poles.
-constexpr int kCpGroups = 256, kCpMerged = 160, kCpDim = 160;
+constexpr int kCpGroups = 128, kCpMerged = 96, kCpDim = 160;
 struct CompactInfo {
     int handled;    // 1: k_lz_compact reduced the chain, 2: k_lz_long did, 0: k_lanczos does
     int q;          // distinct energies, 0 when there are more than kCpGroups
     int np, ng;     // rotated poles, groups
-    int nvec;       // vectors stored in V
+    int nvec;       // vectors stored, np doubles each, from the chain's V on
 };
 struct CompactGroup {
     int p0, m;      // first pole and poles of the group
@@ -166,17 +166,16 @@ struct CompactScratch {
     CompactGroup *grp;   // [kCpMerged]
     double *gram;        // [kCpGroups][kGramEntries] M M^T of every energy's poles, lower triangle
     double *L;           // [kCpMerged][64] Cholesky factors, D x D row-major
-    double *V;           // [kCpDim][np] stored vectors
 };
 constexpr long long kCpStartOff = 256, kCpGrpOff = kCpStartOff + 4 * (kCpGroups + 4),
                     kCpGramOff = (kCpGrpOff + 20 * kCpMerged + 255) / 256 * 256,
-                    kCpLOff = kCpGramOff + 8LL * kCpGroups * kGramEntries, kCpVOff = kCpLOff + 8LL * 64 * kCpMerged,
-                    kCpBytes = (kCpVOff + 8LL * kCpDim * kCpDim + 255) / 256 * 256;
+                    kCpLOff = kCpGramOff + 8LL * kCpGroups * kGramEntries,
+                    kCpBytes = (kCpLOff + 8LL * 64 * kCpMerged + 255) / 256 * 256;
 static_assert(sizeof(CompactInfo) <= kCpStartOff && sizeof(CompactGroup) == 20, "compact scratch layout");
 __host__ __device__ inline CompactScratch lz_compact(char *b) {
     return CompactScratch{reinterpret_cast<CompactInfo *>(b), reinterpret_cast<int *>(b + kCpStartOff),
                           reinterpret_cast<CompactGroup *>(b + kCpGrpOff), reinterpret_cast<double *>(b + kCpGramOff),
-                          reinterpret_cast<double *>(b + kCpLOff), reinterpret_cast<double *>(b + kCpVOff)};
+                          reinterpret_cast<double *>(b + kCpLOff)};
 }
 
 // Rows of a plain Sigma(2) for the full Dyson matrix (k_plain_rotate): as built, and rotated.

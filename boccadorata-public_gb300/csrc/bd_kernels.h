@@ -85,7 +85,7 @@ cudaError_t launch_lz_groups(const LzChain *d_chains, int nchains, long long gra
 // launch_lz_groups and before launch_lanczos, which leaves out the chains it handled; and
 // the stored vectors of such a chain in the poles' space.
 cudaError_t launch_lz_compact(const LzChain *d_chains, int nchains, double eta, cudaStream_t st);
-cudaError_t launch_lz_expand(const LzChain &chain, cudaStream_t st);
+cudaError_t launch_lz_expand(const LzChain &chain, double *out, cudaStream_t st);
 // The plain Sigma(2) rows of the full Dyson matrix, equal energies rotated (k_compact.cu).
 cudaError_t launch_plain_rotate(const LzChain *d_chains, const PlainIO *d_ios, int nchains, cudaStream_t st);
 void compact_smem_init();

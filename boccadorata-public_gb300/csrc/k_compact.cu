@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
             const double v = w[i] * ixb;
             V[(size_t)nvec * np + i] = v;
             Vf[(size_t)nvec * np + i] = (float)v;
-            S.V[(size_t)nvec * np + i] = v;
+            reinterpret_cast<double *>(C.V)[(size_t)nvec * np + i] = v;   // (np <= N: within the chain's store)
         }
         e2v = sc[2] * ixb * ixb;
         if (tid < NT) {
@@ -407,13 +407,13 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
     for (int g = tid; g < ng; g += kCpThreads) S.grp[g].off = s_off[g];
 }
 
-// The stored vectors of a compact chain in the poles' space, into C.V (slot-major, stride
-// ld): a thread per pole, its group's L^-T v' formed by the D-term back substitution
+// The stored vectors of a compact chain in the poles' space, into out (slot-major, stride
+// C.ld): a thread per pole, its group's L^-T v' formed by the D-term back substitution
 // against the pole's own couplings (y = L^-1 M_p, then v_p = sum_c y_c v'_c).
-__global__ void k_lz_expand(const LzChain C) {
+__global__ void k_lz_expand(const LzChain C, double *out) {
     const CompactScratch S = lz_compact(C.cp);
     const int np = S.info->np, ng = S.info->ng, nvec = S.info->nvec, D = C.D;
-    double *V = reinterpret_cast<double *>(C.V);
+    const double *V = reinterpret_cast<const double *>(C.V);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < C.N; i += gridDim.x * blockDim.x) {
         int lo = 0, hi = ng - 1;   // the last group starting at or before pole i
         while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (S.grp[mid].p0 <= i) lo = mid; else hi = mid - 1; }
@@ -433,7 +433,7 @@ __global__ void k_lz_expand(const LzChain C) {
             }
         }
         for (int t = 0; t < nvec; ++t) {
-            const double *vt = S.V + (size_t)t * np + G.off;
+            const double *vt = V + (size_t)t * np + G.off;
             double s = 0.0;
             if (G.kept) {
                 s = vt[i - G.p0];
@@ -441,7 +441,7 @@ __global__ void k_lz_expand(const LzChain C) {
 #pragma unroll
                 for (int a = 0; a < 8; ++a) if (a < D) s = fma(y[a], vt[a], s);
             }
-            V[(size_t)t * C.ld + i] = s;
+            out[(size_t)t * C.ld + i] = s;
         }
     }
 }
@@ -511,8 +511,8 @@ cudaError_t launch_lz_compact(const LzChain *d_chains, int nchains, double eta, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_lz_expand(const LzChain &chain, cudaStream_t st) {
-    k_lz_expand<<<(chain.N + 127) / 128, 128, 0, st>>>(chain);
+cudaError_t launch_lz_expand(const LzChain &chain, double *out, cudaStream_t st) {
+    k_lz_expand<<<(chain.N + 127) / 128, 128, 0, st>>>(chain, out);
     return cudaGetLastError();
 }
 

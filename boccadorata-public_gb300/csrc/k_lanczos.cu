@@ -1188,13 +1188,17 @@ namespace bd {
 //                kGrpSmall poles cut into Gram pieces of at most kGrpPiece poles;
 //   k_lz_gram    the pieces' partial Gram matrices, spread over the whole GPU (degenerate
 //                shells give a chain a few groups of thousands of poles, and their FP64
-//                sums on one SM would take tens of microseconds);
+//                sums on one SM would take tens of microseconds), and the small groups of
+//                chains of many energies, a thread each;
 //   k_lz_groups  a CTA per chain: one-pole groups, the small groups (a warp each), the
 //                sums of the pieces, the eliminations and the cumulative counts.
 constexpr int kGrpThreads = 512;
 constexpr int kGstartThreads = 512;
 constexpr int kGramThreads = 128;
 constexpr int kGramCtas = 608;   // four per SM
+// Chains of more than kGrpMany energies (dressed propagators: tens of thousands): groups of up
+// to kGrpThread poles are ranked a thread each, over the whole GPU, in k_lz_gram.
+constexpr int kGrpMany = kCpGroups, kGrpThread = 16;
 
 // Block-wide exclusive scan of one int per thread (T threads, a multiple of 32): returns
 // the thread's exclusive prefix and sets total.  ws holds T / 32 ints.
@@ -1284,6 +1288,87 @@ __global__ void __launch_bounds__(kGstartThreads) k_lz_gstart(const LzChain *cha
     }
 }
 
+// Directions of a group of m poles from g0 on that no coupling reaches, m - rank(M), by one
+// thread: warp_rank's scaling, pivots and threshold on the lower triangle in registers (the
+// pivot's column taken by selects, so every index is known).  A warp a group, as the larger ones
+// take, holds the FP64 unit for as long with two of its 32 lanes' worth of work: 2.1 M poles in
+// 0.7 M groups took 2.0 ms on the chains' own CTAs, 0.2 ms here.
+template <int D>
+__device__ __forceinline__ int thread_unreached(const double *M, size_t N, int g0, int m) {
+    constexpr int P = D * (D + 1) / 2;
+    if (m == 1) {
+        bool any = false;
+#pragma unroll
+        for (int a = 0; a < D; ++a) any |= (__double_as_longlong(M[a * N + g0]) << 1) != 0;
+        return any ? 0 : 1;
+    }
+    double h[P];
+#pragma unroll
+    for (int u = 0; u < P; ++u) h[u] = 0.0;
+    for (int i = g0; i < g0 + m; ++i) {
+        double mv[D];
+#pragma unroll
+        for (int a = 0; a < D; ++a) mv[a] = M[a * N + i];
+        int u = 0;
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+#pragma unroll
+            for (int b = 0; b <= a; ++b) { h[u] = fma(mv[a], mv[b], h[u]); ++u; }
+    }
+    auto at = [](int a, int b) { return a >= b ? a * (a + 1) / 2 + b : b * (b + 1) / 2 + a; };
+    long long gbits = 0;
+#pragma unroll
+    for (int a = 0; a < D; ++a) gbits = max(gbits, __double_as_longlong(h[at(a, a)]));
+    if (gbits <= 0 || gbits >= 0x7ff0000000000000LL) return m;   // zero couplings (or not finite)
+    const double scale = __longlong_as_double((long long)max(1, 2046 - (int)(gbits >> 52)) << 52);
+#pragma unroll
+    for (int u = 0; u < P; ++u) h[u] *= scale;
+    const long long thr = __double_as_longlong(1e-12 * (__longlong_as_double(gbits) * scale));
+    unsigned used = 0;
+    int rank = 0;
+#pragma unroll 1
+    for (int st = 0; st < D && rank < m; ++st) {
+        long long best = thr;
+        int pv = -1;
+#pragma unroll
+        for (int a = 0; a < D; ++a) {
+            const long long v = __double_as_longlong(h[at(a, a)]);
+            if (!(used >> a & 1u) && v > best && v < 0x7ff0000000000000LL) { best = v; pv = a; }
+        }
+        if (pv < 0) break;
+        used |= 1u << pv;
+        ++rank;
+        const double p = __longlong_as_double(best);
+        double inv = (double)__frcp_rn((float)p);
+        inv = fma(inv, fma(-p, inv, 1.0), inv);
+        double col[D];
+#pragma unroll
+        for (int a = 0; a < D; ++a) {
+            double x = 0.0;
+#pragma unroll
+            for (int b = 0; b < D; ++b) x = (pv == b) ? h[at(a, b)] : x;
+            col[a] = x;
+        }
+#pragma unroll
+        for (int a = 0; a < D; ++a) {
+            const double f = -col[a] * inv;
+#pragma unroll
+            for (int b = 0; b <= a; ++b)
+                if (!(used >> a & 1u) && !(used >> b & 1u)) h[at(a, b)] = fma(f, col[b], h[at(a, b)]);
+        }
+    }
+    return max(0, m - rank);
+}
+
+template <int D>
+__device__ void rank_chunk(const LzChain &C, int q) {   // group q of chain C, a thread's
+    const int *gInfo = C.gInfo;
+    const int Q = gInfo[0], N = C.N;
+    if (q >= Q) return;
+    const int g0 = gInfo[1 + q], m = ((q + 1 < Q) ? gInfo[2 + q] : N) - g0;
+    if (m <= kGrpThread) const_cast<double *>(C.gE)[N + q] = (double)thread_unreached<D>(C.M, (size_t)N, g0, m);
+}
+
 // One piece's partial Gram matrix (the lower triangle, D(D+1)/2 entries): each thread
 // sums its poles' products, each warp's 32 partial sums of an entry are added by one
 // lane, and the warps' sums in warp order; the order is fixed, so the sums repeat.
@@ -1368,6 +1453,31 @@ __global__ void __launch_bounds__(kGramThreads) k_lz_gram(const LzChain *chains,
             }
         }
         base += tot;
+        __syncthreads();   // pre is rewritten below
+        // the small groups of chains of many energies, 128 a chunk, CTA k chunks k, k + grid, ..
+        int nch = 0;
+        if (c < nchains && chains[c].gE && chains[c].gInfo[0] > kGrpMany) nch = (chains[c].gInfo[0] + kGramThreads - 1) / kGramThreads;
+        pre[threadIdx.x] = block_excl_scan<kGramThreads>(nch, tot, ws);
+        __syncthreads();
+        for (int v = blockIdx.x; v < tot; v += G) {
+            int lo = 0, hi = nc - 1;   // the last chain whose first chunk is <= v
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (pre[mid] <= v) lo = mid; else hi = mid - 1;
+            }
+            const LzChain &C = chains[c0 + lo];
+            const int q = (v - pre[lo]) * kGramThreads + threadIdx.x;
+            switch (C.D) {
+                case 1: rank_chunk<1>(C, q); break;
+                case 2: rank_chunk<2>(C, q); break;
+                case 3: rank_chunk<3>(C, q); break;
+                case 4: rank_chunk<4>(C, q); break;
+                case 5: rank_chunk<5>(C, q); break;
+                case 6: rank_chunk<6>(C, q); break;
+                case 7: rank_chunk<7>(C, q); break;
+                default: rank_chunk<8>(C, q); break;
+            }
+        }
         __syncthreads();   // pre is rewritten for the next chains
     }
 }
@@ -1437,9 +1547,8 @@ __device__ int warp_rank(const double *tri, double *H, int lane) {
 // groups spread over all of them): up to kGrpSmall poles the Gram entries are summed here
 // (lanes over the entries, one FP64 instruction per pole for all of them, when they fit in
 // a warp), beyond that from the pieces' partial sums in piece order; then warp_rank.
-// A dressed propagator's chain has one group per pole, tens of thousands: with each warp
-// walking over its groups one after another to skip the one-pole ones the kernel took
-// 2.47 ms at 2.1 M poles in 52 chains (0.82 ms at 0.9 M in 68).
+// Of a chain with more than kGrpMany energies only the groups of more than kGrpThread poles are
+// left here (k_lz_gram ranks the others).
 template <int D>
 __device__ void group_counts(const LzChain &C, int Q, double *gE, const int *gInfo, const GrpScratch &S, int warp,
                              int lane, double *tri, double *H, double *gram) {
@@ -1504,6 +1613,9 @@ __device__ void group_counts(const LzChain &C, int Q, double *gE, const int *gIn
             m[u] = (q < Q) ? ((q + 1 < Q) ? gInfo[2 + q] : N) - g0[u] : 0;
             any[u] = false;
         }
+#pragma unroll
+        for (int u = 0; u < kGrpPer; ++u)
+            if (Q > kGrpMany && m[u] <= kGrpThread) m[u] = 0;   // k_lz_gram's
 #pragma unroll
         for (int a = 0; a < D; ++a)
 #pragma unroll

@@ -117,3 +117,28 @@ def test_dressed_chains_vectors_and_slices(bdmod, problems):
         e, z = strong_diffs(a[tag], b[tag])
         assert e < 1e-10 and z < 1e-9
     ctx.close()
+
+
+@pytest.mark.parametrize("D,nq", [(1, 300), (3, 300), (7, 270), (8, 129), (3, 128)])
+def test_unreached_directions_of_many_groups(bdmod, D, nq):
+    """Groups of 1 to 24 equal energies, more (and just as many) energies than are ranked by
+    whole warps: an exhausted chain's rows take each group's m - rank(M) directions in order."""
+    rng = np.random.default_rng(D)
+    m = np.arange(nq) % 24 + 1
+    Eq = np.sort(rng.uniform(20.0, 300.0, nq))
+    E = np.repeat(Eq, m)
+    first = np.concatenate([[0], np.cumsum(m)])
+    M = np.zeros((D, len(E)))
+    expect = []
+    for q in range(nq):
+        s = slice(first[q], first[q + 1])
+        if q % 40 == 7:                                    # full rank
+            M[:, s] = rng.standard_normal((D, m[q]))
+        elif q % 40 == 23:                                 # rank one (24 poles)
+            M[:, s] = np.outer(rng.standard_normal(D), rng.standard_normal(m[q]))
+        rank = np.linalg.matrix_rank(M[:, s]) if M[:, s].any() else 0
+        expect += [Eq[q]] * (m[q] - int(rank))
+    got = _run(bdmod, E, M, 60)
+    defl = got[np.abs(got[:, 1:]).max(1) == 0, 0]
+    assert len(defl) > 20
+    assert np.array_equal(defl, np.array(expect)[:len(defl)])
