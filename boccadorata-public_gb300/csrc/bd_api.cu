@@ -284,7 +284,7 @@ struct bd_ctx {
     // into tiles of up to 128 rows; usable when every block's pair count fits
     int *d_tc_blk = nullptr;
     int4 *d_tc_tiles = nullptr;
-    int ntc_tiles = 0, tc_np_fw = 0, tc_np_bk = 0;
+    int ntc_tiles = 0, tc_np = 0, tc_np_fw = 0, tc_np_bk = 0;   // columns of a tile at most, in all and by direction
     bool tc_ok = false;
     bool prop_dressed = false;   // some fragment has more than one non-zero amplitude
     bool last_tc = false;        // the last batched step built the couplings on the tensor cores
@@ -741,14 +741,16 @@ int build_tc_tiles(bd_ctx *c) {
     c->tc_blk.resize(nb);
     for (size_t b = 0; b < nb; ++b) c->tc_blk[first[key((int)b)]++] = (int)b;
     c->tc_tiles.clear();
-    c->tc_np_fw = c->tc_np_bk = 0;
+    c->tc_np = c->tc_np_fw = c->tc_np_bk = 0;
     c->tc_ok = true;
     for (size_t q = 0; q < nb;) {
         const int b0 = c->tc_blk[q];
         const S2Block &B = c->blocks[b0];
         if ((long long)c->no[B.ia] * c->no[B.ib] > 64 || B.nfw > 256 || B.nbk > 256) c->tc_ok = false;
-        c->tc_np_fw = std::max(c->tc_np_fw, (B.nfw + 15) & ~15);
-        c->tc_np_bk = std::max(c->tc_np_bk, (B.nbk + 15) & ~15);
+        const int nf = (B.nfw + 15) & ~15, nk = (B.nbk + 15) & ~15;
+        c->tc_np_fw = std::max(c->tc_np_fw, nf);
+        c->tc_np_bk = std::max(c->tc_np_bk, nk);
+        c->tc_np = std::max(c->tc_np, nf + nk);
         int rows = 0, n = 0;
         size_t e = q;
         while (e < nb && key(c->tc_blk[e]) == key(b0) && rows + c->no[c->blocks[c->tc_blk[e]].ch] <= 128) {
@@ -796,19 +798,19 @@ int launch_sigma2(bd_ctx *ctx, int ch_lo, int ch_hi, cudaStream_t aux = nullptr,
         CU(cudaEventRecord(ctx->ev_fork2, ctx->st));
         CU(cudaStreamWaitEvent(aux, ctx->ev_fork2, 0));
     }
-    if (tc) {   // (all channels: the tiles mix them)
-        for (int dir = 1; dir >= 0; --dir) {
-            const int np = dir == 0 ? ctx->tc_np_fw : ctx->tc_np_bk;
+    if (tc) {   // (all channels and both directions: the tiles mix them)
+        const TcOut fw{ctx->d_Efw, ctx->d_S2fw, ctx->d_Mfw}, bk{ctx->d_Ebk, ctx->d_S2bk, ctx->d_Mbk};
+        // both directions of a tile together, unless some tile's columns exceed the MMA's 256
+        const bool both = ctx->tc_np <= 256;
+        for (int half = 0; half < (both ? 1 : 2); ++half) {
+            const int dirs = both ? 3 : 1 + half;
+            const int np = both ? ctx->tc_np : half == 0 ? ctx->tc_np_fw : ctx->tc_np_bk;
             if (np == 0) continue;
-            const size_t smem = tc_smem_bytes(np);
-            cudaStream_t st = (dir == 1 && aux) ? aux : ctx->st;
-            CU(launch_poles_tc(ctx->dp, ctx->d_blocks, ctx->d_tc_blk, ctx->d_tc_tiles, ctx->ntc_tiles, ctx->d_cs, dir,
-                               ctx->d_vp, dir == 0 ? ctx->d_Efw : ctx->d_Ebk, dir == 0 ? ctx->d_S2fw : ctx->d_S2bk,
-                               dir == 0 ? ctx->d_Mfw : ctx->d_Mbk, ctx->d_lzstat + 3, smem, st));
+            CU(launch_poles_tc(ctx->dp, ctx->d_blocks, ctx->d_tc_blk, ctx->d_tc_tiles, ctx->ntc_tiles, ctx->d_cs, ctx->d_vp,
+                               fw, bk, dirs, ctx->d_lzstat + 3, tc_smem_bytes(np), ctx->st));
             ctx->launches += 1;
-            if (dir == 1 && aux) CU(cudaEventRecord(ctx->ev_join2, aux));
         }
-        if (aux && ctx->tc_np_bk == 0) CU(cudaEventRecord(ctx->ev_join2, aux));
+        if (aux) CU(cudaEventRecord(ctx->ev_join2, aux));
         return BD_OK;
     }
     if (nk > 0) {

@@ -12,8 +12,9 @@
 // operand of 128 rows (their D rows each): one tile is one 128 x N x K product, N the
 // block's poles padded to 16, K = pairs x orbitals of ig.
 //
-// Each tile: a CTA of four warps stages A (V') and B in shared memory in the canonical
-// no-swizzle K-major layout (8-row x 16-byte core matrices), 64 K columns at a time; every
+// Each tile, both directions at once (the forward poles' columns, then the backward ones':
+// they share A): a CTA of four warps stages A (V') and B in shared memory in the canonical
+// no-swizzle K-major layout (8-row x 16-byte core matrices), 16 K columns at a time; every
 // value is split into two TF32 parts, hi + lo, and thread 0 issues three tcgen05.mma
 // (kind::tf32, M = 128) per 8 columns, hi*hi + hi*lo + lo*hi, accumulating in FP32 in
 // tensor memory (about 2^-21 relative per product, against the FP32 Lanczos vectors'
@@ -22,6 +23,11 @@
 // CTA forms the poles' energies (FP64, the reference's operations: the same bits as
 // k_poles) and S2 = sum_d M^2.  Every FP64 -> FP32 conversion of the staging is done on
 // the integer pipe (the double's bits truncated): the FP64 unit issues at 1/64 of FP32.
+// A tile is a few dozen MMAs, so its time is the staging and the chains in front of it: a
+// thread (two, four) per row with the row's address and the columns' offsets looked up once,
+// the rows' table from a scan over the blocks, no row or column staged that nobody reads.
+// Sigma(2) phase of a dressed step, N_max = 8, one fragment: 5.2 -> 1.0 ms (64 columns a round:
+// 1.9, 32: 1.2); two fragments 5.7 -> 1.1; N_max = 4: 0.30 -> 0.09.
 #include "bd_common.cuh"
 #include "bd_kernels.h"
 
@@ -30,9 +36,9 @@ namespace bd {
 namespace {
 
 constexpr int kTcRows = 128;     // MMA M: rows of a tile
-constexpr int kTcKc = 64;        // K columns staged per round
+constexpr int kTcKc = 16;        // K columns staged per round (a tile is short: the rounds of eight CTAs an SM overlap)
 constexpr int kTcThreads = 128;  // four warps: one per 32 lanes of tensor memory
-constexpr int kTcPairs = 64;     // (alpha, beta) pairs of a block at most (orbitals <= 8)
+constexpr int kTcKMax = 64 * 8;  // columns at most: 64 (alpha, beta) pairs, 8 orbitals
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -131,111 +137,156 @@ __device__ __forceinline__ void pole_frags(const S2Block &B, int t, int nAa, int
 }  // namespace
 
 __global__ void __launch_bounds__(kTcThreads) k_poles_tc(DevProblem P, const S2Block *blk, const int *tile_blk,
-                                                         const int4 *tiles, int ntiles, const ChanSig *cs, int dir,
-                                                         const double *vp, double *E, double *S2, double *M,
-                                                         int *err) {
+                                                         const int4 *tiles, int ntiles, const ChanSig *cs,
+                                                         const double *vp, TcOut fw, TcOut bk, int dirs, int *err) {
     const int tile = blockIdx.x;
     if (tile >= ntiles) return;
     const int4 T4 = tiles[tile];   // first entry in tile_blk, blocks, rows
     const int b_first = T4.x, nblk = T4.y, rows = T4.z;
     const S2Block B0 = blk[tile_blk[b_first]];
-    const int T = dir == 0 ? B0.nfw : B0.nbk;   // poles of each block of the tile
-    if (T <= 0) return;
+    // poles of each block of the tile, forward and backward (dirs: which of the two)
+    const int Tn[2] = {(dirs & 1) ? B0.nfw : 0, (dirs & 2) ? B0.nbk : 0};
+    if (Tn[0] <= 0 && Tn[1] <= 0) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int NS = P.nspb;
-    const int *nA = dir == 0 ? P.np : P.nh, *nGv = dir == 0 ? P.nh : P.np;
-    const int *sA = dir == 0 ? P.p_start : P.h_start, *sG = dir == 0 ? P.h_start : P.p_start;
-    const double *eA = dir == 0 ? P.ep : P.eh, *eG = dir == 0 ? P.eh : P.ep;
-    const double *fA = dir == 0 ? P.fqp : P.fqh, *fG = dir == 0 ? P.fqh : P.fqp;
     const int ia = B0.ia, ib = B0.ib, ig = B0.ig;
     const int noa = P.no[ia], nob = P.no[ib], nog = P.no[ig];
-    const int nAa = nA[ia], nAb = nA[ib], nG = nGv[ig];
-    const int Np = (T + 15) & ~15;
+    const int col0[2] = {0, (Tn[0] + 15) & ~15};   // first column of each direction
+    const int Np = col0[1] + ((Tn[1] + 15) & ~15);
 
     extern __shared__ __align__(1024) unsigned char smc[];
     float *Ahi = reinterpret_cast<float *>(smc);           // [kTcRows][kTcKc] K-major core matrices
     float *Alo = Ahi + kTcRows * kTcKc;
     float *Bhi = Alo + kTcRows * kTcKc;                    // [Np][kTcKc]
     float *Blo = Bhi + Np * kTcKc;
-    __shared__ int s_pa[kTcPairs], s_pb[kTcPairs];          // (alpha, beta) of pair p
-    __shared__ int s_np;
+    __shared__ __align__(16) int s_k[kTcKMax];                            // column k: offset in a row of V' | gamma << 16 | alpha << 20 | beta << 24, or -1
     __shared__ short s_rblk[kTcRows], s_rd[kTcRows];        // block (in the tile) and d of every row
+    __shared__ int s_wsum[kTcThreads / 32];
     __shared__ uint32_t s_taddr;
     __shared__ __align__(8) uint64_t s_bar;
 
-    if (tid == 0) {
-        int n = 0;
-        for (int a = 0; a < noa; ++a)
-            for (int b = (ia == ib) ? a + B0.nJab : 0; b < nob; ++b)
-                if (n < kTcPairs) { s_pa[n] = a; s_pb[n] = b; ++n; }
-        s_np = n;
-        int r = 0;
-        for (int q = 0; q < nblk && r < kTcRows; ++q) {
-            const int D = P.no[blk[tile_blk[b_first + q]].ch];
-            for (int d = 0; d < D && r < kTcRows; ++d, ++r) { s_rblk[r] = (short)q; s_rd[r] = (short)d; }
-        }
-        mbar_init(&s_bar);
-    }
+    const int npair = ia == ib ? noa * (noa + 1) / 2 - B0.nJab * noa : noa * nob;   // (alpha, beta), beta >= alpha + nJab for ia == ib
+    const int K = npair * nog;
     const int ncols = Np <= 32 ? 32 : Np <= 64 ? 64 : Np <= 128 ? 128 : 256;
+    if (tid == 0) mbar_init(&s_bar);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      :: "r"(smem_addr(&s_taddr)), "r"(ncols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
+    // the rows of the tile's blocks, a block each: their first rows by a scan over the blocks' D
+    {
+        const int Dq = tid < nblk ? P.no[blk[tile_blk[b_first + tid]].ch] : 0;
+        int v = Dq;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += y;
+        }
+        if (lane == 31) s_wsum[warp] = v;
+        __syncthreads();
+        int r = v - Dq;
+        for (int w = 0; w < warp; ++w) r += s_wsum[w];
+        for (int d = 0; d < Dq && r + d < kTcRows; ++d) { s_rblk[r + d] = (short)tid; s_rd[r + d] = (short)d; }
+    }
+    // the columns
+    const int Kp = min((K + 7) & ~7, kTcKMax);
+    for (int k = tid; k < Kp; k += kTcThreads) {
+        int v = -1;
+        if (k < K) {
+            const int p = k / nog, gam = k - p * nog;
+            int a, b;
+            if (ia == ib) {
+                int q = p;
+                a = 0;
+                while (q >= noa - a - B0.nJab) { q -= noa - a - B0.nJab; ++a; }
+                b = a + B0.nJab + q;
+            } else {
+                a = p / nob;
+                b = p - a * nob;
+            }
+            v = ((a * nob + b) * nog + gam) | gam << 16 | a << 20 | b << 24;
+        }
+        s_k[k] = v;
+    }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t taddr = s_taddr;
-    const int npair = s_np, K = npair * nog;
     const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(Np >> 3) << 17) |
                            ((uint32_t)(kTcRows >> 4) << 24);   // F32 += TF32 x TF32, K-major, M = 128, N = Np
+    // A's staging: one, two or four threads per row, each with its row's V' and excluded gamma
+    const int RP = rows <= 32 ? 32 : rows <= 64 ? 64 : 128, r_ = tid % RP, part = tid / RP, nparts = kTcThreads / RP;
+    const double *vrow = nullptr;
+    int excl = -1;
+    if (r_ < rows) {
+        const S2Block &Bb = blk[tile_blk[b_first + s_rblk[r_]]];
+        const int d = s_rd[r_];
+        vrow = vp + Bb.vp_first + (size_t)d * noa * nob * nog;
+        if (Bb.nJgd) excl = P.orb_start[Bb.ch] + d - P.orb_start[ig];
+    }
     bool ok = true;
     int phase = 0;
     for (int kc0 = 0; kc0 < K; kc0 += kTcKc) {
-        // A: V' of every row's block at columns k = p * nog + gamma (the reference's
-        // excluded gamma == d terms as zeros), split into TF32 hi + lo
-        for (int u = tid; u < kTcRows * kTcKc; u += kTcThreads) {
-            const int r = u / kTcKc, kk = u - r * kTcKc, k = kc0 + kk;
-            float x = 0.0f;
-            if (r < rows && k < K) {
-                const S2Block &Bb = blk[tile_blk[b_first + s_rblk[r]]];
-                const int d = s_rd[r], p = k / nog, gam = k - p * nog;
-                const bool excl = (P.orb_start[ig] + gam == P.orb_start[Bb.ch] + d) && Bb.nJgd;
-                if (!excl) x = f64_to_f32(__ldg(vp + Bb.vp_first + (((size_t)d * noa + s_pa[p]) * nob + s_pb[p]) * nog + gam));
+        const int kn = min(kTcKc, Kp - kc0);   // columns of this round, a multiple of 8
+        // A: V' of every row's block at columns k = (p, gamma) (the reference's excluded
+        // gamma == d terms as zeros), split into TF32 hi + lo, four columns at a time.  Rows
+        // beyond the tile's stay as they are: they only reach accumulators nobody reads.
+        if (r_ < rows)
+            for (int kk = 4 * part; kk < kn; kk += 4 * nparts) {
+                const int4 kv = *reinterpret_cast<const int4 *>(s_k + kc0 + kk);
+                double x[4];
+                const int ke[4] = {kv.x, kv.y, kv.z, kv.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[e] = (ke[e] >= 0 && ((ke[e] >> 16) & 15) != excl) ? __ldg(vrow + (ke[e] & 0xffff)) : 0.0;
+                float hi[4], lo[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) tf32_split(f64_to_f32(x[e]), hi[e], lo[e]);
+                *reinterpret_cast<float4 *>(Ahi + tc_off(r_, kk)) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<float4 *>(Alo + tc_off(r_, kk)) = make_float4(lo[0], lo[1], lo[2], lo[3]);
             }
-            float hi, lo;
-            tf32_split(x, hi, lo);
-            Ahi[tc_off(r, kk)] = hi;
-            Alo[tc_off(r, kk)] = lo;
-        }
-        // B: column t = pole (na, nb, ng), row k = (p, gamma): x4 x2(p) f_ng[gamma]
-        for (int u = tid; u < Np * kTcKc; u += kTcThreads) {
-            const int t = u / kTcKc, kk = u - t * kTcKc, k = kc0 + kk;
-            float x = 0.0f;
-            if (t < T && k < K) {
+        // B: column t = pole (na, nb, ng) of a direction, row k = (p, gamma): x4 x2(p) f_ng[gamma]
+#pragma unroll
+        for (int dir = 0; dir < 2; ++dir) {
+            const int T = Tn[dir];
+            const int *nA = dir == 0 ? P.np : P.nh, *nGv = dir == 0 ? P.nh : P.np;
+            const int *sA = dir == 0 ? P.p_start : P.h_start, *sG = dir == 0 ? P.h_start : P.p_start;
+            const double *fA = dir == 0 ? P.fqp : P.fqh, *fG = dir == 0 ? P.fqh : P.fqp;
+            const int kq = kn >> 2;
+            for (int u = tid; u < T * kq; u += kTcThreads) {
+                const int t = u / kq, kk = 4 * (u - t * kq);
                 int na, nb, ng;
-                pole_frags(B0, t, nAa, nAb, nG, na, nb, ng);
-                const int p = k / nog, gam = k - p * nog, a = s_pa[p], b = s_pb[p];
+                pole_frags(B0, t, nA[ia], nA[ib], nGv[ig], na, nb, ng);
                 const double *fa = fA + (size_t)(sA[ia] + na) * NS, *fb = fA + (size_t)(sA[ib] + nb) * NS;
-                float x2 = f64_to_f32(__ldg(fa + a)) * f64_to_f32(__ldg(fb + b));
-                if (ia == ib) {
-                    x2 += (B0.nJab ? -1.0f : 1.0f) * f64_to_f32(__ldg(fa + b)) * f64_to_f32(__ldg(fb + a));
-                    if (a == b) x2 *= 0.70710678118654752f;
-                    if (na == nb) x2 *= 0.70710678118654752f;
+                const double *fg = fG + (size_t)(sG[ig] + ng) * NS;
+                float hi[4], lo[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int kv = s_k[kc0 + kk + e];
+                    float x = 0.0f;
+                    if (kv >= 0) {
+                        const int gam = (kv >> 16) & 15, a = (kv >> 20) & 15, b = (kv >> 24) & 15;
+                        float x2 = f64_to_f32(__ldg(fa + a)) * f64_to_f32(__ldg(fb + b));
+                        if (ia == ib) {
+                            x2 += (B0.nJab ? -1.0f : 1.0f) * f64_to_f32(__ldg(fa + b)) * f64_to_f32(__ldg(fb + a));
+                            if (a == b) x2 *= 0.70710678118654752f;
+                            if (na == nb) x2 *= 0.70710678118654752f;
+                        }
+                        x = x2 * f64_to_f32(__ldg(fg + gam));
+                    }
+                    tf32_split(x, hi[e], lo[e]);
                 }
-                x = x2 * f64_to_f32(__ldg(fG + (size_t)(sG[ig] + ng) * NS + gam));
+                const int o = tc_off(col0[dir] + t, kk);
+                *reinterpret_cast<float4 *>(Bhi + o) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<float4 *>(Blo + o) = make_float4(lo[0], lo[1], lo[2], lo[3]);
             }
-            float hi, lo;
-            tf32_split(x, hi, lo);
-            Bhi[tc_off(t, kk)] = hi;
-            Blo[tc_off(t, kk)] = lo;
         }
         asm volatile("fence.proxy.async.shared::cta;");   // the staged tiles, to the tensor cores
         asm volatile("tcgen05.fence::before_thread_sync;");
         __syncthreads();
         asm volatile("tcgen05.fence::after_thread_sync;");
         if (tid == 0) {
-            const int nstep = (min(kTcKc, K - kc0) + 7) / 8;
+            const int nstep = kn / 8;
             const uint32_t sbo = (kTcKc / 4) * 128;   // next 8-row group
             for (int s = 0; s < nstep; ++s) {
                 const uint32_t off = (uint32_t)s * 256;   // two 128-byte core matrices of K per step
@@ -260,42 +311,52 @@ __global__ void __launch_bounds__(kTcThreads) k_poles_tc(DevProblem P, const S2B
     // every row's accumulators: warp w reads lanes 32w .. 32w + 31, sixteen columns at a time
     const int r = 32 * warp + lane;
     const bool has_row = r < rows;
-    const S2Block Br = blk[tile_blk[b_first + (has_row ? s_rblk[r] : 0)]];
+    const S2Block &Br = blk[tile_blk[b_first + (has_row ? s_rblk[r] : 0)]];
     const ChanSig Cr = cs[Br.ch];
-    const int Nr = dir == 0 ? Cr.nfw : Cr.nbk;
-    double *Mrow = M + (dir == 0 ? Cr.mfw_off : Cr.mbk_off) + (size_t)(has_row ? s_rd[r] : 0) * Nr +
-                   ((dir == 0 ? Br.fw_first : Br.bk_first) - (dir == 0 ? Cr.fw_off : Cr.bk_off));
-    for (int c0 = 0; c0 < Np; c0 += 16) {
-        uint32_t v[16];
-        if (ok && K > 0) {
-            tc_ld16(taddr + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0, v);
-        } else {
+    if (32 * warp < rows)
 #pragma unroll
-            for (int q = 0; q < 16; ++q) v[q] = 0u;
+        for (int dir = 0; dir < 2; ++dir) {
+            const int T = Tn[dir], Nr = dir == 0 ? Cr.nfw : Cr.nbk;
+            double *Mrow = (dir == 0 ? fw.M : bk.M) + (dir == 0 ? Cr.mfw_off : Cr.mbk_off) + (size_t)(has_row ? s_rd[r] : 0) * Nr +
+                           ((dir == 0 ? Br.fw_first : Br.bk_first) - (dir == 0 ? Cr.fw_off : Cr.bk_off));
+            for (int c0 = 0; c0 < T; c0 += 16) {
+                uint32_t v[16];
+                if (ok && K > 0) {
+                    tc_ld16(taddr + ((uint32_t)(32 * warp) << 16) + (uint32_t)(col0[dir] + c0), v);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 16; ++q) v[q] = 0u;
+                }
+                if (has_row)
+#pragma unroll
+                    for (int q = 0; q < 16; ++q)
+                        if (c0 + q < T) Mrow[c0 + q] = f32_to_f64(__uint_as_float(v[q]));
+            }
         }
-        if (has_row)
-#pragma unroll
-            for (int q = 0; q < 16; ++q)
-                if (c0 + q < T) Mrow[c0 + q] = f32_to_f64(__uint_as_float(v[q]));
-    }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(taddr), "r"(ncols));
     // energies (the reference's FP64 operations) and S2 = sum_d M^2 of every pole of the tile
     __threadfence_block();
-    for (int u = tid; u < nblk * T; u += kTcThreads) {
-        const int q = u / T, t = u - q * T;
-        const S2Block Bq = blk[tile_blk[b_first + q]];
-        const ChanSig Cq = cs[Bq.ch];
-        int na, nb, ng;
-        pole_frags(Bq, t, nAa, nAb, nG, na, nb, ng);
-        const long long g = (dir == 0 ? Bq.fw_first : Bq.bk_first) + t;
-        E[g] = __dsub_rn(__dadd_rn(eA[sA[ia] + na], eA[sA[ib] + nb]), eG[sG[ig] + ng]);
-        const int Nq = dir == 0 ? Cq.nfw : Cq.nbk;
-        const double *Mq = M + (dir == 0 ? Cq.mfw_off : Cq.mbk_off) + (g - (dir == 0 ? Cq.fw_off : Cq.bk_off));
-        float s2 = 0.0f;
-        for (int d = 0; d < P.no[Bq.ch]; ++d) { const float m = f64_to_f32(Mq[(size_t)d * Nq]); s2 = fmaf(m, m, s2); }
-        S2[g] = f32_to_f64(s2);
+    for (int dir = 0; dir < 2; ++dir) {
+        const int T = Tn[dir];
+        const int *nA = dir == 0 ? P.np : P.nh, *nGv = dir == 0 ? P.nh : P.np;
+        const int *sA = dir == 0 ? P.p_start : P.h_start, *sG = dir == 0 ? P.h_start : P.p_start;
+        const double *eA = dir == 0 ? P.ep : P.eh, *eG = dir == 0 ? P.eh : P.ep;
+        for (int u = tid; u < nblk * T; u += kTcThreads) {
+            const int q = u / T, t = u - q * T;
+            const S2Block &Bq = blk[tile_blk[b_first + q]];
+            const ChanSig Cq = cs[Bq.ch];
+            int na, nb, ng;
+            pole_frags(B0, t, nA[ia], nA[ib], nGv[ig], na, nb, ng);
+            const long long g = (dir == 0 ? Bq.fw_first : Bq.bk_first) + t;
+            (dir == 0 ? fw.E : bk.E)[g] = __dsub_rn(__dadd_rn(eA[sA[ia] + na], eA[sA[ib] + nb]), eG[sG[ig] + ng]);
+            const int Nq = dir == 0 ? Cq.nfw : Cq.nbk;
+            const double *Mq = (dir == 0 ? fw.M : bk.M) + (dir == 0 ? Cq.mfw_off : Cq.mbk_off) + (g - (dir == 0 ? Cq.fw_off : Cq.bk_off));
+            float s2 = 0.0f;
+            for (int d = 0; d < Cq.D; ++d) { const float m = f64_to_f32(Mq[(size_t)d * Nq]); s2 = fmaf(m, m, s2); }
+            (dir == 0 ? fw.S2 : bk.S2)[g] = f32_to_f64(s2);
+        }
     }
 }
 
@@ -308,12 +369,12 @@ size_t tc_smem_bytes(int np) {
 }
 
 cudaError_t launch_poles_tc(const DevProblem &P, const S2Block *blk, const int *tile_blk, const int4 *tiles,
-                            int ntiles, const ChanSig *cs, int dir, const double *vp, double *E, double *S2, double *M,
-                            int *err, size_t smem, cudaStream_t st) {
+                            int ntiles, const ChanSig *cs, const double *vp, const TcOut &fw, const TcOut &bk,
+                            int dirs, int *err, size_t smem, cudaStream_t st) {
     if (ntiles <= 0) return cudaSuccess;
     cudaError_t e = allow_dynamic_smem((const void *)k_poles_tc);
     if (e != cudaSuccess) return e;
-    k_poles_tc<<<ntiles, kTcThreads, smem, st>>>(P, blk, tile_blk, tiles, ntiles, cs, dir, vp, E, S2, M, err);
+    k_poles_tc<<<ntiles, kTcThreads, smem, st>>>(P, blk, tile_blk, tiles, ntiles, cs, vp, fw, bk, dirs, err);
     return cudaGetLastError();
 }
 

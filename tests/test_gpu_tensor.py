@@ -75,3 +75,32 @@ def test_tensor_core_couplings_in_graph_replay(bdmod, problems):
             for k in ("qp", "qh", "koltun"):
                 assert np.array_equal(a[k], b[k]), k
     ctx.close()
+
+
+def test_many_fragments_take_a_direction_at_a_time(synth, problems, bdmod):
+    """Six fragments a side: a tile's forward and backward poles exceed the 256 columns of one
+    product and go in two launches."""
+    p = problems(2, 20.0, 1, 6)
+    rng = np.random.default_rng(3)
+    ns, nspb, f = p.ms.nsubsh, p.prop.nspb, 6
+    amp = np.zeros((2, ns, f, nspb))
+    for s in range(ns):
+        D = int(p.ms.no[s])
+        amp[:, s, :, :D] = 0.4 * rng.standard_normal((2, f, D))
+    ep, eh = np.sort(rng.uniform(20, 120, (ns, f)))[:, ::-1], np.sort(rng.uniform(-90, -25, (ns, f)))[:, ::-1]
+    n = np.full(ns, f, np.int32)
+    q = synth.propagator_from_arrays(nspb, n, n, ep.reshape(-1), eh.reshape(-1), amp[0].reshape(-1, nspb),
+                                     amp[1].reshape(-1, nspb))
+    got = []
+    for fp64 in (False, True):
+        ctx = bdmod.Context().upload(p).upload_propagator(q)
+        ctx.run_all(lanczos=True, mixed=True, fp64_couplings=fp64)
+        assert ctx.tensor_couplings() == (not fp64)
+        got.append((ctx.koltun_all(), [ctx.result(i) for i in range(ns)]))
+        ctx.close()
+    # TF32 in three products: 2^-21 of the couplings, far inside the mixed form's targets
+    np.testing.assert_allclose(got[0][0].sum(0), got[1][0].sum(0), rtol=1e-5)
+    for a, b in zip(got[0][1], got[1][1]):
+        for tag in ("qp", "qh"):
+            e, z = strong_diffs(b[tag], a[tag], zmin=1e-2, etol=1e-5)
+            assert e * 300.0 < 1e-3 and z < 1e-4
