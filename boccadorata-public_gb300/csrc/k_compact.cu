@@ -31,6 +31,7 @@
 #include <cfloat>
 #include "bd_common.cuh"
 #include "bd_kernels.h"
+#include "lz_fixed.cuh"
 
 namespace bd {
 
@@ -110,30 +111,6 @@ __device__ int merge_groups(const double *gE, int Q, int *s_first, int *ws) {
 
 static_assert(kCpThreads >= kCpGroups, "a thread per exact group");
 
-// A warp's sums of NV values at once (see warp_sums in k_lanczos.cu): lane L ends with the
-// total of value L >> (5 - log2 NV).
-template <int NV>
-__device__ __forceinline__ double warp_sums_d(double *v, int lane) {
-#pragma unroll
-    for (int lev = 0; lev < 5; ++lev) {
-        const int o = 16 >> lev;
-        const int n = NV >> (lev + 1);
-        if (n >= 1) {
-            const bool up = (lane & o) != 0;
-#pragma unroll
-            for (int i = 0; i < (NV >> 1); ++i)
-                if (i < n) {
-                    const double send = up ? v[i] : v[i + n];
-                    const double keep = up ? v[i + n] : v[i];
-                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-                }
-        } else {
-            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-        }
-    }
-    return v[0];
-}
-
 }  // namespace
 
 // ------------------------------------------------------------------ Lanczos
@@ -141,13 +118,14 @@ __device__ __forceinline__ double warp_sums_d(double *v, int lane) {
 // chain that would need what only the full space has (a restart vector, a direction no
 // group has left) is left to k_lanczos as a whole.
 //
-// A step is bound by the FP64 unit (a warp instruction holds an SM sub-partition's for ~64
-// cycles) and by its barriers, so: every vector of the basis in shared memory, a warp per
-// group of four dot products, four barriers a step; and the sweep's update, whose
-// coefficients are rounding-sized after the three-term recurrence, in FP32 from an FP32
-// copy of the basis where |c| <= 1e-9 |w| (its error is below 2^-24 1e-9 |w| < eps |w|).
+// A step is a chain of short phases between barriers, and an FP64 instruction holds an SM
+// sub-partition's FP64 unit for ~64 cycles, so FP64 is kept to what needs it: the sweep's dot
+// products are fixed-point sums (lz_fixed.cuh; four vectors a warp), its update FP32 where the
+// coefficients are rounding-sized (|c| <= 1e-9 |w|: an error below 2^-24 1e-9 |w|) and fixed
+// point otherwise, and one warp takes the decision.  The norm, alpha, m, g and the recurrence
+// are FP64.
 // Measured (N_max = 10, 100 iterations per pivot): the reduction of all 84 chains takes
-// 0.49 ms against 3.59 ms in the poles' space (N_max = 12: 0.73 against 12.2).
+// CPMS against 3.59 ms in the poles' space.
 __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains, int nchains, double eta2) {
     const int cid = blockIdx.x;
     if (cid >= nchains) return;
@@ -161,9 +139,10 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
     __shared__ int ws[kCpWarps];
     __shared__ int s_first[kCpGroups + 1], s_off[kCpGroups + 1];
     __shared__ int s_bad;
+    __shared__ unsigned s_rng[2];
     __shared__ double s_tri[kCpWarps][kGramEntries], s_l[kCpWarps][64];
     extern __shared__ double sm[];
-    if (tid == 0) s_bad = 0;
+    if (tid == 0) { s_bad = 0; s_rng[0] = 0; s_rng[1] = 0; }
     const int ng = merge_groups(C.gE, Q, s_first, ws);
     if (ng > kCpMerged) return;
     // 1. every merged group's coordinates: its own poles (kept), or the columns of L
@@ -201,26 +180,42 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
         __syncthreads();
     }
     const int R = min(L, np);               // vectors, at most
-    const int rq = (R + 4) & ~3;
-    // shared layout (doubles): E[np] | M[D][np] | w[np] | ew[np] | c[rq + 4] | sc[20] | V[R][np],
-    // then floats cf[rq] | Vf[R][np], ints rowslot[L]
-    const size_t need = sizeof(double) * ((size_t)(D + 3) * np + rq + 4 + 20 + (size_t)R * np) +
-                        sizeof(float) * (rq + (size_t)R * np) + sizeof(int) * (size_t)L;
+    const int rq = (R + 4) & ~3, np4 = (np + 3) & ~3;
+    const int nla = max(C.n_used - 1, 0);   // chains whose last vector later ones refer to
+    // shared layout (doubles): E[np4] | M[D][np4] | w[np4] | ew[np4] | ring[2][np4] | last[nla][np4] |
+    // c[rq + 4] | sc[20], then ints wa[np4] | wb[np4] | Va[R][np4] | Vb[R][np4], floats cf[rq + 4] |
+    // Vf[R][np4], ints rowslot[L]
+    const size_t need = sizeof(double) * ((size_t)(D + 5 + nla) * np4 + rq + 4 + 20) +
+                        sizeof(int) * ((size_t)(2 + 3 * R) * np4 + rq + 4 + (size_t)L);
     if (s_bad || np > kCpDim || need > (size_t)kCpSmem) return;
-    double *E = sm, *M = E + np, *w = M + (size_t)D * np, *ew = w + np, *c = ew + np, *sc = c + rq + 4, *V = sc + 20;
-    float *cf = reinterpret_cast<float *>(V + (size_t)R * np), *Vf = cf + rq;
-    int *rowslot = reinterpret_cast<int *>(Vf + (size_t)R * np);
+    double *E = sm, *M = E + np4, *w = M + (size_t)D * np4, *ew = w + np4, *ring = ew + np4, *lasts = ring + 2 * np4,
+           *c = lasts + (size_t)nla * np4, *sc = c + rq + 4;
+    int *wa = reinterpret_cast<int *>(sc + 20), *wb = wa + np4, *Va = wb + np4, *Vb = Va + (size_t)R * np4;
+    float *cf = reinterpret_cast<float *>(Vb + (size_t)R * np4), *Vf = cf + rq + 4;
+    int *rowslot = reinterpret_cast<int *>(Vf + (size_t)R * np4);
+    unsigned me = 0, mm = 0;   // upper words of the largest |E| and |M|
     for (int g = warp; g < ng; g += kCpWarps) {
         const CompactGroup G = S.grp[g];
         const double e0 = C.E[G.p0], eg = 0.5 * (e0 + C.E[G.p0 + G.m - 1]);
         for (int i = lane; i < G.c; i += 32) {
-            E[s_off[g] + i] = G.kept ? C.E[G.p0 + i] : eg;
-            for (int d = 0; d < D; ++d)
-                M[(size_t)d * np + s_off[g] + i] = G.kept ? C.M[(size_t)d * N + G.p0 + i] : S.L[(size_t)g * 64 + d * D + i];
+            const double e = G.kept ? C.E[G.p0 + i] : eg;
+            E[s_off[g] + i] = e;
+            me = max(me, (unsigned)__double2hiint(e) & 0x7fffffffu);
+            for (int d = 0; d < D; ++d) {
+                const double m = G.kept ? C.M[(size_t)d * N + G.p0 + i] : S.L[(size_t)g * 64 + d * D + i];
+                M[(size_t)d * np4 + s_off[g] + i] = m;
+                mm = max(mm, (unsigned)__double2hiint(m) & 0x7fffffffu);
+            }
         }
     }
-    __shared__ int s_start[10], s_last[10], lslot[8], lt[16];
-    __shared__ double lc[16], s_row[32];
+    me = __reduce_max_sync(0xffffffffu, me);
+    mm = __reduce_max_sync(0xffffffffu, mm);
+    if (lane == 0) { atomicMax(&s_rng[0], me); atomicMax(&s_rng[1], mm); }
+    __syncthreads();
+    if (!fixed_range(s_rng[0]) || !fixed_range(s_rng[1])) return;   // (fixed-point and FP32 parts)
+    __shared__ int s_start[10], s_last[10], lslot[8], lt[16], lq[16], s_fl;
+    __shared__ double lc[16], s_row[32], s_n[3];   // s_n: 1/|w|, |w|, |E v|^2 of the kept vector
+    __shared__ float s_f[kCpWarps];
     if (tid <= C.n_used && tid < 10) s_start[tid] = C.start[tid];
     if (tid < C.n_used && tid < 10) s_last[tid] = C.last[tid];
     const int Qg = C.gInfo[0];
@@ -234,16 +229,13 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
     int dcur = 0, ndefl = 0, nvec = 0, extra = 0, k = -1;
     double e2v = 0.0;            // |E v|^2 of the last built vector
     int nl0 = 0;                 // vectors of the next recurrence (lt, lc)
-    // <a_u, b_u> of a warp's four items at once (lane 8 u holds item u's sum)
-    auto dots4 = [&](const double *const *a, const double *const *b, int nu) {
-        double acc[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) acc[u] = 0.0;
-        for (int i = lane; i < np; i += 32)
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (u < nu) acc[u] = fma(a[u][i], b[u][i], acc[u]);
-        return warp_sums_d<4>(acc, lane);
+    // stored vector t as doubles: the two newest, or the last one of chain q
+    auto vecd = [&](int t, int q) -> const double * { return t >= nvec - 2 ? ring + (t & 1) * np4 : lasts + (size_t)q * np4; };
+    int wbias = 1023;   // exponent field of the power of two w is split against
+    auto split_w = [&](int i, double x) {
+        const int2 f = fixed_of(x, wbias);
+        wa[i] = f.x;
+        wb[i] = f.y;
     };
     __syncthreads();
     for (int j = 0; j < L; ++j) {
@@ -252,93 +244,151 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
         const int nq = k;
         if (tid < nq) lslot[tid] = rowslot[s_last[tid]];
         // w = M p, or E v_{j-1} less its known components
-        for (int i = tid; i < np; i += kCpThreads) {
-            double x = 0.0;
-            if (newv) {
-                const double *p = C.piv + (size_t)k * D;
-                for (int d = 0; d < D; ++d) x = fma(M[(size_t)d * np + i], p[d], x);
-            } else {
-                x = V[(size_t)lt[0] * np + i] * E[i];
-                for (int t = 0; t < nl0; ++t) x = fma(-lc[t], V[(size_t)lt[t] * np + i], x);
-            }
-            w[i] = x;
-        }
-        __syncthreads();
-        int fl, nfull = 0;
-        double wn2_first = e2v, x2 = 0.0, ixb = 0.0;
-        for (;;) {
-            // c_t = <v_t, w> for every stored vector, and |w|^2 as item nvec
-            for (int t0 = 4 * warp; t0 <= nvec; t0 += 4 * kCpWarps) {
-                const double *a[4], *b[4];
-                const int nu = min(4, nvec + 1 - t0);
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    a[u] = (t0 + u < nvec) ? V + (size_t)(t0 + u) * np : w;
-                    b[u] = w;
-                }
-                const double r = dots4(a, b, nu);
-                if ((lane & 7) == 0 && (lane >> 3) < nu) {
-                    c[t0 + (lane >> 3)] = r;
-                    if (t0 + (lane >> 3) < nvec) cf[t0 + (lane >> 3)] = (float)r;
-                }
-            }
-            __syncthreads();
-            const double wn2 = c[nvec];
-            if (newv && nfull == 0) wn2_first = wn2;
-            // the sweep's size in FP32 (only the choice of the update's arithmetic), then the update
-            float c2 = 0.0f;
-            for (int t = lane; t < nvec; t += 32) c2 = fmaxf(c2, fabsf(cf[t]));
-            for (int o = 16; o > 0; o >>= 1) c2 = fmaxf(c2, __shfl_xor_sync(0xffffffffu, c2, o));
-            const float wf = (float)wn2;
-            const bool small = (c2 * 1e9f) * (c2 * 1e9f) * (float)max(nvec, 1) <= wf && wf > 1e-30f;
+        double wn2 = 0.0, wn2_first = e2v;   // |w|^2 before the sweep, and of E v_{j-1} / M p (thresholds' scales)
+        if (newv) {
+            float s2 = 0.0f;
             for (int i = tid; i < np; i += kCpThreads) {
-                double x = w[i];
-                if (small) {
-                    float s0 = 0.0f, s1 = 0.0f;
-                    int t = 0;
-                    for (; t + 1 < nvec; t += 2) {
-                        s0 = fmaf(cf[t], Vf[(size_t)t * np + i], s0);
-                        s1 = fmaf(cf[t + 1], Vf[(size_t)(t + 1) * np + i], s1);
-                    }
-                    if (t < nvec) s0 = fmaf(cf[t], Vf[(size_t)t * np + i], s0);
-                    x -= (double)(s0 + s1);
-                } else {
-                    double s = 0.0;
-                    for (int t = 0; t < nvec; ++t) s = fma(c[t], V[(size_t)t * np + i], s);
-                    x -= s;
-                }
+                const double *p = C.piv + (size_t)k * D;
+                double x = 0.0;
+                for (int d = 0; d < D; ++d) x = fma(M[(size_t)d * np4 + i], p[d], x);
                 w[i] = x;
-                ew[i] = E[i] * x;
+                const float f = (float)x;
+                s2 = fmaf(f, f, s2);
+            }
+            for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+            if (lane == 0) s_f[warp] = s2;
+            __syncthreads();
+            s2 = 0.0f;
+#pragma unroll
+            for (int h = 0; h < kCpWarps; ++h) s2 += s_f[h];
+            wn2 = wn2_first = (double)s2;
+            wbias = bias_above(wn2);
+            for (int i = tid; i < np; i += kCpThreads) split_w(i, w[i]);
+        } else {
+            wbias = bias_above(e2v);
+            const double *v0 = ring + (lt[0] & 1) * np4;
+            for (int i = tid; i < np; i += kCpThreads) {
+                double x = v0[i] * E[i];
+                for (int t = 0; t < nl0; ++t) x = fma(-lc[t], vecd(lt[t], lq[t])[i], x);
+                w[i] = x;
+                split_w(i, x);
+            }
+        }
+        int fl, nfull = 0;
+        for (;;) {
+            __syncthreads();
+            // c_t = <v_t, w> for every stored vector, four a warp; after a recurrence |w|^2 as item
+            // nvec (read against the swept norm and the coefficients only: FP32)
+            const bool want_n = !newv && nfull == 0;
+            for (int t0 = 4 * warp; t0 < nvec + (want_n ? 1 : 0); t0 += 4 * kCpWarps) {
+                const int nu = min(4, nvec - t0);
+                if (nu > 0) {
+                    FixedSum acc[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) acc[u] = FixedSum{0, 0};
+                    const int *va = Va + (size_t)t0 * np4, *vb = Vb + (size_t)t0 * np4;
+                    for (int i = lane; i < np; i += 32) {
+                        const int xa = wa[i], xb = wb[i];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (u < nu) fixed_step(acc[u], va[u * np4 + i], vb[u * np4 + i], xa, xb);
+                    }
+                    const FixedSum r = warp_sums_of<4>(acc, lane, fixed_add, fixed_shfl);
+                    if ((lane & 7) == 0 && (lane >> 3) < nu) {
+                        const double x = fixed_value(r, wbias);
+                        c[t0 + (lane >> 3)] = x;
+                        cf[t0 + (lane >> 3)] = (float)x;
+                    }
+                }
+                if (want_n && nvec >= t0 && nvec < t0 + 4) {
+                    float s2 = 0.0f;
+                    for (int i = lane; i < np; i += 32) { const float f = (float)w[i]; s2 = fmaf(f, f, s2); }
+                    for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+                    if (lane == 0) { c[nvec] = (double)s2; cf[nvec] = s2; }
+                }
             }
             __syncthreads();
-            // the scalars of the updated w: |w|^2, <w|E|w>, |E w|^2, <M_d|w>, <v_last(q)|E|w>
-            const int nsc = 3 + D + nq;
-            for (int t0 = 4 * warp; t0 < nsc; t0 += 4 * kCpWarps) {
-                const double *a[4], *b[4];
-                const int nu = min(4, nsc - t0);
+            if (want_n) wn2 = c[nvec];
+            if (warp * 32 < np) {   // (whole warps: the sweep's size needs their lanes)
+                float cm = 0.0f;
+                for (int t = lane; t < nvec; t += 32) cm = fmaxf(cm, fabsf(cf[t]));
+                for (int o = 16; o > 0; o >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, o));
+                const float wf = want_n ? cf[nvec] : 0.0f;
+                const bool small = (cm * 1e9f) * (cm * 1e9f) * (float)max(nvec, 1) <= wf && wf > 1e-30f;
+                for (int i = tid; i < np; i += kCpThreads) {
+                    double x = w[i];
+                    if (small) {
+                        float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                        int t = 0;
+                        for (; t + 3 < nvec; t += 4)
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
+                            for (int u = 0; u < 4; ++u) a[u] = fmaf(cf[t + u], Vf[(size_t)(t + u) * np4 + i], a[u]);
+                        for (; t < nvec; ++t) a[0] = fmaf(cf[t], Vf[(size_t)t * np4 + i], a[0]);
+                        x -= (double)((a[0] + a[1]) + (a[2] + a[3]));
+                    } else {
+                        FixedSum acc{0, 0};
+                        for (int t = 0; t < nvec; ++t) {
+                            const int2 ct = fixed_of(c[t], wbias);
+                            fixed_step(acc, Va[(size_t)t * np4 + i], Vb[(size_t)t * np4 + i], ct.x, ct.y);
+                        }
+                        x -= fixed_value(acc, wbias);
+                    }
+                    w[i] = x;
+                    ew[i] = E[i] * x;
+                }
+            }
+            __syncthreads();
+            // the scalars of the updated w: |w|^2, <w|E|w>, |E w|^2, <M_d|w>, <v_last(q)|E|w>, two a warp
+            // and round
+            const int nsc = 3 + D + nq;
+            for (int t0 = 2 * warp; t0 < nsc; t0 += 2 * kCpWarps) {
+                const double *a[2], *b[2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
                     const int t = t0 + u;
                     a[u] = w;
                     b[u] = w;
                     if (t == 1) b[u] = ew;
                     else if (t == 2) { a[u] = ew; b[u] = ew; }
-                    else if (t >= 3 && t < 3 + D) a[u] = M + (size_t)(t - 3) * np;
-                    else if (t >= 3 + D && t < nsc && lslot[t - 3 - D] >= 0) { a[u] = V + (size_t)lslot[t - 3 - D] * np; b[u] = ew; }
+                    else if (t >= 3 && t < 3 + D) a[u] = M + (size_t)(t - 3) * np4;
+                    else if (t >= 3 + D && t < nsc && lslot[t - 3 - D] >= 0) { a[u] = vecd(lslot[t - 3 - D], t - 3 - D); b[u] = ew; }
                 }
-                const double r = dots4(a, b, nu);
-                const int t = t0 + (lane >> 3);
-                if ((lane & 7) == 0 && t < nsc) sc[t] = (t >= 3 + D && lslot[t - 3 - D] < 0) ? 0.0 : r;
+                double x[2] = {0.0, 0.0};
+                for (int i = lane; i < np; i += 32) {
+                    x[0] = fma(a[0][i], b[0][i], x[0]);
+                    x[1] = fma(a[1][i], b[1][i], x[1]);
+                }
+                const double r = warp_sums_of<2>(x, lane, [](double p, double q) { return p + q; },
+                                                 [](double p, int o) { return __shfl_xor_sync(0xffffffffu, p, o); });
+                const int t = t0 + (lane >> 4);
+                if ((lane & 15) == 0 && t < nsc) sc[t] = (t >= 3 + D && lslot[t - 3 - D] < 0) ? 0.0 : r;
             }
             __syncthreads();
-            // k_lanczos's decision, by every thread alike
-            x2 = sc[0];
-            if (nvec > 0 && nfull + 1 < 4 && x2 < eta2 * wn2) fl = 1;
-            else if (x2 <= thr_exh * wn2_first || x2 == 0.0) fl = (dcur < dtot) ? 2 : 3;
-            else if (!(x2 <= tau * wn2_first) && x2 <= DBL_MAX) fl = 0;
-            else fl = 3;   // (not finite)
+            // k_lanczos's decision, by warp 0 (its lanes take one threshold each); exhaustion first:
+            // further sweeps of a w that holds nothing leave nothing
+            if (warp == 0) {
+                const double x2 = sc[0];
+                const double lim = lane == 0 ? eta2 * wn2 : (lane == 1 ? thr_exh : tau) * wn2_first;
+                const unsigned lt_ = __ballot_sync(0xffffffffu, x2 < lim), le = __ballot_sync(0xffffffffu, x2 <= lim);
+                const long long xb = __double_as_longlong(x2);
+                const bool zero = (xb << 1) == 0, fin = (xb & 0x7ff0000000000000LL) != 0x7ff0000000000000LL;
+                int f;
+                if ((le & 2u) || zero) f = (dcur < dtot) ? 2 : 3;
+                else if (nvec > 0 && nfull + 1 < 4 && (lt_ & 1u)) f = 1;
+                else if (!(le & 4u) && fin) f = 0;
+                else f = 3;   // (not finite)
+                const double r = rsqrt_newton(x2);
+                const double y = (lane == 0 ? 1.0 : lane == 1 ? x2 : sc[2] * r) * r;
+                if (lane < 3) s_n[lane] = y;
+                if (lane == 0) s_fl = f;
+            }
+            __syncthreads();
+            fl = s_fl;
             if (nfull++ > 0) ++extra;
             if (fl != 1) break;
+            wn2 = sc[0];   // another sweep, of the updated w
+            wbias = bias_above(wn2);
+            for (int i = tid; i < np; i += kCpThreads) split_w(i, w[i]);
         }
         if (fl == 3) return;   // the full space's (handled stays 0)
         if (fl == 2) {
@@ -361,18 +411,25 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
         }
         if (nvec >= R) return;   // (beyond the space's dimension: not reached with exact arithmetic)
         // normalise and store; the row
-        ixb = rsqrt_newton(x2);
-        for (int i = tid; i < np; i += kCpThreads) {
-            const double v = w[i] * ixb;
-            V[(size_t)nvec * np + i] = v;
-            Vf[(size_t)nvec * np + i] = (float)v;
-            reinterpret_cast<double *>(C.V)[(size_t)nvec * np + i] = v;   // (np <= N: within the chain's store)
+        const double ixb = s_n[0];
+        e2v = s_n[2];
+        {
+            double *rg = ring + (nvec & 1) * np4, *rl = (j == s_last[k] && k < nla) ? lasts + (size_t)k * np4 : nullptr;
+            for (int i = tid; i < np; i += kCpThreads) {
+                const double v = w[i] * ixb;
+                const int2 f = fixed_of(v, 1023);
+                Va[(size_t)nvec * np4 + i] = f.x;
+                Vb[(size_t)nvec * np4 + i] = f.y;
+                Vf[(size_t)nvec * np4 + i] = (float)f.x * 0x1p-30f;
+                rg[i] = v;
+                if (rl) rl[i] = v;
+                reinterpret_cast<double *>(C.V)[(size_t)nvec * np + i] = v;   // (np <= N: within the chain's store)
+            }
         }
-        e2v = sc[2] * ixb * ixb;
         if (tid < NT) {
             double x = 0.0;
             if (tid == 0) x = sc[1] * ixb * ixb;
-            else if (tid == 1) x = (newv && k >= 1) ? sc[3 + D + (k - 1)] * ixb : x2 * ixb;
+            else if (tid == 1) x = (newv && k >= 1) ? sc[3 + D + (k - 1)] * ixb : s_n[1];
             else if (tid < 2 + k) x = sc[3 + D + (tid - 2)] * ixb;
             else if (tid >= C.nden_out && tid < C.nden_out + D) x = sc[3 + (tid - C.nden_out)] * ixb;
             s_row[tid] = x;
@@ -384,10 +441,10 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
             if (lane == 0) {
                 rowslot[j] = nvec;
                 int n = 0;
-                lt[n] = nvec; lc[n++] = s_row[0];
-                if (j >= 1 && rowslot[j - 1] >= 0) { lt[n] = rowslot[j - 1]; lc[n++] = s_row[1]; }
+                lt[n] = nvec; lq[n] = -1; lc[n++] = s_row[0];
+                if (j >= 1 && rowslot[j - 1] >= 0) { lt[n] = rowslot[j - 1]; lq[n] = -1; lc[n++] = s_row[1]; }
                 for (int q = 0; q < k; ++q)
-                    if (s_last[q] < j - 1 && rowslot[s_last[q]] >= 0) { lt[n] = rowslot[s_last[q]]; lc[n++] = s_row[2 + q]; }
+                    if (s_last[q] < j - 1 && rowslot[s_last[q]] >= 0) { lt[n] = rowslot[s_last[q]]; lq[n] = q; lc[n++] = s_row[2 + q]; }
                 lt[15] = n;
             }
         }

@@ -35,6 +35,7 @@
 #include <cooperative_groups.h>
 #include "bd_common.cuh"
 #include "bd_kernels.h"
+#include "lz_fixed.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -46,64 +47,9 @@ constexpr int kLongThreads = 512, kMaxWarps = kLongThreads / 32;
 constexpr int kMaxSc = 20;             // |w|^2, <w|E|w>, 8 m, 8 g; the last: |E w|^2
 constexpr float kSmall = 1e-10f;
 
-// x 2^-(bias - 1023) as (a 2^27 + b) 2^-57, |x| at most 2^(bias - 1023), to nearest and with b
-// in [-2^26, 2^26): E v_{j-1} and v_{j-1} have their signs in common, so truncated bits or a
-// dropped product of one sign would add up.  bias is the exponent field of one.
-__device__ __forceinline__ int2 fixed_of(double x, int bias) {
-    const int hi = __double2hiint(x);
-    const unsigned lo = (unsigned)__double2loint(x);
-    const unsigned long long m = ((unsigned long long)((hi & 0xfffff) | 0x100000) << 32 | lo) << 6;
-    // one bit more than kept; + half a unit, + half of a's unit
-    const unsigned long long f = (m >> min((unsigned)(bias - ((hi >> 20) & 0x7ff)), 63u)) + (1 + (1 << 27));
-    const int a = (int)(f >> 28), b = ((int)(f >> 1) & 0x7ffffff) - (1 << 26);
-    return hi < 0 ? make_int2(-a, -b) : make_int2(a, b);
-}
-// (s + l 2^-27) 2^-60 for sums s of a a' and l of a b' + b a' (the b b' dropped)
-struct FixedSum { long long s, l; };
-__device__ __forceinline__ void fixed_step(FixedSum &acc, int va, int vb, int wa, int wb) {
-    acc.s += (long long)va * wa;
-    acc.l += (long long)va * wb;
-    acc.l += (long long)vb * wa;
-}
-__device__ __forceinline__ double fixed_value(FixedSum r, int bias) {   // times 2^(bias - 1023)
-    return ((double)(r.s + (r.l >> 27)) + (double)(r.l & 0x7ffffff) * 0x1p-27) * __hiloint2double((bias - 60) << 20, 0);
-}
-// a stored element as a double (abs. error 2^-58)
-__device__ __forceinline__ double fixed_to_double(int a, int b) { return fma((double)b, 0x1p-57, (double)a * 0x1p-30); }
-
-// x to FP32 from its bits, truncated; below 2^-70 zero
-__device__ __forceinline__ float f32_trunc(double x) {
-    const unsigned hi = (unsigned)__double2hiint(x);
-    const unsigned b = (hi & 0x80000000u) | ((__funnelshift_l((unsigned)__double2loint(x), hi, 3) - (384u << 23)) & 0x7fffffffu);
-    return (hi & 0x7fffffffu) >= 953u << 20 ? __uint_as_float(b) : 0.0f;
-}
-
 __device__ __forceinline__ int4 ld4(const int *p) { return *reinterpret_cast<const int4 *>(p); }
 __device__ __forceinline__ double2 ld2(const double *p) { return *reinterpret_cast<const double2 *>(p); }
 __device__ __forceinline__ void st2(double *p, double a, double b) { *reinterpret_cast<double2 *>(p) = make_double2(a, b); }
-
-// Warp sums of NV values at once: lane L ends with the total of value L >> (5 - log2 NV).
-template <int NV, typename T, typename Add, typename Shf>
-__device__ __forceinline__ T warp_sums_of(T *v, int lane, Add add, Shf shf) {
-#pragma unroll
-    for (int lev = 0; lev < 5; ++lev) {
-        const int o = 16 >> lev;
-        const int n = NV >> (lev + 1);
-        if (n >= 1) {
-            const bool up = (lane & o) != 0;
-#pragma unroll
-            for (int i = 0; i < (NV >> 1); ++i)
-                if (i < n) {
-                    const T send = up ? v[i] : v[i + n];
-                    const T keep = up ? v[i + n] : v[i];
-                    v[i] = add(keep, shf(send, o));
-                }
-        } else {
-            v[0] = add(v[0], shf(v[0], o));
-        }
-    }
-    return v[0];
-}
 
 // shared memory before the slices: A[2][rq] partials, c[rq], sp[2][kMaxSc], red[16][kMaxSc] (doubles),
 // cf[rq] (floats), rowslot[lq] (ints)
@@ -188,8 +134,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
             mm = max(mm, p[1]);
         }
         cluster.sync();   // peers have read s_rng (a CTA that leaves frees its shared memory)
-        auto in = [](unsigned m) { return m >= (1023u - 40) << 20 && m <= (1023u + 40) << 20; };
-        if (!in(me) || !in(mm)) return;
+        if (!fixed_range(me) || !fixed_range(mm)) return;
     }
     int nvec = 0;
     // planes of stored vector t: a at the address, b pl(t) behind it
@@ -219,8 +164,6 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
         *reinterpret_cast<int2 *>(ws + i) = make_int2(x.x, y.x);
         *reinterpret_cast<int2 *>(ws + S + i) = make_int2(x.y, y.y);
     };
-    // |x|^2 = m 2^e with e in the field of hi: the field of 2^(floor(e / 2) + 1), above |x|
-    auto bias_above = [](double x2) { return ((__double2hiint(x2) >> 20) - 1023 + 2048) / 2 - 1024 + 1023 + 1; };
     auto csum = [&](const double *buf, int t) -> double {   // over the cluster, a fixed tree
         double x[16];
 #pragma unroll
@@ -340,11 +283,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
                                 fixed_step(acc[u], x[u].w, y[u].w, a.w, b.w);
                             }
                     }
-                    const FixedSum r = warp_sums_of<NU>(acc, lane,
-                        [](FixedSum p, FixedSum q) { return FixedSum{p.s + q.s, p.l + q.l}; },
-                        [](FixedSum p, int o) {
-                            return FixedSum{__shfl_xor_sync(0xffffffffu, p.s, o), __shfl_xor_sync(0xffffffffu, p.l, o)};
-                        });
+                    const FixedSum r = warp_sums_of<NU>(acc, lane, fixed_add, fixed_shfl);
                     const int u = lane >> 3;
                     if ((lane & 7) == 0 && u < nu) Ap[t0 + u * NW] = fixed_value(r, wbias);
                 }
@@ -503,8 +442,8 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
                     const long long xb = __double_as_longlong(x2);
                     const bool zero = (xb << 1) == 0, fin = (xb & 0x7ff0000000000000LL) != 0x7ff0000000000000LL;
                     int f;
-                    if (nvec > 0 && nfull + 1 < 4 && (lt_ & 1u)) f = 1;
-                    else if ((le & 2u) || zero) f = (dcur < dtot) ? 2 : 3;
+                    if ((le & 2u) || zero) f = (dcur < dtot) ? 2 : 3;   // (further sweeps leave no more)
+                    else if (nvec > 0 && nfull + 1 < 4 && (lt_ & 1u)) f = 1;
                     else if (!(le & 4u) && fin) f = 0;
                     else f = 3;
                     const double r = rsqrt_newton(x2);

@@ -1,0 +1,78 @@
+// lz_fixed.cuh -- fixed-point sweeps of the FP64 Lanczos reductions (k_lanczos_long.cu,
+// k_compact.cu): a basis vector's elements are at most one in size and the sweep's
+// coefficients are needed to a fixed part of |w|, so both become pairs of 32-bit integers and
+// a dot product an exact 64-bit integer sum.  GB300 issues FP64 at 1/64 of the FP32 rate.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace bd {
+
+// x 2^-(bias - 1023) as (a 2^27 + b) 2^-57, |x| at most 2^(bias - 1023), to nearest and with b
+// in [-2^26, 2^26): E v_{j-1} and v_{j-1} have their signs in common, so truncated bits or a
+// dropped product of one sign would add up.  bias is the exponent field of one.
+__device__ __forceinline__ int2 fixed_of(double x, int bias) {
+    const int hi = __double2hiint(x);
+    const unsigned lo = (unsigned)__double2loint(x);
+    const unsigned long long m = ((unsigned long long)((hi & 0xfffff) | 0x100000) << 32 | lo) << 6;
+    // one bit more than kept; + half a unit, + half of a's unit
+    const unsigned long long f = (m >> min((unsigned)(bias - ((hi >> 20) & 0x7ff)), 63u)) + (1 + (1 << 27));
+    const int a = (int)(f >> 28), b = ((int)(f >> 1) & 0x7ffffff) - (1 << 26);
+    return hi < 0 ? make_int2(-a, -b) : make_int2(a, b);
+}
+// (s + l 2^-27) 2^-60 for sums s of a a' and l of a b' + b a' (the b b' dropped)
+struct FixedSum { long long s, l; };
+__device__ __forceinline__ void fixed_step(FixedSum &acc, int va, int vb, int wa, int wb) {
+    acc.s += (long long)va * wa;
+    acc.l += (long long)va * wb;
+    acc.l += (long long)vb * wa;
+}
+__device__ __forceinline__ double fixed_value(FixedSum r, int bias) {   // times 2^(bias - 1023)
+    return ((double)(r.s + (r.l >> 27)) + (double)(r.l & 0x7ffffff) * 0x1p-27) * __hiloint2double((bias - 60) << 20, 0);
+}
+// a stored element as a double (abs. error 2^-58)
+__device__ __forceinline__ double fixed_to_double(int a, int b) { return fma((double)b, 0x1p-57, (double)a * 0x1p-30); }
+
+// x to FP32 from its bits, truncated; below 2^-70 zero
+__device__ __forceinline__ float f32_trunc(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x);
+    const unsigned b = (hi & 0x80000000u) | ((__funnelshift_l((unsigned)__double2loint(x), hi, 3) - (384u << 23)) & 0x7fffffffu);
+    return (hi & 0x7fffffffu) >= 953u << 20 ? __uint_as_float(b) : 0.0f;
+}
+
+// whether a set of values whose largest has this upper word (sign cleared) keeps to the
+// exponents FP32 has room for (2^+-40)
+__device__ __forceinline__ bool fixed_range(unsigned hi) { return hi >= (1023u - 40) << 20 && hi <= (1023u + 40) << 20; }
+// the exponent field of a power of two above |x|, from |x|^2
+__device__ __forceinline__ int bias_above(double x2) {
+    return ((__double2hiint(x2) >> 20) - 1023 + 2048) / 2 - 1024 + 1023 + 1;
+}
+
+// Warp sums of NV values at once: lane L ends with the total of value L >> (5 - log2 NV).
+template <int NV, typename T, typename Add, typename Shf>
+__device__ __forceinline__ T warp_sums_of(T *v, int lane, Add add, Shf shf) {
+#pragma unroll
+    for (int lev = 0; lev < 5; ++lev) {
+        const int o = 16 >> lev;
+        const int n = NV >> (lev + 1);
+        if (n >= 1) {
+            const bool up = (lane & o) != 0;
+#pragma unroll
+            for (int i = 0; i < (NV >> 1); ++i)
+                if (i < n) {
+                    const T send = up ? v[i] : v[i + n];
+                    const T keep = up ? v[i + n] : v[i];
+                    v[i] = add(keep, shf(send, o));
+                }
+        } else {
+            v[0] = add(v[0], shf(v[0], o));
+        }
+    }
+    return v[0];
+}
+
+__device__ __forceinline__ FixedSum fixed_add(FixedSum p, FixedSum q) { return FixedSum{p.s + q.s, p.l + q.l}; }
+__device__ __forceinline__ FixedSum fixed_shfl(FixedSum p, int o) {
+    return FixedSum{__shfl_xor_sync(0xffffffffu, p.s, o), __shfl_xor_sync(0xffffffffu, p.l, o)};
+}
+
+}  // namespace bd
