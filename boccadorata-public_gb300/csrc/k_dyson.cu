@@ -519,11 +519,11 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_df(const DyJob *jobs
                 const float sg = pow2_f32(-e);
                 const df alt{al.h * sg, al.l * sg}, s2t{(s2.h * sg) * sg, (s2.l * sg) * sg};
                 const df x2 = dfm::fma(alt, alt, s2t);   // in [1, 12)
-                const df r = dfm::rsqrt(x2, 2), nx = dfm::mul(x2, r);
+                const df r = dfm::rsqrt2(x2), nx = dfm::mul(x2, r);
                 const bool ng = signbit(alt.h);
                 const df aa = ng ? dfm::neg(alt) : alt;
                 tau = dfm::fma(aa, r, one);
-                df st = dfm::rcp(dfm::add(aa, nx), 2);   // 1 / (alpha~ - beta~)
+                df st = dfm::rcp2(dfm::add(aa, nx));   // 1 / (alpha~ - beta~)
                 if (ng) st = dfm::neg(st);
                 scal = df{st.h * sg, st.l * sg};         // 1 / (alpha - beta)
                 const df bt = ng ? nx : dfm::neg(nx);
@@ -806,11 +806,11 @@ __global__ void __launch_bounds__(kTsThreads) k_tridiag_small(const DyJob *jobs,
             if (lane == 0) {
                 const df al = s_col[par][0], s2 = s_col[par][1];
                 const df x2 = dfm::fma(al, al, s2);   // in [1, 12)
-                const df r = dfm::rsqrt(x2, 1), nx = dfm::mul(x2, r);
+                const df r = dfm::rsqrt2(x2), nx = dfm::mul(x2, r);
                 const bool ng = signbit(al.h);
                 const df aa = ng ? dfm::neg(al) : al;
                 const df tau = dfm::fma(aa, r, df{1.0f, 0.0f});   // (beta - alpha) / beta = 1 + |alpha| / |x|
-                df s = dfm::rcp(dfm::add(aa, nx), 1);               // 1 / (alpha - beta) = sign(alpha) / (|alpha| + |x|)
+                df s = dfm::rcp2(dfm::add(aa, nx));               // 1 / (alpha - beta) = sign(alpha) / (|alpha| + |x|)
                 if (ng) s = dfm::neg(s);
                 s_sc[0] = tau;
                 s_sc[1] = s;

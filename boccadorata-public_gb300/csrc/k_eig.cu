@@ -265,7 +265,7 @@ __device__ void invit_vector_df(const DyJob &J, int k, int b0, int b1, const dfm
     const float pt = (float)tl.pertol;
     // Reciprocals by one Newton step from the FP32 seed (~2^-44): the factors only need
     // to keep the shifted matrix's direction, far looser than that.
-    auto rcp1 = [&](df p) { return dfm::rcp(p, 1); };
+    auto rcp1 = [&](df p) { return dfm::rcp2(p); };
     auto clamp_piv = [&](df p) {   // pivots no smaller than pertol
         return (fabsf(p.h) < pt) ? df{p.h < 0.0f ? -pt : pt, 0.0f} : p;
     };
@@ -275,50 +275,48 @@ __device__ void invit_vector_df(const DyJob &J, int k, int b0, int b1, const dfm
     // and the kept pivot's are the same unless the pivot is below pertol); each row's
     // factors go to shared memory for the solves as soon as they are final.  The
     // tridiagonal comes in double-float from dt, et (shared memory).
+    // The pivoting is by selects (the lanes disagree about it row by row), and the forward half of
+    // the first solve runs along, its right-hand side from the hash.
+    auto start = [&](int i) {
+        return df{0.5f + (float)(hash32((unsigned)(i * 2654435761u) ^ (unsigned)(k * 97 + 13)) & 0xffff) / 65536.0f, 0.0f};
+    };
+    auto sel = [](bool c, df p, df q) { return df{c ? p.h : q.h, c ? p.l : q.l}; };
     df cur_d = df_sub(dt[b0], x);                 // dd(i) as updated so far
     df cur_u = (b0 < b1) ? et[b0] : zero;         // u1(i) as updated so far
+    df cur_y = start(b0);
     for (int i = b0; i < b1; ++i) {
-        const df di = cur_d, li = et[i], ui = cur_u;
-        const df nd = df_sub(dt[i + 1], x);                     // dd(i+1) before this row
-        const df nu = (i + 1 < b1) ? et[i + 1] : zero;          // u1(i+1) before this row
-        if (fabsf(di.h) >= fabsf(li.h)) {
-            a.set_pv(i, false);
-            const df cp = clamp_piv(di), r = rcp1(cp);
-            const df f = (di.h != 0.0f) ? dfm::mul(li, (cp.h == di.h) ? r : rcp1(di)) : zero;
-            a.ll(i) = f;
-            a.u1(i) = ui;
-            a.u2(i) = zero;
-            a.dd(i) = r;
-            cur_d = dfm::fma(dfm::neg(f), ui, nd);
-            cur_u = nu;
-        } else {
-            a.set_pv(i, true);
-            const df cp = clamp_piv(li), r = rcp1(cp);
-            const df f = dfm::mul(di, (cp.h == li.h) ? r : rcp1(li));
-            a.ll(i) = f;
-            a.u1(i) = nd;
-            a.u2(i) = nu;
-            a.dd(i) = r;
-            cur_d = dfm::fma(dfm::neg(f), nd, ui);
-            cur_u = dfm::mul(dfm::neg(f), nu);
-        }
+        const df li = et[i], nd = df_sub(dt[i + 1], x), nu = (i + 1 < b1) ? et[i + 1] : zero, yn = start(i + 1);
+        const bool sw = fabsf(cur_d.h) < fabsf(li.h);
+        const df piv = sel(sw, li, cur_d), oth = sel(sw, cur_d, li), cp = clamp_piv(piv), r = rcp1(cp);
+        const df f = (cp.h == piv.h) ? dfm::mul(oth, r) : (piv.h != 0.0f) ? dfm::mul(oth, rcp1(piv)) : zero;
+        const df ui = sel(sw, nd, cur_u), uo = sel(sw, cur_u, nd), yi = sel(sw, yn, cur_y), yo = sel(sw, cur_y, yn);
+        const df nf = dfm::neg(f);
+        a.set_pv(i, sw);
+        a.ll(i) = f;
+        a.u1(i) = ui;
+        a.u2(i) = sel(sw, nu, zero);
+        a.dd(i) = r;
+        a.y(i) = yi;
+        cur_y = dfm::fma(nf, yi, yo);
+        cur_d = dfm::fma(nf, ui, uo);
+        cur_u = sel(sw, dfm::mul(nf, nu), nu);
     }
     a.u1(b1) = zero;
     a.u2(b1) = zero;
     a.dd(b1) = rcp1(clamp_piv(cur_d));
-    for (int i = b0; i <= b1; ++i)
-        a.y(i) = df{0.5f + (float)(hash32((unsigned)(i * 2654435761u) ^ (unsigned)(k * 97 + 13)) & 0xffff) / 65536.0f, 0.0f};
+    a.y(b1) = cur_y;
     for (int it = 0; it < 2; ++it) {
-        df cur = a.y(b0);
-        for (int i = b0; i < b1; ++i) {   // L^-1 with the interchanges, y(i) carried in a register
-            df bi = cur, bi1 = a.y(i + 1);
-            const df f = a.ll(i);
-            if (!a.pv(i)) bi1 = dfm::fma(dfm::neg(f), bi, bi1);
-            else { const df tt = bi; bi = bi1; bi1 = dfm::fma(dfm::neg(f), bi1, tt); }
-            a.y(i) = bi;
-            cur = bi1;
+        if (it == 1) {
+            df cur = a.y(b0);
+            for (int i = b0; i < b1; ++i) {   // L^-1 with the interchanges, y(i) carried in a register
+                const df y1 = a.y(i + 1);
+                const bool sw = a.pv(i);
+                const df bi = sel(sw, y1, cur);
+                a.y(i) = bi;
+                cur = dfm::fma(dfm::neg(a.ll(i)), bi, sel(sw, cur, y1));
+            }
+            a.y(b1) = cur;
         }
-        a.y(b1) = cur;
         // U y = b, two superdiagonals: the term of y(i+2) first, off the chain through y(i+1)
         df y1 = zero, y2 = zero;
         float nrm = 0.0f;
