@@ -933,7 +933,7 @@ int launch_lanczos_range(bd_ctx *ctx, int ch_lo, int ch_hi, bool fp32) {
     // rounding of the stored vectors is part of the result.)
     const bool compact = !fp32 && ctx->lz_slices == 0;
     std::vector<LzChain> ch;
-    int Smax = 1, rmax = 1, long_rmax = 0;
+    int Smax = 1, rmax = 1;
     for (int I = ch_lo; I < ch_hi; ++I) {
         Chan &C = ctx->chans[I];
         for (int dir = 0; dir < 2; ++dir) {
@@ -969,7 +969,6 @@ int launch_lanczos_range(bd_ctx *ctx, int ch_lo, int ch_hi, bool fp32) {
             ch.push_back(z);
             Smax = std::max(Smax, z.S);
             rmax = std::max(rmax, P.L + 1);
-            if (z.N >= kLzLong) long_rmax = std::max(long_rmax, P.L + 1);
         }
     }
     if (ch.empty()) return BD_OK;
@@ -995,11 +994,10 @@ int launch_lanczos_range(bd_ctx *ctx, int ch_lo, int ch_hi, bool fp32) {
     if (compact) {
         CU(launch_lz_compact(d_ch, (int)ch.size(), ctx->eta, ctx->st));
         ctx->launches += 1;
-        const size_t smem = long_rmax > 0 ? lanczos_long_smem(Smax, rmax, true) : 0;
-        if (smem > 0) {
-            CU(launch_lanczos_long(d_ch, (int)ch.size(), rmax, CL, ctx->eta, smem, ctx->st));
-            ctx->launches += 1;
-        }
+        int forms = 0;
+        for (const LzChain &z : ch) if (z.N >= kLzLong) forms |= lanczos_long_form(z.N, rmax, CL);
+        CU(launch_lanczos_long(d_ch, (int)ch.size(), rmax, CL, ctx->eta, forms, ctx->st));
+        ctx->launches += (forms & 1) + (forms >> 1);
     }
     // chains whose slices do not fit next to the scalars keep them in global memory
     const bool gslices = ctx->lz_slices == 2 || (ctx->lz_slices == 0 && lanczos_smem_bytes(Smax, rmax) > kLanczosSmemSliceCap);
@@ -2830,7 +2828,7 @@ extern "C" int bd_lanczos_chain_noalloc(const double *d_E, const double *d_M, in
     if (e == cudaSuccess) e = launch_lz_groups(reinterpret_cast<const LzChain *>(base), 1, lz_gram_cap(N), st);
     if (e == cudaSuccess && !fp32 && N >= kLzLong)
         e = launch_lanczos_long(reinterpret_cast<const LzChain *>(base), 1, P.L + 1, kNoallocCluster, kNoallocEta,
-                                lanczos_long_smem(S, P.L + 1, false), st);
+                                lanczos_long_form(N, P.L + 1, kNoallocCluster) & 1, st);
     if (e == cudaSuccess)
         e = launch_lanczos(reinterpret_cast<const LzChain *>(base), 1, S, P.L + 1, fp32, kNoallocCluster, kNoallocEta,
                            false, st);

@@ -22,14 +22,18 @@
 // host launches behind this kernel.
 //
 // Work split: a cluster per chain, CTA r the pole rows [r S, (r+1) S), 512 threads and an SM to
-// itself; a warp per vector in the dot products, a thread per four poles everywhere else.  A
-// step is two cluster reductions.
+// itself; a part of four vectors a warp in the dot products, a thread per two or four poles
+// everywhere else.  A step is two cluster reductions.  With an SM's whole shared memory taken by
+// the slices L1 is a few KB, so what does not fit in registers costs an L2 access: the uniform
+// state is read from shared memory where it is used and the loads in flight are unconditional
+// (with 250 bytes a thread spilled the step below took 9.4 ms).
 // Bound by the planes' traffic and the phases around it in batches (12 bytes a stored element
-// and step: 2.1 M poles in 52 chains, 20 iterations a pivot, 18.3 -> 10.4 ms against 3.2 at the
-// copy bandwidth) and by the chain of phases for one chain on its 16 SMs (20 000 poles, 80
-// vectors: the call 5.36 -> 2.36 ms).  The same kernel with FP64 dot products took 17.1 and
-// 4.2 ms, with double-float ones formed from the doubles' bits 12.5 and 3.1 (off by 2e-15 |w|
-// where this is off by 5e-16, as FP64 is).
+// and step: 2.1 M poles in 52 chains, 20 iterations a pivot, 18.3 -> 7.7 ms against 3.2 at the
+// copy bandwidth; two thirds of a 41 000-pole chain's step are the sweep's loads, a fifth the
+// FP64 instructions) and by the chain of phases for one chain on its 16 SMs (20 000 poles, 80
+// vectors: the call 5.36 -> 2.26 ms).  FP64 dot products took 17.1 and 4.2 ms, double-float ones
+// formed from the doubles' bits 12.5 and 3.1 (off by 2e-15 |w| where this is off by 5e-16, as
+// FP64 is).
 #include <algorithm>
 #include <cfloat>
 #include <cooperative_groups.h>
@@ -51,62 +55,98 @@ __device__ __forceinline__ int4 ld4(const int *p) { return *reinterpret_cast<con
 __device__ __forceinline__ double2 ld2(const double *p) { return *reinterpret_cast<const double2 *>(p); }
 __device__ __forceinline__ void st2(double *p, double a, double b) { *reinterpret_cast<double2 *>(p) = make_double2(a, b); }
 
-// shared memory before the slices: A[2][rq] partials, c[rq], sp[2][kMaxSc], red[16][kMaxSc] (doubles),
-// cf[rq] (floats), rowslot[lq] (ints)
+// warps that share a vector's dot product, each a part of the elements: the vectors then divide
+// among the warps more evenly (17 of them: 5 quarters a warp against 2 wholes; 5164 elements of 30
+// vectors 72 000 clocks against 88 000), while a part below 512 elements is mostly remainder (1252
+// elements: halves 15 000, quarters 17 000) and the parts' sums of many rows would take the room
+// of the slices
+__host__ __device__ inline int long_parts_max(int rmax) { return rmax <= 160 ? 4 : 1; }
+__host__ __device__ inline int long_parts(int rmax, int S) { return min(long_parts_max(rmax), S >= 2048 ? 4 : 2); }
+// shared memory before the slices: A[2][at most parts_max][rq] sums (FixedSum), c[rq], sp[2][kMaxSc], red[16][kMaxSc]
+// (doubles), cf[rq] (floats), rowslot[rq] (ints)
 __host__ __device__ inline size_t long_fixed(int rmax) {
     const size_t rq = ((size_t)rmax + 4) & ~(size_t)3;
-    return sizeof(double) * (3 * rq + 2 * kMaxSc + kMaxWarps * kMaxSc) + 8 * rq;
+    return sizeof(FixedSum) * 2 * long_parts_max(rmax) * rq + sizeof(double) * (rq + 2 * kMaxSc + kMaxWarps * kMaxSc) + 8 * rq;
+}
+// A warp's part of four dot products (the last vector again where there are fewer): elements
+// [0, n) of this lane's start (n less that start), va the vectors' first planes there, pb from
+// those to the second planes.
+__device__ __forceinline__ void long_dots(FixedSum (&acc)[4], const int *const (&va)[4], int pb, const int *wa,
+                                          int S, int n) {
+#pragma unroll 1
+    for (int i = 0; i < n; i += 128) {
+        int4 x[4], y[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            x[u] = ld4(va[u] + i);
+            y[u] = ld4(va[u] + pb + i);
+        }
+        const int4 a = ld4(wa + i), b = ld4(wa + S + i);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            fixed_step(acc[u], x[u].x, y[u].x, a.x, b.x);
+            fixed_step(acc[u], x[u].y, y[u].y, a.y, b.y);
+            fixed_step(acc[u], x[u].z, y[u].z, a.z, b.z);
+            fixed_step(acc[u], x[u].w, y[u].w, a.w, b.w);
+        }
+    }
 }
 
 }  // namespace
 
+// CTAs a chain where the slices are in shared memory: at one CTA an SM the GPCs hold 15 clusters of
+// nine as of eight, so nine put 135 SMs to work for 120.  (Ten: 13 clusters.)
+__host__ __device__ inline int long_cluster(int cluster) { return cluster == 8 ? 9 : cluster; }
+__host__ __device__ inline int long_slice(int N, int cluster) { return ((N + cluster - 1) / cluster + 3) / 4 * 4; }
+__host__ __device__ inline bool long_fits(int N, int cluster, int rmax, size_t smem) {
+    return long_fixed(rmax) + 32 * (size_t)long_slice(N, long_cluster(cluster)) <= smem;
+}
+
+// SS: w, its split and the two newest vectors in shared memory (else in the chain's global scratch).
+template <bool SS>
 __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chains, int nchains, int rmax, double eta2,
                                                     int smem_bytes) {
     cg::cluster_group cluster = cg::this_cluster();
-    const int CL = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
-    const int cid = blockIdx.x / CL;
+    const int CL = (int)cluster.num_blocks(), rank = (int)cluster.block_rank(), cid = blockIdx.x / CL;
     if (cid >= nchains) return;
-    const LzChain C = chains[cid];
+    __shared__ LzChain C;   // (registers are short: what does not fit goes to an L1 of a few KB)
+    if (threadIdx.x < sizeof(LzChain) / 4)
+        reinterpret_cast<int *>(&C)[threadIdx.x] = reinterpret_cast<const int *>(chains + cid)[threadIdx.x];
+    __syncthreads();
     if (!C.done || *C.done || C.N < kLzLong) return;   // (the whole cluster leaves together)
-    const int N = C.N, D = C.D, L = C.L, NT = C.nden_out + C.D, S = C.S, i0 = rank * S;
-    const int ns = max(0, min(N, i0 + S) - i0);
+    if (long_fits(C.N, CL, rmax, smem_bytes) != SS) return;   // the other form's
+    const int S = long_slice(C.N, CL), i0 = rank * S;
     constexpr int T = kLongThreads, NW = kMaxWarps;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     extern __shared__ double sm[];
     const int rq = (rmax + 4) & ~3;
-    double *A = sm, *c = A + 2 * rq, *sp = c + rq, *red = sp + 2 * kMaxSc;
+    const int np = long_parts(rmax, S), cl2 = 32 - __clz(CL - 1);   // 2^cl2 lanes for the CTAs
+    FixedSum *A = reinterpret_cast<FixedSum *>(sm);
+    double *c = reinterpret_cast<double *>(A + 2 * long_parts_max(rmax) * rq), *sp = c + rq, *red = sp + 2 * kMaxSc;
     float *cf = reinterpret_cast<float *>(red + kMaxWarps * kMaxSc);
     int *rowslot = reinterpret_cast<int *>(cf + rq);
-    char *free_ = reinterpret_cast<char *>(sm) + long_fixed(rmax);
-    char *const end = reinterpret_cast<char *>(sm) + smem_bytes;
-    // slices: w, its split (two planes) and the two newest vectors in shared memory, or in the
-    // chain's global scratch; E and M beside them when they fit; then the first vectors' planes,
-    // as many as fit
-    double *w, *ring;
-    int *ws;
-    const size_t sb = sizeof(double) * (size_t)S;
-    if ((size_t)(end - free_) >= 4 * sb) {
-        w = reinterpret_cast<double *>(free_);
-        free_ += 4 * sb;
-    } else {
-        w = reinterpret_cast<double *>(C.slice + (size_t)rank * C.slice_stride);
+    // slices: w, the two newest vectors and w's split (two planes); E and M beside them when they
+    // fit, and the earlier chains' last vectors as doubles (the recurrence and the g read them)
+    double *const w = SS ? sm + long_fixed(rmax) / sizeof(double)
+                         : reinterpret_cast<double *>(C.slice + (size_t)rank * C.slice_stride);
+    double *const ring = w + S;
+    int *const ws = reinterpret_cast<int *>(w + 3 * (size_t)S);
+    __shared__ int s_oE, s_oM, s_oL, s_nl;   // where in sm, -1: not there; last vectors held
+    if (tid == 0) {
+        int o = (int)(long_fixed(rmax) / sizeof(double)) + (SS ? 4 * S : 0);
+        const int end = smem_bytes / (int)sizeof(double);
+        s_oE = s_oM = -1;
+        if (end - o >= S) { s_oE = o; o += S; }
+        if (end - o >= C.D * S) { s_oM = o; o += C.D * S; }
+        s_oL = o;
+        s_nl = min(max(C.n_used - 1, 0), (end - o) / S);
     }
-    ring = w + S;
-    ws = reinterpret_cast<int *>(w + 3 * (size_t)S);
-    double *Es = nullptr, *Ms = nullptr;
-    if ((size_t)(end - free_) >= sb) { Es = reinterpret_cast<double *>(free_); free_ += sb; }
-    if ((size_t)(end - free_) >= D * sb) { Ms = reinterpret_cast<double *>(free_); free_ += D * sb; }
-    // the earlier chains' last vectors as doubles (the recurrence and the g read them), the rest planes
-    int nlast = min(max(C.n_used - 1, 0), (int)((size_t)(end - free_) / sb));
-    double *lasts = reinterpret_cast<double *>(free_);
-    free_ += nlast * sb;
-    const int ccap = (int)((size_t)(end - free_) / sb);
-    int *cache = reinterpret_cast<int *>(free_);
     __shared__ int s_start[10], s_last[10], lslot[8], lt[16], lq[16];
     __shared__ double lc[16], s_row[32], s_tot[kMaxSc];
     __shared__ double s_n[3];   // 1/|w|, |w|, |E v|^2 of the kept vector
     __shared__ int s_fl;        // 0 keep, 1 sweep again, 2 exhausted, 3 the full space's
     __shared__ unsigned s_rng[2];
+    __shared__ float4 s_w2[2][NW / 4];   // the warps' parts of |w|^2, by the parity of A
     if (tid < 2) s_rng[tid] = 0;
     if (tid <= C.n_used && tid < 10) s_start[tid] = C.start[tid];
     if (tid < C.n_used && tid < 10) s_last[tid] = C.last[tid];
@@ -114,13 +154,13 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
     {   // energies and couplings inside 2^+-40 (the largest of each): FP32's exponents hold all that follows
         unsigned me = 0, mm = 0;
         for (int i = tid; i < S; i += T) {
-            const bool in = i < ns;
+            const bool in = i < min(S, C.N - i0);
             const double e = in ? C.E[i0 + i] : 0.0;
-            if (Es) Es[i] = e;
+            if (s_oE >= 0) sm[s_oE + i] = e;
             me = max(me, (unsigned)__double2hiint(e) & 0x7fffffffu);
-            for (int d = 0; d < D; ++d) {
-                const double m = in ? C.M[(size_t)d * N + i0 + i] : 0.0;
-                if (Ms) Ms[(size_t)d * S + i] = m;
+            for (int d = 0; d < C.D; ++d) {
+                const double m = in ? C.M[(size_t)d * C.N + i0 + i] : 0.0;
+                if (s_oM >= 0) sm[s_oM + d * S + i] = m;
                 mm = max(mm, (unsigned)__double2hiint(m) & 0x7fffffffu);
             }
         }
@@ -137,42 +177,31 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
         if (!fixed_range(me) || !fixed_range(mm)) return;
     }
     int nvec = 0;
-    // planes of stored vector t: a at the address, b pl(t) behind it
+    // planes of stored vector t: a at the address, b C.ld behind it
     int *Vg = reinterpret_cast<int *>(C.V) + i0;
-    auto plane = [&](int t) -> int * { return t < ccap ? cache + 2 * (size_t)t * S : Vg + 2 * (size_t)t * C.ld; };
-    auto pl = [&](int t) -> int { return t < ccap ? S : C.ld; };
+    auto plane = [&](int t) -> int * { return Vg + 2 * (size_t)t * C.ld; };
     // elements i, i + 1 of vector t as doubles (q: the chain it is the last vector of, or -1)
     auto vec2 = [&](int t, int q, int i) -> double2 {
         if (t >= nvec - 2) return ld2(ring + (size_t)(t & 1) * S + i);
-        if (q >= 0 && q < nlast) return ld2(lasts + (size_t)q * S + i);
+        if (q >= 0 && q < s_nl) return ld2(sm + s_oL + q * S + i);
         const int *p = plane(t) + i;
-        const int2 x = *reinterpret_cast<const int2 *>(p), y = *reinterpret_cast<const int2 *>(p + pl(t));
+        const int2 x = *reinterpret_cast<const int2 *>(p), y = *reinterpret_cast<const int2 *>(p + C.ld);
         return make_double2(fixed_to_double(x.x, y.x), fixed_to_double(x.y, y.y));
     };
     auto energy2 = [&](int i) -> double2 {   // of poles i, i + 1 of the slice
-        if (Es) return ld2(Es + i);
-        return make_double2(i < ns ? C.E[i0 + i] : 0.0, i + 1 < ns ? C.E[i0 + i + 1] : 0.0);
+        if (s_oE >= 0) return ld2(sm + s_oE + i);
+        return make_double2(i < min(S, C.N - i0) ? C.E[i0 + i] : 0.0, i + 1 < min(S, C.N - i0) ? C.E[i0 + i + 1] : 0.0);
     };
     auto coupling2 = [&](int d, int i) -> double2 {
-        if (Ms) return ld2(Ms + (size_t)d * S + i);
-        const double *p = C.M + (size_t)d * N + i0 + i;
-        return make_double2(i < ns ? p[0] : 0.0, i + 1 < ns ? p[1] : 0.0);
+        if (s_oM >= 0) return ld2(sm + s_oM + d * S + i);
+        const double *p = C.M + (size_t)d * C.N + i0 + i;
+        return make_double2(i < min(S, C.N - i0) ? p[0] : 0.0, i + 1 < min(S, C.N - i0) ? p[1] : 0.0);
     };
     int wbias = 1023;   // exponent field of the power of two w is split against
     auto split_w = [&](int i, double a, double b) {
         const int2 x = fixed_of(a, wbias), y = fixed_of(b, wbias);
         *reinterpret_cast<int2 *>(ws + i) = make_int2(x.x, y.x);
         *reinterpret_cast<int2 *>(ws + S + i) = make_int2(x.y, y.y);
-    };
-    auto csum = [&](const double *buf, int t) -> double {   // over the cluster, a fixed tree
-        double x[16];
-#pragma unroll
-        for (int r = 0; r < 16; ++r) x[r] = (r < CL) ? cluster.map_shared_rank(const_cast<double *>(buf), r)[t] : 0.0;
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1)
-#pragma unroll
-            for (int r = 0; r < o; ++r) x[r] += x[r + o];
-        return x[0];
     };
     const int Qg = C.gE ? C.gInfo[0] : 0;
     const int dtot = Qg > 0 ? C.gInfo[Qg] : 0;
@@ -185,7 +214,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
     int dcur = 0, ndefl = 0, extra = 0, k = -1, dpar = 0, spar = 0, nl0 = 0;
     double e2v = 0.0;
     bool ok = true;
-    for (int j = 0; j < L; ++j) {
+    for (int j = 0; j < C.L; ++j) {
         const bool newv = (k + 1 < C.n_used) && (j == s_start[k + 1]);
         if (newv) ++k;
         const int nq = k;
@@ -195,13 +224,13 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
         if (newv) {
             double p[8];
 #pragma unroll
-            for (int d = 0; d < 8; ++d) p[d] = d < D ? C.piv[(size_t)k * D + d] : 0.0;
+            for (int d = 0; d < 8; ++d) p[d] = d < C.D ? C.piv[(size_t)k * C.D + d] : 0.0;
             float s2 = 0.0f;
             for (int i = 2 * tid; i < S; i += 2 * T) {
                 double a = 0.0, b = 0.0;
 #pragma unroll
                 for (int d = 0; d < 8; ++d)
-                    if (d < D) {
+                    if (d < C.D) {
                         const double2 m = coupling2(d, i);
                         a = fma(m.x, p[d], a);
                         b = fma(m.y, p[d], b);
@@ -219,7 +248,11 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
                 sp[(size_t)spar * kMaxSc] = x;
             }
             cluster.sync();
-            if (tid == 0) s_n[0] = csum(sp + (size_t)spar * kMaxSc, 0);
+            if (warp == 0) {
+                double x = lane < CL ? *cluster.map_shared_rank(sp + (size_t)spar * kMaxSc, lane) : 0.0;
+                for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+                if (lane == 0) s_n[0] = x;
+            }
             spar ^= 1;
             __syncthreads();
             wn2 = wn2_first = s_n[0];
@@ -231,79 +264,90 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
         } else {
             wbias = bias_above(e2v);
             const double *v0 = ring + (size_t)(lt[0] & 1) * S;
-            for (int i = 2 * tid; i < S; i += 2 * T) {
-                const double2 e = energy2(i), x = ld2(v0 + i);
-                double a = x.x * e.x, b = x.y * e.y;
-#pragma unroll 4
+            float s2 = 0.0f;   // |w|^2 is read against the swept norm and the coefficients only
+#pragma unroll 1
+            for (int b = 2 * tid; b < S; b += 4 * T) {   // two poles here and two 2 T on, loads first
+                const int i[2] = {b, b + 2 * T < S ? b + 2 * T : b};
+                double2 x[2], e[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) { e[h] = energy2(i[h]); x[h] = ld2(v0 + i[h]); }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) { x[h].x *= e[h].x; x[h].y *= e[h].y; }
+#pragma unroll 1
                 for (int t = 0; t < nl0; ++t) {
-                    const double2 y = vec2(lt[t], lq[t], i);
-                    const double ct = lc[t];
-                    a = fma(-ct, y.x, a);
-                    b = fma(-ct, y.y, b);
+                    const double ct = -lc[t];
+                    double2 y[2];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) y[h] = vec2(lt[t], lq[t], i[h]);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) { x[h].x = fma(ct, y[h].x, x[h].x); x[h].y = fma(ct, y[h].y, x[h].y); }
                 }
-                st2(w + i, a, b);
-                split_w(i, a, b);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    if (h == 0 || b + 2 * T < S) {
+                        st2(w + i[h], x[h].x, x[h].y);
+                        split_w(i[h], x[h].x, x[h].y);
+                        const float p = f32_trunc(x[h].x), q = f32_trunc(x[h].y);
+                        s2 = fmaf(q, q, fmaf(p, p, s2));
+                    }
             }
+            for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+            if (lane == 0) reinterpret_cast<float *>(s_w2[dpar])[warp] = s2;
         }
         int fl, nfull = 0;
         for (;;) {
             __syncthreads();
-            // c_t = <v_t, w> for every stored vector, a warp each, four at a time; after a
-            // recurrence also |w|^2 as item nvec (read against the swept norm and the
-            // coefficients only: FP32)
-            double *Ap = A + (size_t)dpar * rq;
-            dpar ^= 1;
+            // c_t = <v_t, w> for every stored vector: np warps a vector, each its part of the
+            // elements, four vectors at a time
+            FixedSum *Ap = A + (size_t)dpar * np * rq;
             const bool want_n = !newv && nfull == 0;
-            const int items = nvec + (want_n ? 1 : 0);
-            constexpr int NU = 4;
-            for (int t0 = warp; t0 < items; t0 += NU * NW) {
-                const int nu = min(NU, (nvec - 1 - t0 + NW) / NW);   // stored vectors t0, t0 + NW, ..
-                if (nu > 0) {
-                    const int *va[NU], *vb[NU];
+            {
+                const int part = warp % np, nw = NW / np;
+                const int pe = (S / 4 + np - 1) / np * 4, e0 = min(part * pe, S), pn_ = min(pe, S - e0);
+                const int *wa = ws + e0 + 4 * lane;
+                for (int t0 = warp / np; t0 < nvec; t0 += 4 * nw) {
+                    const int nu = min(4, (nvec - 1 - t0) / nw + 1);   // stored vectors t0, t0 + nw, ..
+                    const int *va[4];
+                    FixedSum acc[4];
 #pragma unroll
-                    for (int u = 0; u < NU; ++u) {
-                        const int t = min(t0 + u * NW, nvec - 1);
-                        va[u] = plane(t);
-                        vb[u] = va[u] + pl(t);
+                    for (int u = 0; u < 4; ++u) {
+                        const int t = min(t0 + u * nw, nvec - 1);
+                        va[u] = plane(t) + e0 + 4 * lane;
+                        acc[u] = FixedSum{0, 0};
                     }
-                    FixedSum acc[NU];
-#pragma unroll
-                    for (int u = 0; u < NU; ++u) acc[u] = FixedSum{0, 0};
-                    for (int i = 4 * lane; i < S; i += 128) {
-                        int4 x[NU], y[NU];
-#pragma unroll
-                        for (int u = 0; u < NU; ++u) if (u < nu) { x[u] = ld4(va[u] + i); y[u] = ld4(vb[u] + i); }
-                        const int4 a = ld4(ws + i), b = ld4(ws + S + i);
-#pragma unroll
-                        for (int u = 0; u < NU; ++u)
-                            if (u < nu) {
-                                fixed_step(acc[u], x[u].x, y[u].x, a.x, b.x);
-                                fixed_step(acc[u], x[u].y, y[u].y, a.y, b.y);
-                                fixed_step(acc[u], x[u].z, y[u].z, a.z, b.z);
-                                fixed_step(acc[u], x[u].w, y[u].w, a.w, b.w);
-                            }
-                    }
-                    const FixedSum r = warp_sums_of<NU>(acc, lane, fixed_add, fixed_shfl);
+                    long_dots(acc, va, C.ld, wa, S, pn_ - 4 * lane);
+                    const FixedSum r = warp_sums_of<4>(acc, lane, fixed_add, fixed_shfl);
                     const int u = lane >> 3;
-                    if ((lane & 7) == 0 && u < nu) Ap[t0 + u * NW] = fixed_value(r, wbias);
+                    if ((lane & 7) == 0 && u < nu) Ap[part * rq + t0 + u * nw] = r;
                 }
-                if (want_n && (nvec - t0) % NW == 0 && nvec >= t0 && nvec < t0 + NU * NW) {
-                    float x2 = 0.0f;
-                    for (int i = 2 * lane; i < S; i += 64) {
-                        const double2 x = ld2(w + i);
-                        const float a = f32_trunc(x.x), b = f32_trunc(x.y);
-                        x2 = fmaf(b, b, fmaf(a, a, x2));
-                    }
-                    for (int o = 16; o > 0; o >>= 1) x2 += __shfl_xor_sync(0xffffffffu, x2, o);
-                    if (lane == 0) Ap[nvec] = (double)x2;
-                }
+            }
+            if (np > 1) {   // the parts' sums here: reads of the other CTAs cost more
+                __syncthreads();
+                for (int t = tid; t < nvec; t += T)
+                    for (int q = 1; q < np; ++q) Ap[t] = fixed_add(Ap[t], Ap[q * rq + t]);
             }
             cluster.sync();
-            for (int t = tid; t < items; t += T) {
-                const double x = csum(Ap, t);
-                c[t] = x;
-                cf[t] = t < nvec ? f32_trunc(x) * 0x1p-30f : f32_trunc(x);   // (against the a planes)
+            // the CTAs' sums, one a lane: exact, so in any order
+            for (int u0 = warp * 32; u0 < nvec << cl2; u0 += T) {
+                const int u = u0 + lane, t = min(u >> cl2, nvec - 1), r = u & ((1 << cl2) - 1);
+                FixedSum x = r < CL ? cluster.map_shared_rank(Ap, r)[t] : FixedSum{0, 0};
+                for (int o = (1 << cl2) >> 1; o > 0; o >>= 1) x = fixed_add(x, fixed_shfl(x, o));
+                if (r == 0 && u < nvec << cl2) {
+                    const double ct = fixed_value(x, wbias);
+                    c[t] = ct;
+                    cf[t] = f32_trunc(ct) * 0x1p-30f;   // (against the a planes)
+                }
             }
+            if (want_n && warp == NW - 1) {   // four lanes a CTA
+                float x2 = 0.0f;
+                for (int r = lane >> 2; r < CL; r += 8) {
+                    const float4 q = cluster.map_shared_rank(&s_w2[dpar][0], r)[lane & 3];
+                    x2 += (q.x + q.y) + (q.z + q.w);
+                }
+                for (int o = 16; o > 0; o >>= 1) x2 += __shfl_xor_sync(0xffffffffu, x2, o);
+                if (lane == 0) { c[nvec] = (double)x2; cf[nvec] = x2; }
+            }
+            dpar ^= 1;
             __syncthreads();
             if (want_n) wn2 = c[nvec];
             // the update and, of the updated w, this thread's part of the scalars
@@ -311,10 +355,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
             for (int t = lane; t < nvec; t += 32) cm = fmaxf(cm, fabsf(cf[t]));
             for (int o = 16; o > 0; o >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, o));
             const bool small = want_n && cm * 0x1p30f <= kSmall * sqrtf(cf[nvec]);
-            double pn = 0.0, sa = 0.0, m_[8], g_[8];
-            float se = 0.0f;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) { m_[q] = 0.0; g_[q] = 0.0; }
+#pragma unroll 1
             for (int i = 4 * tid; i < S; i += 4 * T) {
                 double x[4];
                 {
@@ -329,19 +370,20 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
                         a[2] = fmaf(ct, (float)v.z, a[2]);
                         a[3] = fmaf(ct, (float)v.w, a[3]);
                     };
-                    int t = 0;
-                    const int tc = min(ccap, nvec);
-                    for (; t < tc; ++t) step(cf[t], ld4(cache + 2 * (size_t)t * S + i));
-                    for (; t + 7 < nvec; t += 8) {
-                        int4 v[8];
+                    constexpr int NB = 8;   // vectors a round
+#pragma unroll 1
+                    for (int t = 0; t < nvec; t += NB) {
+                        int4 v[NB];
+                        const int *q = Vg + 2 * (size_t)t * C.ld + i;
 #pragma unroll
-                        for (int r = 0; r < 8; ++r) v[r] = ld4(Vg + 2 * (size_t)(t + r) * C.ld + i);
+                        for (int r = 0; r < NB; ++r)
+                            v[r] = ld4(q + 2 * (size_t)min(r, nvec - 1 - t) * C.ld);
 #pragma unroll
-                        for (int r = 0; r < 8; ++r) step(cf[t + r], v[r]);
+                        for (int r = 0; r < NB; ++r)
+                            step(t + r < nvec ? cf[t + r] : 0.0f, v[r]);
                     }
-                    for (; t < nvec; ++t) step(cf[t], ld4(Vg + 2 * (size_t)t * C.ld + i));
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) x[e] -= (double)a[e];
+                    for (int e = 0; e < 4; ++e) x[e] -= f32_to_double(a[e]);
                 } else {
                     FixedSum a[4];
 #pragma unroll
@@ -350,7 +392,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
                     for (int t = 0; t < nvec; ++t) {
                         const int2 ct = fixed_of(c[t], wbias);
                         const int *q = plane(t) + i;
-                        const int4 v = ld4(q), u = ld4(q + pl(t));
+                        const int4 v = ld4(q), u = ld4(q + C.ld);
                         fixed_step(a[0], v.x, u.x, ct.x, ct.y);
                         fixed_step(a[1], v.y, u.y, ct.x, ct.y);
                         fixed_step(a[2], v.z, u.z, ct.x, ct.y);
@@ -361,31 +403,41 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
                 }
                 st2(w + i, x[0], x[1]);
                 st2(w + i + 2, x[2], x[3]);
+            }
+            // the scalars' parts, a loop of its own (the thread's same poles): registers
+            double pn = 0.0, sa = 0.0, m_[8], g_[8];
+            float se = 0.0f;
 #pragma unroll
-                for (int e = 0; e < 4; e += 2) {
-                    const double2 ee = energy2(i + e);
-                    const double t0 = ee.x * x[e], t1 = ee.y * x[e + 1];
-                    pn = fma(x[e + 1], x[e + 1], fma(x[e], x[e], pn));
-                    sa = fma(t1, x[e + 1], fma(t0, x[e], sa));
+            for (int q = 0; q < 8; ++q) { m_[q] = 0.0; g_[q] = 0.0; }
+            for (int i = 4 * tid; i < S; i += 4 * T) {
+                double2 e[2], m0[2];   // (more of the couplings ahead would spill)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) { e[h] = energy2(i + 2 * h); m0[h] = coupling2(0, i + 2 * h); }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const double2 x = ld2(w + i + 2 * h);
+                    const double t0 = e[h].x * x.x, t1 = e[h].y * x.y;
+                    pn = fma(x.y, x.y, fma(x.x, x.x, pn));
+                    sa = fma(t1, x.y, fma(t0, x.x, sa));
                     const float f0 = f32_trunc(t0), f1 = f32_trunc(t1);   // |E w|^2 is a threshold's scale
                     se = fmaf(f1, f1, fmaf(f0, f0, se));
 #pragma unroll
                     for (int d = 0; d < 8; ++d)
-                        if (d < D) {
-                            const double2 m = coupling2(d, i + e);
-                            m_[d] = fma(m.y, x[e + 1], fma(m.x, x[e], m_[d]));
+                        if (d < C.D) {
+                            const double2 m = d == 0 ? m0[h] : coupling2(d, i + 2 * h);
+                            m_[d] = fma(m.y, x.y, fma(m.x, x.x, m_[d]));
                         }
 #pragma unroll
                     for (int q = 0; q < 8; ++q)
                         if (q < nq && lslot[q] >= 0) {
-                            const double2 v = vec2(lslot[q], q, i + e);
+                            const double2 v = vec2(lslot[q], q, i + 2 * h);
                             g_[q] = fma(v.y, t1, fma(v.x, t0, g_[q]));
                         }
                 }
             }
             {   // the warp's sums: values 0 |w|^2, 1 alpha, 2 + d m_d, 2 + D + q g_q, eight or all at a time;
                 // |E w|^2 in FP32
-                const int nv = 2 + D + nq;
+                const int nv = 2 + C.D + nq;
                 auto addd = [](double p, double q) { return p + q; };
                 auto shfd = [](double p, int o) { return __shfl_xor_sync(0xffffffffu, p, o); };
                 double v[18];
@@ -394,9 +446,9 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
                 for (int q = 2; q < 18; ++q) {   // (registers: every index known)
                     double x = 0.0;
 #pragma unroll
-                    for (int d = 0; d < 8; ++d) if (q == 2 + d && d < D) x = m_[d];
+                    for (int d = 0; d < 8; ++d) if (q == 2 + d && d < C.D) x = m_[d];
 #pragma unroll
-                    for (int h = 0; h < 8; ++h) if (q - 2 - D == h && h < nq) x = g_[h];
+                    for (int h = 0; h < 8; ++h) if (q - 2 - C.D == h && h < nq) x = g_[h];
                     v[q] = x;
                 }
                 if (nv <= 8) {
@@ -429,7 +481,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
                     double x = sub < CL ? cluster.map_shared_rank(Sp, sub)[sl] : 0.0;
 #pragma unroll
                     for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-                    if (sub == 0 && slot <= nv) s_tot[sl] = (sl >= 2 + D && sl < nv && lslot[sl - 2 - D] < 0) ? 0.0 : x;
+                    if (sub == 0 && slot <= nv) s_tot[sl] = (sl >= 2 + C.D && sl < nv && lslot[sl - 2 - C.D] < 0) ? 0.0 : x;
                 }
                 __syncthreads();
                 // k_lanczos's decision, by warp 0 of every CTA alike (an FP64 instruction of all the
@@ -468,8 +520,8 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
         if (fl == 3) { ok = false; break; }
         if (fl == 2) {
             // exhausted: the rest of this pivot chain takes unreached directions
-            const int jend = (k + 1 < C.n_used) ? min(L, s_start[k + 1]) : L;
-            const int nr = jend - j;
+            const int jend = (k + 1 < C.n_used) ? min(C.L, s_start[k + 1]) : C.L;
+            const int nr = jend - j, NT = C.nden_out + C.D;
             for (int r = tid; r < nr; r += T) {
                 const int d = dcur + r;
                 if (rank == 0) {
@@ -488,9 +540,9 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
         // normalise and store; the row
         const double ixb = s_n[0];
         {
-            int *q = plane(nvec), *qb = q + pl(nvec);
+            int *q = plane(nvec), *qb = q + C.ld;
             double *rg = ring + (size_t)(nvec & 1) * S;
-            double *rl = (j == s_last[k] && k < nlast) ? lasts + (size_t)k * S : nullptr;
+            double *rl = (j == s_last[k] && k < s_nl) ? sm + s_oL + k * S : nullptr;
             for (int i = 4 * tid; i < S; i += 4 * T) {
                 int4 a, b;
                 const double2 x = ld2(w + i), y = ld2(w + i + 2);
@@ -504,19 +556,16 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
                 f = fixed_of(v3, 1023); a.w = f.x; b.w = f.y;
                 *reinterpret_cast<int4 *>(q + i) = a;
                 *reinterpret_cast<int4 *>(qb + i) = b;
-                if (nvec < ccap) {   // (the host reads the basis back from V)
-                    *reinterpret_cast<int4 *>(Vg + 2 * (size_t)nvec * C.ld + i) = a;
-                    *reinterpret_cast<int4 *>(Vg + 2 * (size_t)nvec * C.ld + C.ld + i) = b;
-                }
             }
         }
         e2v = s_n[2];
-        if (tid < NT) {
+        if (tid < C.nden_out + C.D) {
+            const int NT = C.nden_out + C.D;
             double x = 0.0;
             if (tid == 0) x = s_tot[1] * ixb * ixb;
-            else if (tid == 1) x = (newv && k >= 1) ? s_tot[2 + D + (k - 1)] * ixb : s_n[1];
-            else if (tid < 2 + k) x = s_tot[2 + D + (tid - 2)] * ixb;
-            else if (tid >= C.nden_out && tid < C.nden_out + D) x = s_tot[2 + (tid - C.nden_out)] * ixb;
+            else if (tid == 1) x = (newv && k >= 1) ? s_tot[2 + C.D + (k - 1)] * ixb : s_n[1];
+            else if (tid < 2 + k) x = s_tot[2 + C.D + (tid - 2)] * ixb;
+            else if (tid >= C.nden_out && tid < C.nden_out + C.D) x = s_tot[2 + (tid - C.nden_out)] * ixb;
             s_row[tid] = x;
             if (rank == 0) C.out[(size_t)j * NT + tid] = x;
         }
@@ -539,7 +588,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
     }
     if (rank == 0 && ok) {
         if (C.rowslot)
-            for (int q = tid; q < L; q += T) C.rowslot[q] = rowslot[q];
+            for (int q = tid; q < C.L; q += T) C.rowslot[q] = rowslot[q];
         if (tid == 0) {
             atomicAdd(&C.stat[0], extra);
             atomicAdd(&C.stat[2], ndefl);
@@ -549,21 +598,18 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
     cluster.sync();   // no CTA leaves while peers may still read its shared memory
 }
 
-size_t lanczos_long_smem(int S, int rmax, bool have_slices) {
-    const size_t cap = (size_t)216 * 1024, fixed = long_fixed(rmax);
-    return fixed + (have_slices ? 0 : 32 * (size_t)S) <= cap ? cap : 0;
-}
-
-cudaError_t launch_lanczos_long(const LzChain *d_chains, int nchains, int rmax, int cluster, double eta, size_t smem,
-                                cudaStream_t st) {
-    if (nchains <= 0 || smem == 0) return cudaSuccess;
-    cudaError_t e = allow_dynamic_smem((const void *)k_lz_long);
-    if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(k_lz_long, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+namespace {
+constexpr size_t kLongSmem = (size_t)225 * 1024;
+template <bool SS>
+cudaError_t launch_form(const LzChain *d_chains, int nchains, int rmax, int cluster, double eta, cudaStream_t st) {
+    if (SS) cluster = long_cluster(cluster);
+    cudaError_t e = allow_dynamic_smem((const void *)k_lz_long<SS>);
+    if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(k_lz_long<SS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nchains * cluster, 1, 1);
     cfg.blockDim = dim3(kLongThreads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = kLongSmem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -572,9 +618,25 @@ cudaError_t launch_lanczos_long(const LzChain *d_chains, int nchains, int rmax, 
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_lz_long, d_chains, nchains, rmax, eta * eta, (int)smem);
+    return cudaLaunchKernelEx(&cfg, k_lz_long<SS>, d_chains, nchains, rmax, eta * eta, (int)kLongSmem);
+}
+}  // namespace
+
+int lanczos_long_form(int N, int rmax, int cluster) {
+    return long_fixed(rmax) > kLongSmem ? 0 : long_fits(N, cluster, rmax, kLongSmem) ? 1 : 2;
 }
 
-void lanczos_long_smem_init() { allow_dynamic_smem((const void *)k_lz_long); }
+cudaError_t launch_lanczos_long(const LzChain *d_chains, int nchains, int rmax, int cluster, double eta, int forms,
+                                cudaStream_t st) {
+    cudaError_t e = cudaSuccess;
+    if (forms & 1) e = launch_form<true>(d_chains, nchains, rmax, cluster, eta, st);
+    if (e == cudaSuccess && (forms & 2)) e = launch_form<false>(d_chains, nchains, rmax, cluster, eta, st);
+    return e;
+}
+
+void lanczos_long_smem_init() {
+    allow_dynamic_smem((const void *)k_lz_long<true>);
+    allow_dynamic_smem((const void *)k_lz_long<false>);
+}
 
 }  // namespace bd

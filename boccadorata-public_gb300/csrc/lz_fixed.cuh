@@ -29,8 +29,22 @@ __device__ __forceinline__ void fixed_step(FixedSum &acc, int va, int vb, int wa
 __device__ __forceinline__ double fixed_value(FixedSum r, int bias) {   // times 2^(bias - 1023)
     return ((double)(r.s + (r.l >> 27)) + (double)(r.l & 0x7ffffff) * 0x1p-27) * __hiloint2double((bias - 60) << 20, 0);
 }
-// a stored element as a double (abs. error 2^-58)
-__device__ __forceinline__ double fixed_to_double(int a, int b) { return fma((double)b, 0x1p-57, (double)a * 0x1p-30); }
+// a stored element as a double (abs. error 2^-58, or half a unit in the last place), from its bits
+__device__ __forceinline__ double fixed_to_double(int a, int b) {
+    const long long q = ((long long)a << 27) + b;   // v 2^57, |q| <= 2^57
+    const unsigned long long m = (unsigned long long)(q < 0 ? -q : q);
+    const int z = __clzll((long long)m);   // 6 .. 64
+    // the leading bit at bit 63, less itself, and half a unit; the carry goes to the exponent
+    const unsigned long long f = ((m << (z & 63)) & 0x7fffffffffffffffull) + (1u << 10);
+    const unsigned long long r = (f >> 11) + ((unsigned long long)(unsigned)(1023 + 6 - z) << 52);
+    return __longlong_as_double(m == 0 ? 0 : (long long)(r | (q < 0 ? 0x8000000000000000ull : 0)));
+}
+// a normal float as a double, from its bits; what FP32 has as denormal is zero
+__device__ __forceinline__ double f32_to_double(float x) {
+    const unsigned u = __float_as_uint(x), m = u & 0x7fffffffu;
+    if (m < 0x00800000u) return 0.0;
+    return __hiloint2double((int)((u & 0x80000000u) | ((m >> 3) + (896u << 20))), (int)(m << 29));
+}
 
 // x to FP32 from its bits, truncated; below 2^-70 zero
 __device__ __forceinline__ float f32_trunc(double x) {
