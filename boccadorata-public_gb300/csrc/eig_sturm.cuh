@@ -151,12 +151,40 @@ BD_HD void split(double x, float &h, float &l) {
     l = (float)(x - (double)h);
 }
 
-// FP32 count of eigenvalues below x (d, e2 of a scaled block of order m >= 1).
-BD_HD int count_f(const float *d, const float *e2, int m, float x) {
-    float pp = 1.0f, p = d[0] - x;
+// The counts run from both ends of a block at once, two chains of half the length (a lane each
+// on the device): rows 0 .. t give p_t = P0 and p_{t+1} = P1, rows m-1 .. t+1 from below the
+// trailing determinants R of rows t+1 .. m-1 and R' of rows t+2 .. m-1, t = (m - 1) / 2.  Then
+//   det(T - x I) = P1 R - e2_t P0 R',
+// and, eliminating from both ends into row t, whose pivot is det / (P0 R), the number of
+// eigenvalues below x is the sign changes of P up to P0, those of R, and one if that pivot is
+// negative.  Rows of a half: d[d0 + s i], e2 of rows i - 1 and i at e2[e0 + s i].
+struct Half {   // where a half of a block of m >= 2 rows starts, and its length
+    int d0, e0, s, len;
+    BD_HD Half(int m, bool below) {
+        const int t = (m - 1) / 2;
+        d0 = below ? m - 1 : 0;
+        e0 = below ? m - 1 : -1;
+        s = below ? -1 : 1;
+        len = below ? m - 1 - t : t + 1;
+    }
+};
+struct EndF { float p, q; int c; };                       // last value, the one before, sign changes
+struct EndDF { float ph, pl, qh, ql; int c, E; };         // the same times 2^E
+
+// FP32 half of a count at x (d, e2 of a scaled block).  The entries are asked for two rows ahead:
+// the chain of a row is shorter than the loads' latency.
+BD_HD EndF half_f(const float *d, const float *e2, Half h, float x) {
+    float pp = 1.0f, p = d[h.d0] - x;
     int c = (int)sign_bit(p);
-    for (int i = 1; i < m; ++i) {
-        const float np = fmaf(d[i] - x, p, -(e2[i - 1] * pp));
+    auto at = [&](int i) { return i < h.len ? i : h.len - 1; };
+    auto e_at = [&](int i) { return h.len > 1 ? e2[h.e0 + h.s * at(i)] : 0.0f; };
+    float d1 = d[h.d0 + h.s * at(1)], d2 = d[h.d0 + h.s * at(2)], e1 = e_at(1), e2n = e_at(2);
+    for (int i = 1; i < h.len; ++i) {
+        const float di = d1, ei = e1;
+        d1 = d2; e1 = e2n;
+        d2 = d[h.d0 + h.s * at(i + 2)];
+        e2n = e2[h.e0 + h.s * at(i + 2)];
+        const float np = fmaf(di - x, p, -(ei * pp));
         c += (int)(sign_bit(np) ^ sign_bit(p));
         pp = p;
         p = np;
@@ -164,34 +192,44 @@ BD_HD int count_f(const float *d, const float *e2, int m, float x) {
         if (a > 0x1p40f) { p *= 0x1p-64f; pp *= 0x1p-64f; }
         else if (a < 0x1p-40f) { p *= 0x1p64f; pp *= 0x1p64f; }
     }
-    return c;
+    return EndF{p, pp, c};
 }
 
-// Double-float count of eigenvalues below x = xh + xl; also p_m(x) as fh * 2^fe
-// (fh the hi part).  A zero p_i counts with the sign its bits carry: the change it
-// adds or drops at i is returned at i + 1, where p_{i+1} = -e2 p_{i-1}.
-BD_HD int count_df(const float *dh, const float *dl, const float *eh, const float *el, int m, float xh, float xl,
-                   float *fh, int *fe) {
+// the count from its halves, g = e2_t
+BD_HD int join_f(EndF P, EndF R, float g) {
+    const float f = fmaf(P.p, R.p, -(g * P.q) * R.q);
+    return P.c - (int)(sign_bit(P.p) ^ sign_bit(P.q)) + R.c + (int)(sign_bit(f) ^ sign_bit(P.q) ^ sign_bit(R.p));
+}
+
+// Double-float half of a count at x = xh + xl.  A zero p_i counts with the sign its bits carry:
+// the change it adds or drops at i is returned at i + 1, where p_{i+1} = -e2 p_{i-1}.
+BD_HD EndDF half_df(const float *dh, const float *dl, const float *eh, const float *el, Half h, float xh, float xl) {
     float ph, pl;
     {
         float s, r;
-        two_sum(dh[0], -xh, s, r);
-        r = add_rn(r, add_rn(dl[0], -xl));
+        two_sum(dh[h.d0], -xh, s, r);
+        r = add_rn(r, add_rn(dl[h.d0], -xl));
         two_sum(s, r, ph, pl);
     }
     float qh = 1.0f, ql = 0.0f;   // p_{i-1}
     int c = (int)sign_bit(ph), E = 0;
-    for (int i = 1; i < m; ++i) {
+    auto at = [&](int i) { return i < h.len ? i : h.len - 1; };
+    auto e_at = [&](const float *e, int i) { return h.len > 1 ? e[h.e0 + h.s * at(i)] : 0.0f; };
+    float dn = dh[h.d0 + h.s * at(1)], dnl = dl[h.d0 + h.s * at(1)], en = e_at(eh, 1), enl = e_at(el, 1);
+    for (int i = 1; i < h.len; ++i) {
+        const float di = dn, dil = dnl, g = en, gl = enl;
+        const int n = h.s * at(i + 1);   // the next row's entries
+        dn = dh[h.d0 + n]; dnl = dl[h.d0 + n];
+        en = eh[h.e0 + n]; enl = el[h.e0 + n];
         // t = d_i - x, left unnormalised: where the hi parts cancel, |t| < 2^-23 |d_i|
         // and an FP32-relative error in t * p stays below 2^-47 |d_i| |p|
         float th, tl;
-        two_sum(dh[i], -xh, th, tl);
-        tl = add_rn(tl, add_rn(dl[i], -xl));
+        two_sum(di, -xh, th, tl);
+        tl = add_rn(tl, add_rn(dil, -xl));
         const float ah = mul_rn(th, ph);
         float al = fma_rn(th, ph, -ah);
         al = fma_rn(th, pl, al);
         al = fma_rn(tl, ph, al);
-        const float g = eh[i - 1], gl = el[i - 1];
         const float bh = mul_rn(g, qh);
         float bl = fma_rn(g, qh, -bh);
         bl = fma_rn(g, ql, bl);
@@ -211,27 +249,58 @@ BD_HD int count_df(const float *dh, const float *dl, const float *eh, const floa
             ph *= 0x1p64f; pl *= 0x1p64f; qh *= 0x1p64f; ql *= 0x1p64f; E -= 64;
         }
     }
-    *fh = ph;
+    return EndDF{ph, pl, qh, ql, c, E};
+}
+
+// the count from its halves, g + gl = e2_t; also the determinant as fh * 2^fe (fh the hi part)
+BD_HD int join_df(const EndDF &P, const EndDF &R, float g, float gl, float *fh, int *fe) {
+    const float ah = mul_rn(P.ph, R.ph);
+    float al = fma_rn(P.ph, R.ph, -ah);
+    al = fma_rn(P.ph, R.pl, al);
+    al = fma_rn(P.pl, R.ph, al);
+    const float bh = mul_rn(g, P.qh);
+    float bl = fma_rn(g, P.qh, -bh);
+    bl = fma_rn(g, P.ql, bl);
+    bl = fma_rn(gl, P.qh, bl);
+    const float ch = mul_rn(bh, R.qh);
+    float cl = fma_rn(bh, R.qh, -ch);
+    cl = fma_rn(bh, R.ql, cl);
+    cl = fma_rn(bl, R.qh, cl);
+    float s, r, f, l;
+    two_sum(ah, -ch, s, r);
+    r = add_rn(r, add_rn(al, -cl));
+    two_sum(s, r, f, l);
+    const int c = P.c - (int)(sign_bit(P.ph) ^ sign_bit(P.qh)) + R.c +
+                  (int)(sign_bit(f) ^ sign_bit(P.qh) ^ sign_bit(R.ph));
+    int E = P.E + R.E;
+    for (int q = 0; q < 2; ++q) {   // a product of two numbers in 2^+-42, and what cancellation leaves
+        const float a = fabsf(f);
+        if (a > 0x1p40f) { f *= 0x1p-64f; E += 64; }
+        else if (a < 0x1p-40f && a != 0.0f) { f *= 0x1p64f; E -= 64; }
+    }
+    *fh = f;
     *fe = E;
     return c;
 }
 
-// Evaluators of four points per pass.  LaneEval4 (device): four lanes of a warp each
-// count one point and exchange the results by shuffles within their group.
+// Evaluators of four points per pass.  LaneEval4 (device): eight lanes of a warp, a point's
+// two halves on neighbours, exchange the results by shuffles within their group.
 // SeqEval4 (host and device): one thread counts the four points one after another.
 // The bisection below is written against either, so the host check runs the same
-// driver as the device.
+// driver and the same arithmetic as the device.
 struct SeqEval4 {
     const float *dh, *dl, *eh, *el;
     int m;
     BD_HD void f(const float *x, int *c) const {
-        for (int j = 0; j < 4; ++j) c[j] = count_f(dh, eh, m, x[j]);
+        for (int j = 0; j < 4; ++j)
+            c[j] = join_f(half_f(dh, eh, Half(m, false), x[j]), half_f(dh, eh, Half(m, true), x[j]), eh[(m - 1) / 2]);
     }
     BD_HD void df(const double *x, int *c, float *fh, int *fe) const {
         for (int j = 0; j < 4; ++j) {
             float h, l;
             split(x[j], h, l);
-            c[j] = count_df(dh, dl, eh, el, m, h, l, &fh[j], &fe[j]);
+            c[j] = join_df(half_df(dh, dl, eh, el, Half(m, false), h, l), half_df(dh, dl, eh, el, Half(m, true), h, l),
+                           eh[(m - 1) / 2], el[(m - 1) / 2], &fh[j], &fe[j]);
         }
     }
 };
@@ -240,24 +309,33 @@ struct SeqEval4 {
 struct LaneEval4 {
     const float *dh, *dl, *eh, *el;
     int m;
-    int sub;          // this lane's point, 0..3
+    int sub;          // this lane's place in its group: point sub / 2, the lower half if odd
     int base;         // lane index of the group's first lane
-    unsigned mask;    // the group's four lanes
+    unsigned mask;    // the group's eight lanes
+    __device__ float point(const float *x) const { return sub < 4 ? (sub < 2 ? x[0] : x[1]) : (sub < 6 ? x[2] : x[3]); }
+    __device__ double point(const double *x) const { return sub < 4 ? (sub < 2 ? x[0] : x[1]) : (sub < 6 ? x[2] : x[3]); }
     __device__ void f(const float *x, int *c) const {
-        const int mine = count_f(dh, eh, m, x[sub]);
+        const bool below = sub & 1;
+        const EndF a = half_f(dh, eh, Half(m, below), point(x));
+        const EndF b{__shfl_xor_sync(mask, a.p, 1), __shfl_xor_sync(mask, a.q, 1), __shfl_xor_sync(mask, a.c, 1)};
+        const int mine = join_f(below ? b : a, below ? a : b, eh[(m - 1) / 2]);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) c[j] = __shfl_sync(mask, mine, base + j);
+        for (int j = 0; j < 4; ++j) c[j] = __shfl_sync(mask, mine, base + 2 * j);
     }
     __device__ void df(const double *x, int *c, float *fh, int *fe) const {
+        const bool below = sub & 1;
         float h, l, f;
         int e;
-        split(x[sub], h, l);
-        const int mine = count_df(dh, dl, eh, el, m, h, l, &f, &e);
+        split(point(x), h, l);
+        const EndDF a = half_df(dh, dl, eh, el, Half(m, below), h, l);
+        const EndDF b{__shfl_xor_sync(mask, a.ph, 1), __shfl_xor_sync(mask, a.pl, 1), __shfl_xor_sync(mask, a.qh, 1),
+                      __shfl_xor_sync(mask, a.ql, 1), __shfl_xor_sync(mask, a.c, 1), __shfl_xor_sync(mask, a.E, 1)};
+        const int mine = join_df(below ? b : a, below ? a : b, eh[(m - 1) / 2], el[(m - 1) / 2], &f, &e);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            c[j] = __shfl_sync(mask, mine, base + j);
-            fh[j] = __shfl_sync(mask, f, base + j);
-            fe[j] = __shfl_sync(mask, e, base + j);
+            c[j] = __shfl_sync(mask, mine, base + 2 * j);
+            fh[j] = __shfl_sync(mask, f, base + 2 * j);
+            fe[j] = __shfl_sync(mask, e, base + 2 * j);
         }
     }
 };

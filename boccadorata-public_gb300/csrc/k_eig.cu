@@ -6,7 +6,7 @@
 //   k_qrows   R = first D rows of Q = H_0 H_1 ... H_{n-3} from the reflectors k_tridiag
 //             keeps in A's rows (the other reductions form R themselves)
 //   k_bisect_prep  splits T into unreduced blocks at negligible off-diagonals
-//   k_bisect  W_k by bisection on Sturm counts over its block, four threads per
+//   k_bisect  W_k by bisection on Sturm counts over its block, eight threads per
 //             eigenvalue (eig_sturm.cuh): an FP32 bracket, checked and finished in
 //             double-float arithmetic (FP64 issues at 1/64 of the FP32 rate) to
 //             max(1e-12 |W|, 1e-13 |T_b|)
@@ -170,18 +170,19 @@ __device__ inline int job_of(const long long *row_first, int njobs, long long g)
     return lo;
 }
 
-// Four threads per position: the eigenvalue of its block with the position's local
+// Eight threads per position: the eigenvalue of its block with the position's local
 // index, by sturm::bisect4 (FP32 bracket, double-float finish, four points per pass,
-// one per lane; no FP64 in the counts).  A matrix's eigenvalues are few hundred at
-// most, so the per-eigenvalue chain is the latency that matters; four lanes shorten
-// it and still leave most of the GPU's sub-partitions idle.
-constexpr int kBisectThreads = 128;   // 32 positions per CTA
+// the recurrence from both ends of the block, a lane each; no FP64 in the counts).  A
+// matrix's eigenvalues are a few hundred at most, so the per-eigenvalue chain is the
+// latency that matters; the lanes shorten it and leave one or two warps a sub-partition.
+constexpr int kBisectLanes = 8;
+constexpr int kBisectThreads = 128;   // 16 positions per CTA
 
 __global__ void __launch_bounds__(kBisectThreads) k_bisect(const DyJob *jobs, int njobs, const long long *row_first,
                                                            long long total, double *work, const long long *work_first) {
     const long long g4 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const long long g = g4 >> 2;   // the group's position; its four lanes share every branch
-    const int sub = (int)(g4 & 3);
+    const long long g = g4 / kBisectLanes;   // the group's position; its lanes share every branch of the driver
+    const int sub = (int)(g4 % kBisectLanes);
     if (g >= total) return;
     const int lo = job_of(row_first, njobs, g);
     const DyJob J = jobs[lo];
@@ -193,8 +194,8 @@ __global__ void __launch_bounds__(kBisectThreads) k_bisect(const DyJob *jobs, in
         W = J.d[t];
     } else {
         const BisectTables T = bisect_tables(work + work_first[lo], n);
-        const int lane = threadIdx.x & 31, base = lane & ~3;
-        const sturm::LaneEval4 ev{T.dh + b0, T.dl + b0, T.eh + b0, T.el + b0, m, sub, base, 0xFu << base};
+        const int lane = threadIdx.x & 31, base = lane & ~(kBisectLanes - 1);
+        const sturm::LaneEval4 ev{T.dh + b0, T.dl + b0, T.eh + b0, T.el + b0, m, sub, base, 0xFFu << base};
         W = sturm::bisect4(ev, k, T.glo[b0], T.ghi[b0], T.sx[b0], nullptr);
     }
     if (sub == 0) J.sol[(size_t)t * (2 + J.D)] = W;   // eigenvalue parked in the W slot of its position
@@ -263,8 +264,8 @@ __device__ void invit_vector_df(const DyJob &J, int k, int b0, int b1, const dfm
     const df x = dfm::from_double(xs);
     const df zero{0.0f, 0.0f};
     const float pt = (float)tl.pertol;
-    // Reciprocals by one Newton step from the FP32 seed (~2^-44): the factors only need
-    // to keep the shifted matrix's direction, far looser than that.
+    // Reciprocals by one second-order correction of the FP32 seed: the factors only need to
+    // keep the shifted matrix's direction, far looser than that.
     auto rcp1 = [&](df p) { return dfm::rcp2(p); };
     auto clamp_piv = [&](df p) {   // pivots no smaller than pertol
         return (fabsf(p.h) < pt) ? df{p.h < 0.0f ? -pt : pt, 0.0f} : p;
@@ -840,7 +841,7 @@ cudaError_t launch_eig(const DyJob *d_jobs, int njobs, const long long *d_row_fi
     if (nmax > nlim) k_qrows<<<njobs, kEigThreads, 0, st>>>(d_jobs, njobs, nlim);
     k_bisect_prep<<<njobs, 256, 0, st>>>(d_jobs, njobs, work, d_work_first);
     // four lanes per eigenvalue; a matrix's few hundred eigenvalues spread over many SMs
-    k_bisect<<<(unsigned)((total_rows * 4 + kBisectThreads - 1) / kBisectThreads), kBisectThreads, 0, st>>>(
+    k_bisect<<<(unsigned)((total_rows * kBisectLanes + kBisectThreads - 1) / kBisectThreads), kBisectThreads, 0, st>>>(
         d_jobs, njobs, d_row_first, total_rows, work, d_work_first);
     if (nmax > kTsMax) {
         const size_t smem = sizeof(double) * 2 * (size_t)(nmax < kIvTri ? nmax : kIvTri);
