@@ -8,6 +8,28 @@
 
 namespace bd {
 
+// A kernel beside the one launched before it on the stream, where neither reads what the other
+// writes and each alone leaves SMs idle.  The first calls beside_release (its dependent starts
+// once every CTA of it has, or has left); the second is started with launch_beside and calls
+// beside_wait before it leaves, on every path, so that it ends after the first and what follows
+// on the stream sees both.  (Without a first kernel beside_wait returns at once.)
+__device__ __forceinline__ void beside_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void beside_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+inline cudaError_t launch_beside(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // Lets a kernel take all the dynamic shared memory a CTA may opt into, once per kernel
 // in the process.  The limit is a property of the function, not of a launch: set to a
 // launch's own size, contexts on other host threads (other problem sizes) could lower

@@ -366,6 +366,7 @@ constexpr int kIvTri = 6144;   // rows of the tridiagonal kept in shared memory
 
 __global__ void __launch_bounds__(kIvLarge) k_invit(const DyJob *jobs, int njobs, const long long *row_first,
                                                     long long total, double *work, const long long *work_first) {
+    beside_release();
     const long long g = blockIdx.x * (long long)kIvLarge + threadIdx.x;
     extern __shared__ double smi[];
     // the CTA's positions usually belong to one matrix: its tridiagonal in shared memory
@@ -517,7 +518,7 @@ __global__ void __launch_bounds__(kIvThreads) k_invit_small(const DyJob *jobs, i
     if (jid >= njobs) return;
     const DyJob J = jobs[jid];
     const int n = J.nc, lane = threadIdx.x, k = blockIdx.y * kIvThreads + lane;
-    if (n > kTsMax || blockIdx.y * kIvThreads >= n) return;   // uniform over the CTA
+    if (n > kTsMax || blockIdx.y * kIvThreads >= n) { beside_wait(); return; }   // uniform over the CTA
     extern __shared__ double smi[];
     const int cap = kTsMax * kIvThreads;
     dfm::df *sd = reinterpret_cast<dfm::df *>(smi);
@@ -530,12 +531,17 @@ __global__ void __launch_bounds__(kIvThreads) k_invit_small(const DyJob *jobs, i
         et[i] = dfm::from_double(J.e[i]);
     }
     __syncthreads();
-    if (k >= n) return;
-    const int b0 = J.blk[k], b1 = J.blk[n + k];
-    double *Y = J.A;
-    if (b0 == b1) { Y[(size_t)b0 * n + k] = 1.0; return; }
-    invit_vector_df(J, k, b0, b1, dt, et, a);
-    for (int i = b0; i <= b1; ++i) Y[(size_t)i * n + k] = dfm::to_double(a.y(i));
+    if (k < n) {
+        const int b0 = J.blk[k], b1 = J.blk[n + k];
+        double *Y = J.A;
+        if (b0 == b1) {
+            Y[(size_t)b0 * n + k] = 1.0;
+        } else {
+            invit_vector_df(J, k, b0, b1, dt, et, a);
+            for (int i = b0; i <= b1; ++i) Y[(size_t)i * n + k] = dfm::to_double(a.y(i));
+        }
+    }
+    beside_wait();
 }
 
 // kOrthCtas CTAs per matrix.  Each takes 256 positions at a time, a thread per
@@ -840,7 +846,7 @@ cudaError_t launch_eig(const DyJob *d_jobs, int njobs, const long long *d_row_fi
                        int nlim, double *work, const long long *d_work_first, cudaStream_t st) {
     if (nmax > nlim) k_qrows<<<njobs, kEigThreads, 0, st>>>(d_jobs, njobs, nlim);
     k_bisect_prep<<<njobs, 256, 0, st>>>(d_jobs, njobs, work, d_work_first);
-    // four lanes per eigenvalue; a matrix's few hundred eigenvalues spread over many SMs
+    // eight lanes per eigenvalue; a matrix's few hundred eigenvalues spread over many SMs
     k_bisect<<<(unsigned)((total_rows * kBisectLanes + kBisectThreads - 1) / kBisectThreads), kBisectThreads, 0, st>>>(
         d_jobs, njobs, d_row_first, total_rows, work, d_work_first);
     if (nmax > kTsMax) {
@@ -854,7 +860,14 @@ cudaError_t launch_eig(const DyJob *d_jobs, int njobs, const long long *d_row_fi
         const int smem = (int)(sizeof(double) * 5 * kTsMax * kIvThreads + kTsMax * kIvThreads + sizeof(double) * 2 * kTsMax);
         cudaError_t e = allow_dynamic_smem((const void *)k_invit_small);
         if (e != cudaSuccess) return e;
-        k_invit_small<<<dim3(njobs, (kTsMax + kIvThreads - 1) / kIvThreads), kIvThreads, smem, st>>>(d_jobs, njobs);
+        // beside k_invit where that runs: the two take different matrices
+        const dim3 grid(njobs, (kTsMax + kIvThreads - 1) / kIvThreads);
+        if (nmax > kTsMax) {
+            e = launch_beside(k_invit_small, grid, dim3(kIvThreads), smem, st, d_jobs, njobs);
+            if (e != cudaSuccess) return e;
+        } else {
+            k_invit_small<<<grid, kIvThreads, smem, st>>>(d_jobs, njobs);
+        }
     }
     k_cluster_orth<<<(unsigned)(njobs * kOrthCtas), kEigThreads, 0, st>>>(d_jobs, njobs);
     k_post<<<(unsigned)((total_rows * 4 + 127) / 128), 128, 0, st>>>(d_jobs, njobs, d_row_first, total_rows);
