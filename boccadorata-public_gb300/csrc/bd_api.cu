@@ -303,9 +303,6 @@ struct bd_ctx {
     int4 *d_chunks_fw = nullptr, *d_chunks_bk = nullptr;   // chunk tables of the shared-memory sort
     long long chunk_cap_fw = 0, chunk_cap_bk = 0;
     int *d_sorti_fw = nullptr, *d_sorti_bk = nullptr;       // its sorted indices
-    unsigned long long *d_rkey[2] = {nullptr, nullptr};   // radix sort ping-pong buffers (long channels)
-    unsigned *d_rval[2] = {nullptr, nullptr};
-    void *d_rscratch = nullptr;
     double *d_sighf = nullptr, *d_sig1b = nullptr;  // per channel D*D at chan_dd_off
     double *d_efermi = nullptr;   // per channel: the Fermi energy of the input propagator (Seek_EFermi)
     bool ef_override = false;     // a per-channel Dyson call with the caller's Fermi energy
@@ -879,32 +876,32 @@ int launch_sort(bd_ctx *ctx, int ch_lo, int ch_hi, bool ref_order) {
         const int nseg = ch_hi - ch_lo;
         int seg_max = 0;
         for (int I = ch_lo; I < ch_hi; ++I) seg_max = std::max(seg_max, rel[I - ch_lo + 1] - rel[I - ch_lo]);
-        cudaError_t e;
-        if (seg_max <= kSortMax) {   // chunks sorted in shared memory, then ranked
-            std::vector<int4> chunks;
-            for (int I = ch_lo; I < ch_hi; ++I) {
-                const int s0 = rel[I - ch_lo], sl = rel[I - ch_lo + 1] - s0;
-                for (int c0 = 0; c0 < sl; c0 += kSortChunk) chunks.push_back(make_int4(s0 + c0, std::min(kSortChunk, sl - c0), s0, sl));
-            }
-            int4 *dch = dir == 0 ? ctx->d_chunks_fw : ctx->d_chunks_bk;
-            if ((long long)chunks.size() > (dir == 0 ? ctx->chunk_cap_fw : ctx->chunk_cap_bk))
-                return fail(ctx, BD_ERR_STATE, "sort chunk table overflow");
-            if (int rc = h2d_table(ctx, dch, chunks.data(), sizeof(int4) * chunks.size())) return rc;
-            unsigned long long *tk = reinterpret_cast<unsigned long long *>(ctx->d_keys_tmp);
-            int *ti = dir == 0 ? ctx->d_sorti_fw : ctx->d_sorti_bk;
-            k_chunk_sort<<<(unsigned)chunks.size(), kSortThreads, 0, ctx->st>>>(E + n0, dch, dir == 1, n0, tk, ti);
-            k_chunk_place<<<(unsigned)((n + 255) / 256), 256, 0, ctx->st>>>(tk, ti, dch, (int)chunks.size(), n, n0,
-                                                                          perm + n0);
-            e = cudaGetLastError();
-            ctx->launches += 2;
-        } else {   // a channel beyond shared memory: radix sorts over the range
-            int nl = 0;
-            e = launch_pole_radix(E, dir == 0 ? ctx->d_seg_fw : ctx->d_seg_bk, ch_lo, nseg, n0, n, dir == 1,
-                                  ctx->d_rkey[0], ctx->d_rval[0], ctx->d_rkey[1], ctx->d_rval[1], ctx->d_rscratch,
-                                  perm, &nl, ctx->st);
-            ctx->launches += nl;
+        std::vector<int4> chunks;
+        for (int I = ch_lo; I < ch_hi; ++I) {
+            const int s0 = rel[I - ch_lo], sl = rel[I - ch_lo + 1] - s0;
+            for (int c0 = 0; c0 < sl; c0 += kSortChunk) chunks.push_back(make_int4(s0 + c0, std::min(kSortChunk, sl - c0), s0, sl));
         }
-        CU(e);
+        int4 *dch = dir == 0 ? ctx->d_chunks_fw : ctx->d_chunks_bk;
+        if ((long long)chunks.size() > (dir == 0 ? ctx->chunk_cap_fw : ctx->chunk_cap_bk))
+            return fail(ctx, BD_ERR_STATE, "sort chunk table overflow");
+        if (int rc = h2d_table(ctx, dch, chunks.data(), sizeof(int4) * chunks.size())) return rc;
+        // the passes' second buffers: the range's own sorted copies, which k_permute_soa writes last
+        unsigned long long *tk[2] = {reinterpret_cast<unsigned long long *>(ctx->d_keys_tmp),
+                                     reinterpret_cast<unsigned long long *>((dir == 0 ? ctx->d_Efw_s : ctx->d_Ebk_s) + n0)};
+        int *ti[2] = {dir == 0 ? ctx->d_sorti_fw : ctx->d_sorti_bk,
+                      reinterpret_cast<int *>(dir == 0 ? ctx->d_Mfw_f + A.mfw_off : ctx->d_Mbk_f + A.mbk_off)};
+        const unsigned nch = (unsigned)chunks.size();
+        k_chunk_sort<<<nch, kSortThreads, 0, ctx->st>>>(E + n0, dch, dir == 1, n0, tk[0], ti[0],
+                                                        seg_max <= kSortChunk ? perm + n0 : nullptr);
+        ctx->launches += 1;
+        int b = 0;
+        for (unsigned run = kSortChunk; run < (unsigned)seg_max; run *= 2, b ^= 1) {
+            const bool last = 2ull * run >= (unsigned)seg_max;
+            k_run_merge<<<nch, kSortThreads, 0, ctx->st>>>(tk[b], ti[b], dch, run, tk[b ^ 1], ti[b ^ 1],
+                                                            last ? perm + n0 : nullptr);
+            ctx->launches += 1;
+        }
+        CU(cudaGetLastError());
         if (ref_order) {
             CU(launch_heap_order(E, d_off, nseg, seg_max, n0, perm, ctx->st));
             ctx->launches += 1;
@@ -1646,16 +1643,6 @@ int upload_propagator(bd_ctx *ctx, const bd_propagator *prop) {
     if ((rc = dalloc(ctx, &ctx->d_Mbk_s, ctx->tot_mbk))) return rc;
     if ((rc = dalloc(ctx, &ctx->d_Mfw_f, ctx->tot_mfw))) return rc;
     if ((rc = dalloc(ctx, &ctx->d_Mbk_f, ctx->tot_mbk))) return rc;
-    {   // radix sort buffers, used when a channel exceeds the shared-memory chunk sort
-        long long seg_max = 0;
-        for (int I = 0; I < ns; ++I) seg_max = std::max<long long>(seg_max, std::max(ctx->chans[I].nfw, ctx->chans[I].nbk));
-        const long long nr = seg_max > kSortMax ? std::max<long long>(1, std::max(ctx->tot_fw, ctx->tot_bk)) : 1;
-        for (int b = 0; b < 2; ++b) {
-            if ((rc = dalloc(ctx, &ctx->d_rkey[b], (size_t)nr))) return rc;
-            if ((rc = dalloc(ctx, &ctx->d_rval[b], (size_t)nr))) return rc;
-        }
-        if ((rc = dalloc(ctx, reinterpret_cast<char **>(&ctx->d_rscratch), radix_scratch_bytes(nr)))) return rc;
-    }
     // one-body (diag xe, Trel=7 ExtU1=1) and static self-energy, per channel D x D
     ctx->chan_dd_off.assign(ns, 0);
     std::vector<double> s1b;

@@ -36,11 +36,12 @@ size_t tc_smem_bytes(int np);
 cudaError_t launch_poles_tc(const DevProblem &P, const S2Block *blk, const int *tile_blk, const int4 *tiles,
                             int ntiles, const ChanSig *cs, const double *vp, const TcOut &fw, const TcOut &bk,
                             int dirs, int *err, size_t smem, cudaStream_t st);
-constexpr int kSortThreads = 512;
+constexpr int kSortThreads = 256;
 constexpr int kSortChunk = 2048;  // poles per chunk of the shared-memory sort
-constexpr int kSortMax = 16384;   // longest channel sorted by chunks (longer: radix sort)
 __global__ void k_chunk_sort(const double *E, const int4 *chunks, bool desc, long long base, unsigned long long *tk,
-                             int *ti);
+                             int *ti, int *perm);
+__global__ void k_run_merge(const unsigned long long *kin, const int *vin, const int4 *chunks, unsigned run,
+                            unsigned long long *kout, int *vout, int *perm);
 // Stable LSD radix sort of (key, value) pairs over key bits [bit0, bit1), eight per pass
 // (k_sort.cu).  keys / vals and ktmp / vtmp are ping-pong buffers of n entries: on
 // return keys / vals point at the sorted pairs.  scratch: radix_scratch_bytes(n).
@@ -57,9 +58,6 @@ __global__ void k_vpp_canon(const int4 *abcd, const int *Jv, long long n, const 
 __global__ void k_vpp_first(const unsigned long long *key, long long n, unsigned *keep);
 __global__ void k_vpp_place(const unsigned long long *key, const unsigned *val, const unsigned *pos, const unsigned *keep,
                             long long n, const double *Vin, const signed char *sign, int *iabJ, int *icdJ, double *V);
-cudaError_t launch_pole_radix(const double *E, const int *seg_of, int ch_lo, int nseg, long long n0, long long n,
-                              bool desc, unsigned long long *k0, unsigned *v0, unsigned long long *k1, unsigned *v1,
-                              void *scratch, int *perm, int *launches, cudaStream_t st);
 __global__ void k_dressed_select(const double *sol, const long long *sol_off, const int *nq, const int *D_of, int ns,
                                  double z_cut, int max_frag, int cap, int *cnt, int *sel);
 __global__ void k_dressed_write(const double *sol, const long long *sol_off, const int *nq, const int *D_of,

@@ -330,83 +330,154 @@ __global__ void k_pair_rank(const int *iabJ, const int *icdJ, int n, int norb, c
     prank[((size_t)c * norb + d) * nJ + J] = i - s0;
 }
 
-// Stable sort of each channel's poles by energy (ascending, or descending with desc),
-// for channels of at most kSortMax poles, in two kernels over chunks of kSortChunk
-// consecutive poles of one channel (the chunk table lists, per chunk, its first pole
-// and length and its channel's first pole and length, relative to the range):
-//   k_chunk_sort   one CTA per chunk sorts (key, index) pairs with a bitonic network
-//                  in shared memory, the key the order-preserving integer image of the
-//                  double (sign bit set: all bits flipped, else the sign bit set; the
-//                  radix sort's mapping, -0 before +0), complemented for descending
+// Stable sort of each channel's poles by energy (ascending, or descending with desc), over
+// chunks of kSortChunk consecutive poles of one channel (the chunk table lists, per chunk,
+// its first pole and length and its channel's first pole and length, relative to the range):
+//   k_chunk_sort   one CTA per chunk sorts (key, index) pairs in shared memory, each thread
+//                  its eight, then by merging runs of 8, 16, .. pairs; the key the order-preserving integer image of the
+//                  double (sign bit set: all bits flipped, else the sign bit set: -0
+//                  before +0), complemented for descending
 //                  order, the index (the pole's global index) breaking ties;
-//   k_chunk_place  one thread per pole: its rank in the channel is the number of
-//                  pairs below its own in every chunk of the channel (binary searches
-//                  in the sorted chunks), so perm[rank] = its global index.
-// (key, index) pairs are distinct, so the order is the stable sort's.
+//   k_run_merge    pairs of sorted runs of a channel merged, one CTA per chunk of the output:
+//                  a 32-way search finds the parts of the two runs that fill it, they are
+//                  merged in shared memory; the runs' length doubles until the longest
+//                  channel is one, and the last pass writes the indices to perm.
+// (key, index) pairs are distinct, and the earlier run holds the smaller indices, so the order is
+// the stable sort's.  Bound by the steps' latency (a chunk's eight merges, a pass's search and
+// merge).  480 000 poles in channels up to 16 000: 20 us and 3 x 9 (a bitonic network 50, ranks by
+// binary searches in every other chunk 47); 1.05 M poles in channels up to 52 000: 31 us and 5 x 11
+// (a radix sort of energies, then channels, 320).
 __device__ inline unsigned long long sort_key(double e, bool desc) {
     unsigned long long u = (unsigned long long)__double_as_longlong(e);
     u = (u >> 63) ? ~u : (u | (1ull << 63));
     return desc ? ~u : u;
 }
 
-__global__ void __launch_bounds__(kSortThreads) k_chunk_sort(const double *E, const int4 *chunks, bool desc,
-                                                             long long base, unsigned long long *tk, int *ti) {
-    const int4 ch = chunks[blockIdx.x];   // first pole, length, channel's first pole, channel's length
-    __shared__ unsigned long long skey[kSortChunk];
-    __shared__ int sidx[kSortChunk];
-    const int n = ch.y;
-    int P = 32;
-    while (P < n) P <<= 1;
-    for (int t = threadIdx.x; t < P; t += kSortThreads) {
-        unsigned long long k = ~0ull;
-        int ix = INT_MAX;
-        if (t < n) { k = sort_key(E[ch.x + t], desc); ix = (int)(base + ch.x + t); }
-        skey[t] = k;
-        sidx[t] = ix;
+// Merging in shared memory: kMergePer outputs a thread, from output diag on, of the sorted runs
+// sk[A, A + nA) and sk[B, B + nB) (the first run's first among equals).  Element i is kept at
+// merge_at(i): threads read and write eight consecutive ones each.
+constexpr int kMergePer = kSortChunk / kSortThreads;
+constexpr int kMergeRoom = kSortChunk + kSortChunk / kMergePer;
+static_assert(kMergePer == 8, "the sorting of a thread's own pairs and merge_at are for eight");
+__device__ __forceinline__ int merge_at(int i) { return i + (i >> 3); }
+__device__ __forceinline__ void merge_part(const unsigned long long *sk, const int *sv, int A, int nA, int B, int nB, int diag,
+                                           unsigned long long (&key)[kMergePer], int (&val)[kMergePer]) {
+    int lo = max(0, diag - nB), hi = min(diag, nA);
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (sk[merge_at(A + mid)] <= sk[merge_at(B + diag - 1 - mid)]) lo = mid + 1; else hi = mid;
     }
-    __syncthreads();
-    for (int kk = 2; kk <= P; kk <<= 1)
-        for (int j = kk >> 1; j > 0; j >>= 1) {
-            for (int t = threadIdx.x; t < P; t += kSortThreads) {
-                const int u = t ^ j;
-                if (u <= t) continue;
-                const unsigned long long ka = skey[t], kb = skey[u];
-                const int ia = sidx[t], ib = sidx[u];
-                const bool gt = (ka > kb) || (ka == kb && ia > ib);
-                if (((t & kk) == 0) ? gt : !gt) { skey[t] = kb; skey[u] = ka; sidx[t] = ib; sidx[u] = ia; }
-            }
-            __syncthreads();
-        }
-    for (int t = threadIdx.x; t < n; t += kSortThreads) { tk[ch.x + t] = skey[t]; ti[ch.x + t] = sidx[t]; }
+    int i = A + lo, j = B + diag - lo;
+    const int iE = A + nA, jE = B + nB;
+    unsigned long long ka = i < iE ? sk[merge_at(i)] : 0ull, kb = j < jE ? sk[merge_at(j)] : 0ull;
+#pragma unroll
+    for (int r = 0; r < kMergePer; ++r) {
+        if (i >= iE && j >= jE) break;
+        const bool first = j >= jE || (i < iE && ka <= kb);
+        key[r] = first ? ka : kb;
+        val[r] = sv[merge_at(first ? i : j)];
+        if (first) { ++i; if (i < iE) ka = sk[merge_at(i)]; }
+        else { ++j; if (j < jE) kb = sk[merge_at(j)]; }
+    }
 }
 
-__global__ void k_chunk_place(const unsigned long long *tk, const int *ti, const int4 *chunks, int nchunks,
-                              long long n, long long base, int *perm) {
-    const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (g >= n) return;
-    int lo = 0, hi = nchunks - 1;   // the chunk holding g
-    while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (chunks[mid].x <= g) lo = mid; else hi = mid - 1; }
-    const int4 me = chunks[lo];
-    const unsigned long long key = tk[g];
-    const int idx = ti[g];
-    int rank = (int)(g - me.x);   // pairs below it in its own chunk
-    // the channel's other chunks (a channel's chunks are consecutive in the table)
-    int c0 = lo, c1 = lo;
-    while (c0 > 0 && chunks[c0 - 1].z == me.z) --c0;
-    while (c1 + 1 < nchunks && chunks[c1 + 1].z == me.z) ++c1;
-    for (int c = c0; c <= c1; ++c) {
-        if (c == lo) continue;
-        const int4 o = chunks[c];
-        int a = 0, b = o.y;   // first pair of chunk c not below (key, idx)
-        while (a < b) {
-            const int mid = (a + b) >> 1;
-            const unsigned long long km = tk[o.x + mid];
-            const bool below = km < key || (km == key && ti[o.x + mid] < idx);
-            if (below) a = mid + 1; else b = mid;
-        }
-        rank += a;
+__global__ void __launch_bounds__(kSortThreads) k_chunk_sort(const double *E, const int4 *chunks, bool desc,
+                                                             long long base, unsigned long long *tk, int *ti, int *perm) {
+    const int4 ch = chunks[blockIdx.x];   // first pole, length, channel's first pole, channel's length
+    __shared__ unsigned long long sk[kMergeRoom];
+    __shared__ int sv[kMergeRoom];
+    const int n = ch.y, n8 = (n + kMergePer - 1) / kMergePer * kMergePer, tid = threadIdx.x, diag = kMergePer * tid;
+    for (int t = tid; t < n8; t += kSortThreads) {   // past the end the largest key, after all equal ones
+        sk[merge_at(t)] = t < n ? sort_key(E[ch.x + t], desc) : ~0ull;
+        sv[merge_at(t)] = t < n ? (int)(base + ch.x + t) : INT_MAX;
     }
-    perm[me.z + rank] = idx;
+    __syncthreads();
+    unsigned long long key[kMergePer];
+    int val[kMergePer];
+    if (diag < n8) {   // a thread's own pairs: exchanges of neighbours, strictly out of order (stable)
+#pragma unroll
+        for (int r = 0; r < kMergePer; ++r) { key[r] = sk[merge_at(diag + r)]; val[r] = sv[merge_at(diag + r)]; }
+#pragma unroll
+        for (int p = 0; p < kMergePer; ++p)
+#pragma unroll
+            for (int r = p & 1; r + 1 < kMergePer; r += 2) {
+                const bool gt = key[r] > key[r + 1];
+                const unsigned long long k0 = gt ? key[r + 1] : key[r], k1 = gt ? key[r] : key[r + 1];
+                const int v0 = gt ? val[r + 1] : val[r], v1 = gt ? val[r] : val[r + 1];
+                key[r] = k0; key[r + 1] = k1; val[r] = v0; val[r + 1] = v1;
+            }
+#pragma unroll
+        for (int r = 0; r < kMergePer; ++r) { sk[merge_at(diag + r)] = key[r]; sv[merge_at(diag + r)] = val[r]; }
+    }
+    for (int run = kMergePer; run < n8; run *= 2) {
+        __syncthreads();
+        if (diag < n8) {
+            const int A = diag / (2 * run) * (2 * run), nA = min(run, n8 - A), nB = max(0, min(run, n8 - A - run));
+            merge_part(sk, sv, A, nA, A + run, nB, diag - A, key, val);
+        }
+        __syncthreads();
+        if (diag < n8)
+#pragma unroll
+            for (int r = 0; r < kMergePer; ++r) { sk[merge_at(diag + r)] = key[r]; sv[merge_at(diag + r)] = val[r]; }
+    }
+    __syncthreads();
+    for (int t = tid; t < n; t += kSortThreads) {
+        if (perm) { perm[ch.x + t] = sv[merge_at(t)]; continue; }   // no channel longer than a chunk
+        tk[ch.x + t] = sk[merge_at(t)];
+        ti[ch.x + t] = sv[merge_at(t)];
+    }
+}
+
+// Outputs [c0, c0 + len) of the channel are the chunk's place in it; they lie in one pair of runs.
+__global__ void __launch_bounds__(kSortThreads) k_run_merge(const unsigned long long *kin, const int *vin,
+                                                             const int4 *chunks, unsigned run, unsigned long long *kout,
+                                                             int *vout, int *perm) {
+    const int4 ch = chunks[blockIdx.x];
+    __shared__ unsigned long long sk[kMergeRoom];
+    __shared__ int sv[kMergeRoom], s_a[2];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned c0 = (unsigned)(ch.x - ch.z), len = (unsigned)ch.y, w = (unsigned)ch.w;
+    const unsigned base = (unsigned)(c0 / (2ull * run) * (2ull * run));
+    const int nA = (int)min(run, w - base), nB = w - base > run ? (int)min(run, w - base - run) : 0;
+    const unsigned long long *A = kin + ch.z + base, *B = A + run;
+    const int *Av = vin + ch.z + base, *Bv = Av + run;
+    if (warp < 2) {   // how many of A are among the first d outputs: 32 probes at a time
+        const int d = (int)(c0 - base) + (warp ? (int)len : 0);
+        int lo = max(0, d - nB), hi = min(d, nA);
+        while (lo < hi) {
+            const long long span = hi - lo;
+            const int p = lo + (int)(span * lane / 32);
+            const int t = __popc(__ballot_sync(0xffffffffu, A[p] <= B[d - 1 - p]));   // true up to some p
+            if (t == 0) break;
+            hi = t < 32 ? lo + (int)(span * t / 32) : hi;
+            lo += (int)(span * (t - 1) / 32) + 1;
+        }
+        if (lane == 0) s_a[warp] = lo;
+    }
+    __syncthreads();
+    const int a0 = s_a[0], na = s_a[1] - a0, b0 = (int)(c0 - base) - a0, nb = (int)len - na;
+    for (int t = tid; t < (int)len; t += kSortThreads) {
+        sk[merge_at(t)] = t < na ? A[a0 + t] : B[b0 + t - na];
+        sv[merge_at(t)] = t < na ? Av[a0 + t] : Bv[b0 + t - na];
+    }
+    __syncthreads();
+    const int diag = min(kMergePer * tid, (int)len);
+    unsigned long long key[kMergePer];
+    int val[kMergePer];
+    merge_part(sk, sv, 0, na, na, nb, diag, key, val);
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kMergePer; ++r)
+        if (diag + r < (int)len) { sk[merge_at(diag + r)] = key[r]; sv[merge_at(diag + r)] = val[r]; }
+    __syncthreads();
+    for (int t = tid; t < (int)len; t += kSortThreads) {
+        if (perm) {
+            perm[ch.x + t] = sv[merge_at(t)];
+        } else {
+            kout[ch.x + t] = sk[merge_at(t)];
+            vout[ch.x + t] = sv[merge_at(t)];
+        }
+    }
 }
 
 // Channel of every pole (offsets off[0..ns], off[ns] = n) and the identity order.
@@ -632,45 +703,6 @@ __global__ void __launch_bounds__(kHeapThreads) k_heap_order(const double *E, co
         if (loc >= n) loc = p;   // a permutation of the channel by construction
         pm[p] = (int)(gbase + loc);
     }
-}
-
-// Channels longer than kSortMax poles: a stable radix sort of the range by the energies'
-// integer images (k_sort.cu), then a stable one by channel, so each channel's poles end
-// in energy order and equal energies keep their build order.
-__global__ void k_pole_keys(const double *E, long long n0, long long n, bool desc, unsigned long long *key,
-                            unsigned *val) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    key[i] = sort_key(E[n0 + i], desc);
-    val[i] = (unsigned)(n0 + i);
-}
-__global__ void k_pole_chan(const unsigned *val, const int *seg_of, int ch_lo, long long n, unsigned long long *key) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    key[i] = (unsigned long long)(seg_of[val[i]] - ch_lo);
-}
-__global__ void k_perm_out(const unsigned *val, long long n0, long long n, int *perm) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    perm[n0 + i] = (int)val[i];
-}
-
-cudaError_t launch_pole_radix(const double *E, const int *seg_of, int ch_lo, int nseg, long long n0, long long n,
-                              bool desc, unsigned long long *k0, unsigned *v0, unsigned long long *k1, unsigned *v1,
-                              void *scratch, int *perm, int *launches, cudaStream_t st) {
-    const unsigned nb = (unsigned)((n + 255) / 256);
-    k_pole_keys<<<nb, 256, 0, st>>>(E, n0, n, desc, k0, v0);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    int p1 = 0, p2 = 0;
-    if ((e = radix_sort_pairs(k0, v0, k1, v1, n, 0, 64, false, scratch, &p1, st)) != cudaSuccess) return e;
-    k_pole_chan<<<nb, 256, 0, st>>>(v0, seg_of, ch_lo, n, k0);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    const int cbits = nseg <= 256 ? 8 : 16;
-    if ((e = radix_sort_pairs(k0, v0, k1, v1, n, 0, cbits, false, scratch, &p2, st)) != cudaSuccess) return e;
-    k_perm_out<<<nb, 256, 0, st>>>(v0, n0, n, perm);
-    if (launches) *launches += 3 + radix_launches(p1, false) + radix_launches(p2, false);
-    return cudaGetLastError();
 }
 
 // The next iteration's propagator on the device (bd_dressed_propagator): one warp per

@@ -1,7 +1,6 @@
 // k_sort.cu -- stable least-significant-digit radix sort of (64-bit key, 32-bit value)
-// pairs, eight bits per pass, used where a sort is longer than a CTA's shared memory:
-// channels of more than kSortMax poles (dressed propagators) and the interaction's
-// canonical keys (VppInt_t::prepare_for_reading, source/BcDor-Vpp_potential.cpp:440-501).
+// pairs, eight bits per pass, for the interaction's canonical keys
+// (VppInt_t::prepare_for_reading, source/BcDor-Vpp_potential.cpp:440-501).
 //
 // One pass over digit [shift, shift + 8):
 //   k_rs_hist     one CTA per tile of kRsTile pairs: the tile's 256 digit counts,
