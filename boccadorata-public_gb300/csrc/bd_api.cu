@@ -298,10 +298,9 @@ struct bd_ctx {
     float *d_Mfw_f = nullptr, *d_Mbk_f = nullptr;                                           // FP32 sorted M
     int *d_seg_fw = nullptr, *d_seg_bk = nullptr, *d_idx_fw = nullptr, *d_idx_bk = nullptr, *d_perm_fw = nullptr,
         *d_perm_bk = nullptr;
-    double *d_keys_tmp = nullptr;
     int *d_segoff_fw = nullptr, *d_segoff_bk = nullptr;
-    int4 *d_chunks_fw = nullptr, *d_chunks_bk = nullptr;   // chunk tables of the shared-memory sort
-    long long chunk_cap_fw = 0, chunk_cap_bk = 0;
+    int4 *d_chunks = nullptr;   // chunk table of the sort, forward then backward
+    long long chunk_cap = 0;
     int *d_sorti_fw = nullptr, *d_sorti_bk = nullptr;       // its sorted indices
     double *d_sighf = nullptr, *d_sig1b = nullptr;  // per channel D*D at chan_dd_off
     double *d_efermi = nullptr;   // per channel: the Fermi energy of the input propagator (Seek_EFermi)
@@ -860,59 +859,66 @@ int launch_ehf(bd_ctx *ctx, int ch_lo, int ch_hi, cudaStream_t st = nullptr) {
 // (the FP64 path) k_heap_order then puts equal energies in the order the reference's
 // heap sorts leave them (source/BcDor-Utilities.cpp:25-94).
 int launch_sort(bd_ctx *ctx, int ch_lo, int ch_hi, bool ref_order) {
+    const Chan &A = ctx->chans[ch_lo], &Z = ctx->chans[ch_hi - 1];
+    const int nseg = ch_hi - ch_lo;
+    SortSides S{};
+    std::vector<int4> chunks;
+    std::vector<int> rel[2];
+    int seg_max[2] = {0, 0};
     for (int dir = 0; dir < 2; ++dir) {
-        const Chan &A = ctx->chans[ch_lo], &Z = ctx->chans[ch_hi - 1];
-        const long long n0 = dir == 0 ? A.fw_off : A.bk_off;
-        const long long n = (dir == 0 ? Z.fw_off + Z.nfw : Z.bk_off + Z.nbk) - n0;
-        if (n <= 0) continue;
-        std::vector<int> rel(ch_hi - ch_lo + 1);
+        SortSide &D = S.s[dir];
+        D.n0 = dir == 0 ? A.fw_off : A.bk_off;
+        D.n = (dir == 0 ? Z.fw_off + Z.nfw : Z.bk_off + Z.nbk) - D.n0;
+        D.E = dir == 0 ? ctx->d_Efw : ctx->d_Ebk;
+        D.M = dir == 0 ? ctx->d_Mfw : ctx->d_Mbk;
+        D.Es = dir == 0 ? ctx->d_Efw_s : ctx->d_Ebk_s;
+        D.Ms = dir == 0 ? ctx->d_Mfw_s : ctx->d_Mbk_s;
+        D.Mf = dir == 0 ? ctx->d_Mfw_f : ctx->d_Mbk_f;
+        D.seg_of = dir == 0 ? ctx->d_seg_fw : ctx->d_seg_bk;
+        D.perm = dir == 0 ? ctx->d_perm_fw : ctx->d_perm_bk;
+        // the range's own part of the sorted copies (at least one coupling a pole)
+        const long long m0 = dir == 0 ? A.mfw_off : A.mbk_off;
+        D.k[0] = reinterpret_cast<unsigned long long *>(D.Ms + m0);
+        D.k[1] = reinterpret_cast<unsigned long long *>(D.Es + D.n0);
+        D.v[0] = dir == 0 ? ctx->d_sorti_fw : ctx->d_sorti_bk;
+        D.v[1] = reinterpret_cast<int *>(D.Mf + m0);
+        const size_t c = chunks.size();
+        rel[dir].resize(nseg + 1);
         for (int I = ch_lo; I < ch_hi; ++I)
-            rel[I - ch_lo] = (int)((dir == 0 ? ctx->chans[I].fw_off : ctx->chans[I].bk_off) - n0);
-        rel[ch_hi - ch_lo] = (int)n;
-        int *d_off = dir == 0 ? ctx->d_segoff_fw : ctx->d_segoff_bk;
-        if (int rc = h2d_table(ctx, d_off, rel.data(), sizeof(int) * rel.size())) return rc;
-        double *E = dir == 0 ? ctx->d_Efw : ctx->d_Ebk;
-        int *perm = dir == 0 ? ctx->d_perm_fw : ctx->d_perm_bk;
-        const int nseg = ch_hi - ch_lo;
-        int seg_max = 0;
-        for (int I = ch_lo; I < ch_hi; ++I) seg_max = std::max(seg_max, rel[I - ch_lo + 1] - rel[I - ch_lo]);
-        std::vector<int4> chunks;
-        for (int I = ch_lo; I < ch_hi; ++I) {
-            const int s0 = rel[I - ch_lo], sl = rel[I - ch_lo + 1] - s0;
+            rel[dir][I - ch_lo] = (int)((dir == 0 ? ctx->chans[I].fw_off : ctx->chans[I].bk_off) - D.n0);
+        rel[dir][nseg] = (int)D.n;
+        for (int I = 0; I < nseg; ++I) {
+            const int s0 = rel[dir][I], sl = rel[dir][I + 1] - s0;
+            seg_max[dir] = std::max(seg_max[dir], sl);
             for (int c0 = 0; c0 < sl; c0 += kSortChunk) chunks.push_back(make_int4(s0 + c0, std::min(kSortChunk, sl - c0), s0, sl));
         }
-        int4 *dch = dir == 0 ? ctx->d_chunks_fw : ctx->d_chunks_bk;
-        if ((long long)chunks.size() > (dir == 0 ? ctx->chunk_cap_fw : ctx->chunk_cap_bk))
-            return fail(ctx, BD_ERR_STATE, "sort chunk table overflow");
-        if (int rc = h2d_table(ctx, dch, chunks.data(), sizeof(int4) * chunks.size())) return rc;
-        // the passes' second buffers: the range's own sorted copies, which k_permute_soa writes last
-        unsigned long long *tk[2] = {reinterpret_cast<unsigned long long *>(ctx->d_keys_tmp),
-                                     reinterpret_cast<unsigned long long *>((dir == 0 ? ctx->d_Efw_s : ctx->d_Ebk_s) + n0)};
-        int *ti[2] = {dir == 0 ? ctx->d_sorti_fw : ctx->d_sorti_bk,
-                      reinterpret_cast<int *>(dir == 0 ? ctx->d_Mfw_f + A.mfw_off : ctx->d_Mbk_f + A.mbk_off)};
-        const unsigned nch = (unsigned)chunks.size();
-        k_chunk_sort<<<nch, kSortThreads, 0, ctx->st>>>(E + n0, dch, dir == 1, n0, tk[0], ti[0],
-                                                        seg_max <= kSortChunk ? perm + n0 : nullptr);
-        ctx->launches += 1;
-        int b = 0;
-        for (unsigned run = kSortChunk; run < (unsigned)seg_max; run *= 2, b ^= 1) {
-            const bool last = 2ull * run >= (unsigned)seg_max;
-            k_run_merge<<<nch, kSortThreads, 0, ctx->st>>>(tk[b], ti[b], dch, run, tk[b ^ 1], ti[b ^ 1],
-                                                            last ? perm + n0 : nullptr);
-            ctx->launches += 1;
-        }
-        CU(cudaGetLastError());
-        if (ref_order) {
-            CU(launch_heap_order(E, d_off, nseg, seg_max, n0, perm, ctx->st));
-            ctx->launches += 1;
-        }
-        k_permute_soa<<<(unsigned)((n + 255) / 256), 256, 0, ctx->st>>>(
-            perm, n0, n, dir == 0 ? ctx->d_seg_fw : ctx->d_seg_bk, ctx->d_cs, dir, E, dir == 0 ? ctx->d_Mfw : ctx->d_Mbk,
-            dir == 0 ? ctx->d_Efw_s : ctx->d_Ebk_s, dir == 0 ? ctx->d_Mfw_s : ctx->d_Mbk_s,
-            dir == 0 ? ctx->d_Mfw_f : ctx->d_Mbk_f);
-        CU(cudaGetLastError());
+        D.nch = (int)(chunks.size() - c);
+    }
+    const long long n = S.s[0].n + S.s[1].n;
+    if (n <= 0) return BD_OK;
+    if ((long long)chunks.size() > ctx->chunk_cap) return fail(ctx, BD_ERR_STATE, "sort chunk table overflow");
+    if (int rc = h2d_table(ctx, ctx->d_chunks, chunks.data(), sizeof(int4) * chunks.size())) return rc;
+    const unsigned nch = (unsigned)chunks.size(), longest = (unsigned)std::max(seg_max[0], seg_max[1]);
+    k_chunk_sort<<<nch, kSortThreads, 0, ctx->st>>>(S, ctx->d_chunks, longest <= kSortChunk);
+    ctx->launches += 1;
+    int in = 0;
+    for (unsigned run = kSortChunk; run < longest; run *= 2, in ^= 1) {
+        k_run_merge<<<nch, kSortThreads, 0, ctx->st>>>(S, ctx->d_chunks, run, in, 2ull * run >= longest);
         ctx->launches += 1;
     }
+    CU(cudaGetLastError());
+    if (ref_order)
+        for (int dir = 0; dir < 2; ++dir) {
+            const SortSide &D = S.s[dir];
+            if (D.n <= 0) continue;
+            int *d_off = dir == 0 ? ctx->d_segoff_fw : ctx->d_segoff_bk;
+            if (int rc = h2d_table(ctx, d_off, rel[dir].data(), sizeof(int) * rel[dir].size())) return rc;
+            CU(launch_heap_order(D.E, d_off, nseg, seg_max[dir], D.n0, D.perm, ctx->st));
+            ctx->launches += 1;
+        }
+    k_permute_soa<<<(unsigned)((n + 255) / 256), 256, 0, ctx->st>>>(S, ctx->d_cs);
+    CU(cudaGetLastError());
+    ctx->launches += 1;
     return BD_OK;
 }
 
@@ -1621,15 +1627,12 @@ int upload_propagator(bd_ctx *ctx, const bd_propagator *prop) {
         CU(cudaGetLastError());
         ctx->launches += 1;
     }
-    ctx->chunk_cap_fw = ctx->tot_fw / kSortChunk + ns + 1;
-    ctx->chunk_cap_bk = ctx->tot_bk / kSortChunk + ns + 1;
-    if ((rc = dalloc(ctx, &ctx->d_chunks_fw, (size_t)ctx->chunk_cap_fw))) return rc;
-    if ((rc = dalloc(ctx, &ctx->d_chunks_bk, (size_t)ctx->chunk_cap_bk))) return rc;
+    ctx->chunk_cap = ctx->tot_fw / kSortChunk + ctx->tot_bk / kSortChunk + 2 * ns + 2;
+    if ((rc = dalloc(ctx, &ctx->d_chunks, (size_t)ctx->chunk_cap))) return rc;
     if ((rc = dalloc(ctx, &ctx->d_sorti_fw, ctx->tot_fw))) return rc;
     if ((rc = dalloc(ctx, &ctx->d_sorti_bk, ctx->tot_bk))) return rc;
     if ((rc = dalloc(ctx, &ctx->d_perm_fw, ctx->tot_fw))) return rc;
     if ((rc = dalloc(ctx, &ctx->d_perm_bk, ctx->tot_bk))) return rc;
-    if ((rc = dalloc(ctx, &ctx->d_keys_tmp, std::max(ctx->tot_fw, ctx->tot_bk)))) return rc;
     if ((rc = dalloc(ctx, &ctx->d_vp, ctx->tot_vp))) return rc;
     if ((rc = dalloc(ctx, &ctx->d_Efw, ctx->tot_fw))) return rc;
     if ((rc = dalloc(ctx, &ctx->d_S2fw, ctx->tot_fw))) return rc;

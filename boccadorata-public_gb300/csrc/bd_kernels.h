@@ -22,8 +22,6 @@ __global__ void k_ehf_terms(DevProblem P, const int3 *entries, const long long *
 __global__ void k_ehf_sum(DevProblem P, const int3 *entries, const long long *term_first, int e0, const int *ctab_cmb,
                           const int *ctab_toff, const int *ctab_off, const int *ncomb, const double *terms,
                           const long long *out_off, double *out);
-__global__ void k_permute_soa(const int *perm, long long n0, long long n, const int *seg_of, const ChanSig *cs, int dir,
-                              const double *Ein, const double *Min, double *Eout, double *Mout, float *Mfout);
 __global__ void k_rows_aos(const double *E, const double *S2, const double *M, int N, int D, double *rows);
 __global__ void k_rows_aos_perm(const int *perm, long long off, const double *E, const double *S2, const double *M,
                                 int N, int D, double *rows);
@@ -38,10 +36,24 @@ cudaError_t launch_poles_tc(const DevProblem &P, const S2Block *blk, const int *
                             int dirs, int *err, size_t smem, cudaStream_t st);
 constexpr int kSortThreads = 256;
 constexpr int kSortChunk = 2048;  // poles per chunk of the shared-memory sort
-__global__ void k_chunk_sort(const double *E, const int4 *chunks, bool desc, long long base, unsigned long long *tk,
-                             int *ti, int *perm);
-__global__ void k_run_merge(const unsigned long long *kin, const int *vin, const int4 *chunks, unsigned run,
-                            unsigned long long *kout, int *vout, int *perm);
+// A direction's poles [n0, n0 + n) of a range of channels, sorted by k_chunk_sort and k_run_merge
+// into perm and gathered by k_permute_soa.  k, v: two buffers of n pairs each, the output copies'
+// memory among them (k_permute_soa writes those last).
+struct SortSide {
+    const double *E, *M;          // the direction's poles
+    double *Es, *Ms;              // sorted copies
+    float *Mf;
+    const int *seg_of;            // channel of a pole
+    int *perm;
+    unsigned long long *k[2];
+    int *v[2];
+    long long n0, n;
+    int nch;                      // its chunks; the second direction's follow the first's in the table
+};
+struct SortSides { SortSide s[2]; };   // forward (ascending), backward (descending)
+__global__ void k_chunk_sort(SortSides S, const int4 *chunks, bool only);
+__global__ void k_run_merge(SortSides S, const int4 *chunks, unsigned run, int in, bool last);
+__global__ void k_permute_soa(SortSides S, const ChanSig *cs);
 // Stable LSD radix sort of (key, value) pairs over key bits [bit0, bit1), eight per pass
 // (k_sort.cu).  keys / vals and ktmp / vtmp are ping-pong buffers of n entries: on
 // return keys / vals point at the sorted pairs.  scratch: radix_scratch_bytes(n).

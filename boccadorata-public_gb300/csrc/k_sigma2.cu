@@ -381,15 +381,17 @@ __device__ __forceinline__ void merge_part(const unsigned long long *sk, const i
     }
 }
 
-__global__ void __launch_bounds__(kSortThreads) k_chunk_sort(const double *E, const int4 *chunks, bool desc,
-                                                             long long base, unsigned long long *tk, int *ti, int *perm) {
+__global__ void __launch_bounds__(kSortThreads) k_chunk_sort(SortSides S, const int4 *chunks, bool only) {
     const int4 ch = chunks[blockIdx.x];   // first pole, length, channel's first pole, channel's length
+    const bool desc = (int)blockIdx.x >= S.s[0].nch;
+    const SortSide &D = S.s[desc];
+    const double *E = D.E + D.n0;
     __shared__ unsigned long long sk[kMergeRoom];
     __shared__ int sv[kMergeRoom];
     const int n = ch.y, n8 = (n + kMergePer - 1) / kMergePer * kMergePer, tid = threadIdx.x, diag = kMergePer * tid;
     for (int t = tid; t < n8; t += kSortThreads) {   // past the end the largest key, after all equal ones
         sk[merge_at(t)] = t < n ? sort_key(E[ch.x + t], desc) : ~0ull;
-        sv[merge_at(t)] = t < n ? (int)(base + ch.x + t) : INT_MAX;
+        sv[merge_at(t)] = t < n ? (int)(D.n0 + ch.x + t) : INT_MAX;
     }
     __syncthreads();
     unsigned long long key[kMergePer];
@@ -422,17 +424,19 @@ __global__ void __launch_bounds__(kSortThreads) k_chunk_sort(const double *E, co
     }
     __syncthreads();
     for (int t = tid; t < n; t += kSortThreads) {
-        if (perm) { perm[ch.x + t] = sv[merge_at(t)]; continue; }   // no channel longer than a chunk
-        tk[ch.x + t] = sk[merge_at(t)];
-        ti[ch.x + t] = sv[merge_at(t)];
+        if (only) { D.perm[D.n0 + ch.x + t] = sv[merge_at(t)]; continue; }   // no channel longer than a chunk
+        D.k[0][ch.x + t] = sk[merge_at(t)];
+        D.v[0][ch.x + t] = sv[merge_at(t)];
     }
 }
 
 // Outputs [c0, c0 + len) of the channel are the chunk's place in it; they lie in one pair of runs.
-__global__ void __launch_bounds__(kSortThreads) k_run_merge(const unsigned long long *kin, const int *vin,
-                                                             const int4 *chunks, unsigned run, unsigned long long *kout,
-                                                             int *vout, int *perm) {
+__global__ void __launch_bounds__(kSortThreads) k_run_merge(SortSides S, const int4 *chunks, unsigned run,
+                                                            int in, bool last) {
     const int4 ch = chunks[blockIdx.x];
+    const SortSide &D = S.s[(int)blockIdx.x >= S.s[0].nch];
+    const unsigned long long *kin = D.k[in];
+    const int *vin = D.v[in];
     __shared__ unsigned long long sk[kMergeRoom];
     __shared__ int sv[kMergeRoom], s_a[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -471,11 +475,11 @@ __global__ void __launch_bounds__(kSortThreads) k_run_merge(const unsigned long 
         if (diag + r < (int)len) { sk[merge_at(diag + r)] = key[r]; sv[merge_at(diag + r)] = val[r]; }
     __syncthreads();
     for (int t = tid; t < (int)len; t += kSortThreads) {
-        if (perm) {
-            perm[ch.x + t] = sv[merge_at(t)];
+        if (last) {
+            D.perm[D.n0 + ch.x + t] = sv[merge_at(t)];
         } else {
-            kout[ch.x + t] = sk[merge_at(t)];
-            vout[ch.x + t] = sv[merge_at(t)];
+            D.k[in ^ 1][ch.x + t] = sk[merge_at(t)];
+            D.v[in ^ 1][ch.x + t] = sv[merge_at(t)];
         }
     }
 }
@@ -492,12 +496,18 @@ __global__ void k_pole_index(const int *off, int ns, long long n, int *seg, int 
 
 // Gather rows in a given order into separate SoA arrays (used after the sort), plus an
 // FP32 copy of the couplings for the FP32-vector Lanczos form.
-__global__ void k_permute_soa(const int *perm, long long n0, long long n, const int *seg_of, const ChanSig *cs, int dir,
-                              const double *Ein, const double *Min, double *Eout, double *Mout, float *Mfout) {
-    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (idx >= n) return;
-    const long long g = n0 + idx;
-    const int ch = seg_of[g];
+__global__ void k_permute_soa(SortSides S, const ChanSig *cs) {
+    long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const int dir = idx >= S.s[0].n;
+    const SortSide &T = S.s[dir];
+    if (dir) idx -= S.s[0].n;
+    if (idx >= T.n) return;
+    const double *Ein = T.E, *Min = T.M;
+    double *Eout = T.Es, *Mout = T.Ms;
+    float *Mfout = T.Mf;
+    const int *perm = T.perm;
+    const long long g = T.n0 + idx;
+    const int ch = T.seg_of[g];
     const ChanSig C = cs[ch];
     const long long off = dir == 0 ? C.fw_off : C.bk_off;
     const long long moff = dir == 0 ? C.mfw_off : C.mbk_off;
