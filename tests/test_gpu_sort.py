@@ -115,3 +115,35 @@ def test_sorted_rows_need_a_reduction(bdmod, problems):
         ctx.sigma2_sorted(0)
     assert e.value.code == bdmod.BD_ERR_STATE
     ctx.close()
+
+
+@pytest.mark.parametrize("n_max,dressed", [(4, False), (8, False), (6, True)])
+def test_stable_order_every_channel(bdmod, problems, n_max, dressed):
+    """Channels from a few poles to many chunks of the sort, ragged last chunks, equal and
+    distinct energies, both directions: the first vector of every chain visits the poles in
+    numpy's stable order."""
+    p = problems(n_max, 20.0, 0, 12)
+    ctx = bdmod.Context().upload(p)
+    ctx.run_all(lanczos=True)
+    if dressed:
+        ctx.dressed_propagator(1e-2, 2)
+        ctx.run_all(lanczos=True)
+    pv = p.piv
+    lengths = set()
+    for ish in range(p.ms.nsubsh):
+        rows = ctx.sigma2_build(ish)
+        lz = ctx.lanczos_reduce(ish, pv.vec[ish].copy(), pv.n_fw[ish], pv.n_bk[ish])
+        for d, tag in ((0, "fw"), (1, "bk")):
+            used = np.nonzero(lz["nitr_" + tag] > 0)[0]
+            if not len(rows[d]) or not len(used):
+                continue
+            key = rows[d][:, 0]
+            order = np.argsort(-key if d else key, kind="stable")
+            v0 = rows[d][order, 2:] @ lz["pivots"][int(used[0])]
+            v0 /= np.linalg.norm(v0)
+            V = ctx.lanczos_vectors(ish, d, len(lz["lz_" + tag]), len(key))
+            # couplings and pivots of order one in FP64; the sums behind |M p| have 1e5 terms at most
+            assert np.abs(V[0] - v0).max() < 1e-12, (ish, d, len(key))
+            lengths.add(len(key))
+    assert len(lengths) > 3
+    ctx.close()
