@@ -223,6 +223,12 @@ template <> __device__ inline void load16g<double>(const double *p, double *o) {
 // The reads of those vectors then cost shared-memory latency instead of L2's.  V keeps
 // every vector (the host reads the basis back from it).
 //
+// Loads: a step is a few passes over slices in L2, each a thread's one to three groups, so
+// what a pass costs is the loads' latency times how often it waits: all loads of a group (the
+// recurrence's vectors, the last vectors of a sum) are issued before the first is used, two
+// groups at a time where registers allow, the sums in the same order.  (FP32 vectors, chains
+// of up to 15 000 poles and 54 vectors, N_max=10: 0.92 -> 0.82 ms.)
+//
 // Arithmetic: with FP64 vectors everything is FP64.  With FP32 vectors every
 // per-pole operation (products, the update, the per-thread partial sums of the dot
 // products, norms and scalars) is FP32, and only the sums across warps and CTAs are
@@ -244,7 +250,10 @@ __global__ void __launch_bounds__(kLzThreads, 2) k_lanczos(const LzChain *chains
     const int rank = (int)cluster.block_rank();
     const int cid = blockIdx.x / CL;
     if (cid >= nchains) return;  // whole clusters only: every CTA of a cluster has the same cid
-    const LzChain C = chains[cid];
+    __shared__ LzChain C;   // the slices leave L1 little room: members read again would come from L2
+    if (threadIdx.x < sizeof(LzChain) / 4)
+        reinterpret_cast<int *>(&C)[threadIdx.x] = reinterpret_cast<const int *>(chains + cid)[threadIdx.x];
+    __syncthreads();
     if (sizeof(VT) == 8 && C.done && *C.done) return;   // done by k_lz_compact or k_lz_long (the whole cluster leaves)
     const int N = C.N, D = C.D, L = C.L, NT = C.nden_out + C.D;
     const int S = C.S;                       // multiple of 4
@@ -502,31 +511,50 @@ __global__ void __launch_bounds__(kLzThreads, 2) k_lanczos(const LzChain *chains
             PA acc[2 * NU];
 #pragma unroll
             for (int u = 0; u < 2 * NU; ++u) acc[u] = PS::zero();
-#pragma unroll UNR
-            for (int q = lane; q < nv; q += 32) {
-                VT wq[VW], eq[VW];
-                load16g<VT>(wv + q * VW, wq);
-                load16g<VT>(ev + q * VW, eq);
-                VT x[NU][VW];   // all loads first (items beyond the pass read E w: valid, unused)
+            auto step = [&](int u, const VT *x, const VT *wq, const VT *eq) {
+                if constexpr (kComp) {
+                    CT g = (CT)0, h = (CT)0;
 #pragma unroll
-                for (int u = 0; u < NU; ++u) load16g<VT>(vp[u] + q * VW, x[u]);
+                    for (int e = 0; e < VW; ++e) { g += x[e] * wq[e]; h += x[e] * eq[e]; }
+                    PS::add(acc[u], g);
+                    PS::add(acc[NU + u], h);
+                } else {
 #pragma unroll
-                for (int u = 0; u < NU; ++u)
-                    if (u < nu) {
-                        if constexpr (kComp) {
-                            CT g = (CT)0, h = (CT)0;
-#pragma unroll
-                            for (int e = 0; e < VW; ++e) { g += x[u][e] * wq[e]; h += x[u][e] * eq[e]; }
-                            PS::add(acc[u], g);
-                            PS::add(acc[NU + u], h);
-                        } else {
-#pragma unroll
-                            for (int e = 0; e < VW; ++e) {
-                                acc[u] += x[u][e] * wq[e];
-                                acc[NU + u] += x[u][e] * eq[e];
-                            }
-                        }
+                    for (int e = 0; e < VW; ++e) {
+                        acc[u] += x[e] * wq[e];
+                        acc[NU + u] += x[e] * eq[e];
                     }
+                }
+            };
+            if (NU == 8 && nu <= 4) {   // few vectors: two groups of each in flight
+                for (int q = lane; q < nv; q += 64) {
+                    const int q2 = min(q + 32, nv - 1);
+                    VT x[4][VW], y[4][VW], wq[VW], eq[VW];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) { load16g<VT>(vp[u] + q * VW, x[u]); load16g<VT>(vp[u] + q2 * VW, y[u]); }
+                    load16g<VT>(wv + q * VW, wq);
+                    load16g<VT>(ev + q * VW, eq);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) if (u < nu) step(u, x[u], wq, eq);
+                    if (q + 32 < nv) {
+                        load16g<VT>(wv + q2 * VW, wq);
+                        load16g<VT>(ev + q2 * VW, eq);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) if (u < nu) step(u, y[u], wq, eq);
+                    }
+                }
+            } else {
+#pragma unroll UNR
+                for (int q = lane; q < nv; q += 32) {
+                    VT wq[VW], eq[VW];
+                    load16g<VT>(wv + q * VW, wq);
+                    load16g<VT>(ev + q * VW, eq);
+                    VT x[NU][VW];   // all loads first (items beyond the pass read E w: valid, unused)
+#pragma unroll
+                    for (int u = 0; u < NU; ++u) load16g<VT>(vp[u] + q * VW, x[u]);
+#pragma unroll
+                    for (int u = 0; u < NU; ++u) if (u < nu) step(u, x[u], wq, eq);
+                }
             }
             const PA r = warp_sums<2 * NU>(acc, lane);
             const int vi = lane >> LS2, u = vi % NU, kind = vi / NU;
@@ -672,22 +700,34 @@ __global__ void __launch_bounds__(kLzThreads, 2) k_lanczos(const LzChain *chains
                 for (int u = 0; u < VW; ++u) acc[u] += cr * x[r][u];
             }
         }
-        for (; t + 3 < nl; t += 4) {
-            VT x0[VW], x1[VW], x2[VW], x3[VW];
-            load16g<VT>(vslice(loc ? lt[t] : t) + qo, x0);
-            load16g<VT>(vslice(loc ? lt[t + 1] : t + 1) + qo, x1);
-            load16g<VT>(vslice(loc ? lt[t + 2] : t + 2) + qo, x2);
-            load16g<VT>(vslice(loc ? lt[t + 3] : t + 3) + qo, x3);
-            const CT c0 = cf[t], c1 = cf[t + 1], c2 = cf[t + 2], c3 = cf[t + 3];
+        const int rem = nl - t;   // the last ones' loads together too
+        if (rem > 0) {
+            VT x[7][VW];
 #pragma unroll
-            for (int u = 0; u < VW; ++u) acc[u] += c0 * x0[u] + c1 * x1[u] + c2 * x2[u] + c3 * x3[u];
-        }
-        for (; t < nl; ++t) {
-            VT x0[VW];
-            load16g<VT>(vslice(loc ? lt[t] : t) + qo, x0);
-            const CT c0 = cf[t];
+            for (int r = 0; r < 7; ++r) {
+                const int tt = min(t + r, nl - 1);
+                load16g<VT>(vslice(loc ? lt[tt] : tt) + qo, x[r]);
+            }
+            if (rem >= 4) {
+                const CT c0 = cf[t], c1 = cf[t + 1], c2 = cf[t + 2], c3 = cf[t + 3];
 #pragma unroll
-            for (int u = 0; u < VW; ++u) acc[u] += c0 * x0[u];
+                for (int u = 0; u < VW; ++u) acc[u] += c0 * x[0][u] + c1 * x[1][u] + c2 * x[2][u] + c3 * x[3][u];
+#pragma unroll
+                for (int r = 4; r < 7; ++r)
+                    if (r < rem) {
+                        const CT cr = cf[t + r];
+#pragma unroll
+                        for (int u = 0; u < VW; ++u) acc[u] += cr * x[r][u];
+                    }
+            } else {
+#pragma unroll
+                for (int r = 0; r < 3; ++r)
+                    if (r < rem) {
+                        const CT cr = cf[t + r];
+#pragma unroll
+                        for (int u = 0; u < VW; ++u) acc[u] += cr * x[r][u];
+                    }
+            }
         }
     };
     auto update_pass = [&](bool loc, int nl) {
@@ -732,14 +772,24 @@ __global__ void __launch_bounds__(kLzThreads, 2) k_lanczos(const LzChain *chains
                         const CT e = Es[i];
                         PS::add(sa, e * wi * wi);
                         PS::add(se, e * e * wi * wi);
+                        if (!Msl)
 #pragma unroll
-                        for (int d = 0; d < 8; ++d)
-                            if (d < D) PS::add(sm_[d], (Msl ? Msl[d * S + i] : Mc[(size_t)d * N + i0 + i]) * wi);
+                            for (int d = 0; d < 8; ++d)
+                                if (d < D) PS::add(sm_[d], Mc[(size_t)d * N + i0 + i] * wi);
 #pragma unroll
                         for (int g = 0; g < 8; ++g)
                             if (lok[g]) PS::add(sg[g], e * (CT)(g < 4 ? lv[g & 3][u] : vslice(lslot[g])[i]) * wi);
                     }
                 }
+                if (Msl)   // (zero past the end of the slice, as w is)
+#pragma unroll
+                    for (int d = 0; d < 8; ++d)
+                        if (d < D) {
+                            CT m[VW];
+                            load16g<CT>(Msl + (size_t)d * S + qo, m);
+#pragma unroll
+                            for (int u = 0; u < VW; ++u) PS::add(sm_[d], m[u] * w[qo + u]);
+                        }
             }
         }
         // the 19 sums of the warp at once (values 0 |w|^2, 1 alpha, 2 |E w|^2, 3 + d m_d,
@@ -825,9 +875,14 @@ __global__ void __launch_bounds__(kLzThreads, 2) k_lanczos(const LzChain *chains
         if (newv) {
             const double *p = C.piv + (size_t)k * D;
             for (int i = tid; i < S; i += kLzThreads) {
-                double s = 0.0;
-                if (i < ns)
-                    for (int d = 0; d < D; ++d) s = __dadd_rn(s, __dmul_rn(C.M[(size_t)d * N + i0 + i], p[d]));
+                double s = 0.0, m[8];
+                if (i < ns) {
+#pragma unroll
+                    for (int d = 0; d < 8; ++d) m[d] = d < D ? C.M[(size_t)d * N + i0 + i] : 0.0;
+#pragma unroll
+                    for (int d = 0; d < 8; ++d)
+                        if (d < D) s = __dadd_rn(s, __dmul_rn(m[d], p[d]));
+                }
                 w[i] = (CT)s;
             }
         } else if (rec) {
@@ -835,26 +890,44 @@ __global__ void __launch_bounds__(kLzThreads, 2) k_lanczos(const LzChain *chains
             // (lt, lcf, s_nl), listed by warp 0 when it wrote row j - 1
             const int nl0 = s_nl;
             const VT *vp0 = vslice(lt[0]);
-            for (int q = tid; q < nv; q += kLzThreads) {
-                const int qo = q * VW;
-                VT x0[VW];
-                load16g<VT>(vp0 + qo, x0);
-                CT x[VW];
+            for (int q = tid; q < nv; q += 2 * kLzThreads) {   // two groups a thread, loads first
+                const bool two = q + kLzThreads < nv;
+                const int qo[2] = {q * VW, (two ? q + kLzThreads : q) * VW};
+                CT x[2][VW];
 #pragma unroll
-                for (int u = 0; u < VW; ++u) x[u] = (CT)x0[u] * Es[qo + u];
-#pragma unroll 4
-                for (int t = 0; t < nl0; ++t) {
-                    VT y[VW];
-                    load16g<VT>(vslice(lt[t]) + qo, y);
-                    const CT ct = lcf[t];
+                for (int h = 0; h < 2; ++h) {
+                    VT x0[VW];
+                    load16g<VT>(vp0 + qo[h], x0);
 #pragma unroll
-                    for (int u = 0; u < VW; ++u) x[u] -= ct * (CT)y[u];
+                    for (int u = 0; u < VW; ++u) x[h][u] = (CT)x0[u] * Es[qo[h] + u];
+                }
+                for (int t0 = 0; t0 < nl0; t0 += 4) {   // and four vectors' loads together
+                    VT y[4][2][VW];
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const VT *v = vslice(lt[min(t0 + r, nl0 - 1)]);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) load16g<VT>(v + qo[h], y[r][h]);
+                    }
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        if (t0 + r < nl0) {
+                            const CT ct = lcf[t0 + r];
+#pragma unroll
+                            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                                for (int u = 0; u < VW; ++u) x[h][u] -= ct * (CT)y[r][h][u];
+                        }
                 }
 #pragma unroll
-                for (int u = 0; u < VW; ++u) {
-                    w[qo + u] = x[u];
-                    if constexpr (kFused) ew[qo + u] = Es[qo + u] * x[u];
-                }
+                for (int h = 0; h < 2; ++h)
+                    if (h == 0 || two) {
+#pragma unroll
+                        for (int u = 0; u < VW; ++u) {
+                            w[qo[h] + u] = x[h][u];
+                            if constexpr (kFused) ew[qo[h] + u] = Es[qo[h] + u] * x[h][u];
+                        }
+                    }
             }
         } else {
             const VT *vp = vslice(rowslot[j - 1]);
@@ -1093,17 +1166,18 @@ __global__ void __launch_bounds__(kLzThreads, 2) k_lanczos(const LzChain *chains
         if (warp == 0) {
             __syncwarp();
             const bool next_newv = (k + 1 < C.n_used) && (j + 1 == s_start[k + 1]);
-            if (tid == 0 && !injected && !next_newv) {
-                auto pr = [&](int q) -> CT { if constexpr (kFused) return prowf[q]; else return (CT)prow[q]; };
-                int n = 0;
-                lt[n] = nvec; lcf[n++] = pr(0);
-                if (j >= 1 && rowslot[j - 1] >= 0) { lt[n] = rowslot[j - 1]; lcf[n++] = pr(1); }
-                for (int q = 0; q < k; ++q)
-                    if (s_last[q] < j - 1 && rowslot[s_last[q]] >= 0) {
-                        lt[n] = rowslot[s_last[q]];
-                        lcf[n++] = pr(2 + q);
-                    }
-                s_nl = n;
+            if (!injected && !next_newv) {   // lane 0: v_j, lane 1: v_{j-1}, lane 2 + q: chain q's last
+                int v = -1;
+                if (lane == 0) v = nvec;
+                else if (lane == 1) v = j >= 1 ? rowslot[j - 1] : -1;
+                else if (lane < 2 + k) v = s_last[lane - 2] < j - 1 ? rowslot[s_last[lane - 2]] : -1;
+                const unsigned m = __ballot_sync(0xffffffffu, v >= 0);
+                if (v >= 0) {
+                    const int n = __popc(m & ((1u << lane) - 1u));
+                    lt[n] = v;
+                    if constexpr (kFused) lcf[n] = prowf[lane]; else lcf[n] = (CT)prow[lane];
+                }
+                if (lane == 0) s_nl = __popc(m);
             }
         }
         prow_ok = !injected;
