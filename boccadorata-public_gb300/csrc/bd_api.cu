@@ -1190,7 +1190,7 @@ int launch_dyson_range(bd_ctx *ctx, int ch_lo, int ch_hi, bool lanczos) {
         return rct;
     CU(launch_dyson(ctx->d_jobs + ch_lo, (int)jobs.size(), ctx->d_row_first + ch_lo, rows, nmax, Dmax,
                     dy_cluster_for(ctx, ch_hi - ch_lo), ctx->d_dywork, ctx->d_work_first + ch_lo, ctx->st));
-    ctx->launches += dyson_launch_count(nmax, Dmax, dy_cluster_for(ctx, ch_hi - ch_lo));
+    ctx->launches += dyson_launch_count((int)jobs.size(), nmax, Dmax, dy_cluster_for(ctx, ch_hi - ch_lo));
     return BD_OK;
 }
 
@@ -2046,6 +2046,7 @@ static int dyson_status_error(bd_ctx *ctx, int ish, int st) {
     if (st == kDyStatCapacity)
         return fail(ctx, BD_ERR_CAPACITY,
                     "channel %d: the deflated Dyson matrix is larger than the cluster reduction's shared memory holds", ish);
+    if (st == kDyStatBarrier) return fail(ctx, BD_ERR_CUDA, "channel %d: a barrier of the Householder reduction ran out", ish);
     return fail(ctx, BD_ERR_NUMERIC, "channel %d: the eigensolver did not converge", ish);
 }
 
@@ -2155,7 +2156,7 @@ int bd_dyson_rows(bd_ctx *ctx, int ish, int nden, int n_fw, const double *fw_row
     CU(cudaMemcpyAsync(dwf, zero, sizeof zero, cudaMemcpyHostToDevice, ctx->st));
     CU(cudaMemcpyAsync(drf, zero, sizeof zero, cudaMemcpyHostToDevice, ctx->st));
     CU(launch_dyson(dj, 1, drf, n, n, D, dy_cluster_for(ctx, 1), dwork, dwf, ctx->st));
-    ctx->launches += dyson_launch_count(n, D, dy_cluster_for(ctx, 1));
+    ctx->launches += dyson_launch_count(1, n, D, dy_cluster_for(ctx, 1));
     int nq[2] = {0, 0}, dst = 0;
     double kol[3];
     CU(cudaMemcpyAsync(nq, ctx->d_dynq + 2 * ish, sizeof nq, cudaMemcpyDeviceToHost, ctx->st));

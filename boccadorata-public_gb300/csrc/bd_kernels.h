@@ -111,7 +111,7 @@ cudaError_t launch_lanczos_long(const LzChain *d_chains, int nchains, int rmax, 
                                 cudaStream_t st);
 void lanczos_long_smem_init();
 
-int dyson_launch_count(int nmax, int Dmax, int cluster);
+int dyson_launch_count(int njobs, int nmax, int Dmax, int cluster);
 cudaError_t launch_dyson(const DyJob *d_jobs, int njobs, const long long *d_row_first, long long total_rows,
                          int nmax, int Dmax, int cluster, double *work, const long long *d_work_first, cudaStream_t st);
 // nmax bounds the orders; those beyond nlim come from k_tridiag (reflectors in A), whose first
@@ -129,6 +129,6 @@ void sigma2_smem_init();
 void lanczos_smem_init();
 // DyJob::stat values: the eigensolver did not converge; the deflated matrix is larger
 // than the cluster reduction's shared-memory layout holds (nothing solved)
-constexpr int kDyStatNumeric = 1, kDyStatCapacity = 2;
+constexpr int kDyStatNumeric = 1, kDyStatCapacity = 2, kDyStatBarrier = 3;
 
 }  // namespace bd

@@ -9,6 +9,7 @@
 //                         <= 160 in one CTA's shared memory, with the first D rows of Q,
 //       k_tridiag_df      the same for larger orders, one thread-block cluster per
 //                         matrix (rows split across the CTAs),
+//       k_tridiag_grid    the same for one large matrix alone, a CTA on every SM,
 //       k_tridiag         in FP64 for orders beyond that kernel's shared memory (Q's rows
 //                         by k_qrows),
 //   K4b..K5 (k_eig.cu)    eigenvalues and the first D eigenvector components of T,
@@ -89,6 +90,16 @@ __device__ inline void dy_mark_branch_starts(const DyJob &J, int r, int *flag) {
     }
 }
 
+constexpr int kTdgMax = 256;   // CTAs of k_tridiag_grid at most
+// Its smallest order: a column costs it 5.3 us at any order below 700, the cluster kernel's 16 CTAs
+// less up to orders of 500 (a solve of 300: 2.6 against 2.2 ms, 500: 4.1 and 4.1, 600: 4.9 and 5.3)
+constexpr int kTdgMin = 512;
+// the exchange area in a job's work space (5 n^2 doubles, the spilled rows in the first n^2):
+// y[2][n], row k+1 [2][n], parts of v^T A v [2][kTdgMax], the barrier's count (zeroed by
+// k_dyson_deflate)
+__host__ __device__ inline size_t tdg_exchange(int n) { return 4 * (size_t)n * n; }
+__host__ __device__ inline size_t tdg_count(int n) { return tdg_exchange(n) + 4 * (size_t)n + 2 * kTdgMax; }
+
 // One CTA per matrix: the compact index of every kept row (work area, ints; -1 for a
 // deflated row), the compact order into the job, and the deflated rows' solutions
 // [W, 0, 0 ..] staged behind R after the nc rows the eigensolver will stage.
@@ -103,7 +114,11 @@ __global__ void __launch_bounds__(kDfThreads) k_dyson_deflate(DyJob *jobs, int n
     int *map = reinterpret_cast<int *>(work + work_first[jid]);
     __shared__ int wsum[kDfThreads / 32][2];
     __shared__ int s_keep, s_defl;
-    if (tid == 0) { s_keep = 0; s_defl = 0; }
+    if (tid == 0) {
+        s_keep = 0;
+        s_defl = 0;
+        if (n > kTsMax) *reinterpret_cast<unsigned *>(work + work_first[jid] + tdg_count(n)) = 0u;   // k_tridiag_grid's
+    }
     __syncthreads();
     double *st = J.R + (size_t)D * n;
     int nkept_total = 0;
@@ -679,6 +694,240 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_df(const DyJob *jobs
         for (int j = tid; j < n; j += kTdfThreads) J.R[(size_t)(rank + u * CL) * n + j] = dfm::to_double(R[(size_t)u * n + j]);
 }
 
+// ---------------------------------------------------------------- K4a''' one matrix, the whole GPU
+// A matrix reduced alone leaves a cluster's 16 SMs to do the pass and most of its rows in L2 (order
+// 1 000: 25 000 cycles a column, two thirds of them the pass).  Here every SM takes rows: a
+// cooperative launch, one CTA an SM, row i with CTA (i mod G), and what the CTAs exchange goes
+// through L2.  Step k, with one grid barrier:
+//   pass      as k_tridiag_df's, 1 to 4 warps a row
+//   own rows  y_i = a_i,k+1 + s S_i and the CTA's part of v^T A v; from its owner row k+1; barrier
+//   all rows  v, w, R; from row k+1, which is column k+1, that column after this step's update (x
+//             of the next step, d_{k+1} on the diagonal), and the sum of its squares, by every CTA
+//             for itself
+// Bound by the barrier and what surrounds it in a column (order 1 000, 11 000 cycles: the pass beside
+// the scalars' chain 3 000, y 1 000, the barrier 3 200, L2 and the sum of the parts 2 700, v and w
+// 1 500).  Order 1 000: 12.8 ms by the cluster kernel -> 6.0.
+constexpr int kTdgRowWarps = kTdfWarps - 2;   // the others: R's product, the scalars
+constexpr int kTdgParts = 4;                  // warps a row at most
+constexpr int kTdgPolls = 1 << 20;            // a barrier's reads before it gives up (about a second)
+
+// 8-byte slots before the resident rows: V[2], W, one row of R, S by parts and a_{i,k+1} of own rows
+__host__ __device__ inline size_t tdg_fixed(int n, int G) {
+    return 4 * (size_t)n + (kTdgParts + 1) * (size_t)((n + G - 1) / G) + kTdfWarps + 16;
+}
+__global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_grid(const DyJob *jobs, int nlim, int smem_df, double *work,
+                                                                 const long long *work_first) {
+    using dfm::df;
+    __shared__ DyJob J;
+    __shared__ int s_ok;
+    const int G = gridDim.x, rank = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid < (int)(sizeof(DyJob) / 4)) reinterpret_cast<int *>(&J)[tid] = reinterpret_cast<const int *>(jobs)[tid];
+    if (tid == 0) s_ok = 1;
+    __syncthreads();
+    const int n = J.nc, D = J.D;
+    if (n < kTdgMin || n > nlim) return;   // another kernel's (the whole grid leaves)
+    const int nrm = (n + G - 1) / G, nr = rank < n ? (n - rank + G - 1) / G : 0;   // own rows i = rank + q G
+    extern __shared__ double sm[];
+    df *V = reinterpret_cast<df *>(sm);          // [2][n]
+    df *w = V + 2 * (size_t)n;                   // [n]
+    df *R = w + n;                               // [n] row rank of R, if rank < D
+    df *rs = R + n;                              // [kTdgParts][nrm] parts of S of own rows
+    df *ra = rs + (size_t)kTdgParts * nrm;       // [nrm] a_{i,k+1}
+    df *sb = ra + nrm;                           // [kTdfWarps] partials of |x_1:|^2
+    df *rows = reinterpret_cast<df *>(sm) + tdg_fixed(n, G);
+    const int room = max(0, (smem_df - (int)tdg_fixed(n, G)) / n);
+    const int qs = max(0, nr - room);            // own rows q >= qs in shared memory
+    double *wk = work + work_first[0];
+    df *spill = reinterpret_cast<df *>(wk);
+    auto row = [&](int q) -> df * { return q >= qs ? rows + (size_t)(q - qs) * n : spill + (size_t)(rank + q * G) * n; };
+    df *Yx = reinterpret_cast<df *>(wk + tdg_exchange(J.n)), *Bx = Yx + 2 * (size_t)n, *Kx = Bx + 2 * (size_t)n;
+    unsigned *count = reinterpret_cast<unsigned *>(wk + tdg_count(J.n));
+    __shared__ df s_sc[2], s_rd, s_c;   // tau, s of the step; R_d . x of the own R row, -tau R_d . v
+    const df zero{0.0f, 0.0f}, one{1.0f, 0.0f};
+    const bool own_r = rank < D;
+    auto put = [](double *p, df x) { *reinterpret_cast<float2 *>(p) = make_float2(x.h, x.l); };
+    auto far = [](const df *p) { const float2 f = __ldcg(reinterpret_cast<const float2 *>(p)); return df{f.x, f.y}; };
+    for (int q = warp; q < nr; q += kTdfWarps) {
+        const int i = rank + q * G;
+        df *a = row(q);
+        for (int j = lane; j < n; j += 32) a[j] = df_from_bits(__ldcg(J.A + (j <= i ? (size_t)i * n + j : (size_t)j * n + i)));
+    }
+    df sq0 = zero;
+    for (int j = tid; j < n; j += kTdfThreads) {
+        const df xj = df_from_bits(__ldcg(J.A + (size_t)j * n));   // x of step 0
+        V[j] = xj;
+        V[n + j] = zero;
+        w[j] = zero;
+        R[j] = (j == rank) ? one : zero;
+        if (j >= 2) sq0 = dfm::fma(xj, xj, sq0);
+    }
+    sq0 = dfm::warp_sum(sq0);
+    if (lane == 0) sb[warp] = sq0;
+    if (rank == 0 && tid == 0) put(J.d, V[0]);
+    __syncthreads();
+    int cur = 0;
+    for (int k = 0; k + 2 < n; ++k, cur ^= 1) {
+        df *x = V + (size_t)cur * n, *vp = V + (size_t)(cur ^ 1) * n;
+        df *yk = Yx + (size_t)cur * n, *bk = Bx + (size_t)cur * n, *kb = Kx + (size_t)cur * kTdgMax;
+        const int b0 = k + 1;
+        const int q0 = b0 <= rank ? 0 : (b0 - rank + G - 1) / G;   // first own row >= b0
+        const int na = max(0, nr - q0);
+        const int np = 4 * na <= kTdgRowWarps ? 4 : 2 * na <= kTdgRowWarps ? 2 : 1;
+        // pass
+        if (warp == kTdScal) {
+            df s2 = lane < kTdfWarps ? sb[lane] : zero;
+            s2 = dfm::warp_sum(s2);
+            const df al = x[b0];
+            df tau = zero, scal = zero, beta = al;
+            if (s2.h != 0.0f || s2.l != 0.0f) {
+                const int ea = (al.h != 0.0f) ? f32_exponent(al.h) : -1000;
+                int e = max(ea, f32_exponent(s2.h) >> 1);
+                e = min(max(e, -126), 126);
+                const float sg = pow2_f32(-e);
+                const df alt{al.h * sg, al.l * sg}, s2t{(s2.h * sg) * sg, (s2.l * sg) * sg};
+                const df x2 = dfm::fma(alt, alt, s2t);   // in [1, 12)
+                const df r = dfm::rsqrt2(x2), nx = dfm::mul(x2, r);
+                const bool ng = signbit(alt.h);
+                const df aa = ng ? dfm::neg(alt) : alt;
+                tau = dfm::fma(aa, r, one);
+                df st = dfm::rcp2(dfm::add(aa, nx));   // 1 / (alpha~ - beta~)
+                if (ng) st = dfm::neg(st);
+                scal = df{st.h * sg, st.l * sg};         // 1 / (alpha - beta)
+                const df bt = ng ? nx : dfm::neg(nx);
+                const float un = pow2_f32(e);
+                beta = df{bt.h * un, bt.l * un};
+            }
+            if (lane == 0) {
+                s_sc[0] = tau;
+                s_sc[1] = scal;
+                if (rank == 0) { put(J.e + k, beta); put(J.tau + k, tau); }
+            }
+        } else if (warp == kTdScal - 1) {
+            if (own_r) {   // R_d . x_{1:}
+                df s0 = zero, s1 = zero;
+                int j = b0 + 1 + lane;
+                for (; j + 32 < n; j += 64) { s0 = dfm::fma(R[j], x[j], s0); s1 = dfm::fma(R[j + 32], x[j + 32], s1); }
+                if (j < n) s0 = dfm::fma(R[j], x[j], s0);
+                s0 = dfm::warp_sum(dfm::add(s0, s1));
+                if (lane == 0) s_rd = s0;
+            }
+        } else {
+            for (int u = warp; u < na * np; u += kTdgRowWarps) {
+                const int q = q0 + u / np, part = u % np, i0 = rank + q * G;
+                df *a0 = row(q);
+                const df v0 = vp[i0], w0 = w[i0];
+                df s0 = zero, s1 = zero;   // two columns at a time
+                for (int j = b0 + 32 * part + lane; j < n; j += 64 * np) {
+                    const bool in = j + 32 * np < n;
+                    const int j2 = in ? j + 32 * np : j;
+                    const df p0 = a0[j], p1 = a0[j2];
+                    const df t0 = rank2(p0, v0, w[j], w0, vp[j]), t1 = rank2(p1, v0, w[j2], w0, vp[j2]);
+                    a0[j] = t0;
+                    if (in) a0[j2] = t1;
+                    s0 = dfm::fma(t0, (j == b0) ? zero : x[j], s0);
+                    s1 = dfm::fma(t1, in ? x[j2] : zero, s1);
+                    if (j == b0) ra[q] = t0;
+                }
+                s0 = dfm::warp_sum(dfm::add(s0, s1));
+                if (lane == 0) rs[(size_t)part * nrm + q] = s0;
+            }
+        }
+        __syncthreads();
+        const df tau = s_sc[0], s = s_sc[1];
+        const bool nz = (tau.h != 0.0f);
+        if (warp == 0) {   // y of own rows, and their part of v . y
+            df kv = zero;
+            for (int q = q0 + lane; q < nr; q += 32) {
+                const int i = rank + q * G;
+                df S = rs[q];
+                for (int p = 1; p < np; ++p) S = dfm::add(S, rs[(size_t)p * nrm + q]);
+                const df yi = nz ? dfm::fma(s, S, ra[q]) : zero;
+                yk[i] = yi;
+                kv = (i == b0) ? dfm::add(kv, yi) : dfm::fma(dfm::mul(s, x[i]), yi, kv);
+            }
+            kv = dfm::warp_sum(kv);
+            if (lane == 0) kb[rank] = kv;
+        } else if (b0 % G == rank) {   // row k+1
+            const df *a = row(q0);
+            for (int j = b0 + tid - 32; j < n; j += kTdfThreads - 32) bk[j] = a[j];
+        }
+        // every CTA's count of this step; a CTA that waits in vain marks the job and all leave
+        __syncthreads();
+        if (tid == 0) {
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+            const unsigned want = (unsigned)(k + 1) * (unsigned)G;
+            unsigned c = 0;
+            int polls = 0;
+            do {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
+            } while (c < want && ++polls < kTdgPolls);
+            if (c < want) s_ok = 0;
+        }
+        __syncthreads();
+        if (!s_ok) {
+            if (tid == 0) atomicExch(J.stat, kDyStatBarrier);
+            return;
+        }
+        // all rows: v, w; R; x of the next step
+        {
+            // all that comes from L2 first
+            constexpr int NA = 2;   // rows a thread has ahead
+            df ya[NA], ba[NA], ka[kTdgMax / 32];
+#pragma unroll
+            for (int h = 0; h < NA; ++h) {
+                const int j = min(b0 + tid + h * kTdfThreads, n - 1);
+                ya[h] = far(yk + j);
+                ba[h] = far(bk + j);
+            }
+#pragma unroll
+            for (int h = 0; h < kTdgMax / 32; ++h) ka[h] = lane + 32 * h < G ? far(kb + lane + 32 * h) : zero;
+            const df yb = far(yk + b0);
+#pragma unroll
+            for (int o = kTdgMax / 64; o > 0; o >>= 1)
+#pragma unroll
+                for (int h = 0; h < o; ++h) ka[h] = dfm::add(ka[h], ka[h + o]);
+            const df K = dfm::warp_sum(ka[0]);
+            const df tk = dfm::mul(tau, tau);
+            const df nK = dfm::neg(dfm::mul(df{0.5f * tk.h, 0.5f * tk.l}, K));
+            const df vb = nz ? one : zero, wb = dfm::fma(nK, vb, dfm::mul(tau, yb));
+            if (own_r) {   // (the whole CTA)
+                if (tid == 0) s_c = dfm::neg(dfm::mul(tau, dfm::fma(s, s_rd, R[b0])));
+                __syncthreads();   // R_{b0} changes
+            }
+            df sq = zero;
+            auto one_row = [&](int j, df yj, df bj) {
+                const df vj = !nz ? zero : (j == b0) ? one : dfm::mul(s, x[j]);
+                const df wj = dfm::fma(nK, vj, dfm::mul(tau, yj));
+                const df t = rank2(bj, vj, wb, wj, vb);
+                w[j] = wj;
+                x[j] = vj;
+                vp[j] = t;
+                if (j > b0 + 1) sq = dfm::fma(t, t, sq);
+                if (rank == 0 && j == b0) put(J.d + b0, t);
+                if (rank == 0 && j == b0 + 1 && k + 3 == n) put(J.e + n - 2, t);
+                if (k + 3 == n && j == n - 1 && (n - 1) % G == rank)   // the last step: the last diagonal entry
+                    J.d[n - 1] = dfm::to_double(rank2(row(nr - 1)[n - 1], vj, wj, wj, vj));
+                if (own_r) R[j] = dfm::fma(s_c, vj, R[j]);
+            };
+#pragma unroll
+            for (int h = 0; h < NA; ++h)
+                if (b0 + tid + h * kTdfThreads < n) one_row(b0 + tid + h * kTdfThreads, ya[h], ba[h]);
+            for (int j = b0 + tid + NA * kTdfThreads; j < n; j += kTdfThreads) one_row(j, far(yk + j), far(bk + j));
+            sq = dfm::warp_sum(sq);
+            if (lane == 0) sb[warp] = sq;
+        }
+        __syncthreads();
+    }
+    if (rank == 0)
+        for (int j = tid; j < n; j += kTdfThreads) {
+            auto conv = [](double *p) { const float2 f = __ldcg(reinterpret_cast<const float2 *>(p)); *p = dfm::to_double(df{f.x, f.y}); };
+            if (j + 1 < n) { conv(J.d + j); conv(J.e + j); } else J.e[j] = 0.0;
+            if (j + 2 < n) conv(J.tau + j); else J.tau[j] = 0.0;
+        }
+    if (own_r)
+        for (int j = tid; j < n; j += kTdfThreads) J.R[(size_t)rank * n + j] = dfm::to_double(R[j]);
+}
+
 // the kernel for a cluster size (1, 2, 4, 8 or 16)
 static auto tridiag_df_kernel(int cluster) {
     return cluster == 16 ? k_tridiag_df<16> : cluster == 8 ? k_tridiag_df<8> : cluster == 4 ? k_tridiag_df<4>
@@ -1007,12 +1256,29 @@ int tridiag_df_limit(int cluster, int D) {
     return lo;
 }
 
+// CTAs of k_tridiag_grid: one on every SM (0: the device takes no cooperative launch)
+static int grid_ctas() {
+    static const int g = [] {
+        int dev = 0, sms = 0, coop = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
+            return 0;
+        return std::min(sms, kTdgMax);
+    }();
+    return g;
+}
+
+// One matrix in the launch, of an order that k_tridiag_grid may take
+static bool tridiag_on_grid(int njobs, int nmax, int nlim) {
+    return njobs == 1 && std::min(nmax, nlim) >= kTdgMin && grid_ctas() > 0;
+}
+
 // Kernels launch_dyson starts for matrices of order up to nmax: deflate, assemble, the
 // small-matrix reduction (the cluster one beyond kTsMax, the FP64 one and k_qrows beyond
 // its limit), then launch_eig's.
-int dyson_launch_count(int nmax, int Dmax, int cluster) {
+int dyson_launch_count(int njobs, int nmax, int Dmax, int cluster) {
     const int nlim = tridiag_df_limit(cluster, Dmax);
-    return 3 + (nmax > kTsMax ? 1 : 0) + (nmax > nlim ? 2 : 0) + (nmax > kTsMax ? 8 : 7);
+    return 3 + (nmax > kTsMax ? 1 : 0) + (tridiag_on_grid(njobs, nmax, nlim) ? 1 : 0) + (nmax > nlim ? 2 : 0) + (nmax > kTsMax ? 8 : 7);
 }
 
 cudaError_t launch_dyson(const DyJob *d_jobs, int njobs, const long long *d_row_first, long long total_rows,
@@ -1048,10 +1314,26 @@ cudaError_t launch_dyson(const DyJob *d_jobs, int njobs, const long long *d_row_
         return e == cudaSuccess;
     };
     const int nlim = tridiag_df_limit(cluster, Dmax);
+    const bool grid = tridiag_on_grid(njobs, nmax, nlim);
+    if (grid) {
+        cudaLaunchConfig_t gc = {};
+        gc.gridDim = dim3(grid_ctas(), 1, 1);
+        gc.blockDim = dim3(kTdfThreads, 1, 1);
+        gc.dynamicSmemBytes = kTdfSlots * 8;
+        gc.stream = st;
+        cudaLaunchAttribute ga[1];
+        ga[0].id = cudaLaunchAttributeCooperative;
+        ga[0].val.cooperative = 1;
+        gc.attrs = ga;
+        gc.numAttrs = 1;
+        e = allow_dynamic_smem((const void *)k_tridiag_grid);
+        if (e == cudaSuccess) e = cudaLaunchKernelEx(&gc, k_tridiag_grid, d_jobs, nlim, kTdfSlots, work, d_work_first);
+        if (e != cudaSuccess) return e;
+    }
     {
         // as many slots as the largest order (the full orders bound the deflated ones) needs
         // to keep all its rows, at most kTdfSlots
-        const int nb = std::min(nmax, nlim);
+        const int nb = grid ? kTdgMin - 1 : std::min(nmax, nlim);
         const size_t slots = std::min((size_t)kTdfSlots, tdf_fixed(nb, cluster, Dmax) + (size_t)((nb + cluster - 1) / cluster) * nb);
         cfg.blockDim = dim3(kTdfThreads, 1, 1);
         cfg.dynamicSmemBytes = slots * 8;

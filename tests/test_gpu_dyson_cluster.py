@@ -59,3 +59,35 @@ def test_cluster_sizes_agree(bdmod, problems):
                 assert e < 1e-10 and z < 1e-8, c
             np.testing.assert_allclose(a["koltun"], b["koltun"], rtol=1e-10, atol=1e-11)
     ctx.close()
+
+
+# the smallest order one matrix takes the whole GPU for and one less, orders that are no multiple
+# of its CTAs, rows beyond shared memory; D from the channel
+@pytest.mark.parametrize("n,ish", [(511, 1), (512, 1), (531, 5), (760, 2), (1901, 0)])
+def test_one_matrix_on_the_whole_gpu(bdmod, problems, n, ish):
+    p = problems(6, 20.0, 1, 50)
+    rng = np.random.default_rng(n)
+    ctx = bdmod.Context().upload(p)
+    D = int(p.ms.no[ish])
+    nb = (n - D) // 3
+    nf = n - D - nb
+    fw, bk = np.zeros((nf, 2 + D)), np.zeros((nb, 2 + D))
+    fw[:, 0], bk[:, 0] = rng.uniform(20.0, 300.0, nf), -rng.uniform(60.0, 250.0, nb)
+    fw[:, 2:], bk[:, 2:] = rng.standard_normal((nf, D)) * 0.3, rng.standard_normal((nb, D)) * 0.3
+    s1, hf = np.diag(np.linspace(-20.0, 60.0, D)), np.zeros((D, D))
+    r = ctx.dyson_rows(ish, 2, fw, bk, sig1b=s1, sighf=hf, efermi=-50.0)
+    A = np.diag(np.concatenate([np.zeros(D), fw[:, 0], bk[:, 0]]))
+    A[:D, :D] = s1
+    A[D:, :D] = np.concatenate([fw[:, 2:], bk[:, 2:]])
+    A[:D, D:] = A[D:, :D].T
+    w, v = np.linalg.eigh(A)
+    got = np.concatenate([r["qp"], r["qh"]])
+    assert len(got) == n
+    # the tolerances of the cluster kernel's test above: the arithmetic is the same
+    np.testing.assert_allclose(np.sort(got[:, 0]), w, rtol=1e-11, atol=1e-11 * np.abs(A).sum(0).max())
+    ref = np.concatenate([w[:, None], (v[:D] ** 2).sum(0)[:, None], v[:D].T], 1)
+    e, z = strong_diffs(ref, got)
+    assert e < 1e-10 and z < 1e-8
+    x = got[:, 2:]
+    assert np.abs(x.T @ x - np.eye(D)).max() < 1e-11
+    ctx.close()
