@@ -91,3 +91,37 @@ def test_one_matrix_on_the_whole_gpu(bdmod, problems, n, ish):
     x = got[:, 2:]
     assert np.abs(x.T @ x - np.eye(D)).max() < 1e-11
     ctx.close()
+
+
+def test_whole_gpu_reductions_of_two_threads(bdmod, problems):
+    """Two contexts on two host threads, each solving large matrices that take every SM: the same
+    bits as alone."""
+    import threading
+    p = problems(4, 20.0, 0, 20)
+    D = int(p.ms.no[0])
+    rng = np.random.default_rng(3)
+    jobs = []
+    for n in (600, 777):
+        rows = np.zeros((n, 2 + D))
+        rows[:, 0], rows[:, 2:] = rng.uniform(20.0, 300.0, n), rng.standard_normal((n, D)) * 0.3
+        ctx = bdmod.Context().upload(p)
+
+        def solve(ctx=ctx, rows=rows):
+            r = ctx.dyson_rows(0, 2, rows, np.zeros((0, 2 + D)), sig1b=np.diag(np.linspace(-20.0, 60.0, D)),
+                               sighf=np.zeros((D, D)), efermi=-50.0)
+            return np.concatenate([r["qp"], r["qh"]])
+        jobs.append((ctx, solve, solve()))
+    bad = []
+
+    def work(solve, want):
+        for _ in range(5):
+            if not np.array_equal(solve(), want):
+                bad.append(len(want))
+    threads = [threading.Thread(target=work, args=j[1:]) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+    for j in jobs:
+        j[0].close()
