@@ -121,16 +121,19 @@ static_assert(kCpThreads >= kCpGroups, "a thread per exact group");
 //
 // A step is a chain of short phases between barriers, and an FP64 instruction holds an SM
 // sub-partition's FP64 unit for ~64 cycles, so FP64 is kept to what needs it: the sweep's dot
-// products are fixed-point sums (lz_fixed.cuh; four vectors a warp), its update FP32 where the
-// coefficients are rounding-sized (|c| <= 1e-9 |w|: an error below 2^-24 1e-9 |w|) and fixed
-// point otherwise, and one warp takes the decision.  The norm, alpha, m, g and the recurrence
-// are FP64.
+// products and m are fixed-point sums (lz_fixed.cuh; four vectors a warp), its update FP32 where the
+// coefficients are rounding-sized (|c| <= 1e-9 |w|: an error below 2^-23 1e-9 |w|) and fixed
+// point otherwise, and one warp takes the decision.  The norm, alpha, g and the recurrence are
+// FP64.
 // Measured (N_max = 10, 100 iterations per pivot): the reduction of all 84 chains takes
-// 0.38 ms against 3.59 ms in the poles' space (N_max = 12: 0.57 against 12.2).
+// 0.36 ms against 3.59 ms in the poles' space (N_max = 12: 0.53 against 12.2).
 __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains, int nchains, double eta2) {
     const int cid = blockIdx.x;
     if (cid >= nchains) return;
-    const LzChain C = chains[cid];
+    __shared__ LzChain C;
+    if (threadIdx.x < sizeof(LzChain) / 4)
+        reinterpret_cast<int *>(&C)[threadIdx.x] = reinterpret_cast<const int *>(chains + cid)[threadIdx.x];
+    __syncthreads();
     if (!C.cp || !C.cp_on) return;
     const CompactScratch S = lz_compact(C.cp);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -183,13 +186,14 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
     const int R = min(L, np);               // vectors, at most
     const int rq = (R + 4) & ~3, np4 = (np + 3) & ~3;
     const int nla = max(C.n_used - 1, 0);   // chains whose last vector later ones refer to
-    // shared layout (doubles): E[np4] | M[D][np4] | w[np4] | ew[np4] | ring[2][np4] | last[nla][np4] |
+    // shared layout (doubles): E[np4] | M[D][np4] (two planes of integers against s_mb) | w[np4] | ew[np4] | ring[2][np4] | last[nla][np4] |
     // c[rq + 4] | sc[20], then ints wa[np4] | wb[np4] | Va[R][np4] | Vb[R][np4], floats cf[rq + 4] |
     // Vf[R][np4], ints rowslot[L]
     const size_t need = sizeof(double) * ((size_t)(D + 5 + nla) * np4 + rq + 4 + 20) +
                         sizeof(int) * ((size_t)(2 + 3 * R) * np4 + rq + 4 + (size_t)L);
     if (s_bad || np > kCpDim || need > (size_t)kCpSmem) return;
-    double *E = sm, *M = E + np4, *w = M + (size_t)D * np4, *ew = w + np4, *ring = ew + np4, *lasts = ring + 2 * np4,
+    double *E = sm, *M = E + np4, *w = M + (size_t)D * np4;
+    double *ew = w + np4, *ring = ew + np4, *lasts = ring + 2 * np4,
            *c = lasts + (size_t)nla * np4, *sc = c + rq + 4;
     int *wa = reinterpret_cast<int *>(sc + 20), *wb = wa + np4, *Va = wb + np4, *Vb = Va + (size_t)R * np4;
     float *cf = reinterpret_cast<float *>(Vb + (size_t)R * np4), *Vf = cf + rq + 4;
@@ -209,27 +213,62 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
             }
         }
     }
+    int *Ma = reinterpret_cast<int *>(M), *Mb = Ma + (size_t)D * np4;
+    __syncthreads();
+    __shared__ int s_mb[8];
+    double mv[(8 * kCpDim + kCpThreads - 1) / kCpThreads];   // (the planes take the doubles' place)
+#pragma unroll
+    for (int r = 0; r < (8 * kCpDim + kCpThreads - 1) / kCpThreads; ++r) {
+        const int q = tid + r * kCpThreads;
+        mv[r] = q < D * np ? M[(size_t)(q / np) * np4 + q % np] : 0.0;
+    }
+    if (warp < D) {   // a power of two above |M_d|
+        float m2 = 0.0f;
+        for (int i = lane; i < np; i += 32) { const float f = f32_trunc(M[(size_t)warp * np4 + i]); m2 = fmaf(f, f, m2); }
+        for (int o = 16; o > 0; o >>= 1) m2 += __shfl_xor_sync(0xffffffffu, m2, o);
+        bool any = false;
+        for (int i = lane; i < np; i += 32) any |= M[(size_t)warp * np4 + i] != 0.0;
+        any = __any_sync(0xffffffffu, any);
+        if (lane == 0) {
+            s_mb[warp] = bias_above((double)m2);
+            if (any && m2 < 0x1p-90f) s_bad = 1;   // an orbital coupled far more weakly than the others
+        }
+    }
     me = __reduce_max_sync(0xffffffffu, me);
     mm = __reduce_max_sync(0xffffffffu, mm);
     if (lane == 0) { atomicMax(&s_rng[0], me); atomicMax(&s_rng[1], mm); }
     __syncthreads();
-    if (!fixed_range(s_rng[0]) || !fixed_range(s_rng[1])) return;   // (fixed-point and FP32 parts)
-    __shared__ int s_start[10], s_last[10], lslot[8], lt[16], lq[16], s_fl;
-    __shared__ double lc[16], s_row[32], s_n[3];   // s_n: 1/|w|, |w|, |E v|^2 of the kept vector
+    if (s_bad || !fixed_range(s_rng[0]) || !fixed_range(s_rng[1])) return;   // (fixed-point and FP32 parts)
+#pragma unroll
+    for (int r = 0; r < (8 * kCpDim + kCpThreads - 1) / kCpThreads; ++r) {
+        const int q = tid + r * kCpThreads;
+        if (q < D * np) {
+            const int2 f = fixed_of(mv[r], s_mb[q / np]);
+            Ma[(size_t)(q / np) * np4 + q % np] = f.x;
+            Mb[(size_t)(q / np) * np4 + q % np] = f.y;
+        }
+    }
+    __shared__ int s_start[10], s_last[10], lslot[8], lo_[16], s_nl, s_fl;
+    __shared__ double lc[16], s_n[3];   // s_n: 1/|w|, |w|, |E v|^2 of the kept vector
     __shared__ float s_f[kCpWarps];
     if (tid <= C.n_used && tid < 10) s_start[tid] = C.start[tid];
     if (tid < C.n_used && tid < 10) s_last[tid] = C.last[tid];
-    const int Qg = C.gInfo[0];
-    const int dtot = Qg > 0 ? C.gInfo[Qg] : 0;
+    // the groups' energies and unreached directions, cumulated (Q = gInfo[0])
+    __shared__ int s_cum[kCpGroups];
+    __shared__ double s_gE[kCpGroups];
+    if (tid < Q) { s_cum[tid] = C.gInfo[1 + tid]; s_gE[tid] = C.gE[tid]; }
+    __syncthreads();
+    const int dtot = s_cum[Q - 1];
     auto group_of = [&](int d) {
-        int lo = 0, hi = Qg - 1;
-        while (lo < hi) { const int mid = (lo + hi) >> 1; if (C.gInfo[1 + mid] > d) hi = mid; else lo = mid + 1; }
+        int lo = 0, hi = Q - 1;
+        while (lo < hi) { const int mid = (lo + hi) >> 1; if (s_cum[mid] > d) hi = mid; else lo = mid + 1; }
         return lo;
     };
     constexpr double tau = 1e-48, thr_exh = 1e-20;   // k_lanczos's, FP64 vectors
     int dcur = 0, ndefl = 0, nvec = 0, extra = 0, k = -1;
     double e2v = 0.0;            // |E v|^2 of the last built vector
-    int nl0 = 0;                 // vectors of the next recurrence (lt, lc)
+    int nl0 = 0;                 // vectors of the next recurrence (lo_, lc)
+    bool rough = false;          // w much shorter than what it was split against: swept again
     // stored vector t as doubles: the two newest, or the last one of chain q
     auto vecd = [&](int t, int q) -> const double * { return t >= nvec - 2 ? ring + (t & 1) * np4 : lasts + (size_t)q * np4; };
     int wbias = 1023;   // exponent field of the power of two w is split against
@@ -251,9 +290,11 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
             for (int i = tid; i < np; i += kCpThreads) {
                 const double *p = C.piv + (size_t)k * D;
                 double x = 0.0;
-                for (int d = 0; d < D; ++d) x = fma(M[(size_t)d * np4 + i], p[d], x);
+                for (int d = 0; d < D; ++d)
+                    x = fma(fixed_to_double(Ma[(size_t)d * np4 + i], Mb[(size_t)d * np4 + i]) *
+                                __hiloint2double(s_mb[d] << 20, 0), p[d], x);
                 w[i] = x;
-                const float f = (float)x;
+                const float f = f32_trunc(x);
                 s2 = fmaf(f, f, s2);
             }
             for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
@@ -267,10 +308,20 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
             for (int i = tid; i < np; i += kCpThreads) split_w(i, w[i]);
         } else {
             wbias = bias_above(e2v);
-            const double *v0 = ring + (lt[0] & 1) * np4;
+            const double *v0 = ring + lo_[0];
             for (int i = tid; i < np; i += kCpThreads) {
                 double x = v0[i] * E[i];
-                for (int t = 0; t < nl0; ++t) x = fma(-lc[t], vecd(lt[t], lq[t])[i], x);
+                for (int t0 = 0; t0 < nl0; t0 += 4) {
+                    double y[4], cc[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int t = min(t0 + u, nl0 - 1);
+                        y[u] = ring[lo_[t] + i];
+                        cc[u] = lc[t];
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) if (t0 + u < nl0) x = fma(-cc[u], y[u], x);
+                }
                 w[i] = x;
                 split_w(i, x);
             }
@@ -297,14 +348,14 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
                     const FixedSum r = warp_sums_of<4>(acc, lane, fixed_add, fixed_shfl);
                     if ((lane & 7) == 0 && (lane >> 3) < nu) {
                         const double x = fixed_value(r, wbias);
-                        const float xf = (float)x;
+                        const float xf = f32_trunc(x);
                         c[t0 + (lane >> 3)] = x;
                         cf[t0 + (lane >> 3)] = xf;
                     }
                 }
                 if (want_n && nvec >= t0 && nvec < t0 + 4) {
                     float s2 = 0.0f;
-                    for (int i = lane; i < np; i += 32) { const float f = (float)w[i]; s2 = fmaf(f, f, s2); }
+                    for (int i = lane; i < np; i += 32) { const float f = f32_trunc(w[i]); s2 = fmaf(f, f, s2); }
                     for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
                     if (lane == 0) { c[nvec] = (double)s2; cf[nvec] = s2; }
                 }
@@ -326,7 +377,7 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
 #pragma unroll
                             for (int u = 0; u < 4; ++u) a[u] = fmaf(cf[t + u], Vf[(size_t)(t + u) * np4 + i], a[u]);
                         for (; t < nvec; ++t) a[0] = fmaf(cf[t], Vf[(size_t)t * np4 + i], a[0]);
-                        x -= (double)((a[0] + a[1]) + (a[2] + a[3]));
+                        x -= f32_to_double((a[0] + a[1]) + (a[2] + a[3]));
                     } else {
                         FixedSum acc{0, 0};
                         for (int t = 0; t < nvec; ++t) {
@@ -336,58 +387,81 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
                         x -= fixed_value(acc, wbias);
                     }
                     w[i] = x;
+                    split_w(i, x);   // (for m; the dot products are done)
                     ew[i] = E[i] * x;
                 }
             }
             __syncthreads();
-            // the scalars of the updated w: |w|^2, <w|E|w>, |E w|^2, <M_d|w>, <v_last(q)|E|w>, two a warp
-            // and round
-            const int nsc = 3 + D + nq;
-            for (int t0 = 2 * warp; t0 < nsc; t0 += 2 * kCpWarps) {
-                const double *a[2], *b[2];
+            // the scalars of the updated w: |w|^2, <w|E|w>, |E w|^2, <v_last(q)|E|w> in FP64, two a warp
+            // and round, beside <M_d|w> in fixed point, four a warp
+            const int nsc = 3 + nq;
+            if (warp >= kCpWarps - 2) {
+                const int d0 = 4 * (kCpWarps - 1 - warp);
+                if (d0 < D) {
+                    FixedSum acc[4];
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int t = t0 + u;
-                    a[u] = w;
-                    b[u] = w;
-                    if (t == 1) b[u] = ew;
-                    else if (t == 2) { a[u] = ew; b[u] = ew; }
-                    else if (t >= 3 && t < 3 + D) a[u] = M + (size_t)(t - 3) * np4;
-                    else if (t >= 3 + D && t < nsc && lslot[t - 3 - D] >= 0) { a[u] = vecd(lslot[t - 3 - D], t - 3 - D); b[u] = ew; }
+                    for (int u = 0; u < 4; ++u) acc[u] = FixedSum{0, 0};
+                    for (int i = lane; i < np; i += 32) {
+                        const int xa = wa[i], xb = wb[i];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (d0 + u < D) fixed_step(acc[u], Ma[(size_t)(d0 + u) * np4 + i], Mb[(size_t)(d0 + u) * np4 + i], xa, xb);
+                    }
+                    const FixedSum r = warp_sums_of<4>(acc, lane, fixed_add, fixed_shfl);
+                    const int d = d0 + (lane >> 3);
+                    if ((lane & 7) == 0 && d < D) sc[3 + d] = fixed_value(r, wbias + s_mb[d] - 1023);
                 }
-                double x[2] = {0.0, 0.0};
-                for (int i = lane; i < np; i += 32) {
-                    x[0] = fma(a[0][i], b[0][i], x[0]);
-                    x[1] = fma(a[1][i], b[1][i], x[1]);
+            } else {
+                for (int t0 = 2 * warp; t0 < nsc; t0 += 2 * (kCpWarps - 2)) {
+                    const double *a[2], *b[2];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const int t = t0 + u;
+                        a[u] = w;
+                        b[u] = w;
+                        if (t == 1) b[u] = ew;
+                        else if (t == 2) { a[u] = ew; b[u] = ew; }
+                        else if (t >= 3 && t < nsc && lslot[t - 3] >= 0) { a[u] = vecd(lslot[t - 3], t - 3); b[u] = ew; }
+                    }
+                    double x[2] = {0.0, 0.0};
+                    for (int i = lane; i < np; i += 32) {
+                        x[0] = fma(a[0][i], b[0][i], x[0]);
+                        x[1] = fma(a[1][i], b[1][i], x[1]);
+                    }
+                    const double r = warp_sums_of<2>(x, lane, [](double p, double q) { return p + q; },
+                                                     [](double p, int o) { return __shfl_xor_sync(0xffffffffu, p, o); });
+                    const int t = t0 + (lane >> 4);
+                    if ((lane & 15) == 0 && t < nsc) {
+                        if (t < 3) sc[t] = r;
+                        else sc[D + t] = lslot[t - 3] < 0 ? 0.0 : r;
+                    }
                 }
-                const double r = warp_sums_of<2>(x, lane, [](double p, double q) { return p + q; },
-                                                 [](double p, int o) { return __shfl_xor_sync(0xffffffffu, p, o); });
-                const int t = t0 + (lane >> 4);
-                if ((lane & 15) == 0 && t < nsc) sc[t] = (t >= 3 + D && lslot[t - 3 - D] < 0) ? 0.0 : r;
             }
             __syncthreads();
             // k_lanczos's decision, by warp 0 (its lanes take one threshold each); exhaustion first:
             // further sweeps of a w that holds nothing leave nothing
             if (warp == 0) {
                 const double x2 = sc[0];
-                const double lim = lane == 0 ? eta2 * wn2 : (lane == 1 ? thr_exh : tau) * wn2_first;
+                const double lim = lane == 0 ? eta2 * wn2 : (lane == 1 ? thr_exh : lane == 2 ? tau : kFixedShort) * wn2_first;
                 const unsigned lt_ = __ballot_sync(0xffffffffu, x2 < lim), le = __ballot_sync(0xffffffffu, x2 <= lim);
                 const long long xb = __double_as_longlong(x2);
                 const bool zero = (xb << 1) == 0, fin = (xb & 0x7ff0000000000000LL) != 0x7ff0000000000000LL;
                 int f;
                 if ((le & 2u) || zero) f = (dcur < dtot) ? 2 : 3;
                 else if (nvec > 0 && nfull + 1 < 4 && (lt_ & 1u)) f = 1;
+                else if (nvec > 0 && nfull == 0 && (lt_ & 8u)) f = 4;
                 else if (!(le & 4u) && fin) f = 0;
                 else f = 3;   // (not finite)
-                const double r = rsqrt_newton(x2);
+                const double r = rsqrt_cubic(x2);
                 const double y = (lane == 0 ? 1.0 : lane == 1 ? x2 : sc[2] * r) * r;
                 if (lane < 3) s_n[lane] = y;
                 if (lane == 0) s_fl = f;
             }
             __syncthreads();
             fl = s_fl;
-            if (nfull++ > 0) ++extra;
-            if (fl != 1) break;
+            if (nfull++ > 0 && !rough) ++extra;
+            rough = fl == 4;
+            if (fl != 1 && fl != 4) break;
             wn2 = sc[0];   // another sweep, of the updated w
             wbias = bias_above(wn2);
             for (int i = tid; i < np; i += kCpThreads) split_w(i, w[i]);
@@ -399,7 +473,7 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
             const int nr = jend - j;
             for (int r = tid; r < nr; r += kCpThreads) {
                 const int d = dcur + r;
-                const double a = (d < dtot) ? C.gE[group_of(d)] : C.gE[Qg - 1];
+                const double a = s_gE[d < dtot ? group_of(d) : Q - 1];
                 double *row = C.out + (size_t)(j + r) * NT;
                 for (int e = 0; e < NT; ++e) row[e] = 0.0;
                 row[0] = a;
@@ -431,29 +505,34 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
         // the row, and the next step's recurrence from it, by the last warp (the first ones hold the
         // elements)
         if (warp == kCpWarps - 1) {
+            double x = 0.0;
             if (lane < NT) {
-                double x = 0.0;
-                if (lane == 0) x = sc[1] * ixb * ixb;
-                else if (lane == 1) x = (newv && k >= 1) ? sc[3 + D + (k - 1)] * ixb : s_n[1];
-                else if (lane < 2 + k) x = sc[3 + D + (lane - 2)] * ixb;
-                else if (lane >= C.nden_out && lane < C.nden_out + D) x = sc[3 + (lane - C.nden_out)] * ixb;
-                s_row[lane] = x;
+                int e = -1;   // the row's entry from sc
+                if (lane == 0) e = 1;
+                else if (lane == 1) e = (newv && k >= 1) ? 3 + D + (k - 1) : -1;
+                else if (lane < 2 + k) e = 3 + D + (lane - 2);
+                else if (lane >= C.nden_out && lane < C.nden_out + D) e = 3 + (lane - C.nden_out);
+                if (e >= 0) x = sc[e] * ixb;
+                if (lane == 0) x *= ixb;
+                if (lane == 1 && e < 0) x = s_n[1];
                 C.out[(size_t)j * NT + lane] = x;
             }
-            __syncwarp();
-            if (lane == 0) {
-                rowslot[j] = nvec;
-                int n = 0;
-                lt[n] = nvec; lq[n] = -1; lc[n++] = s_row[0];
-                if (j >= 1 && rowslot[j - 1] >= 0) { lt[n] = rowslot[j - 1]; lq[n] = -1; lc[n++] = s_row[1]; }
-                for (int q = 0; q < k; ++q)
-                    if (s_last[q] < j - 1 && rowslot[s_last[q]] >= 0) { lt[n] = rowslot[s_last[q]]; lq[n] = q; lc[n++] = s_row[2 + q]; }
-                lt[15] = n;
+            // lane 0: v_j, lane 1: v_{j-1}, lane 2 + q: chain q's last
+            int v = -1;
+            if (lane == 0) v = nvec;
+            else if (lane == 1) v = j >= 1 ? rowslot[j - 1] : -1;
+            else if (lane < 2 + k) v = s_last[lane - 2] < j - 1 ? rowslot[s_last[lane - 2]] : -1;
+            const unsigned m = __ballot_sync(0xffffffffu, v >= 0);
+            if (v >= 0) {
+                const int n = __popc(m & ((1u << lane) - 1u));
+                lo_[n] = v >= nvec - 1 ? (v & 1) * np4 : (2 + lane - 2) * np4;   // (lasts behind the ring)
+                lc[n] = x;
             }
+            if (lane == 0) { rowslot[j] = nvec; s_nl = __popc(m); }
         }
         ++nvec;
         __syncthreads();
-        nl0 = lt[15];
+        nl0 = s_nl;
     }
     for (int q = tid; q < L; q += kCpThreads) C.rowslot[q] = rowslot[q];
     if (tid == 0) {

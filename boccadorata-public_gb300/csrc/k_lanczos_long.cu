@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
     __shared__ int s_start[10], s_last[10], lslot[8], lt[16], lq[16];
     __shared__ double lc[16], s_row[32], s_tot[kMaxSc];
     __shared__ double s_n[3];   // 1/|w|, |w|, |E v|^2 of the kept vector
-    __shared__ int s_fl;        // 0 keep, 1 sweep again, 2 exhausted, 3 the full space's
+    __shared__ int s_fl;        // 0 keep, 1 sweep again, 2 exhausted, 3 the full space's, 4 sweep again (split too coarse)
     __shared__ unsigned s_rng[2];
     __shared__ float4 s_w2[2][NW / 4];   // the warps' parts of |w|^2, by the parity of A
     if (tid < 2) s_rng[tid] = 0;
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
     constexpr double tau = 1e-48, thr_exh = 1e-20;   // k_lanczos's, FP64 vectors
     int dcur = 0, ndefl = 0, extra = 0, k = -1, dpar = 0, spar = 0, nl0 = 0;
     double e2v = 0.0;
-    bool ok = true;
+    bool ok = true, rough = false;   // rough: w much shorter than what it was split against, swept again
     for (int j = 0; j < C.L; ++j) {
         const bool newv = (k + 1 < C.n_used) && (j == s_start[k + 1]);
         if (newv) ++k;
@@ -489,16 +489,17 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
                 // one threshold each)
                 if (warp == 0) {
                     const double x2 = s_tot[0];
-                    const double lim = lane == 0 ? eta2 * wn2 : (lane == 1 ? thr_exh : tau) * wn2_first;
+                    const double lim = lane == 0 ? eta2 * wn2 : (lane == 1 ? thr_exh : lane == 2 ? tau : kFixedShort) * wn2_first;
                     const unsigned lt_ = __ballot_sync(0xffffffffu, x2 < lim), le = __ballot_sync(0xffffffffu, x2 <= lim);
                     const long long xb = __double_as_longlong(x2);
                     const bool zero = (xb << 1) == 0, fin = (xb & 0x7ff0000000000000LL) != 0x7ff0000000000000LL;
                     int f;
                     if ((le & 2u) || zero) f = (dcur < dtot) ? 2 : 3;   // (further sweeps leave no more)
                     else if (nvec > 0 && nfull + 1 < 4 && (lt_ & 1u)) f = 1;
+                    else if (nvec > 0 && nfull == 0 && (lt_ & 8u)) f = 4;
                     else if (!(le & 4u) && fin) f = 0;
                     else f = 3;
-                    const double r = rsqrt_newton(x2);
+                    const double r = rsqrt_cubic(x2);
                     const double y = (lane == 0 ? 1.0 : lane == 1 ? x2 : s_tot[kMaxSc - 1] * r) * r;
                     if (lane < 3) s_n[lane] = y;   // 1/|w|, |w|, |E v|^2
                     if (lane == 0) s_fl = f;
@@ -506,8 +507,9 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
                 __syncthreads();
             }
             fl = s_fl;
-            if (nfull++ > 0) ++extra;
-            if (fl != 1) break;
+            if (nfull++ > 0 && !rough) ++extra;
+            rough = fl == 4;
+            if (fl != 1 && fl != 4) break;
             wn2 = s_tot[0];   // another sweep, of the updated w
             wbias = bias_above(wn2);
             for (int i = 4 * tid; i < S; i += 4 * T)

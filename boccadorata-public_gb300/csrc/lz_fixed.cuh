@@ -26,8 +26,32 @@ __device__ __forceinline__ void fixed_step(FixedSum &acc, int va, int vb, int wa
     acc.l += (long long)va * wb;
     acc.l += (long long)vb * wa;
 }
-__device__ __forceinline__ double fixed_value(FixedSum r, int bias) {   // times 2^(bias - 1023)
-    return ((double)(r.s + (r.l >> 27)) + (double)(r.l & 0x7ffffff) * 0x1p-27) * __hiloint2double((bias - 60) << 20, 0);
+// Times 2^(bias - 1023), rounded, from its bits: the FP64 forms of this are six instructions of
+// ~64 cycles in every warp of a sweep.
+__device__ __forceinline__ double fixed_value(FixedSum r, int bias) {
+    long long t = r.s + (r.l >> 27);             // value t + f 2^-27
+    unsigned f = (unsigned)r.l & 0x7ffffffu;
+    const bool neg = t < 0;
+    if (neg) {
+        t = -t - (f != 0);
+        f = (0u - f) & 0x7ffffffu;
+    }
+    unsigned long long m = (unsigned long long)t, lo = (unsigned long long)f << 37;   // m, then lo behind it
+    int z = __clzll((long long)m);
+    if (z == 64) {
+        m = lo;
+        lo = 0;
+        z = __clzll((long long)m);
+        if (z == 64) return 0.0;
+        m <<= z;
+        z += 64;
+    } else if (z > 0) {
+        m = (m << z) | (lo >> (64 - z));
+    }
+    // the leading bit, at bit 63, less itself, and half a unit; the carry goes to the exponent
+    const unsigned long long q = (((m & 0x7fffffffffffffffull) + (1u << 10)) >> 11) +
+                                 ((unsigned long long)(unsigned)(bias + 3 - z) << 52);
+    return __longlong_as_double((long long)(q | (neg ? 0x8000000000000000ull : 0)));
 }
 // a stored element as a double (abs. error 2^-58, or half a unit in the last place), from its bits
 __device__ __forceinline__ double fixed_to_double(int a, int b) {
@@ -46,16 +70,30 @@ __device__ __forceinline__ double f32_to_double(float x) {
     return __hiloint2double((int)((u & 0x80000000u) | ((m >> 3) + (896u << 20))), (int)(m << 29));
 }
 
-// x to FP32 from its bits, truncated; below 2^-70 zero
+// x to FP32 from its bits, truncated; below 2^-126 zero
 __device__ __forceinline__ float f32_trunc(double x) {
     const unsigned hi = (unsigned)__double2hiint(x);
     const unsigned b = (hi & 0x80000000u) | ((__funnelshift_l((unsigned)__double2loint(x), hi, 3) - (384u << 23)) & 0x7fffffffu);
-    return (hi & 0x7fffffffu) >= 953u << 20 ? __uint_as_float(b) : 0.0f;
+    return (hi & 0x7fffffffu) >= 897u << 20 ? __uint_as_float(b) : 0.0f;
+}
+
+// 1/sqrt(x), x > 0: the FP32 seed (2^-23) and one third-order step, five FP64 instructions where
+// two Newton steps with their conversions and comparisons are eleven
+__device__ __forceinline__ double rsqrt_cubic(double x) {
+    const unsigned e = (unsigned)__double2hiint(x) >> 20;
+    if (e < 1023 - 120 || e > 1023 + 120) return 1.0 / sqrt(x);
+    const double y = f32_to_double(__frsqrt_rn(f32_trunc(x)));
+    const double r = fma(-x * y, y, 1.0);
+    return fma(y * r, fma(0.375, r, 0.5), y);
 }
 
 // whether a set of values whose largest has this upper word (sign cleared) keeps to the
 // exponents FP32 has room for (2^+-40)
 __device__ __forceinline__ bool fixed_range(unsigned hi) { return hi >= (1023u - 40) << 20 && hi <= (1023u + 40) << 20; }
+// After a recurrence w is split against |E v_{j-1}|: where it is below 2^-6 of that (its square
+// below this part of the other's), the sums are too coarse for it and the sweep is repeated, split
+// against |w| itself.
+constexpr double kFixedShort = 0x1p-12;
 // the exponent field of a power of two above |x|, from |x|^2
 __device__ __forceinline__ int bias_above(double x2) {
     return ((__double2hiint(x2) >> 20) - 1023 + 2048) / 2 - 1024 + 1023 + 1;
