@@ -171,7 +171,9 @@ int bd_dyson_rows(bd_ctx *ctx, int ish, int nden, int n_fw, const double *fw_row
 
 /* Copy of the Lanczos basis of the last reduction of channel ish (dir 0 forward,
  * 1 backward) as L rows of N doubles; fp32 = 1 if it ran with BD_RUN_MIXED.  Used to
- * check the basis' orthonormality. */
+ * check the basis' orthonormality.  FP64 chains of few distinct energies are reduced in
+ * the space their couplings span and expanded here over the poles; long FP64 chains store
+ * their vectors to 2^-58. */
 int bd_lanczos_vectors(bd_ctx *ctx, int ish, int dir, int fp32, double *out, long long cap);
 
 /* Whole chain for every channel (flags BD_RUN_*), asynchronous on the context's
