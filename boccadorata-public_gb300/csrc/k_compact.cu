@@ -186,18 +186,23 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
     const int R = min(L, np);               // vectors, at most
     const int rq = (R + 4) & ~3, np4 = (np + 3) & ~3;
     const int nla = max(C.n_used - 1, 0);   // chains whose last vector later ones refer to
-    // shared layout (doubles): E[np4] | M[D][np4] (two planes of integers against s_mb) | w[np4] | ew[np4] | ring[2][np4] | last[nla][np4] |
-    // c[rq + 4] | sc[20], then ints wa[np4] | wb[np4] | Va[R][np4] | Vb[R][np4], floats cf[rq + 4] |
-    // Vf[R][np4], ints rowslot[L]
-    const size_t need = sizeof(double) * ((size_t)(D + 5 + nla) * np4 + rq + 4 + 20) +
-                        sizeof(int) * ((size_t)(2 + 3 * R) * np4 + rq + 4 + (size_t)L);
+    // shared layout (doubles): E[np4] | M[D][np4] (two planes of integers against s_mb) | w[np4] |
+    // ew[np4] | ring[2][np4] | last[nla][np4] | c[rq + 4] | sc[20] | part[256] (FixedSum) | wab[np4] (int2),
+    // then ints Va[np][RS] | Vb[np][RS] (element by element: a lane a vector reads consecutive ones, a lane an
+    // element ones an odd stride apart), floats cf[rq + 4], ints rowslot[L]
+    const int RS = R | 1;
+    const size_t need = sizeof(double) * ((size_t)(D + 6 + nla) * np4 + rq + 4 + 20 + 512) +
+                        sizeof(int) * (2 * (size_t)np * RS + rq + 4 + (size_t)L);
     if (s_bad || np > kCpDim || need > (size_t)kCpSmem) return;
     double *E = sm, *M = E + np4, *w = M + (size_t)D * np4;
-    double *ew = w + np4, *ring = ew + np4, *lasts = ring + 2 * np4,
-           *c = lasts + (size_t)nla * np4, *sc = c + rq + 4;
-    int *wa = reinterpret_cast<int *>(sc + 20), *wb = wa + np4, *Va = wb + np4, *Vb = Va + (size_t)R * np4;
-    float *cf = reinterpret_cast<float *>(Vb + (size_t)R * np4), *Vf = cf + rq + 4;
-    int *rowslot = reinterpret_cast<int *>(Vf + (size_t)R * np4);
+    double *ew = w + np4, *ring = ew + np4, *lasts = ring + 2 * np4, *c = lasts + (size_t)nla * np4, *sc = c + rq + 4;
+    FixedSum *part = reinterpret_cast<FixedSum *>(sc + 20);
+    float *fpart = reinterpret_cast<float *>(part);
+    int2 *wab = reinterpret_cast<int2 *>(part + 256);
+    int *Va = reinterpret_cast<int *>(wab + np4), *Vb = Va + (size_t)np * RS;
+    float *cf = reinterpret_cast<float *>(Vb + (size_t)np * RS);
+    int *rowslot = reinterpret_cast<int *>(cf + rq + 4);
+    static_assert(kCpThreads == 256, "part holds a sum a thread");
     unsigned me = 0, mm = 0;   // upper words of the largest |E| and |M|
     for (int g = warp; g < ng; g += kCpWarps) {
         const CompactGroup G = S.grp[g];
@@ -250,7 +255,7 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
     }
     __shared__ int s_start[10], s_last[10], lslot[8], lo_[16], s_nl, s_fl;
     __shared__ double lc[16], s_n[3];   // s_n: 1/|w|, |w|, |E v|^2 of the kept vector
-    __shared__ float s_f[kCpWarps];
+    __shared__ float s_f[kCpWarps], s_cm[kCpWarps];
     if (tid <= C.n_used && tid < 10) s_start[tid] = C.start[tid];
     if (tid < C.n_used && tid < 10) s_last[tid] = C.last[tid];
     // the groups' energies and unreached directions, cumulated (Q = gInfo[0])
@@ -273,10 +278,10 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
     auto vecd = [&](int t, int q) -> const double * { return t >= nvec - 2 ? ring + (t & 1) * np4 : lasts + (size_t)q * np4; };
     int wbias = 1023;   // exponent field of the power of two w is split against
     auto split_w = [&](int i, double x) {
-        const int2 f = fixed_of(x, wbias);
-        wa[i] = f.x;
-        wb[i] = f.y;
+        wab[i] = fixed_of(x, wbias);
     };
+    // the update's threads: an element each, npw apart the groups that share its vectors
+    const int npw = (np + 31) & ~31, tgs = kCpThreads / npw, tgp = tid / npw, ei = tid - tgp * npw;
     __syncthreads();
     for (int j = 0; j < L; ++j) {
         const bool newv = (k + 1 < C.n_used) && (j == s_start[k + 1]);
@@ -309,6 +314,7 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
         } else {
             wbias = bias_above(e2v);
             const double *v0 = ring + lo_[0];
+            float s2 = 0.0f;
             for (int i = tid; i < np; i += kCpThreads) {
                 double x = v0[i] * E[i];
                 for (int t0 = 0; t0 < nl0; t0 += 4) {
@@ -324,117 +330,130 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
                 }
                 w[i] = x;
                 split_w(i, x);
+                const float f = f32_trunc(x);
+                s2 = fmaf(f, f, s2);
             }
+            // |w|^2, read against the swept norm and the coefficients only: FP32
+            for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+            if (lane == 0) s_f[warp] = s2;
         }
         int fl, nfull = 0;
         for (;;) {
             __syncthreads();
-            // c_t = <v_t, w> for every stored vector, four a warp; after a recurrence |w|^2 as item
-            // nvec (read against the swept norm and the coefficients only: FP32)
+            // c_t = <v_t, w>, a lane a vector (no sums across lanes), the warps over groups of 32 vectors
+            // and parts of the elements
             const bool want_n = !newv && nfull == 0;
-            for (int t0 = 4 * warp; t0 < nvec + (want_n ? 1 : 0); t0 += 4 * kCpWarps) {
-                const int nu = min(4, nvec - t0);
-                if (nu > 0) {
-                    FixedSum acc[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) acc[u] = FixedSum{0, 0};
-                    const int *va = Va + (size_t)t0 * np4, *vb = Vb + (size_t)t0 * np4;
-                    for (int i = lane; i < np; i += 32) {
-                        const int xa = wa[i], xb = wb[i];
-#pragma unroll
-                        for (int u = 0; u < 4; ++u)
-                            if (u < nu) fixed_step(acc[u], va[u * np4 + i], vb[u * np4 + i], xa, xb);
+            {
+                const int tg = (nvec + 31) >> 5, P = tg > 0 ? kCpWarps / tg : 0;
+                const int gi = tg > 0 ? warp % tg : 0, pa = tg > 0 ? warp / tg : 1, v = 32 * gi + lane;
+                if (pa < P) {
+                    const int i1 = (pa + 1) * np / P, vc = min(v, nvec - 1);
+                    FixedSum acc{0, 0};
+                    const int *va = Va + vc, *vb = Vb + vc;
+#pragma unroll 4
+                    for (int i = pa * np / P; i < i1; ++i) {
+                        const int2 x = wab[i];
+                        fixed_step(acc, va[(size_t)i * RS], vb[(size_t)i * RS], x.x, x.y);
                     }
-                    const FixedSum r = warp_sums_of<4>(acc, lane, fixed_add, fixed_shfl);
-                    if ((lane & 7) == 0 && (lane >> 3) < nu) {
-                        const double x = fixed_value(r, wbias);
-                        const float xf = f32_trunc(x);
-                        c[t0 + (lane >> 3)] = x;
-                        cf[t0 + (lane >> 3)] = xf;
-                    }
+                    part[pa * 32 * tg + v] = acc;
                 }
-                if (want_n && nvec >= t0 && nvec < t0 + 4) {
-                    float s2 = 0.0f;
-                    for (int i = lane; i < np; i += 32) { const float f = f32_trunc(w[i]); s2 = fmaf(f, f, s2); }
-                    for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-                    if (lane == 0) { c[nvec] = (double)s2; cf[nvec] = s2; }
-                }
-            }
-            __syncthreads();
-            if (want_n) wn2 = c[nvec];
-            if (warp * 32 < np) {   // (whole warps: the sweep's size needs their lanes)
+                __syncthreads();
                 float cm = 0.0f;
-                for (int t = lane; t < nvec; t += 32) cm = fmaxf(cm, fabsf(cf[t]));
-                for (int o = 16; o > 0; o >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, o));
-                const float wf = want_n ? cf[nvec] : 0.0f;
-                const bool small = (cm * 1e9f) * (cm * 1e9f) * (float)max(nvec, 1) <= wf && wf > 1e-30f;
-                for (int i = tid; i < np; i += kCpThreads) {
-                    double x = w[i];
-                    if (small) {
-                        float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                        int t = 0;
-                        for (; t + 3 < nvec; t += 4)
+                for (int q = tid; q < nvec; q += kCpThreads) {
+                    FixedSum x = part[q];
+                    for (int r = 1; r < P; ++r) x = fixed_add(x, part[r * 32 * tg + q]);
+                    const double ct = fixed_value(x, wbias);
+                    c[q] = ct;
+                    cm = f32_trunc(ct);
+                    cf[q] = cm * 0x1p-30f;   // (against the a planes)
+                }
+                cm = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(cm))));
+                if (lane == 0) s_cm[warp] = cm;
+            }
+            __syncthreads();
+            float wf = 0.0f, cm = 0.0f;
 #pragma unroll
-                            for (int u = 0; u < 4; ++u) a[u] = fmaf(cf[t + u], Vf[(size_t)(t + u) * np4 + i], a[u]);
-                        for (; t < nvec; ++t) a[0] = fmaf(cf[t], Vf[(size_t)t * np4 + i], a[0]);
-                        x -= f32_to_double((a[0] + a[1]) + (a[2] + a[3]));
-                    } else {
-                        FixedSum acc{0, 0};
-                        for (int t = 0; t < nvec; ++t) {
-                            const int2 ct = fixed_of(c[t], wbias);
-                            fixed_step(acc, Va[(size_t)t * np4 + i], Vb[(size_t)t * np4 + i], ct.x, ct.y);
-                        }
-                        x -= fixed_value(acc, wbias);
+            for (int q = 0; q < kCpWarps; ++q) { wf += s_f[q]; cm = fmaxf(cm, s_cm[q]); }
+            if (want_n) wn2 = (double)wf;
+            const bool small = want_n && (cm * 1e9f) * (cm * 1e9f) * (float)max(nvec, 1) <= wf && wf > 1e-30f;
+            // the update: every element's sum by tgs threads, each its part of the vectors
+            if (tgp < tgs && ei < np) {
+                const int t0 = tgp * nvec / tgs, t1 = (tgp + 1) * nvec / tgs;
+                const int *va = Va + (size_t)ei * RS, *vb = Vb + (size_t)ei * RS;
+                if (small) {
+                    float a0 = 0.0f, a1 = 0.0f;
+                    int q = t0;
+                    for (; q + 1 < t1; q += 2) {
+                        a0 = fmaf(cf[q], (float)va[q], a0);
+                        a1 = fmaf(cf[q + 1], (float)va[q + 1], a1);
                     }
-                    w[i] = x;
-                    split_w(i, x);   // (for m; the dot products are done)
-                    ew[i] = E[i] * x;
+                    if (q < t1) a0 = fmaf(cf[q], (float)va[q], a0);
+                    fpart[tid] = a0 + a1;
+                } else {
+                    FixedSum acc{0, 0};
+                    for (int q = t0; q < t1; ++q) {
+                        const int2 ct = fixed_of(c[q], wbias);
+                        fixed_step(acc, va[q], vb[q], ct.x, ct.y);
+                    }
+                    part[tid] = acc;
                 }
             }
             __syncthreads();
-            // the scalars of the updated w: |w|^2, <w|E|w>, |E w|^2, <v_last(q)|E|w> in FP64, two a warp
-            // and round, beside <M_d|w> in fixed point, four a warp
-            const int nsc = 3 + nq;
-            if (warp >= kCpWarps - 2) {
-                const int d0 = 4 * (kCpWarps - 1 - warp);
-                if (d0 < D) {
+            for (int i = tid; i < np; i += kCpThreads) {
+                double x = w[i];
+                if (small) {
+                    float a = fpart[i];
+                    for (int r = 1; r < tgs; ++r) a += fpart[r * npw + i];
+                    x -= f32_to_double(a);
+                } else {
+                    FixedSum acc = part[i];
+                    for (int r = 1; r < tgs; ++r) acc = fixed_add(acc, part[r * npw + i]);
+                    x -= fixed_value(acc, wbias);
+                }
+                w[i] = x;
+                split_w(i, x);   // (for |w|^2 and m; the dot products are done)
+                ew[i] = E[i] * x;
+            }
+            __syncthreads();
+            // the scalars of the updated w: <w|E|w> and <v_last(q)|E|w> in FP64, a warp each, beside |w|^2 and
+            // <M_d|w> in fixed point (w is no shorter than kFixedShort allows against what it is split
+            // against), four a warp, and |E w|^2, a threshold's scale, in FP32
+            if (warp >= kCpWarps - 3) {
+                const int f0 = 4 * (kCpWarps - 1 - warp);   // item 0 |w|^2, 1 + d <M_d|w>
+                if (f0 < D + 1) {
                     FixedSum acc[4];
 #pragma unroll
                     for (int u = 0; u < 4; ++u) acc[u] = FixedSum{0, 0};
                     for (int i = lane; i < np; i += 32) {
-                        const int xa = wa[i], xb = wb[i];
+                        const int2 x = wab[i];
 #pragma unroll
-                        for (int u = 0; u < 4; ++u)
-                            if (d0 + u < D) fixed_step(acc[u], Ma[(size_t)(d0 + u) * np4 + i], Mb[(size_t)(d0 + u) * np4 + i], xa, xb);
+                        for (int u = 0; u < 4; ++u) {
+                            const int d = f0 + u - 1;
+                            if (d < 0) fixed_step(acc[u], x.x, x.y, x.x, x.y);
+                            else if (d < D) fixed_step(acc[u], Ma[(size_t)d * np4 + i], Mb[(size_t)d * np4 + i], x.x, x.y);
+                        }
                     }
                     const FixedSum r = warp_sums_of<4>(acc, lane, fixed_add, fixed_shfl);
-                    const int d = d0 + (lane >> 3);
-                    if ((lane & 7) == 0 && d < D) sc[3 + d] = fixed_value(r, wbias + s_mb[d] - 1023);
+                    const int d = f0 + (lane >> 3) - 1;
+                    if ((lane & 7) == 0 && d < D) {
+                        if (d < 0) sc[0] = fixed_value(r, 2 * wbias - 1023);
+                        else sc[3 + d] = fixed_value(r, wbias + s_mb[d] - 1023);
+                    }
+                }
+                if (warp == kCpWarps - 3) {
+                    float s2 = 0.0f;
+                    for (int i = lane; i < np; i += 32) { const float f = f32_trunc(ew[i]); s2 = fmaf(f, f, s2); }
+                    for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+                    if (lane == 0) sc[2] = (double)s2;
                 }
             } else {
-                for (int t0 = 2 * warp; t0 < nsc; t0 += 2 * (kCpWarps - 2)) {
-                    const double *a[2], *b[2];
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        const int t = t0 + u;
-                        a[u] = w;
-                        b[u] = w;
-                        if (t == 1) b[u] = ew;
-                        else if (t == 2) { a[u] = ew; b[u] = ew; }
-                        else if (t >= 3 && t < nsc && lslot[t - 3] >= 0) { a[u] = vecd(lslot[t - 3], t - 3); b[u] = ew; }
-                    }
-                    double x[2] = {0.0, 0.0};
-                    for (int i = lane; i < np; i += 32) {
-                        x[0] = fma(a[0][i], b[0][i], x[0]);
-                        x[1] = fma(a[1][i], b[1][i], x[1]);
-                    }
-                    const double r = warp_sums_of<2>(x, lane, [](double p, double q) { return p + q; },
-                                                     [](double p, int o) { return __shfl_xor_sync(0xffffffffu, p, o); });
-                    const int t = t0 + (lane >> 4);
-                    if ((lane & 15) == 0 && t < nsc) {
-                        if (t < 3) sc[t] = r;
-                        else sc[D + t] = lslot[t - 3] < 0 ? 0.0 : r;
-                    }
+                for (int q = warp - 1; q < nq; q += kCpWarps - 3) {   // q -1: <w|E|w>
+                    const double *a = q < 0 ? w : lslot[q] >= 0 ? vecd(lslot[q], q) : nullptr;
+                    double x = 0.0;
+                    if (a)
+                        for (int i = lane; i < np; i += 32) x = fma(a[i], ew[i], x);
+                    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+                    if (lane == 0) sc[q < 0 ? 1 : 3 + D + q] = x;
                 }
             }
             __syncthreads();
@@ -494,9 +513,8 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
             for (int i = tid; i < np; i += kCpThreads) {
                 const double v = w[i] * ixb;
                 const int2 f = fixed_of(v, 1023);
-                Va[(size_t)nvec * np4 + i] = f.x;
-                Vb[(size_t)nvec * np4 + i] = f.y;
-                Vf[(size_t)nvec * np4 + i] = (float)f.x * 0x1p-30f;
+                Va[(size_t)i * RS + nvec] = f.x;
+                Vb[(size_t)i * RS + nvec] = f.y;
                 rg[i] = v;
                 if (rl) rl[i] = v;
                 reinterpret_cast<double *>(C.V)[(size_t)nvec * np + i] = v;   // (np <= N: within the chain's store)
