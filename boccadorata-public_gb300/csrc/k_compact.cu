@@ -61,7 +61,7 @@ __device__ bool warp_cholesky(const double *tri, int D, double *out, int lane) {
         if (!zero && !(p > kPivot * g && p <= DBL_MAX)) ok = false;
         if (!ok) break;   // the same in every lane
         // (Newton's iteration to a few ulp: FP64 square root and division are chains of their own)
-        const double ri = zero ? 0.0 : rsqrt_newton(p), r = p * ri;
+        const double ri = zero ? 0.0 : rsqrt_cubic(p), r = p * ri;
         __syncwarp();
         if (lane >= s && lane < D) out[lane * D + s] = (lane == s) ? r : out[lane * D + s] * ri;
         __syncwarp();
@@ -120,13 +120,17 @@ static_assert(kCpThreads >= kCpGroups, "a thread per exact group");
 // group has left) is left to k_lanczos as a whole.
 //
 // A step is a chain of short phases between barriers, and an FP64 instruction holds an SM
-// sub-partition's FP64 unit for ~64 cycles, so FP64 is kept to what needs it: the sweep's dot
-// products and m are fixed-point sums (lz_fixed.cuh; four vectors a warp), its update FP32 where the
-// coefficients are rounding-sized (|c| <= 1e-9 |w|: an error below 2^-23 1e-9 |w|) and fixed
-// point otherwise, and one warp takes the decision.  The norm, alpha, g and the recurrence are
-// FP64.
+// sub-partition's FP64 unit for ~64 cycles, so FP64 is kept to what needs it (alpha, g, the
+// recurrence, 1/|w|): the sweep's dot products, |w|^2 and m are fixed-point sums (lz_fixed.cuh),
+// the update is FP32 where the coefficients are rounding-sized (|c| <= 1e-9 |w|: an error below
+// 2^-23 1e-9 |w|) and fixed point otherwise.  Stored vectors lie element by element: in the dot
+// products a lane takes a vector and the warps split the elements, in the update a thread takes
+// an element and the idle ones split the vectors, so neither sums across lanes; one warp takes
+// the decision beside the other warps' sums.
 // Measured (N_max = 10, 100 iterations per pivot): the reduction of all 84 chains takes
-// 0.36 ms against 3.59 ms in the poles' space (N_max = 12: 0.53 against 12.2).
+// 0.30 ms against 3.59 ms in the poles' space (N_max = 12: 0.44 against 12.2); about 8 000 cycles
+// a step of a 54-coordinate chain (11 000 with a warp's lanes summing each dot product and the
+// decision after them).
 __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains, int nchains, double eta2) {
     const int cid = blockIdx.x;
     if (cid >= nchains) return;
@@ -256,6 +260,8 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
     __shared__ int s_start[10], s_last[10], lslot[8], lo_[16], s_nl, s_fl;
     __shared__ double lc[16], s_n[3];   // s_n: 1/|w|, |w|, |E v|^2 of the kept vector
     __shared__ float s_f[kCpWarps], s_cm[kCpWarps];
+    __shared__ double s_piv[80];   // at most 9 pivots of 8
+    for (int q = tid; q < C.n_used * D && q < 80; q += kCpThreads) s_piv[q] = C.piv[q];
     if (tid <= C.n_used && tid < 10) s_start[tid] = C.start[tid];
     if (tid < C.n_used && tid < 10) s_last[tid] = C.last[tid];
     // the groups' energies and unreached directions, cumulated (Q = gInfo[0])
@@ -293,7 +299,7 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
         if (newv) {
             float s2 = 0.0f;
             for (int i = tid; i < np; i += kCpThreads) {
-                const double *p = C.piv + (size_t)k * D;
+                const double *p = s_piv + k * D;
                 double x = 0.0;
                 for (int d = 0; d < D; ++d)
                     x = fma(fixed_to_double(Ma[(size_t)d * np4 + i], Mb[(size_t)d * np4 + i]) *
@@ -415,52 +421,26 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
                 ew[i] = E[i] * x;
             }
             __syncthreads();
-            // the scalars of the updated w: <w|E|w> and <v_last(q)|E|w> in FP64, a warp each, beside |w|^2 and
-            // <M_d|w> in fixed point (w is no shorter than kFixedShort allows against what it is split
-            // against), four a warp, and |E w|^2, a threshold's scale, in FP32
-            if (warp >= kCpWarps - 3) {
-                const int f0 = 4 * (kCpWarps - 1 - warp);   // item 0 |w|^2, 1 + d <M_d|w>
-                if (f0 < D + 1) {
-                    FixedSum acc[4];
+            // the scalars of the updated w: <w|E|w> and <v_last(q)|E|w> in FP64, a warp each, beside <M_d|w> in
+            // fixed point, four a warp; the last warp takes |w|^2, in fixed point too (w is no shorter than
+            // kFixedShort allows against what it is split against), |E w|^2, a threshold's scale, in FP32, and
+            // with them k_lanczos's decision, its lanes one threshold each (exhaustion first: further sweeps of
+            // a w that holds nothing leave nothing)
+            if (warp == kCpWarps - 1) {
+                FixedSum p{0, 0};
+                float s2 = 0.0f;
+                for (int i = lane; i < np; i += 32) {
+                    const int2 x = wab[i];
+                    fixed_step(p, x.x, x.y, x.x, x.y);
+                    const float f = f32_trunc(ew[i]);
+                    s2 = fmaf(f, f, s2);
+                }
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) acc[u] = FixedSum{0, 0};
-                    for (int i = lane; i < np; i += 32) {
-                        const int2 x = wab[i];
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const int d = f0 + u - 1;
-                            if (d < 0) fixed_step(acc[u], x.x, x.y, x.x, x.y);
-                            else if (d < D) fixed_step(acc[u], Ma[(size_t)d * np4 + i], Mb[(size_t)d * np4 + i], x.x, x.y);
-                        }
-                    }
-                    const FixedSum r = warp_sums_of<4>(acc, lane, fixed_add, fixed_shfl);
-                    const int d = f0 + (lane >> 3) - 1;
-                    if ((lane & 7) == 0 && d < D) {
-                        if (d < 0) sc[0] = fixed_value(r, 2 * wbias - 1023);
-                        else sc[3 + d] = fixed_value(r, wbias + s_mb[d] - 1023);
-                    }
+                for (int o = 16; o > 0; o >>= 1) {
+                    p = fixed_add(p, fixed_shfl(p, o));
+                    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
                 }
-                if (warp == kCpWarps - 3) {
-                    float s2 = 0.0f;
-                    for (int i = lane; i < np; i += 32) { const float f = f32_trunc(ew[i]); s2 = fmaf(f, f, s2); }
-                    for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-                    if (lane == 0) sc[2] = (double)s2;
-                }
-            } else {
-                for (int q = warp - 1; q < nq; q += kCpWarps - 3) {   // q -1: <w|E|w>
-                    const double *a = q < 0 ? w : lslot[q] >= 0 ? vecd(lslot[q], q) : nullptr;
-                    double x = 0.0;
-                    if (a)
-                        for (int i = lane; i < np; i += 32) x = fma(a[i], ew[i], x);
-                    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-                    if (lane == 0) sc[q < 0 ? 1 : 3 + D + q] = x;
-                }
-            }
-            __syncthreads();
-            // k_lanczos's decision, by warp 0 (its lanes take one threshold each); exhaustion first:
-            // further sweeps of a w that holds nothing leave nothing
-            if (warp == 0) {
-                const double x2 = sc[0];
+                const double x2 = fixed_value(p, 2 * wbias - 1023);
                 const double lim = lane == 0 ? eta2 * wn2 : (lane == 1 ? thr_exh : lane == 2 ? tau : kFixedShort) * wn2_first;
                 const unsigned lt_ = __ballot_sync(0xffffffffu, x2 < lim), le = __ballot_sync(0xffffffffu, x2 <= lim);
                 const long long xb = __double_as_longlong(x2);
@@ -472,9 +452,34 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
                 else if (!(le & 4u) && fin) f = 0;
                 else f = 3;   // (not finite)
                 const double r = rsqrt_cubic(x2);
-                const double y = (lane == 0 ? 1.0 : lane == 1 ? x2 : sc[2] * r) * r;
+                const double y = (lane == 0 ? 1.0 : lane == 1 ? x2 : f32_to_double(s2) * r) * r;
                 if (lane < 3) s_n[lane] = y;
-                if (lane == 0) s_fl = f;
+                if (lane == 0) { sc[0] = x2; s_fl = f; }
+            } else if (warp >= kCpWarps - 3) {
+                const int d0 = 4 * (kCpWarps - 2 - warp);
+                if (d0 < D) {
+                    FixedSum acc[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) acc[u] = FixedSum{0, 0};
+                    for (int i = lane; i < np; i += 32) {
+                        const int2 x = wab[i];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (d0 + u < D) fixed_step(acc[u], Ma[(size_t)(d0 + u) * np4 + i], Mb[(size_t)(d0 + u) * np4 + i], x.x, x.y);
+                    }
+                    const FixedSum r = warp_sums_of<4>(acc, lane, fixed_add, fixed_shfl);
+                    const int d = d0 + (lane >> 3);
+                    if ((lane & 7) == 0 && d < D) sc[3 + d] = fixed_value(r, wbias + s_mb[d] - 1023);
+                }
+            } else {
+                for (int q = warp - 1; q < nq; q += kCpWarps - 3) {   // q -1: <w|E|w>
+                    const double *a = q < 0 ? w : lslot[q] >= 0 ? vecd(lslot[q], q) : nullptr;
+                    double x = 0.0;
+                    if (a)
+                        for (int i = lane; i < np; i += 32) x = fma(a[i], ew[i], x);
+                    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+                    if (lane == 0) sc[q < 0 ? 1 : 3 + D + q] = x;
+                }
             }
             __syncthreads();
             fl = s_fl;
