@@ -103,7 +103,7 @@ __host__ __device__ inline size_t tdg_count(int n) { return tdg_exchange(n) + 4 
 // One CTA per matrix: the compact index of every kept row (work area, ints; -1 for a
 // deflated row), the compact order into the job, and the deflated rows' solutions
 // [W, 0, 0 ..] staged behind R after the nc rows the eigensolver will stage.
-constexpr int kDfThreads = 256;
+constexpr int kDfThreads = 1024;
 
 __global__ void __launch_bounds__(kDfThreads) k_dyson_deflate(DyJob *jobs, int njobs, double *work,
                                                               const long long *work_first) {

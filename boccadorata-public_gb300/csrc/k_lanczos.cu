@@ -700,33 +700,53 @@ __global__ void __launch_bounds__(kLzThreads, 2) k_lanczos(const LzChain *chains
                 for (int u = 0; u < VW; ++u) acc[u] += cr * x[r][u];
             }
         }
-        const int rem = nl - t;   // the last ones' loads together too
-        if (rem > 0) {
-            VT x[7][VW];
-#pragma unroll
-            for (int r = 0; r < 7; ++r) {
-                const int tt = min(t + r, nl - 1);
-                load16g<VT>(vslice(loc ? lt[tt] : tt) + qo, x[r]);
-            }
-            if (rem >= 4) {
+        if constexpr (sizeof(VT) == 8) {
+            for (; t + 3 < nl; t += 4) {
+                VT x0[VW], x1[VW], x2[VW], x3[VW];
+                load16g<VT>(vslice(loc ? lt[t] : t) + qo, x0);
+                load16g<VT>(vslice(loc ? lt[t + 1] : t + 1) + qo, x1);
+                load16g<VT>(vslice(loc ? lt[t + 2] : t + 2) + qo, x2);
+                load16g<VT>(vslice(loc ? lt[t + 3] : t + 3) + qo, x3);
                 const CT c0 = cf[t], c1 = cf[t + 1], c2 = cf[t + 2], c3 = cf[t + 3];
 #pragma unroll
-                for (int u = 0; u < VW; ++u) acc[u] += c0 * x[0][u] + c1 * x[1][u] + c2 * x[2][u] + c3 * x[3][u];
+                for (int u = 0; u < VW; ++u) acc[u] += c0 * x0[u] + c1 * x1[u] + c2 * x2[u] + c3 * x3[u];
+            }
+            for (; t < nl; ++t) {
+                VT x0[VW];
+                load16g<VT>(vslice(loc ? lt[t] : t) + qo, x0);
+                const CT c0 = cf[t];
 #pragma unroll
-                for (int r = 4; r < 7; ++r)
-                    if (r < rem) {
-                        const CT cr = cf[t + r];
+                for (int u = 0; u < VW; ++u) acc[u] += c0 * x0[u];
+            }
+        } else {
+            const int rem = nl - t;   // the last ones' loads together too
+            if (rem > 0) {
+                VT x[7][VW];
 #pragma unroll
-                        for (int u = 0; u < VW; ++u) acc[u] += cr * x[r][u];
-                    }
-            } else {
+                for (int r = 0; r < 7; ++r) {
+                    const int tt = min(t + r, nl - 1);
+                    load16g<VT>(vslice(loc ? lt[tt] : tt) + qo, x[r]);
+                }
+                if (rem >= 4) {
+                    const CT c0 = cf[t], c1 = cf[t + 1], c2 = cf[t + 2], c3 = cf[t + 3];
 #pragma unroll
-                for (int r = 0; r < 3; ++r)
-                    if (r < rem) {
-                        const CT cr = cf[t + r];
+                    for (int u = 0; u < VW; ++u) acc[u] += c0 * x[0][u] + c1 * x[1][u] + c2 * x[2][u] + c3 * x[3][u];
 #pragma unroll
-                        for (int u = 0; u < VW; ++u) acc[u] += cr * x[r][u];
-                    }
+                    for (int r = 4; r < 7; ++r)
+                        if (r < rem) {
+                            const CT cr = cf[t + r];
+#pragma unroll
+                            for (int u = 0; u < VW; ++u) acc[u] += cr * x[r][u];
+                        }
+                } else {
+#pragma unroll
+                    for (int r = 0; r < 3; ++r)
+                        if (r < rem) {
+                            const CT cr = cf[t + r];
+#pragma unroll
+                            for (int u = 0; u < VW; ++u) acc[u] += cr * x[r][u];
+                        }
+                }
             }
         }
     };
@@ -890,6 +910,26 @@ __global__ void __launch_bounds__(kLzThreads, 2) k_lanczos(const LzChain *chains
             // (lt, lcf, s_nl), listed by warp 0 when it wrote row j - 1
             const int nl0 = s_nl;
             const VT *vp0 = vslice(lt[0]);
+            if constexpr (sizeof(VT) == 8) {   // vectors mostly in shared memory: one group at a time
+                for (int q = tid; q < nv; q += kLzThreads) {
+                    const int qo = q * VW;
+                    VT x0[VW];
+                    load16g<VT>(vp0 + qo, x0);
+                    CT x[VW];
+#pragma unroll
+                    for (int u = 0; u < VW; ++u) x[u] = (CT)x0[u] * Es[qo + u];
+#pragma unroll 4
+                    for (int t = 0; t < nl0; ++t) {
+                        VT y[VW];
+                        load16g<VT>(vslice(lt[t]) + qo, y);
+                        const CT ct = lcf[t];
+#pragma unroll
+                        for (int u = 0; u < VW; ++u) x[u] -= ct * (CT)y[u];
+                    }
+#pragma unroll
+                    for (int u = 0; u < VW; ++u) w[qo + u] = x[u];
+                }
+            } else
             for (int q = tid; q < nv; q += 2 * kLzThreads) {   // two groups a thread, loads first
                 const bool two = q + kLzThreads < nv;
                 const int qo[2] = {q * VW, (two ? q + kLzThreads : q) * VW};
