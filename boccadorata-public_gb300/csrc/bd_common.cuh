@@ -329,17 +329,6 @@ __device__ inline double rcp_newton(double q) {
     return 1.0 / q;
 }
 
-// 1/q to a few ulp (two steps)
-__device__ inline double rcp_newton2(double q) {
-    const double aq = fabs(q);
-    if (aq > 1e-36 && aq < 1e36) {
-        double r = (double)__frcp_rn((float)q);
-        r = fma(r, fma(-q, r, 1.0), r);
-        return fma(r, fma(-q, r, 1.0), r);
-    }
-    return 1.0 / q;
-}
-
 // 1/sqrt(x), x > 0, to a few ulp: the FP32 seed and two steps of y <- y (3/2 - x y^2 / 2)
 __device__ inline double rsqrt_newton(double x) {
     if (x > 1e-36 && x < 1e36) {

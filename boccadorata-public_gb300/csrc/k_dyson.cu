@@ -966,11 +966,6 @@ constexpr int kTsIt = kTsMax / 32;            // column entries per lane of warp
 static_assert(kTsMax % 32 == 0, "warp 0 holds a column in kTsIt entries per lane");
 static_assert(2 * kTsMax <= kTsThreads, "the R update keeps at least half the threads");
 
-__device__ inline double warp_sum(double v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 // Binary exponent of a non-zero float (denormals give -127), and 2^e for -126 <= e <= 127.
 __device__ inline int f32_exp(float x) { return (int)((__float_as_uint(x) >> 23) & 255u) - 127; }
 __device__ inline float f32_pow2(int e) { return __uint_as_float((unsigned)(e + 127) << 23); }

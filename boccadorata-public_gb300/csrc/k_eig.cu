@@ -248,7 +248,6 @@ struct InvitSharedDF {   // shared memory, element i of this thread at i * kIvTh
     __device__ void set_pv(int i, bool b) { PV[i * kIvThreads + lane] = b ? 1 : 0; }
 };
 
-__device__ inline dfm::df df_abs(dfm::df a) { return a.h < 0.0f ? dfm::neg(a) : a; }
 __device__ inline dfm::df df_sub(dfm::df a, dfm::df b) { return dfm::add(a, dfm::neg(b)); }
 
 __device__ void invit_vector_df(const DyJob &J, int k, int b0, int b1, const dfm::df *dt, const dfm::df *et,
