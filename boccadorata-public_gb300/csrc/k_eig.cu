@@ -23,6 +23,7 @@
 #include <climits>
 #include "bd_common.cuh"
 #include "df64.cuh"
+#include "lz_fixed.cuh"
 #include "bd_kernels.h"
 #include "eig_sturm.cuh"
 
@@ -407,7 +408,9 @@ __global__ void __launch_bounds__(kIvLarge) k_invit(const DyJob *jobs, int njobs
     auto mag = [](double v) { return __double_as_longlong(v) & 0x7fffffffffffffffLL; };
     const long long pmag = mag(tl.pertol);
     auto clamp_piv = [&](double p) { return mag(p) < pmag ? (p < 0.0 ? -tl.pertol : tl.pertol) : p; };
-    auto start = [&](int i) { return 0.5 + (double)(hash32((unsigned)(i * 2654435761u) ^ (unsigned)(k * 97 + 13)) & 0xffff) / 65536.0; };
+    auto start = [&](int i) {   // in [0.5, 1.5), exact in FP32
+        return f32_to_double(0.5f + (float)(hash32((unsigned)(i * 2654435761u) ^ (unsigned)(k * 97 + 13)) & 0xffff) * 0x1p-16f);
+    };
     // LU with partial pivoting of T_b - x I (rows i and i+1 may swap); pivots no smaller than
     // pertol, kept as reciprocals
     double cur_d = d[b0] - x, cur_u = e[b0], cur_y = start(b0);
@@ -416,9 +419,9 @@ __global__ void __launch_bounds__(kIvLarge) k_invit(const DyJob *jobs, int njobs
         const double li = e[i], nd = d[i + 1] - x, nu = (i + 1 < b1) ? e[i + 1] : 0.0, yn = start(i + 1);
         const bool sw = mag(cur_d) < mag(li);
         const double piv = sw ? li : cur_d, oth = sw ? cur_d : li, cp = clamp_piv(piv);
-        const double r = rcp_newton(cp);
+        const double r = rcp_cubic(cp);
         // (a pivot below pertol: the multiplier from the pivot itself, zero for a zero pivot)
-        const double f = (__double_as_longlong(cp) == __double_as_longlong(piv)) ? oth * r : (mag(piv) != 0 ? oth * rcp_newton(piv) : 0.0);
+        const double f = (__double_as_longlong(cp) == __double_as_longlong(piv)) ? oth * r : (mag(piv) != 0 ? oth * rcp_cubic(piv) : 0.0);
         const double ui = sw ? nd : cur_u, uo = sw ? cur_u : nd;
         const double yi = sw ? yn : cur_y, yo = sw ? cur_y : yn;
         const size_t o = (size_t)i * n;
@@ -435,7 +438,7 @@ __global__ void __launch_bounds__(kIvLarge) k_invit(const DyJob *jobs, int njobs
     }
     U1[(size_t)b1 * n] = 0.0;
     U2[(size_t)b1 * n] = 0.0;
-    DD[(size_t)b1 * n] = rcp_newton(clamp_piv(cur_d));
+    DD[(size_t)b1 * n] = rcp_cubic(clamp_piv(cur_d));
     Y[(size_t)b1 * n] = cur_y;
     // two sweeps: the shift is within 1e-13 |T_b| of W_k and eigenvalues of a block
     // closer than 1e-6 |T_b| are clustered (orthonormalised together), so each sweep
@@ -462,7 +465,7 @@ __global__ void __launch_bounds__(kIvLarge) k_invit(const DyJob *jobs, int njobs
         }
     };
     back();
-    double sc = nmag > 0 ? rcp_newton(__longlong_as_double(nmag)) : 1.0;
+    double sc = nmag > 0 ? rcp_cubic(__longlong_as_double(nmag)) : 1.0;
     double cur = Y[(size_t)b0 * n] * sc;
     for (int t = b0; t < b1; t += kIvAhead) {   // L^-1 with the interchanges, on the scaled iterate
         double ll[kIvAhead], yn[kIvAhead];
@@ -484,7 +487,7 @@ __global__ void __launch_bounds__(kIvLarge) k_invit(const DyJob *jobs, int njobs
     }
     Y[(size_t)b1 * n] = cur;
     back();
-    sc = nmag > 0 ? rcp_newton(__longlong_as_double(nmag)) : 1.0;
+    sc = nmag > 0 ? rcp_cubic(__longlong_as_double(nmag)) : 1.0;
     double s2a = 0.0, s2b = 0.0;   // two chains
     for (int t = b0; t <= b1; t += kIvAhead) {
         double yy[kIvAhead];

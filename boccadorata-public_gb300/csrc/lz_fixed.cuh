@@ -87,6 +87,15 @@ __device__ __forceinline__ double rsqrt_cubic(double x) {
     return fma(y * r, fma(0.375, r, 0.5), y);
 }
 
+// 1/q: the FP32 seed and one third-order step, three FP64 instructions
+__device__ __forceinline__ double rcp_cubic(double q) {
+    const unsigned e = ((unsigned)__double2hiint(q) >> 20) & 0x7ffu;
+    if (e < 1023 - 120 || e > 1023 + 120) return 1.0 / q;
+    const double y = f32_to_double(__frcp_rn(f32_trunc(q)));
+    const double r = fma(-q, y, 1.0);
+    return fma(y, fma(r, r, r), y);
+}
+
 // whether a set of values whose largest has this upper word (sign cleared) keeps to the
 // exponents FP32 has room for (2^+-40)
 __device__ __forceinline__ bool fixed_range(unsigned hi) { return hi >= (1023u - 40) << 20 && hi <= (1023u + 40) << 20; }
