@@ -314,7 +314,10 @@ __device__ inline double vget(const DevProblem &P, int ia, int ib, int ic, int i
     return 0.0;
 }
 
-// 1/sqrt(x), x > 0, to a few ulp: the FP32 seed and two steps of y <- y (3/2 - x y^2 / 2)
+// FP64 division and square root are dependent chains of about ten FP64 instructions,
+// each of which holds an SM sub-partition's FP64 unit for ~64 cycles on this GPU; where
+// a few ulp suffice an FP32 seed refined by Newton's iteration replaces them.
+// 1/sqrt(x), x > 0: two steps of y <- y (3/2 - x y^2 / 2)
 __device__ inline double rsqrt_newton(double x) {
     if (x > 1e-36 && x < 1e36) {
         const double hx = 0.5 * x;

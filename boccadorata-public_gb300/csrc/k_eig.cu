@@ -359,7 +359,7 @@ __device__ void invit_vector_df(const DyJob &J, int k, int b0, int b1, const dfm
 // rows' factors before they use them: the L2 round trips overlap instead of adding one to
 // every row.  The pivoting is by selects (a warp's lanes disagree about it row by row).  What
 // is left is the FP64 unit, about twenty instructions a row at ~64 cycles each; 1 000
-// positions are 32 warps, one an SM.  Order 1 000: 4.06 -> 1.43 ms.
+// positions are 32 warps, one an SM.  Order 1 000: 4.06 -> 1.32 ms.
 constexpr int kIvAhead = 8;
 constexpr int kIvLarge = 32;   // positions per CTA
 constexpr int kIvTri = 6144;   // rows of the tridiagonal kept in shared memory
