@@ -743,6 +743,7 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_grid(const DyJob *jo
     df *Yx = reinterpret_cast<df *>(wk + tdg_exchange(J.n)), *Bx = Yx + 2 * (size_t)n, *Kx = Bx + 2 * (size_t)n;
     unsigned *count = reinterpret_cast<unsigned *>(wk + tdg_count(J.n));
     __shared__ df s_sc[2], s_rd, s_c;   // tau, s of the step; R_d . x of the own R row, -tau R_d . v
+    __shared__ df s_k[2];               // -(tau^2 / 2) v^T A v, w_{k+1}
     const df zero{0.0f, 0.0f}, one{1.0f, 0.0f};
     const bool own_r = rank < D;
     auto put = [](double *p, df x) { *reinterpret_cast<float2 *>(p) = make_float2(x.h, x.l); };
@@ -870,30 +871,36 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_grid(const DyJob *jo
         }
         // all rows: v, w; R; x of the next step
         {
-            // all that comes from L2 first
+            // all that comes from L2 first; the parts' sum and what follows from it by one warp (by every
+            // warp it takes the FP32 pipe from the others: 2 700 cycles)
             constexpr int NA = 2;   // rows a thread has ahead
-            df ya[NA], ba[NA], ka[kTdgMax / 32];
+            df ya[NA], ba[NA];
 #pragma unroll
             for (int h = 0; h < NA; ++h) {
                 const int j = min(b0 + tid + h * kTdfThreads, n - 1);
                 ya[h] = far(yk + j);
                 ba[h] = far(bk + j);
             }
+            const df vb = nz ? one : zero;
+            if (warp == 0) {
+                df ka[kTdgMax / 32];
 #pragma unroll
-            for (int h = 0; h < kTdgMax / 32; ++h) ka[h] = lane + 32 * h < G ? far(kb + lane + 32 * h) : zero;
-            const df yb = far(yk + b0);
+                for (int h = 0; h < kTdgMax / 32; ++h) ka[h] = lane + 32 * h < G ? far(kb + lane + 32 * h) : zero;
+                const df yb = far(yk + b0);
 #pragma unroll
-            for (int o = kTdgMax / 64; o > 0; o >>= 1)
+                for (int o = kTdgMax / 64; o > 0; o >>= 1)
 #pragma unroll
-                for (int h = 0; h < o; ++h) ka[h] = dfm::add(ka[h], ka[h + o]);
-            const df K = dfm::warp_sum(ka[0]);
-            const df tk = dfm::mul(tau, tau);
-            const df nK = dfm::neg(dfm::mul(df{0.5f * tk.h, 0.5f * tk.l}, K));
-            const df vb = nz ? one : zero, wb = dfm::fma(nK, vb, dfm::mul(tau, yb));
-            if (own_r) {   // (the whole CTA)
-                if (tid == 0) s_c = dfm::neg(dfm::mul(tau, dfm::fma(s, s_rd, R[b0])));
-                __syncthreads();   // R_{b0} changes
+                    for (int h = 0; h < o; ++h) ka[h] = dfm::add(ka[h], ka[h + o]);
+                const df K = dfm::warp_sum(ka[0]);
+                const df tk = dfm::mul(tau, tau);
+                const df nk = dfm::neg(dfm::mul(df{0.5f * tk.h, 0.5f * tk.l}, K));
+                const df wk1 = dfm::fma(nk, vb, dfm::mul(tau, yb));
+                if (lane == 0) { s_k[0] = nk; s_k[1] = wk1; }
+            } else if (warp == 1 && own_r && lane == 0) {
+                s_c = dfm::neg(dfm::mul(tau, dfm::fma(s, s_rd, R[b0])));
             }
+            __syncthreads();   // (R_{b0} changes behind it too)
+            const df nK = s_k[0], wb = s_k[1];
             df sq = zero;
             auto one_row = [&](int j, df yj, df bj) {
                 const df vj = !nz ? zero : (j == b0) ? one : dfm::mul(s, x[j]);
