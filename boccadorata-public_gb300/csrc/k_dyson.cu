@@ -91,9 +91,10 @@ __device__ inline void dy_mark_branch_starts(const DyJob &J, int r, int *flag) {
 }
 
 constexpr int kTdgMax = 256;   // CTAs of k_tridiag_grid at most
-// Its smallest order: a column costs it 5.3 us at any order below 700, the cluster kernel's 16 CTAs
-// less up to orders of 500 (a solve of 300: 2.6 against 2.2 ms, 500: 4.1 and 4.1, 600: 4.9 and 5.3)
-constexpr int kTdgMin = 512;
+// Its smallest order: a column costs it about the same at any order below 700, the cluster kernel's
+// 16 CTAs less up to orders of 350 (a solve of 300: 2.25 against 2.14 ms, 400: 2.90 and 2.99, 500: 3.6
+// and 4.0)
+constexpr int kTdgMin = 384;
 // the exchange area in a job's work space (5 n^2 doubles, the spilled rows in the first n^2):
 // y[2][n], row k+1 [2][n], parts of v^T A v [2][kTdgMax], the barrier's count (zeroed by
 // k_dyson_deflate)
@@ -704,9 +705,9 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_df(const DyJob *jobs
 //   all rows  v, w, R; from row k+1, which is column k+1, that column after this step's update (x
 //             of the next step, d_{k+1} on the diagonal), and the sum of its squares, by every CTA
 //             for itself
-// Bound by the barrier and what surrounds it in a column (order 1 000, 11 000 cycles: the pass beside
-// the scalars' chain 3 000, y 1 000, the barrier 3 200, L2 and the sum of the parts 2 700, v and w
-// 1 500).  Order 1 000: 12.8 ms by the cluster kernel -> 6.0.
+// Bound by the barrier and what surrounds it in a column (order 1 000, 9 000 cycles: the pass beside
+// the scalars' chain 3 000, y 1 000, the barrier 3 200, then L2, the sum of the parts, v and w).
+// Order 1 000: 12.8 ms by the cluster kernel -> 4.7.
 constexpr int kTdgRowWarps = kTdfWarps - 2;   // the others: R's product, the scalars
 constexpr int kTdgParts = 4;                  // warps a row at most
 constexpr int kTdgPolls = 1 << 20;            // a barrier's reads before it gives up (about a second)

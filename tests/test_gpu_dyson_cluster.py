@@ -63,7 +63,7 @@ def test_cluster_sizes_agree(bdmod, problems):
 
 # the smallest order one matrix takes the whole GPU for and one less, orders that are no multiple
 # of its CTAs, rows beyond shared memory; D from the channel
-@pytest.mark.parametrize("n,ish", [(511, 1), (512, 1), (531, 5), (760, 2), (1901, 0)])
+@pytest.mark.parametrize("n,ish", [(383, 1), (384, 1), (511, 1), (512, 1), (531, 5), (760, 2), (1901, 0)])
 def test_one_matrix_on_the_whole_gpu(bdmod, problems, n, ish):
     p = problems(6, 20.0, 1, 50)
     rng = np.random.default_rng(n)
