@@ -20,6 +20,7 @@
 //   k_post    x_k[0:D] = R y_k, Z_k = sum_d x_k[d]^2
 //   k_place   quasiparticle / quasihole split by E_F with both lists by descending W
 //   k_koltun  Koltun partial sums (Calc_En, source/BcDor-DysonMatrix.cpp:542-594)
+#include <cfloat>
 #include <climits>
 #include "bd_common.cuh"
 #include "df64.cuh"
@@ -111,6 +112,8 @@ __device__ inline BisectTables bisect_tables(double *work, int n) {
     return t;
 }
 
+constexpr int kPrepBits = 8192;   // positions whose ends are kept as bits in shared memory
+
 __global__ void k_bisect_prep(const DyJob *jobs, int njobs, double *work, const long long *work_first) {
     const int jid = blockIdx.x;
     if (jid >= njobs) return;
@@ -131,8 +134,30 @@ __global__ void k_bisect_prep(const DyJob *jobs, int njobs, double *work, const 
         T.glo[i] = lo; T.ghi[i] = hi; T.rn[i] = r;
     }
     __syncthreads();
-    // 2. block bounds: one integer pass
-    if (threadIdx.x == 0) {
+    // 2. block bounds, from the ends' bits (orders beyond what they hold: one integer pass)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    __shared__ unsigned s_end[kPrepBits / 32];
+    if (n <= kPrepBits) {
+        for (int q = warp; 32 * q < n; q += nw) {
+            const unsigned m = __ballot_sync(0xffffffffu, 32 * q + lane < n && T.flag[32 * q + lane]);
+            if (lane == 0) s_end[q] = m;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            int first = 0;
+            if (i > 0) {   // behind the last end before i
+                int q = (i - 1) >> 5;
+                unsigned m = s_end[q] & (0xffffffffu >> (31 - ((i - 1) & 31)));
+                while (m == 0 && q > 0) m = s_end[--q];
+                if (m) first = 32 * q + 32 - __clz(m);
+            }
+            int q = i >> 5;
+            unsigned m = s_end[q] & (0xffffffffu << (i & 31));
+            while (m == 0) m = s_end[++q];   // (the last position is an end)
+            bs[i] = first;
+            be[i] = 32 * q + __ffs(m) - 1;
+        }
+    } else if (threadIdx.x == 0) {
         int b0 = 0;
         for (int i = 0; i < n; ++i)
             if (T.flag[i]) {
@@ -141,15 +166,24 @@ __global__ void k_bisect_prep(const DyJob *jobs, int njobs, double *work, const 
             }
     }
     __syncthreads();
-    // 3. each block's first position reduces its block and picks the scale
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    // 3. a warp per block reduces it and picks the scale
+    for (int i = warp; i < n; i += nw) {
         if (bs[i] != i) continue;
         const int b1 = be[i];
-        float lo = T.glo[i], hi = T.ghi[i], r = T.rn[i];
-        for (int q = i + 1; q <= b1; ++q) { lo = fminf(lo, T.glo[q]); hi = fmaxf(hi, T.ghi[q]); r = fmaxf(r, T.rn[q]); }
-        const int s = sturm::scale_exponent(fmaxf(fabsf(lo), fabsf(hi)));
-        const float sc = sturm::pow2f(-s);
-        T.glo[i] = lo * sc; T.ghi[i] = hi * sc; T.rn[i] = r; T.sx[i] = s;
+        float lo = FLT_MAX, hi = -FLT_MAX, r = 0.0f;
+        for (int q = i + lane; q <= b1; q += 32) { lo = fminf(lo, T.glo[q]); hi = fmaxf(hi, T.ghi[q]); r = fmaxf(r, T.rn[q]); }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+            r = fmaxf(r, __shfl_xor_sync(0xffffffffu, r, o));
+        }
+        if (lane == 0) {
+            const int s = sturm::scale_exponent(fmaxf(fabsf(lo), fabsf(hi)));
+            const float sc = sturm::pow2f(-s);
+            T.glo[i] = lo * sc; T.ghi[i] = hi * sc; T.rn[i] = r; T.sx[i] = s;
+        }
+        __syncwarp();
     }
     __syncthreads();
     // 4. scaled FP32 pairs; split off-diagonals back into J.e; block norms into J.tau
