@@ -998,8 +998,11 @@ int launch_lanczos_range(bd_ctx *ctx, int ch_lo, int ch_hi, bool fp32) {
         CU(launch_lz_compact(d_ch, (int)ch.size(), ctx->eta, ctx->st));
         ctx->launches += 1;
         int forms = 0;
-        for (const LzChain &z : ch) if (z.N >= kLzLong) forms |= lanczos_long_form(z.N, rmax, CL);
-        CU(launch_lanczos_long(d_ch, (int)ch.size(), rmax, CL, ctx->eta, forms, ctx->st));
+        int longest = 0;
+        for (const LzChain &z : ch) longest = std::max(longest, z.N);
+        const int nmin = lz_long_from(ch.size(), longest);
+        for (const LzChain &z : ch) if (z.N >= nmin) forms |= lanczos_long_form(z.N, rmax, CL);
+        CU(launch_lanczos_long(d_ch, (int)ch.size(), rmax, nmin, CL, ctx->eta, forms, ctx->st));
         ctx->launches += (forms & 1) + (forms >> 1);
     }
     // chains whose slices do not fit next to the scalars keep them in global memory
@@ -2818,7 +2821,7 @@ extern "C" int bd_lanczos_chain_noalloc(const double *d_E, const double *d_M, in
         e = launch_to_float(d_M, reinterpret_cast<float *>(base + mf_off), (long long)D * N, st);
     if (e == cudaSuccess) e = launch_lz_groups(reinterpret_cast<const LzChain *>(base), 1, lz_gram_cap(N), st);
     if (e == cudaSuccess && !fp32 && N >= kLzLong)
-        e = launch_lanczos_long(reinterpret_cast<const LzChain *>(base), 1, P.L + 1, kNoallocCluster, kNoallocEta,
+        e = launch_lanczos_long(reinterpret_cast<const LzChain *>(base), 1, P.L + 1, kLzLong, kNoallocCluster, kNoallocEta,
                                 lanczos_long_form(N, P.L + 1, kNoallocCluster) & 1, st);
     if (e == cudaSuccess)
         e = launch_lanczos(reinterpret_cast<const LzChain *>(base), 1, S, P.L + 1, fp32, kNoallocCluster, kNoallocEta,

@@ -1,6 +1,7 @@
 // bd_common.cuh -- device-side data structures shared by the kernels of the
 // Sigma(2) -> Lanczos -> Dyson chain (sm_103a).
 #pragma once
+#include <climits>
 #include <cstdint>
 #include <mutex>
 #include <unordered_set>
@@ -137,7 +138,16 @@ struct LzChain {
     int *done;              // set by the kernel that reduced the chain ahead of k_lanczos (k_lz_compact's
                             // CompactInfo::handled in a context); nullptr: k_lanczos alone
 };
-constexpr int kLzLong = 2048;   // poles from which k_lz_long takes a chain with FP64 vectors
+// Poles from which k_lz_long takes a chain with FP64 vectors.  In a launch of more chains than its
+// clusters are resident (kLzLongFew) only where the longest has kLzLongBatch poles: k_lanczos keeps two
+// and a half times as many clusters resident, which is worth more to short chains (the dressed steps'
+// chains of at most 3 500, 6 500, 11 200 and 18 000 poles, 15 iterations: 1.6, 2.9, 2.7 and 4.0 ms by
+// k_lz_long, 1.1, 2.0, 3.9 and 7.5 by k_lanczos; some chains by each, one kernel after the other, is
+// slower than either).  INT_MAX: no chain.
+constexpr int kLzLong = 2048, kLzLongBatch = 8192, kLzLongFew = 15;
+inline int lz_long_from(size_t nchains, int longest) {
+    return nchains > (size_t)kLzLongFew && longest < kLzLongBatch ? INT_MAX : kLzLong;
+}
 
 // Energy-group scratch of a chain of N poles, behind gE [2N doubles] and gInfo [N + 1
 // ints]: the Gram pieces of the groups of more than kGrpSmall poles (a piece is at most

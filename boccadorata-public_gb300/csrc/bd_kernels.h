@@ -102,12 +102,12 @@ cudaError_t launch_lz_expand(const LzChain &chain, double *out, cudaStream_t st)
 // The plain Sigma(2) rows of the full Dyson matrix, equal energies rotated (k_compact.cu).
 cudaError_t launch_plain_rotate(const LzChain *d_chains, const PlainIO *d_ios, int nchains, cudaStream_t st);
 void compact_smem_init();
-// FP64 vectors, long chains (k_lanczos_long.cu): chains with done set and at least kLzLong
-// poles, before launch_lanczos.  lanczos_long_form: which form of it takes a chain, 0 none
+// FP64 vectors, long chains (k_lanczos_long.cu): chains with done set and at least nmin
+// poles (lz_long_from), before launch_lanczos.  lanczos_long_form: which form of it takes a chain, 0 none
 // (rows beyond shared memory), 1 slices in shared memory, 2 in the chain.s scratch; forms: all of
 // a launch (1 | 2).  Their stored vectors are two planes of integers (k_lanczos_long.cu) per slot.
 int lanczos_long_form(int N, int rmax, int cluster);
-cudaError_t launch_lanczos_long(const LzChain *d_chains, int nchains, int rmax, int cluster, double eta, int forms,
+cudaError_t launch_lanczos_long(const LzChain *d_chains, int nchains, int rmax, int nmin, int cluster, double eta, int forms,
                                 cudaStream_t st);
 void lanczos_long_smem_init();
 

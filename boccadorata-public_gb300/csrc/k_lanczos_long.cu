@@ -18,7 +18,7 @@
 // The recurrence, the norm, alpha, m and g stay FP64 with as few instructions as they take.
 //
 // What a chain needs beyond that -- a restart vector, energies or couplings outside 2^+-40,
-// fewer than kLzLong poles -- is left to k_lanczos as a whole (C.done stays 0), which the
+// fewer poles than lz_long_from says -- is left to k_lanczos as a whole (C.done stays 0), which the
 // host launches behind this kernel.
 //
 // Work split: a cluster per chain, CTA r the pole rows [r S, (r+1) S), 512 threads and an SM to
@@ -104,7 +104,7 @@ __host__ __device__ inline bool long_fits(int N, int cluster, int rmax, size_t s
 
 // SS: w, its split and the two newest vectors in shared memory (else in the chain's global scratch).
 template <bool SS>
-__global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chains, int nchains, int rmax, double eta2,
+__global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chains, int nchains, int rmax, int nmin, double eta2,
                                                     int smem_bytes) {
     cg::cluster_group cluster = cg::this_cluster();
     const int CL = (int)cluster.num_blocks(), rank = (int)cluster.block_rank(), cid = blockIdx.x / CL;
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
     if (threadIdx.x < sizeof(LzChain) / 4)
         reinterpret_cast<int *>(&C)[threadIdx.x] = reinterpret_cast<const int *>(chains + cid)[threadIdx.x];
     __syncthreads();
-    if (!C.done || *C.done || C.N < kLzLong) return;   // (the whole cluster leaves together)
+    if (!C.done || *C.done || C.N < nmin) return;   // (the whole cluster leaves together)
     if (long_fits(C.N, CL, rmax, smem_bytes) != SS) return;   // the other form's
     const int S = long_slice(C.N, CL), i0 = rank * S;
     constexpr int T = kLongThreads, NW = kMaxWarps;
@@ -603,7 +603,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
 namespace {
 constexpr size_t kLongSmem = (size_t)225 * 1024;
 template <bool SS>
-cudaError_t launch_form(const LzChain *d_chains, int nchains, int rmax, int cluster, double eta, cudaStream_t st) {
+cudaError_t launch_form(const LzChain *d_chains, int nchains, int rmax, int nmin, int cluster, double eta, cudaStream_t st) {
     if (SS) cluster = long_cluster(cluster);
     cudaError_t e = allow_dynamic_smem((const void *)k_lz_long<SS>);
     if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(k_lz_long<SS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -620,7 +620,7 @@ cudaError_t launch_form(const LzChain *d_chains, int nchains, int rmax, int clus
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_lz_long<SS>, d_chains, nchains, rmax, eta * eta, (int)kLongSmem);
+    return cudaLaunchKernelEx(&cfg, k_lz_long<SS>, d_chains, nchains, rmax, nmin, eta * eta, (int)kLongSmem);
 }
 }  // namespace
 
@@ -628,11 +628,11 @@ int lanczos_long_form(int N, int rmax, int cluster) {
     return long_fixed(rmax) > kLongSmem ? 0 : long_fits(N, cluster, rmax, kLongSmem) ? 1 : 2;
 }
 
-cudaError_t launch_lanczos_long(const LzChain *d_chains, int nchains, int rmax, int cluster, double eta, int forms,
+cudaError_t launch_lanczos_long(const LzChain *d_chains, int nchains, int rmax, int nmin, int cluster, double eta, int forms,
                                 cudaStream_t st) {
     cudaError_t e = cudaSuccess;
-    if (forms & 1) e = launch_form<true>(d_chains, nchains, rmax, cluster, eta, st);
-    if (e == cudaSuccess && (forms & 2)) e = launch_form<false>(d_chains, nchains, rmax, cluster, eta, st);
+    if (forms & 1) e = launch_form<true>(d_chains, nchains, rmax, nmin, cluster, eta, st);
+    if (e == cudaSuccess && (forms & 2)) e = launch_form<false>(d_chains, nchains, rmax, nmin, cluster, eta, st);
     return e;
 }
 
