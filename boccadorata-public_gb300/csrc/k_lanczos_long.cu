@@ -17,7 +17,8 @@
 //     kSmall sqrt(R) |w|.  Otherwise (new pivots, further sweeps) it is fixed point too.
 // The recurrence, the norm, alpha, m and g stay FP64 with as few instructions as they take.
 //
-// What a chain needs beyond that -- a restart vector, energies or couplings outside 2^+-40,
+// What a chain needs beyond that -- a restart vector, energies or couplings outside 2^+-40, a
+// vector (a weakly coupled orbital's, say) whose |w|^2 the FP32 scale does not hold (kFixedWeak),
 // fewer poles than lz_long_from says -- is left to k_lanczos as a whole (C.done stays 0), which the
 // host launches behind this kernel.
 //
@@ -494,7 +495,8 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
                     const long long xb = __double_as_longlong(x2);
                     const bool zero = (xb << 1) == 0, fin = (xb & 0x7ff0000000000000LL) != 0x7ff0000000000000LL;
                     int f;
-                    if ((le & 2u) || zero) f = (dcur < dtot) ? 2 : 3;   // (further sweeps leave no more)
+                    if (!zero && wn2_first < kFixedWeak) f = 3;   // split against a scale FP32 lost
+                    else if ((le & 2u) || zero) f = (dcur < dtot) ? 2 : 3;   // (further sweeps leave no more)
                     else if (nvec > 0 && nfull + 1 < 4 && (lt_ & 1u)) f = 1;
                     else if (nvec > 0 && nfull == 0 && (lt_ & 8u)) f = 4;
                     else if (!(le & 4u) && fin) f = 0;

@@ -103,6 +103,10 @@ __device__ __forceinline__ bool fixed_range(unsigned hi) { return hi >= (1023u -
 // below this part of the other's), the sums are too coarse for it and the sweep is repeated, split
 // against |w| itself.
 constexpr double kFixedShort = 0x1p-12;
+// |E v_{j-1}|^2 and |M p|^2, the scales of the split and the thresholds, are FP32 sums of squares: below
+// this they lose elements to FP32's range (squares under 2^-149), down to a scale of zero for a w that is
+// not, and the split puts nothing in its place.
+constexpr double kFixedWeak = 0x1p-90;
 // the exponent field of a power of two above |x|, from |x|^2
 __device__ __forceinline__ int bias_above(double x2) {
     return ((__double2hiint(x2) >> 20) - 1023 + 2048) / 2 - 1024 + 1023 + 1;

@@ -142,3 +142,44 @@ def test_unreached_directions_of_many_groups(bdmod, D, nq):
     defl = got[np.abs(got[:, 1:]).max(1) == 0, 0]
     assert len(defl) > 20
     assert np.array_equal(defl, np.array(expect)[:len(defl)])
+
+
+def _run_pivots(bdmod, E, M, piv, nits):
+    D, N = M.shape
+    tE, tM = torch.from_numpy(E).cuda(), torch.from_numpy(np.ascontiguousarray(M)).cuda()
+    out = torch.full((int(sum(nits)), len(piv) + 1 + D), float("nan"), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    L, *_ = bdmod.lanczos_chain_noalloc(tE.data_ptr(), tM.data_ptr(), N, D, piv, np.array(nits, np.int32), out.data_ptr(),
+                                        len(out))
+    return out.cpu().numpy()[:L]
+
+
+# the second orbital's couplings below the first's by as much as FP32's squares hold, and beyond (|M p|^2 from
+# 2^-90 down); a second pivot in which couplings cancel down to their last bits (an exact difference); a second
+# pivot that lives on poles next to zero (|E v|^2)
+@pytest.mark.parametrize("kind,size", [("orbital", 1e-11), ("orbital", 1e-14), ("orbital", 1e-20), ("orbital", 1e-24),
+                                       ("orbital", 1e-40), ("cancelling", 1e-11), ("energies", 1e-24)])
+def test_weakly_coupled_orbital(bdmod, kind, size):
+    rng = np.random.default_rng(11)
+    N, nit = 2500, 8
+    E = np.sort(rng.uniform(20.0, 300.0, N))
+    M = rng.standard_normal((2, N))
+    piv = np.eye(2)
+    if kind == "orbital":
+        M[1] *= size
+    elif kind == "cancelling":
+        M = np.concatenate([M * size, np.zeros((2, N))])
+        M[1] = M[0] * (1.0 + 2.0 ** -52 * rng.integers(-3, 4, N))
+        piv = np.array([[1.0, 0.0, 0.0, 0.0], [0.5, -0.5, 0.5, -0.5]])
+    else:
+        E[:40] = np.sort(rng.uniform(1.0, 2.0, 40)) * size
+        M[0, :40] = 0.0
+        M[1, 40:] = 0.0
+    got = _run_pivots(bdmod, E, M, piv, [nit, nit])
+    ref = _reference(E, piv @ M, nit)
+    for c in (0, 1):   # every chain on the scale of the energies it lives on
+        r = slice(c * nit, (c + 1) * nit)
+        scale = np.abs(ref[r, 0]).max()
+        assert np.abs(got[r, 0] - ref[r, 0]).max() < 1e-11 * scale, c
+        assert np.abs(got[r, 1][1:] - ref[r, 1][1:]).max() < 1e-11 * scale, c
+        assert np.abs(got[r, 2] - ref[r, 2]).max() < 1e-11 * 300.0, c
