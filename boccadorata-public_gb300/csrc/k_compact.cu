@@ -111,6 +111,7 @@ __device__ int merge_groups(const double *gE, int Q, int *s_first, int *ws) {
 }
 
 static_assert(kCpThreads >= kCpGroups, "a thread per exact group");
+static_assert(kCpDim <= kFixedRun, "a chain's sums are one run");
 
 }  // namespace
 

@@ -10,8 +10,10 @@
 //     newest vectors, which the recurrence reads, are kept as doubles besides;
 //   - w is split the same way against a power of two above |w| (above |E v_{j-1}| after a
 //     recurrence, of which w is a projection), and a dot product is three 32 x 32 -> 64 bit
-//     multiply-adds an element, exact sums (they are bounded by |v| |w|) on the integer pipe: c_t
-//     is off by about 2^-57 |w|, where FP64's own sum is off by 1e-16 |w|;
+//     multiply-adds an element, exact sums on the integer pipe (run by run of what a word holds,
+//     lz_fixed.cuh): c_t is off by about 2^-57 |w|, where FP64's own sum is off by 1e-16 |w|.  w's words are
+//     dithered, so that elements of one size leave no sum of their low words' products (which at the most
+//     would be n 2^-62 |w|; as a fourth product an element they cost a chain of 20 000 poles 4.7 %);
 //   - the update w -= sum c_t v_t runs in FP32 from the a planes alone (4 bytes a pole) where
 //     every |c_t| <= kSmall |w|, which after a recurrence is the rule: its error is below 2^-23
 //     kSmall sqrt(R) |w|.  Otherwise (new pivots, further sweeps) it is fixed point too.
@@ -75,21 +77,27 @@ __host__ __device__ inline size_t long_fixed(int rmax) {
 __device__ __forceinline__ void long_dots(FixedSum (&acc)[4], const int *const (&va)[4], int pb, const int *wa,
                                           int S, int n) {
 #pragma unroll 1
-    for (int i = 0; i < n; i += 128) {
-        int4 x[4], y[4];
+    for (int r = 0; r < n; r += 32 * kFixedRun) {
+        const int end = min(n, r + 32 * kFixedRun);
+#pragma unroll 1
+        for (int i = r; i < end; i += 128) {
+            int4 x[4], y[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            x[u] = ld4(va[u] + i);
-            y[u] = ld4(va[u] + pb + i);
-        }
-        const int4 a = ld4(wa + i), b = ld4(wa + S + i);
+            for (int u = 0; u < 4; ++u) {
+                x[u] = ld4(va[u] + i);
+                y[u] = ld4(va[u] + pb + i);
+            }
+            const int4 a = ld4(wa + i), b = ld4(wa + S + i);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            fixed_step(acc[u], x[u].x, y[u].x, a.x, b.x);
-            fixed_step(acc[u], x[u].y, y[u].y, a.y, b.y);
-            fixed_step(acc[u], x[u].z, y[u].z, a.z, b.z);
-            fixed_step(acc[u], x[u].w, y[u].w, a.w, b.w);
+            for (int u = 0; u < 4; ++u) {
+                fixed_step(acc[u], x[u].x, y[u].x, a.x, b.x);
+                fixed_step(acc[u], x[u].y, y[u].y, a.y, b.y);
+                fixed_step(acc[u], x[u].z, y[u].z, a.z, b.z);
+                fixed_step(acc[u], x[u].w, y[u].w, a.w, b.w);
+            }
         }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[u] = fixed_carry(acc[u]);
     }
 }
 
@@ -200,7 +208,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
     };
     int wbias = 1023;   // exponent field of the power of two w is split against
     auto split_w = [&](int i, double a, double b) {
-        const int2 x = fixed_of(a, wbias), y = fixed_of(b, wbias);
+        const int2 x = fixed_dithered(a, wbias, i), y = fixed_dithered(b, wbias, i + 1);
         *reinterpret_cast<int2 *>(ws + i) = make_int2(x.x, y.x);
         *reinterpret_cast<int2 *>(ws + S + i) = make_int2(x.y, y.y);
     };
@@ -387,17 +395,26 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
                     for (int e = 0; e < 4; ++e) x[e] -= f32_to_double(a[e]);
                 } else {
                     FixedSum a[4];
+                    int h[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) a[e] = FixedSum{0, 0};
+#pragma unroll 1
+                    for (int r = 0; r < nvec; r += kFixedRun) {
+                        const int end = min(nvec, r + kFixedRun);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) h[e] = 0;
 #pragma unroll 2
-                    for (int t = 0; t < nvec; ++t) {
-                        const int2 ct = fixed_of(c[t], wbias);
-                        const int *q = plane(t) + i;
-                        const int4 v = ld4(q), u = ld4(q + C.ld);
-                        fixed_step(a[0], v.x, u.x, ct.x, ct.y);
-                        fixed_step(a[1], v.y, u.y, ct.x, ct.y);
-                        fixed_step(a[2], v.z, u.z, ct.x, ct.y);
-                        fixed_step(a[3], v.w, u.w, ct.x, ct.y);
+                        for (int t = r; t < end; ++t) {
+                            const int2 ct = fixed_of(c[t], wbias);
+                            const int *q = plane(t) + i;
+                            const int4 v = ld4(q), u = ld4(q + C.ld);
+                            fixed_step(a[0], h[0], v.x, u.x, ct.x, ct.y);
+                            fixed_step(a[1], h[1], v.y, u.y, ct.x, ct.y);
+                            fixed_step(a[2], h[2], v.z, u.z, ct.x, ct.y);
+                            fixed_step(a[3], h[3], v.w, u.w, ct.x, ct.y);
+                        }
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) a[e] = fixed_carry(a[e], h[e]);
                     }
 #pragma unroll
                     for (int e = 0; e < 4; ++e) x[e] -= fixed_value(a[e], wbias);

@@ -19,12 +19,40 @@ __device__ __forceinline__ int2 fixed_of(double x, int bias) {
     const int a = (int)(f >> 28), b = ((int)(f >> 1) & 0x7ffffff) - (1 << 26);
     return hi < 0 ? make_int2(-a, -b) : make_int2(a, b);
 }
-// (s + l 2^-27) 2^-60 for sums s of a a' and l of a b' + b a' (the b b' dropped)
+// The same value with a rounded up or down by element i's place in a sequence that fills the unit interval
+// evenly, b in (-2^27, 2^27): over elements of one size b is zero in the mean, where to nearest it is the
+// same word n times.
+__device__ __forceinline__ int2 fixed_dithered(double x, int bias, int i) {
+    const int hi = __double2hiint(x);
+    const unsigned lo = (unsigned)__double2loint(x);
+    const unsigned long long m = ((unsigned long long)((hi & 0xfffff) | 0x100000) << 32 | lo) << 6;
+    const unsigned long long f = (m >> min((unsigned)(bias - ((hi >> 20) & 0x7ff)), 63u)) + 1;
+    const int a = (int)((f + ((unsigned)i * 0x9e3779b9u >> 4)) >> 28), b = (int)((unsigned)(f >> 1) - ((unsigned)a << 27));
+    return hi < 0 ? make_int2(-a, -b) : make_int2(a, b);
+}
+// (s + l 2^-27) 2^-60 for sums s of a a' and l of what is below.  A thread's l is in [0, 2^27) at last, the rest
+// carried into s, so 2^36 threads' sums can be added as they are.
 struct FixedSum { long long s, l; };
+// A thread's running sums of a a' and of a b' + b a'.  Where the low words of all elements have one sign (vectors
+// of elements of one size) the second does not cancel: it grows by up to 3 2^56 |v| |w| sqrt(n) and would wrap
+// beyond n of some thousand.  A run of at most kFixedRun elements keeps it inside its word.  The products b b'
+// are left out: below n 2^-62 together for one sign, sqrt(n) 2^-63 with one factor dithered.
+constexpr int kFixedRun = 1024;
 __device__ __forceinline__ void fixed_step(FixedSum &acc, int va, int vb, int wa, int wb) {
     acc.s += (long long)va * wa;
     acc.l += (long long)va * wb;
     acc.l += (long long)vb * wa;
+}
+// with the upper words of b b' (units of 2^32 2^-114), for a vector against itself, where they have one sign, and
+// where a sum is short
+__device__ __forceinline__ void fixed_step(FixedSum &acc, int &h, int va, int vb, int wa, int wb) {
+    fixed_step(acc, va, vb, wa, wb);
+    h += __mulhi(vb, wb);
+}
+// what a run has summed, carried
+__device__ __forceinline__ FixedSum fixed_carry(FixedSum r, int h = 0) {
+    const long long l = r.l + ((long long)h << 5);
+    return FixedSum{r.s + (l >> 27), l & 0x7ffffff};
 }
 // Times 2^(bias - 1023), rounded, from its bits: the FP64 forms of this are six instructions of
 // ~64 cycles in every warp of a sweep.

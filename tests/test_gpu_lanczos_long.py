@@ -183,3 +183,24 @@ def test_weakly_coupled_orbital(bdmod, kind, size):
         assert np.abs(got[r, 0] - ref[r, 0]).max() < 1e-11 * scale, c
         assert np.abs(got[r, 1][1:] - ref[r, 1][1:]).max() < 1e-11 * scale, c
         assert np.abs(got[r, 2] - ref[r, 2]).max() < 1e-11 * 300.0, c
+
+
+# A vector of equal elements against one of two values: the fixed-point words of all elements have one sign, so
+# neither their cross products (1 and 4 times 2^63) nor the products of their low words (4e-14 |w|) cancel.
+@pytest.mark.parametrize("overlap", [0.694, 0.678])
+def test_elements_of_one_size(bdmod, overlap):
+    N = 111230   # (an element 1 / sqrt(N) whose low word is the largest there is)
+    rng = np.random.default_rng(1)
+    E = np.sort(rng.uniform(20.0, 300.0, N))
+    s = np.where(np.arange(N) < N // 2, 1.0, -1.0)
+    M = np.array([np.ones(N), overlap + np.sqrt(1.0 - overlap ** 2) * s])
+    got = _run_pivots(bdmod, E, M, np.eye(2), [1, 3])
+    u = M[1] - M[1].mean()
+    u = u / np.linalg.norm(u)
+    g = np.dot(np.full(N, 1.0 / np.sqrt(N)), E * u)
+    # FP64 sums of a hundred thousand terms over a tree of at most some 64 additions in a row: 64 eps of the terms' sizes
+    tol = 64 * 2.2e-16
+    assert abs(got[1, 0] - np.dot(u, E * u)) < tol * 300.0
+    assert abs(got[1, 1] - g) < tol * 300.0
+    assert abs(got[1, 3]) < tol * np.sqrt(N)          # <M_0|u>, nothing
+    assert abs(got[1, 4] - np.dot(M[1], u)) < tol * np.sqrt(N)
