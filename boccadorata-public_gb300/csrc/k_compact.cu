@@ -262,7 +262,13 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
     __shared__ double lc[16], s_n[3];   // s_n: 1/|w|, |w|, |E v|^2 of the kept vector
     __shared__ float s_f[kCpWarps], s_cm[kCpWarps];
     __shared__ double s_piv[80];   // at most 9 pivots of 8
-    for (int q = tid; q < C.n_used * D && q < 80; q += kCpThreads) s_piv[q] = C.piv[q];
+    bool bad_piv = false;   // (a pivot of zeros is NaN here: the integers of the split would hide it)
+    for (int q = tid; q < C.n_used * D && q < 80; q += kCpThreads) {
+        const double p = C.piv[q];
+        s_piv[q] = p;
+        bad_piv |= (__double2hiint(p) & 0x7ff00000) == 0x7ff00000;
+    }
+    if (__syncthreads_or(bad_piv)) return;
     if (tid <= C.n_used && tid < 10) s_start[tid] = C.start[tid];
     if (tid < C.n_used && tid < 10) s_last[tid] = C.last[tid];
     // the groups' energies and unreached directions, cumulated (Q = gInfo[0])
@@ -286,6 +292,13 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
     int wbias = 1023;   // exponent field of the power of two w is split against
     auto split_w = [&](int i, double x) {
         wab[i] = fixed_of(x, wbias);
+    };
+    // a scale that FP32 may have lost (from its upper word), and a w that is not zero
+    auto weak = [](double x2) { return __double2hiint(x2) < __double2hiint(kFixedWeak); };
+    auto lost = [&]() {
+        bool any = false;
+        for (int i = tid; i < np; i += kCpThreads) any |= (__double_as_longlong(w[i]) << 1) != 0;
+        return __syncthreads_or(any) != 0;
     };
     // the update's threads: an element each, npw apart the groups that share its vectors
     const int npw = (np + 31) & ~31, tgs = kCpThreads / npw, tgp = tid / npw, ei = tid - tgp * npw;
@@ -317,6 +330,7 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
             for (int h = 0; h < kCpWarps; ++h) s2 += s_f[h];
             wn2 = wn2_first = (double)s2;
             wbias = bias_above(wn2);
+            if (weak(wn2) && lost()) return;
             for (int i = tid; i < np; i += kCpThreads) split_w(i, w[i]);
         } else {
             wbias = bias_above(e2v);
@@ -343,6 +357,7 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
             // |w|^2, read against the swept norm and the coefficients only: FP32
             for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
             if (lane == 0) s_f[warp] = s2;
+            if (weak(e2v) && lost()) return;
         }
         int fl, nfull = 0;
         for (;;) {

@@ -92,3 +92,25 @@ def test_rotated_full_dyson_equals_plain_rows(bdmod, problems, nmax, hw, kind):
             assert e < 1e-10 and z < 1e-10, (ish, tag, e, z)
         np.testing.assert_allclose(a["koltun"], b["koltun"], rtol=1e-10, atol=1e-11)
     ctx.close()
+
+
+@pytest.mark.parametrize("lead", [False, True])
+def test_pivot_of_zeros_as_in_the_full_space(bdmod, problems, lead):
+    """A pivot without direction (the chain's first, or a later one): its rows are not finite, as those of the
+    reduction over the poles, and not an exhausted chain's."""
+    p = problems(4, 20.0, 3, 4)
+    ctx = bdmod.Context().upload(p)
+    ish = 0
+    D = int(p.ms.no[ish])
+    piv = np.eye(D)
+    piv[0 if lead else D - 1] = 0.0
+    rows = []
+    for mode in (0, 1):
+        ctx.set_lanczos_slices(mode)
+        ctx.sigma2_build(ish, copy=False)
+        lz = ctx.lanczos_reduce(ish, piv, np.full(D, 4), np.full(D, 4))
+        rows.append((lz["lz_fw"], lz["lz_bk"]))
+    for a, b in zip(*rows):
+        assert not np.isfinite(b).all()
+        assert np.array_equal(np.isfinite(a), np.isfinite(b))
+    ctx.close()
