@@ -445,12 +445,14 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
             if (warp == kCpWarps - 1) {
                 FixedSum p{0, 0};
                 float s2 = 0.0f;
+                int h = 0;   // (the low words' squares have one sign)
                 for (int i = lane; i < np; i += 32) {
                     const int2 x = wab[i];
-                    fixed_step(p, x.x, x.y, x.x, x.y);
+                    fixed_step(p, h, x.x, x.y, x.x, x.y);
                     const float f = f32_trunc(ew[i]);
                     s2 = fmaf(f, f, s2);
                 }
+                p = fixed_carry(p, h);
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) {
                     p = fixed_add(p, fixed_shfl(p, o));

@@ -114,3 +114,21 @@ def test_pivot_of_zeros_as_in_the_full_space(bdmod, problems, lead):
         assert not np.isfinite(b).all()
         assert np.array_equal(np.isfinite(a), np.isfinite(b))
     ctx.close()
+
+
+@pytest.mark.parametrize("shift", [0.0, 1500.0, 2500.0])
+def test_norms_of_vectors_short_beside_the_energies(bdmod, synth, shift):
+    """Energies far from zero: w is E v less its projections and much shorter (down to 2^-6, where the sweep is
+    repeated), so |w|^2 is made of the low words.  The stored vectors' norms are off by the rounding of 1/|w|
+    and of the elements and of the sum's terms only: a few eps."""
+    p = synth.make_problem(8, 16.0, 1, 6)
+    p.prop.ep[:] += shift
+    p.prop.eh[:] += shift
+    ctx = bdmod.Context().upload(p)
+    D = int(p.ms.no[0])
+    ctx.sigma2_build(0, copy=False)
+    nit = np.full(D, 6, np.int32)
+    lz = ctx.lanczos_reduce(0, np.eye(D), nit, nit)
+    V = ctx.lanczos_vectors(0, 0, len(lz["lz_fw"]), ctx.count_poles(0)[0]).astype(np.longdouble)
+    assert np.abs((V ** 2).sum(1) - 1.0).max() < 8 * 2.2e-16
+    ctx.close()
