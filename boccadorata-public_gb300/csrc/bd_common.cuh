@@ -197,12 +197,12 @@ struct CompactScratch {
     int *start;          // [kCpGroups + 1] first pole of every energy, then N
     CompactGroup *grp;   // [kCpMerged]
     double *gram;        // [kCpGroups][kGramEntries] M M^T of every energy's poles, lower triangle
-    double *L;           // [kCpMerged][64] Cholesky factors, D x D row-major
+    double *L;           // [kCpGroups][64] the groups' factors, D x D row-major
 };
 constexpr long long kCpStartOff = 256, kCpGrpOff = kCpStartOff + 4 * (kCpGroups + 4),
                     kCpGramOff = (kCpGrpOff + 20 * kCpMerged + 255) / 256 * 256,
                     kCpLOff = kCpGramOff + 8LL * kCpGroups * kGramEntries,
-                    kCpBytes = (kCpLOff + 8LL * 64 * kCpMerged + 255) / 256 * 256;
+                    kCpBytes = (kCpLOff + 8LL * 64 * kCpGroups + 255) / 256 * 256;
 static_assert(sizeof(CompactInfo) <= kCpStartOff && sizeof(CompactGroup) == 20, "compact scratch layout");
 __host__ __device__ inline CompactScratch lz_compact(char *b) {
     return CompactScratch{reinterpret_cast<CompactInfo *>(b), reinterpret_cast<int *>(b + kCpStartOff),

@@ -26,8 +26,16 @@
 // (sums of FP64 products in a fixed order).  A group keeps its poles as they are when it
 // has at most kKeep, or at most kGrpSmall and a pivot that loses digits (below kPivot of
 // its diagonal entry); a larger group with such a pivot leaves the whole chain to
-// k_lanczos.  The reduction depends on a group through G_g only, so the Cholesky factor's
-// backward error, a few eps of G's diagonal, is the rounding of the result.
+// k_lanczos.
+//
+// The reduction depends on a group through L only, but a Gram matrix holds L's rows to the
+// rounding of their squares: where an orbital's couplings lie close to the others' (a pivot
+// of the fraction p of its diagonal entry) L is off by about 1e-17 / p, and alpha and beta
+// with it (1.7e-11 of the energies at p = 2e-6, where the reduction over the poles is off by
+// 3e-15).  So a factor with a pivot below kLossy is formed a second time from its own poles,
+// factor_again: Q = L^-1 M_g has rows that are orthonormal but for L's error, and with
+// Q Q^T = L2 L2^T the product L L2 is M_g's factor to FP64's rounding of M_g (Cholesky QR
+// taken twice).
 #include <cfloat>
 #include "bd_common.cuh"
 #include "bd_kernels.h"
@@ -41,15 +49,15 @@ constexpr int kCpThreads = 256;
 constexpr int kCpWarps = kCpThreads / 32;
 constexpr int kKeep = 12;
 constexpr double kMergeUlp = 16.0;
-constexpr double kPivot = 1e-6;
+constexpr double kPivot = 1e-6, kLossy = 0.125;
 constexpr int kCpSmem = 200 * 1024;
 
 // Lower-triangular factor of a D x D Gram matrix (lower triangle in tri), a warp; L (D x D,
 // row-major, zero above the diagonal) to out.  A row without couplings (zero diagonal
-// entry) gives a zero column.  False when a pivot falls below kPivot of its diagonal entry
-// or anything is not finite; then out is not to be used.
-__device__ bool warp_cholesky(const double *tri, int D, double *out, int lane) {
-    bool ok = true;
+// entry) gives a zero column.  0 when a pivot falls below kPivot of its diagonal entry
+// or anything is not finite, and out is not to be used; 2 when one falls below kLossy of it.
+__device__ int warp_cholesky(const double *tri, int D, double *out, int lane) {
+    int res = 1;
     for (int e = lane; e < D * D; e += 32) {
         const int a = e / D, b = e % D;
         out[e] = (b <= a) ? tri[a * (a + 1) / 2 + b] : 0.0;
@@ -58,8 +66,8 @@ __device__ bool warp_cholesky(const double *tri, int D, double *out, int lane) {
     for (int s = 0; s < D; ++s) {
         const double p = out[s * D + s], g = tri[s * (s + 1) / 2 + s];
         const bool zero = (g == 0.0);
-        if (!zero && !(p > kPivot * g && p <= DBL_MAX)) ok = false;
-        if (!ok) break;   // the same in every lane
+        if (!zero && !(p > kPivot * g && p <= DBL_MAX)) return 0;   // the same in every lane
+        if (!zero && p < kLossy * g) res = 2;
         // (Newton's iteration to a few ulp: FP64 square root and division are chains of their own)
         const double ri = zero ? 0.0 : rsqrt_cubic(p), r = p * ri;
         __syncwarp();
@@ -71,7 +79,89 @@ __device__ bool warp_cholesky(const double *tri, int D, double *out, int lane) {
         }
         __syncwarp();
     }
-    return ok;
+    return res;
+}
+
+// The factor L (D x D, row-major, global) of the couplings M of poles [p0, p0 + m) formed again
+// from Q = L^-1 M, by the whole CTA: a thread per pole and round, D (D + 1) FP64 instructions a
+// pole.  (N_max = 10 with every subshell's orbitals close, all groups formed again: the Lanczos phase
+// 0.39 -> 0.52 ms; none of them: no change.)
+template <int D>
+__device__ __noinline__ void factor_again(const double *M, size_t N, int p0, int m, double *L, double (*s_l)[64],
+                                          double (*s_tri)[kGramEntries]) {
+    constexpr int P = D * (D + 1) / 2;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid < D * D) s_l[0][tid] = L[tid];
+    if (tid < D) s_l[1][tid] = L[tid * D + tid] != 0.0 ? 1.0 / L[tid * D + tid] : 0.0;
+    __syncthreads();
+    double G[P];
+#pragma unroll
+    for (int u = 0; u < P; ++u) G[u] = 0.0;
+    for (int i = tid; i < m; i += kCpThreads) {
+        double y[D];
+#pragma unroll
+        for (int a = 0; a < D; ++a) y[a] = M[a * N + p0 + i];
+#pragma unroll
+        for (int a = 0; a < D; ++a) {
+#pragma unroll
+            for (int b = 0; b < a; ++b) y[a] = fma(-s_l[0][a * D + b], y[b], y[a]);
+            y[a] *= s_l[1][a];
+        }
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+#pragma unroll
+            for (int b = 0; b <= a; ++b) G[a * (a + 1) / 2 + b] = fma(y[a], y[b], G[a * (a + 1) / 2 + b]);
+    }
+    auto add = [](double p, double q) { return p + q; };
+    auto shf = [](double p, int o) { return __shfl_xor_sync(0xffffffffu, p, o); };
+    constexpr int NV = P <= 4 ? 4 : P <= 8 ? 8 : P <= 16 ? 16 : 32, W = 32 / NV;
+    double v[NV];
+#pragma unroll
+    for (int u = 0; u < NV; ++u) v[u] = u < P ? G[u < P ? u : 0] : 0.0;
+    const double r = warp_sums_of<NV>(v, lane, add, shf);   // lane L: value L / W
+    if (lane % W == 0 && lane / W < P) s_tri[warp][lane / W] = r;
+    if constexpr (P > 32) {
+        double x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = G[32 + u];
+        const double r2 = warp_sums_of<4>(x, lane, add, shf);
+        if (lane % 8 == 0) s_tri[warp][32 + lane / 8] = r2;
+    }
+    __syncthreads();
+    if (tid < P) {
+        double s = s_tri[0][tid];
+        for (int w = 1; w < kCpWarps; ++w) s += s_tri[w][tid];
+        s_tri[0][tid] = s;
+    }
+    __syncthreads();
+    if (warp == 0 && warp_cholesky(s_tri[0], D, s_l[2], lane))
+        for (int e = lane; e < D * D; e += 32) {
+            const int a = e / D, b = e % D;
+            double s = 0.0;
+            for (int c = b; c <= a; ++c) s = fma(s_l[0][a * D + c], s_l[2][c * D + b], s);
+            L[e] = s;
+        }
+    __syncthreads();
+}
+
+// The factors that state marks as lossy (2), S.L[g] of groups [S.start[first[g]], S.start[first[g + 1]]).
+__device__ void lossy_factors(const LzChain &C, const CompactScratch &S, const int *first, int ng, const int *state,
+                              double (*s_l)[64], double (*s_tri)[kGramEntries]) {
+    for (int g = 0; g < ng; ++g) {
+        if (state[g] != 2) continue;
+        const int p0 = S.start[first[g]], m = S.start[first[g + 1]] - p0;
+        double *L = S.L + (size_t)g * 64;
+        switch (C.D) {
+            case 1: factor_again<1>(C.M, C.N, p0, m, L, s_l, s_tri); break;
+            case 2: factor_again<2>(C.M, C.N, p0, m, L, s_l, s_tri); break;
+            case 3: factor_again<3>(C.M, C.N, p0, m, L, s_l, s_tri); break;
+            case 4: factor_again<4>(C.M, C.N, p0, m, L, s_l, s_tri); break;
+            case 5: factor_again<5>(C.M, C.N, p0, m, L, s_l, s_tri); break;
+            case 6: factor_again<6>(C.M, C.N, p0, m, L, s_l, s_tri); break;
+            case 7: factor_again<7>(C.M, C.N, p0, m, L, s_l, s_tri); break;
+            default: factor_again<8>(C.M, C.N, p0, m, L, s_l, s_tri); break;
+        }
+    }
 }
 
 // Exclusive scan over one int per thread of the CTA.
@@ -146,7 +236,7 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
     const int Q = S.info->q;
     if (Q < 1) return;   // too many distinct energies (k_lz_groups cleared S.info->handled)
     __shared__ int ws[kCpWarps];
-    __shared__ int s_first[kCpGroups + 1], s_off[kCpGroups + 1];
+    __shared__ int s_first[kCpGroups + 1], s_off[kCpGroups + 1], s_state[kCpMerged];
     __shared__ int s_bad;
     __shared__ unsigned s_rng[2];
     __shared__ double s_tri[kCpWarps][kGramEntries], s_l[kCpWarps][64];
@@ -167,7 +257,8 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
                 s_tri[warp][e] = s;
             }
             __syncwarp();
-            const bool ok = warp_cholesky(s_tri[warp], D, s_l[warp], lane);
+            const int ok = warp_cholesky(s_tri[warp], D, s_l[warp], lane);
+            if (lane == 0) s_state[g] = ok;
             if (ok) {
                 G.kept = 0;
                 G.c = D;
@@ -176,10 +267,14 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
                 if (lane == 0) s_bad = 1;
             }
             __syncwarp();
+        } else if (lane == 0) {
+            s_state[g] = 0;
         }
         if (lane == 0) { S.grp[g] = G; s_off[g] = G.c; }
     }
     __syncthreads();
+    if (s_bad) return;
+    lossy_factors(C, S, s_first, ng, s_state, s_l, s_tri);
     int np;
     {
         const int x = (tid < ng) ? s_off[tid] : 0;
@@ -198,7 +293,7 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
     const int RS = R | 1;
     const size_t need = sizeof(double) * ((size_t)(D + 6 + nla) * np4 + rq + 4 + 20 + 512) +
                         sizeof(int) * (2 * (size_t)np * RS + rq + 4 + (size_t)L);
-    if (s_bad || np > kCpDim || need > (size_t)kCpSmem) return;
+    if (np > kCpDim || need > (size_t)kCpSmem) return;
     double *E = sm, *M = E + np4, *w = M + (size_t)D * np4;
     double *ew = w + np4, *ring = ew + np4, *lasts = ring + 2 * np4, *c = lasts + (size_t)nla * np4, *sc = c + rq + 4;
     FixedSum *part = reinterpret_cast<FixedSum *>(sc + 20);
@@ -653,11 +748,11 @@ __global__ void __launch_bounds__(kCpThreads) k_plain_rotate(const LzChain *chai
         for (size_t i = tid; i < (size_t)D * N; i += kCpThreads) io.M[i] = io.M0[i];
         return;
     }
+    __shared__ int s_state[kCpGroups];
     for (int g = warp; g < ng; g += kCpWarps) {
         const int q0 = s_first[g], q1 = s_first[g + 1];
-        const int p0 = S.start[q0], m = S.start[q1] - p0;
-        bool rot = false;
-        if (m > kKeep) {
+        int rot = 0;
+        if (S.start[q1] - S.start[q0] > kKeep) {
             for (int e = lane; e < D * (D + 1) / 2; e += 32) {
                 double s = 0.0;
                 for (int q = q0; q < q1; ++q) s += S.gram[(size_t)q * kGramEntries + e];
@@ -666,14 +761,24 @@ __global__ void __launch_bounds__(kCpThreads) k_plain_rotate(const LzChain *chai
             __syncwarp();
             rot = warp_cholesky(s_tri[warp], D, s_l[warp], lane);
             __syncwarp();
+            if (rot)
+                for (int e = lane; e < D * D; e += 32) S.L[(size_t)g * 64 + e] = s_l[warp][e];
         }
+        if (lane == 0) s_state[g] = rot;
+        __syncwarp();
+    }
+    __syncthreads();
+    lossy_factors(C, S, s_first, ng, s_state, s_l, s_tri);
+    for (int g = warp; g < ng; g += kCpWarps) {
+        const int p0 = S.start[s_first[g]], m = S.start[s_first[g + 1]] - p0;
+        const bool rot = s_state[g] != 0;
+        const double *L = S.L + (size_t)g * 64;
         const double eg = 0.5 * (C.E[p0] + C.E[p0 + m - 1]);
         for (int i = lane; i < m; i += 32) {
             io.E[p0 + i] = (rot && i < D) ? eg : C.E[p0 + i];
             for (int d = 0; d < D; ++d)
-                io.M[(size_t)d * N + p0 + i] = !rot ? C.M[(size_t)d * N + p0 + i] : i < D ? s_l[warp][d * D + i] : 0.0;
+                io.M[(size_t)d * N + p0 + i] = !rot ? C.M[(size_t)d * N + p0 + i] : i < D ? L[d * D + i] : 0.0;
         }
-        __syncwarp();
     }
 }
 

@@ -132,3 +132,68 @@ def test_norms_of_vectors_short_beside_the_energies(bdmod, synth, shift):
     V = ctx.lanczos_vectors(0, 0, len(lz["lz_fw"]), ctx.count_poles(0)[0]).astype(np.longdouble)
     assert np.abs((V ** 2).sum(1) - 1.0).max() < 8 * 2.2e-16
     ctx.close()
+
+
+def _close_orbitals(synth, p, delta):
+    """The problem with matrix elements that hardly depend on the radial quantum numbers: every subshell's
+    orbitals couple alike but for the part delta."""
+    v, sh = p.vpp, p.ms.orb_sh
+    J = v.iabJ % synth.JMULT
+    (a, b), (c, d) = ((k // synth.JMULT // synth.ABMULT, k // synth.JMULT % synth.ABMULT) for k in (v.iabJ, v.icdJ))
+    k1, k2 = sh[a] * 64 + sh[b], sh[c] * 64 + sh[d]
+    key = (np.minimum(k1, k2).astype(np.int64) * 4096 + np.maximum(k1, k2)) * synth.JMULT + J
+    u, inv = np.unique(key, return_inverse=True)
+    rng = np.random.default_rng(len(u))
+    z = rng.standard_normal(len(u))[inv]
+    z[((sh[a] == sh[b]) | (sh[c] == sh[d])) & (J % 2 == 1)] = 0.0   # (sign changes under exchange)
+    p.vpp = synth.Interaction(v.iabJ, v.icdJ, z * (1.0 + delta * rng.standard_normal(len(z))))
+    return p
+
+
+def _reference_rows(E, M, nit):
+    """Rows of the reduction with unit pivots in extended precision, two Gram-Schmidt sweeps a step."""
+    E, M = E.astype(np.longdouble), M.astype(np.longdouble)
+    D = len(M)
+    V, rows, last = [], [], []
+    for p in range(D):
+        for k in range(nit):
+            w = M[p].copy() if k == 0 else E * V[-1]
+            for _ in range(2):
+                for t in V:
+                    w = w - (t * w).sum() * t
+            beta = np.sqrt((w * w).sum())
+            u = w / beta
+            g = [(V[t] * E * u).sum() for t in last]
+            row = np.zeros(2 * D + 1, np.longdouble)
+            row[0], row[1] = (u * E * u).sum(), g[-1] if k == 0 and g else beta
+            row[2:2 + len(g)] = g
+            row[D + 1:] = M @ u
+            V.append(u)
+            rows.append(row)
+        last.append(len(V) - 1)
+    return np.array(rows)
+
+
+# orbitals whose couplings are alike: pivots of the groups' Gram matrices at about delta^2 of their diagonal entries,
+# from those that are taken as they are to just above the least one that is rotated at all (1e-6)
+@pytest.mark.parametrize("nmax,hw,delta", [(4, 20.0, 1.0), (4, 23.1, 3e-3), (6, 17.3, 0.3), (6, 20.0, 3e-2), (6, 13.7, 3e-3),
+                                           (8, 16.0, 3e-3)])
+def test_rows_of_close_orbitals(bdmod, synth, nmax, hw, delta):
+    p = synth.make_problem(nmax, hw, 3, 3)
+    if delta < 1.0:
+        _close_orbitals(synth, p, delta)
+    ctx = bdmod.Context().upload(p)
+    D = int(p.ms.no[0])
+    nit = np.full(D, 3, np.int32)
+    err = []
+    for mode in (0, 1):
+        ctx.set_lanczos_slices(mode)
+        fw, bk = ctx.sigma2_build(0)
+        lz = ctx.lanczos_reduce(0, np.eye(D), nit, nit)
+        for sig, tag in ((fw, "lz_fw"), (bk, "lz_bk")):
+            E, M = sig[:, 0], np.ascontiguousarray(sig[:, 2:].T)
+            d = np.abs(lz[tag] - _reference_rows(E, M, 3))
+            err.append([float(d[:, :D + 1].max() / np.abs(E).max()), float(d[:, D + 1:].max() / np.abs(lz[tag][:, D + 1:]).max())])
+    ctx.close()
+    # what the reduction over the poles makes of the same rows, within the scatter of two roundings
+    assert np.all(np.array(err[:2]) <= 8 * np.array(err[2:]) + 1e-15), err
