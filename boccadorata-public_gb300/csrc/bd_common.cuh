@@ -198,16 +198,17 @@ struct CompactScratch {
     CompactGroup *grp;   // [kCpMerged]
     double *gram;        // [kCpGroups][kGramEntries] M M^T of every energy's poles, lower triangle
     double *L;           // [kCpGroups][64] the groups' factors, D x D row-major
+    double *M;           // [8][kCpDim] the rotated poles' couplings
 };
 constexpr long long kCpStartOff = 256, kCpGrpOff = kCpStartOff + 4 * (kCpGroups + 4),
                     kCpGramOff = (kCpGrpOff + 20 * kCpMerged + 255) / 256 * 256,
                     kCpLOff = kCpGramOff + 8LL * kCpGroups * kGramEntries,
-                    kCpBytes = (kCpLOff + 8LL * 64 * kCpGroups + 255) / 256 * 256;
+                    kCpMOff = kCpLOff + 8LL * 64 * kCpGroups, kCpBytes = (kCpMOff + 8LL * 8 * kCpDim + 255) / 256 * 256;
 static_assert(sizeof(CompactInfo) <= kCpStartOff && sizeof(CompactGroup) == 20, "compact scratch layout");
 __host__ __device__ inline CompactScratch lz_compact(char *b) {
     return CompactScratch{reinterpret_cast<CompactInfo *>(b), reinterpret_cast<int *>(b + kCpStartOff),
                           reinterpret_cast<CompactGroup *>(b + kCpGrpOff), reinterpret_cast<double *>(b + kCpGramOff),
-                          reinterpret_cast<double *>(b + kCpLOff)};
+                          reinterpret_cast<double *>(b + kCpLOff), reinterpret_cast<double *>(b + kCpMOff)};
 }
 
 // Rows of a plain Sigma(2) for the full Dyson matrix (k_plain_rotate): as built, and rotated.

@@ -314,6 +314,7 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
             for (int d = 0; d < D; ++d) {
                 const double m = G.kept ? C.M[(size_t)d * N + G.p0 + i] : S.L[(size_t)g * 64 + d * D + i];
                 M[(size_t)d * np4 + s_off[g] + i] = m;
+                S.M[d * kCpDim + s_off[g] + i] = m;   // for w = M p (the planes are for m)
                 mm = max(mm, (unsigned)__double2hiint(m) & 0x7fffffffu);
             }
         }
@@ -409,10 +410,12 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
             float s2 = 0.0f;
             for (int i = tid; i < np; i += kCpThreads) {
                 const double *p = s_piv + k * D;
-                double x = 0.0;
-                for (int d = 0; d < D; ++d)
-                    x = fma(fixed_to_double(Ma[(size_t)d * np4 + i], Mb[(size_t)d * np4 + i]) *
-                                __hiloint2double(s_mb[d] << 20, 0), p[d], x);
+                double x = 0.0, m[8];
+#pragma unroll
+                for (int d = 0; d < 8; ++d) m[d] = d < D ? S.M[d * kCpDim + i] : 0.0;
+#pragma unroll
+                for (int d = 0; d < 8; ++d)
+                    if (d < D) x = fma(m[d], p[d], x);
                 w[i] = x;
                 const float f = f32_trunc(x);
                 s2 = fmaf(f, f, s2);
