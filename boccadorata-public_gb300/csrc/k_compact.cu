@@ -21,8 +21,11 @@
 //                  orthonormalising clusters of a hundred equal eigenvalues, takes 0.92).
 //
 // Energies that differ by rounding only (e1 + e2 - e3 of orbits of the same shells added
-// in another order, a few ulp) count as one group: kMergeUlp ulp of the largest energy, a
-// relative change of E below its own rounding.  The Gram matrices come from k_lz_groups
+// in another order: over hbar omega of 5 to 40 MeV and N_max of 4 to 12 a shell's differ by at
+// most 2.2 eps of the largest energy) count as one group, whose poles take the middle of it.
+// All of a group lies within kMergeUlp eps, so that moves E by no more than the rounding of the
+// sum; a set in which neighbours lie that close and the whole run does not is not one of such
+// shells, and is left as it is.  The Gram matrices come from k_lz_groups
 // (sums of FP64 products in a fixed order).  A group keeps its poles as they are when it
 // has at most kKeep, or at most kGrpSmall and a pivot that loses digits (below kPivot of
 // its diagonal entry); a larger group with such a pivot leaves the whole chain to
@@ -48,7 +51,7 @@ namespace {
 constexpr int kCpThreads = 256;
 constexpr int kCpWarps = kCpThreads / 32;
 constexpr int kKeep = 12;
-constexpr double kMergeUlp = 16.0;
+constexpr double kMergeUlp = 4.0;
 constexpr double kPivot = 1e-6, kLossy = 0.125;
 constexpr int kCpSmem = 200 * 1024;
 
@@ -187,7 +190,8 @@ __device__ __forceinline__ int scan_ints(int x, int &total, int *ws) {
 }
 
 // The merged groups of a chain (first exact group of each, s_first[0 .. n], s_first[n] = Q)
-// from the exact groups' energies; returns their number.  One thread per exact group.
+// from the exact groups' energies; returns their number, 0 when one spans more than kMergeUlp.
+// One thread per exact group.
 __device__ int merge_groups(const double *gE, int Q, int *s_first, int *ws) {
     const int tid = threadIdx.x;
     const double tol = kMergeUlp * DBL_EPSILON * fmax(fabs(gE[0]), fabs(gE[Q - 1]));
@@ -197,7 +201,8 @@ __device__ int merge_groups(const double *gE, int Q, int *s_first, int *ws) {
     if (brk) s_first[pos] = tid;
     if (tid == 0) s_first[n] = Q;
     __syncthreads();
-    return n;
+    const bool wide = tid < n && fabs(gE[s_first[tid + 1] - 1] - gE[s_first[tid]]) > tol;
+    return __syncthreads_or(wide) ? 0 : n;
 }
 
 static_assert(kCpThreads >= kCpGroups, "a thread per exact group");
@@ -243,7 +248,7 @@ __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains
     extern __shared__ double sm[];
     if (tid == 0) { s_bad = 0; s_rng[0] = 0; s_rng[1] = 0; }
     const int ng = merge_groups(C.gE, Q, s_first, ws);
-    if (ng > kCpMerged) return;
+    if (ng < 1 || ng > kCpMerged) return;
     // 1. every merged group's coordinates: its own poles (kept), or the columns of L
     for (int g = warp; g < ng; g += kCpWarps) {
         const int q0 = s_first[g], q1 = s_first[g + 1];

@@ -197,3 +197,21 @@ def test_rows_of_close_orbitals(bdmod, synth, nmax, hw, delta):
     ctx.close()
     # what the reduction over the poles makes of the same rows, within the scatter of two roundings
     assert np.all(np.array(err[:2]) <= 8 * np.array(err[2:]) + 1e-15), err
+
+
+# steps of energies that are rounding's one by one (3 eps) and not as a run, and steps just beyond rounding
+@pytest.mark.parametrize("step", [3.0, 12.0])
+def test_energies_a_few_eps_apart(bdmod, synth, step):
+    """Levels of a shell a few eps apart: no pole's energy moves by more than its own rounding."""
+    p = synth.make_problem(4, 20.0, 3, 3)
+    p.prop.ep[:] += (np.arange(len(p.prop.ep)) % 3) * step * 2.0 ** -52 * 200.0
+    ctx = bdmod.Context().upload(p)
+    D = int(p.ms.no[0])
+    nit = np.full(D, 3, np.int32)
+    fw, _ = ctx.sigma2_build(0)
+    lz = ctx.lanczos_reduce(0, np.eye(D), nit, nit)["lz_fw"]
+    ctx.close()
+    E = fw[:, 0]
+    ref = _reference_rows(E, np.ascontiguousarray(fw[:, 2:].T), 3)
+    # alpha is a mean of the energies: their half span in a group (2 eps), and the rounding of its sum
+    assert np.abs(lz[:, 0] - ref[:, 0]).max() < 6 * 2.2e-16 * np.abs(E).max()
