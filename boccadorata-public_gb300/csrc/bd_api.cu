@@ -60,7 +60,8 @@ struct Chan {
     ChainPlan lz[2];
     // resident results of the per-channel API
     int state = ST_NONE;
-    bool ref_sorted = false;   // the sort permutation holds the reference's order of equal energies
+    bool ref_sorted = false;   // the sorted poles and their permutation are in the reference's order of equal energies
+    bool lz_ref = false;       // they were when the channel was last reduced
 };
 
 // Host array in page-locked memory (grown by reallocation, contents not kept), so a
@@ -1129,6 +1130,7 @@ int launch_plain(bd_ctx *ctx, int ch_lo, int ch_hi) {
     if (ch.empty()) return BD_OK;
     int rc;
     if ((rc = launch_sort(ctx, ch_lo, ch_hi, false))) return rc;
+    for (int I = ch_lo; I < ch_hi; ++I) ctx->chans[I].ref_sorted = false;
     LzChain *d_ch = ctx->d_dychains + 2 * ch_lo;   // this range's own slots
     PlainIO *d_io = ctx->d_dyio + 2 * ch_lo;
     if ((rc = h2d_table(ctx, d_ch, ch.data(), sizeof(LzChain) * ch.size()))) return rc;
@@ -2028,7 +2030,7 @@ int bd_lanczos_reduce(bd_ctx *ctx, int ish, int n_pvt, double *pivots, int *n_it
     const bool fp32 = (flags & BD_RUN_MIXED) != 0;
     const bool ref_order = !fp32 && (flags & BD_RUN_REF_ORDER);
     if ((rc = launch_sort(ctx, ish, ish + 1, ref_order))) return rc;
-    C.ref_sorted = ref_order;
+    C.ref_sorted = C.lz_ref = ref_order;
     if ((rc = launch_lanczos_range(ctx, ish, ish + 1, fp32))) return rc;
     for (int dir = 0; dir < 2; ++dir) {
         const ChainPlan &P = C.lz[dir];
@@ -2209,7 +2211,11 @@ int bd_lanczos_vectors(bd_ctx *ctx, int ish, int dir, int fp32, double *out, lon
         CU(cudaMemcpy(&info, cp, sizeof info, cudaMemcpyDeviceToHost));
         handled = info.handled;
         if (handled == 1) {
-            const Chan &C = ctx->chans[ish];
+            Chan &C = ctx->chans[ish];
+            if (C.ref_sorted != C.lz_ref) {   // the sorted couplings in the order the chain was reduced in
+                if ((rc = launch_sort(ctx, ish, ish + 1, C.lz_ref))) return rc;
+                C.ref_sorted = C.lz_ref;
+            }
             CU(cudaMallocAsync(&expanded, sizeof(double) * (size_t)P.L * ld, ctx->st));
             LzChain z{};
             z.N = P.N; z.D = C.D; z.ld = ld; z.V = ctx->d_lzV + ctx->lz_v_off[dir][ish]; z.cp = cp;
@@ -2366,6 +2372,7 @@ int bd_run_all(bd_ctx *ctx, int flags) {
     for (int I = 0; I < ns; ++I) {
         ctx->chans[I].state = lanczos ? ST_LANCZOS : ST_SIGMA;
         ctx->chans[I].ref_sorted = lanczos && (flags & BD_RUN_REF_ORDER) && !(flags & BD_RUN_MIXED);
+        if (lanczos) ctx->chans[I].lz_ref = ctx->chans[I].ref_sorted;
     }
     ctx->last_lanczos_flags = flags;
     ctx->results_valid = true;

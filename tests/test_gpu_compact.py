@@ -215,3 +215,26 @@ def test_energies_a_few_eps_apart(bdmod, synth, step):
     ref = _reference_rows(E, np.ascontiguousarray(fw[:, 2:].T), 3)
     # alpha is a mean of the energies: their half span in a group (2 eps), and the rounding of its sum
     assert np.abs(lz[:, 0] - ref[:, 0]).max() < 6 * 2.2e-16 * np.abs(E).max()
+
+
+@pytest.mark.parametrize("ref_order", [False, True])
+@pytest.mark.parametrize("nmax,hw,nit", [(3, 13.7, 7), (5, 20.0, 3)])
+def test_vectors_keep_the_reduction_s_order(bdmod, problems, nmax, hw, nit, ref_order):
+    """The stored vectors read back before and after the sorted poles were put in another order of their equal
+    energies: the same, pole by pole."""
+    p = problems(nmax, hw, 3, nit)
+    ctx = bdmod.Context().upload(p)
+    pv = p.piv
+    for ish in range(p.ms.nsubsh):
+        n = ctx.count_poles(ish)
+        ctx.sigma2_build(ish, copy=False)
+        lz = ctx.lanczos_reduce(ish, pv.vec[ish], pv.n_fw[ish], pv.n_bk[ish], ref_order=ref_order)
+        L = (len(lz["lz_fw"]), len(lz["lz_bk"]))
+        before = [ctx.lanczos_vectors(ish, d, L[d], n[d]) for d in (0, 1) if L[d]]
+        sorted_rows = ctx.sigma2_sorted(ish)
+        after = [ctx.lanczos_vectors(ish, d, L[d], n[d]) for d in (0, 1) if L[d]]
+        for a, b in zip(before, after):
+            assert np.array_equal(a, b), ish
+        for a, b in zip(sorted_rows, ctx.sigma2_sorted(ish)):
+            assert np.array_equal(a, b), ish
+    ctx.close()
