@@ -10,8 +10,8 @@
 //       k_tridiag_df      the same for larger orders, one thread-block cluster per
 //                         matrix (rows split across the CTAs),
 //       k_tridiag_grid    the same for one large matrix alone, a CTA on every SM,
-//       k_tridiag         in FP64 for orders beyond that kernel's shared memory (Q's rows
-//                         by k_qrows),
+//       k_tridiag         in FP64 for launches of orders beyond about 2 300, and beyond those
+//                         kernels' shared memory (Q's rows by k_qrows),
 //   K4b..K5 (k_eig.cu)    eigenvalues and the first D eigenvector components of T,
 //                         back-transformed, split by E_F, Koltun sums.
 #include <algorithm>
@@ -1248,9 +1248,15 @@ void tridiag_fit_warm() {
 }
 
 // Shared memory of k_tridiag_df (8-byte slots, at most kTdfSlots: 224 KB) and the largest
-// order whose vectors fit in it (the rows may spill).
+// order it takes in a launch of orders up to nmax: as far as its vectors fit (the rows may
+// spill), where all of the launch's orders leave k_tridiag room for a partial vector a warp
+// (orders up to about 2 300); kTsMax, none, beyond.  There FP64 stays: double-float is twelve
+// times as fast (a solve of order 2 500, 38 ms against 465) but its rounding, 2^-48 a step,
+// grows with the order beside the bisection's 1e-13 |T| (eigenvector components off by 1.8e-14
+// against 1.0e-15 in the median, 8.6e-11 against 3.5e-12 at the most).
 constexpr int kTdfSlots = 224 * 1024 / 8;
-int tridiag_df_limit(int cluster, int D) {
+int tridiag_df_limit(int nmax, int cluster, int D) {
+    if (tridiag_npriv(std::min(nmax, tridiag_fit_order(cluster)), cluster) < kTdThreads / 32) return kTsMax;
     int lo = kTsMax, hi = 1 << 16;
     while (lo < hi) {
         const int mid = lo + (hi - lo + 1) / 2;
@@ -1280,8 +1286,8 @@ static bool tridiag_on_grid(int njobs, int nmax, int nlim) {
 // small-matrix reduction (the cluster one beyond kTsMax, the FP64 one and k_qrows beyond
 // its limit), then launch_eig's.
 int dyson_launch_count(int njobs, int nmax, int Dmax, int cluster) {
-    const int nlim = tridiag_df_limit(cluster, Dmax);
-    return 3 + (nmax > kTsMax ? 1 : 0) + (tridiag_on_grid(njobs, nmax, nlim) ? 1 : 0) + (nmax > nlim ? 2 : 0) + (nmax > kTsMax ? 8 : 7);
+    const int nlim = tridiag_df_limit(nmax, cluster, Dmax);
+    return 3 + (nmax > kTsMax && nlim > kTsMax ? 1 : 0) + (tridiag_on_grid(njobs, nmax, nlim) ? 1 : 0) + (nmax > nlim ? 2 : 0) + (nmax > kTsMax ? 8 : 7);
 }
 
 cudaError_t launch_dyson(const DyJob *d_jobs, int njobs, const long long *d_row_first, long long total_rows,
@@ -1316,7 +1322,7 @@ cudaError_t launch_dyson(const DyJob *d_jobs, int njobs, const long long *d_row_
         if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         return e == cudaSuccess;
     };
-    const int nlim = tridiag_df_limit(cluster, Dmax);
+    const int nlim = tridiag_df_limit(nmax, cluster, Dmax);
     const bool grid = tridiag_on_grid(njobs, nmax, nlim);
     if (grid) {
         cudaLaunchConfig_t gc = {};
@@ -1333,7 +1339,11 @@ cudaError_t launch_dyson(const DyJob *d_jobs, int njobs, const long long *d_row_
         if (e == cudaSuccess) e = cudaLaunchKernelEx(&gc, k_tridiag_grid, d_jobs, nlim, kTdfSlots, work, d_work_first);
         if (e != cudaSuccess) return e;
     }
-    {
+    if (nlim == kTsMax) {
+        k_tridiag_small<<<njobs, kTsThreads, ssmem, st>>>(d_jobs, njobs);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    } else {
         // as many slots as the largest order (the full orders bound the deflated ones) needs
         // to keep all its rows, at most kTdfSlots
         const int nb = grid ? kTdgMin - 1 : std::min(nmax, nlim);

@@ -125,3 +125,30 @@ def test_whole_gpu_reductions_of_two_threads(bdmod, problems):
     assert not bad
     for j in jobs:
         j[0].close()
+
+
+def test_orders_beyond_2300_in_fp64(bdmod, problems):
+    """The eigenvector components of an order that is reduced in FP64: off by LAPACK's own rounding in the median
+    (about 1e-15), where double-float's 2^-48 leaves 1.8e-14."""
+    p = problems(6, 20.0, 1, 50)
+    n, ish = 2403, 0
+    rng = np.random.default_rng(n)
+    ctx = bdmod.Context().upload(p)
+    D = int(p.ms.no[ish])
+    nb = n // 5
+    nf = n - D - nb
+    fw, bk = np.zeros((nf, 2 + D)), np.zeros((nb, 2 + D))
+    fw[:, 0], bk[:, 0] = rng.uniform(20.0, 300.0, nf), -rng.uniform(60.0, 250.0, nb)
+    fw[:, 2:], bk[:, 2:] = (rng.standard_normal((k, D)) * (4.0 / np.sqrt(nf)) for k in (nf, nb))
+    s1, hf = np.diag(np.linspace(-20.0, 60.0, D)), np.zeros((D, D))
+    r = ctx.dyson_rows(ish, 2, fw, bk, sig1b=s1, sighf=hf, efermi=-50.0)
+    ctx.close()
+    A = np.diag(np.concatenate([np.zeros(D), fw[:, 0], bk[:, 0]]))
+    A[:D, :D] = s1
+    A[D:, :D] = np.concatenate([fw[:, 2:], bk[:, 2:]])
+    A[:D, D:] = A[D:, :D].T
+    w, v = np.linalg.eigh(A)
+    got = np.concatenate([r["qp"], r["qh"]])
+    got, ref = got[np.argsort(got[:, 0])], v[:D].T
+    x = got[:, 2:] * np.where((got[:, 2:] * ref).sum(1) < 0.0, -1.0, 1.0)[:, None]
+    assert np.median(np.abs(x - ref).max(1)) < 6e-15
