@@ -20,6 +20,7 @@
 #include "bd_common.cuh"
 #include "bd_kernels.h"
 #include "df64.cuh"
+#include "lz_fixed.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -388,14 +389,14 @@ __global__ void __launch_bounds__(kTdThreads) k_tridiag(const DyJob *jobs, int n
 // Rows live in shared memory, the last ones first (they stay longest); those that do not fit
 // in the job's work area.  Step k (trailing rows and columns > k) takes one pass over the
 // matrix instead of a product and an update: the pass applies step k-1's rank-2 update and
-// multiplies by step k's column as it goes.  The column is used unscaled, as in
-// k_tridiag_small, so the reflector's scalars are formed by one warp beside the pass:
+// multiplies by step k's column as it goes.  The column is used as it is (v is x but for a power
+// of two and its first entry), so the reflector's scalars are formed by one warp beside the pass:
 //   pass      a_ij -= v'_i w'_j + w'_i v'_j (v', w' of step k-1), S_i = sum_{j>k+1} a_ij x_j, two
 //             rows a warp; the same product for this CTA's rows of R; warp kTdScal: |x|^2 from
-//             the CTAs' partial sums, then tau and s
-//   own rows  y_i = a_i,k+1 + s S_i = (A v)_i to every CTA, with the warps' partials of v^T A v;
+//             the CTAs' partial sums, then h, v_0 and g
+//   own rows  y_i = v_0 a_i,k+1 + g S_i = (A v)_i to every CTA, with the warps' partials of v^T A v;
 //             cluster barrier
-//   all rows  v = s x, w = tau y - (tau^2 / 2) (v^T A v) v; R -= tau (R v) v^T
+//   all rows  v = g x, w = h y - (h^2 / 2) (v^T A v) v; R -= h (R v) v^T (R in FP64)
 //   own rows  column k+1 of the updated matrix to every CTA (x of the next step, d_{k+1} from
 //             the diagonal), with the partials of its square; cluster barrier
 // Bound by these two cluster barriers and the chains between them (about 4 000 cycles a
@@ -426,6 +427,9 @@ __device__ inline dfm::df df_from_bits(double x) {
     return dfm::renorm(hi, lo);
 }
 
+// a pair's value, one FP64 instruction (the conversions from the words' bits)
+__device__ __forceinline__ double df_value(dfm::df a) { return f32_to_double(a.h) + f32_to_double(a.l); }
+
 __device__ inline int f32_exponent(float x) { return (int)((__float_as_uint(x) >> 23) & 255u) - 127; }
 __device__ inline float pow2_f32(int e) { return __uint_as_float((unsigned)(e + 127) << 23); }
 
@@ -436,6 +440,32 @@ constexpr int kTdfThreads = 512, kTdfWarps = kTdfThreads / 32, kTdScal = kTdfWar
 __host__ __device__ inline size_t tdf_fixed(int n, int CL, int D) {
     const int nrm = (n + CL - 1) / CL;
     return (size_t)(4 + (D + CL - 1) / CL) * n + 2 * (size_t)nrm + 2 * (size_t)CL * kTdfWarps + 32;
+}
+
+__device__ __forceinline__ dfm::df scaled(dfm::df a, float g) { return dfm::df{dfm::fmul(a.h, g), dfm::fmul(a.l, g)}; }
+
+// The reflector H = 1 - h v v^T that takes a column x = (alpha, x_1, ..) to (beta, 0, ..): v = g x
+// but for v_0 = g (alpha - beta), with g a power of two that brings |x| to about one, so v holds
+// x's own bits and the products A x formed before the scalars were known are A v's.  s2: |x_1:|^2;
+// h is zero when there is nothing to reflect.
+struct Reflector { dfm::df h, v0, beta; float g; };
+__device__ __forceinline__ Reflector reflector(dfm::df al, dfm::df s2) {
+    using dfm::df;
+    Reflector o{df{0.0f, 0.0f}, df{0.0f, 0.0f}, al, 1.0f};
+    if (s2.h != 0.0f || s2.l != 0.0f) {
+        const int ea = (al.h != 0.0f) ? f32_exponent(al.h) : -1000;
+        int e = max(ea, f32_exponent(s2.h) >> 1);
+        e = min(max(e, -126), 126);
+        o.g = pow2_f32(-e);
+        const df alt = scaled(al, o.g), x2 = dfm::fma(alt, alt, scaled(scaled(s2, o.g), o.g));   // in [1, 12)
+        const df r = dfm::rsqrt2(x2), nx = dfm::mul(x2, r);
+        const bool ng = signbit(alt.h);
+        const df u = dfm::add(ng ? dfm::neg(alt) : alt, nx);   // |alpha| + |x|
+        o.h = dfm::mul(r, dfm::rcp2(u));                       // 2 / v^T v
+        o.v0 = ng ? dfm::neg(u) : u;
+        o.beta = scaled(ng ? nx : dfm::neg(nx), pow2_f32(e));
+    }
+    return o;
 }
 
 // a - (vi wj + wi vj): both products exact to ~2^-48, summed before they meet a; the same bits
@@ -477,18 +507,19 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_df(const DyJob *jobs
     df *W = V + 2 * (size_t)n;                   // [2][n]
     df *kb = W + 2 * (size_t)n;                  // [kTdfWarps][CL] partials of v . y
     df *sb = kb + (size_t)CL * kTdfWarps;        // [kTdfWarps][CL] partials of |x_1:|^2
-    df *R = sb + (size_t)CL * kTdfWarps;         // [NRR][n]
-    df *rs = R + (size_t)((D + CL - 1) / CL) * n;   // [nrm] S of own rows
+    double *R = reinterpret_cast<double *>(sb + (size_t)CL * kTdfWarps);   // [NRR][n]
+    df *rs = reinterpret_cast<df *>(R + (size_t)((D + CL - 1) / CL) * n);   // [nrm] S of own rows
     df *ra = rs + nrm;                           // [nrm] a_{i,k+1}
     df *rows = reinterpret_cast<df *>(sm) + tdf_fixed(n, CL, D);
     const int room = max(0, (smem_df - (int)tdf_fixed(n, CL, D)) / n);
     const int qs = max(0, nr - room);            // own rows q >= qs in shared memory
     df *spill = reinterpret_cast<df *>(work + work_first[jid]);
     auto row = [&](int q) -> df * { return q >= qs ? rows + (size_t)(q - qs) * n : spill + (size_t)(rank + q * CL) * n; };
-    __shared__ df s_sc[2];      // tau, s of the step
-    __shared__ df s_rd[8];      // R_d . v of own R rows
-    const df zero{0.0f, 0.0f}, one{1.0f, 0.0f};
-    // d, e and tau stay double-float pairs in their FP64 slots until the end: a conversion is
+    __shared__ df s_sc[2];      // h, v_0 of the step
+    __shared__ float s_g;       // and the power of two that scales x
+    __shared__ double s_rd[8], s_c[8];   // R_d . x_{1:} of own R rows, -h R_d . v
+    const df zero{0.0f, 0.0f};
+    // d and e stay double-float pairs in their FP64 slots until the end: a conversion is
     // two FP64 instructions on a chain that other warps wait for
     auto put = [](double *p, df x) { *reinterpret_cast<float2 *>(p) = make_float2(x.h, x.l); };
     // the sum of cnt values by a warp, the same in every lane
@@ -509,7 +540,7 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_df(const DyJob *jobs
         V[j] = xj;
         V[n + j] = zero;
         W[n + j] = zero;
-        for (int u = 0; u < NRR; ++u) R[(size_t)u * n + j] = (j == rank + u * CL) ? one : zero;
+        for (int u = 0; u < NRR; ++u) R[(size_t)u * n + j] = (j == rank + u * CL) ? 1.0 : 0.0;
         if (j >= 2) sq0 = dfm::fma(xj, xj, sq0);
     }
     // the squares of column 0, summed by every CTA for itself
@@ -527,30 +558,12 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_df(const DyJob *jobs
         // pass
         if (warp == kTdScal) {
             const df s2 = sum_of(sb, nsb);
-            const df al = x[b0];
-            df tau = zero, scal = zero, beta = al;
-            if (s2.h != 0.0f || s2.l != 0.0f) {
-                const int ea = (al.h != 0.0f) ? f32_exponent(al.h) : -1000;
-                int e = max(ea, f32_exponent(s2.h) >> 1);
-                e = min(max(e, -126), 126);
-                const float sg = pow2_f32(-e);
-                const df alt{al.h * sg, al.l * sg}, s2t{(s2.h * sg) * sg, (s2.l * sg) * sg};
-                const df x2 = dfm::fma(alt, alt, s2t);   // in [1, 12)
-                const df r = dfm::rsqrt2(x2), nx = dfm::mul(x2, r);
-                const bool ng = signbit(alt.h);
-                const df aa = ng ? dfm::neg(alt) : alt;
-                tau = dfm::fma(aa, r, one);
-                df st = dfm::rcp2(dfm::add(aa, nx));   // 1 / (alpha~ - beta~)
-                if (ng) st = dfm::neg(st);
-                scal = df{st.h * sg, st.l * sg};         // 1 / (alpha - beta)
-                const df bt = ng ? nx : dfm::neg(nx);
-                const float un = pow2_f32(e);
-                beta = df{bt.h * un, bt.l * un};
-            }
+            const Reflector r = reflector(x[b0], s2);
             if (lane == 0) {
-                s_sc[0] = tau;
-                s_sc[1] = scal;
-                if (rank == 0) { put(J.e + k, beta); put(J.tau + k, tau); }
+                s_sc[0] = r.h;
+                s_sc[1] = r.v0;
+                s_g = r.g;
+                if (rank == 0) put(J.e + k, r.beta);
             }
         }
         {   // the active own rows in runs of consecutive ones, one run a warp (the scalars' warp
@@ -607,30 +620,31 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_df(const DyJob *jobs
             // R_d . x_{1:} of own R rows, from the warps before the scalars' one
             if (warp < kTdScal && kTdScal - 1 - warp < NRR) {
                 const int u = kTdScal - 1 - warp;
-                const df *r = R + (size_t)u * n;
-                df s0 = zero, s1 = zero;
-                int j = b0 + 1 + lane;
-                for (; j + 32 < n; j += 64) { s0 = dfm::fma(r[j], x[j], s0); s1 = dfm::fma(r[j + 32], x[j + 32], s1); }
-                if (j < n) s0 = dfm::fma(r[j], x[j], s0);
-                s0 = dfm::warp_sum(dfm::add(s0, s1));
-                if (lane == 0) s_rd[u] = s0;
+                const double *r = R + (size_t)u * n;
+                double t = 0.0;
+                for (int j = b0 + 1 + lane; j < n; j += 32) t = fma(r[j], df_value(x[j]), t);
+                for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+                if (lane == 0) s_rd[u] = t;
             }
         }
         __syncthreads();
-        const df tau = s_sc[0], s = s_sc[1];
-        const bool nz = (tau.h != 0.0f);
+        const df hs = s_sc[0], v0 = s_sc[1];
+        const float g = s_g;
+        const bool nz = (hs.h != 0.0f);
         // own rows, a lane per (row, receiving CTA): y to every CTA, partials of v . y (of the
         // warp's RW rows, the same count of warps in every CTA)
         const int wpk = min(kTdfWarps, (int)((unsigned)((n - b0 + CL - 1) / CL + RW - 1) / RW));
         const int to = lane % CL, q_ = q0 + warp * RW + lane / CL;
+        if (warp == kTdScal && lane < NRR)
+            s_c[lane] = -df_value(hs) * fma(df_value(v0), R[(size_t)lane * n + b0], (double)g * s_rd[lane]);
         if (warp < wpk) {
             df kv = zero;
             df *yr = cluster.map_shared_rank(y, to);
             for (int q = q_; q < nr; q += kTdfWarps * RW) {
                 const int i = rank + q * CL;
-                const df yi = nz ? dfm::fma(s, rs[q], ra[q]) : zero;
+                const df yi = nz ? dfm::fma(v0, ra[q], scaled(rs[q], g)) : zero;
                 yr[i] = yi;
-                kv = (i == b0) ? dfm::add(kv, yi) : dfm::fma(dfm::mul(s, x[i]), yi, kv);
+                kv = dfm::fma((i == b0) ? v0 : scaled(x[i], g), yi, kv);
             }
 #pragma unroll
             for (int o = 16; o >= CL; o >>= 1) kv = dfm::add(kv, dfm::shfl_xor(kv, o));
@@ -640,24 +654,16 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_df(const DyJob *jobs
         // all rows: v, w; R
         {
             const df K = sum_of(kb, wpk * CL);
-            const df tk = dfm::mul(tau, tau);
-            const df nK = dfm::neg(dfm::mul(df{0.5f * tk.h, 0.5f * tk.l}, K));
+            const df hh = dfm::mul(hs, hs);
+            const df nK = dfm::neg(dfm::mul(df{0.5f * hh.h, 0.5f * hh.l}, K));
             for (int j = b0 + tid; j < n; j += kTdfThreads) {
-                const df vj = !nz ? zero : (j == b0) ? one : dfm::mul(s, x[j]);
-                y[j] = dfm::fma(nK, vj, dfm::mul(tau, y[j]));
+                const df vj = !nz ? zero : (j == b0) ? v0 : scaled(x[j], g);
+                y[j] = dfm::fma(nK, vj, dfm::mul(hs, y[j]));
                 x[j] = vj;
-                for (int u = 0; u < NRR; ++u) {
-                    df &r = R[(size_t)u * n + j];
-                    const df c = dfm::neg(dfm::mul(tau, dfm::fma(s, s_rd[u], R[(size_t)u * n + b0])));
-                    if (j != b0) r = dfm::fma(c, vj, r);
-                }
+                for (int u = 0; u < NRR; ++u) R[(size_t)u * n + j] = fma(s_c[u], df_value(vj), R[(size_t)u * n + j]);
             }
         }
         __syncthreads();
-        if (tid < NRR && nz) {   // R_d[b0], read by every thread above
-            df &r = R[(size_t)tid * n + b0];
-            r = dfm::fma(dfm::neg(dfm::mul(tau, dfm::fma(s, s_rd[tid], r))), one, r);
-        }
         // own rows: column k+1 of the updated matrix
         if (warp < wpk) {
             const df vb = x[b0], wb = y[b0];
@@ -689,32 +695,34 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_df(const DyJob *jobs
             auto conv = [](double *p) { const float2 f = __ldcg(reinterpret_cast<const float2 *>(p)); *p = dfm::to_double(df{f.x, f.y}); };
             conv(J.d + j);
             if (j + 1 < n) conv(J.e + j); else J.e[j] = 0.0;
-            if (j + 2 < n) conv(J.tau + j); else J.tau[j] = 0.0;
         }
     for (int u = 0; u < NRR; ++u)
-        for (int j = tid; j < n; j += kTdfThreads) J.R[(size_t)(rank + u * CL) * n + j] = dfm::to_double(R[(size_t)u * n + j]);
+        for (int j = tid; j < n; j += kTdfThreads) J.R[(size_t)(rank + u * CL) * n + j] = R[(size_t)u * n + j];
 }
 
 // ---------------------------------------------------------------- K4a''' one matrix, the whole GPU
 // A matrix reduced alone leaves a cluster's 16 SMs to do the pass and most of its rows in L2 (order
-// 1 000: 25 000 cycles a column, two thirds of them the pass).  Here every SM takes rows: a
-// cooperative launch, one CTA an SM, row i with CTA (i mod G), and what the CTAs exchange goes
-// through L2.  Step k, with one grid barrier:
-//   pass      as k_tridiag_df's, 1 to 4 warps a row
-//   own rows  y_i = a_i,k+1 + s S_i and the CTA's part of v^T A v; from its owner row k+1; barrier
+// 1 000: 25 000 cycles a column, two thirds of them the pass).  Here every SM takes part: a
+// cooperative launch, one CTA an SM, row i with CTA (i mod H), and what the CTAs exchange goes
+// through L2.  The last D CTAs have a row of R each and none of the matrix: R is FP64, and 2 n of
+// its instructions a column beside a CTA's own rows would hold up the barrier (order 1 000: 5.6 ms
+// for 4.7), in the time the others take for the pass they do not.  Step k, with one grid barrier:
+//   pass      as k_tridiag_df's, 1 to 4 warps a row; R_d . x
+//   own rows  y_i = v_0 a_i,k+1 + g S_i and the CTA's part of v^T A v; from its owner row k+1; barrier
 //   all rows  v, w, R; from row k+1, which is column k+1, that column after this step's update (x
 //             of the next step, d_{k+1} on the diagonal), and the sum of its squares, by every CTA
 //             for itself
 // Bound by the barrier and what surrounds it in a column (order 1 000, 9 000 cycles: the pass beside
 // the scalars' chain 3 000, y 1 000, the barrier 3 200, then L2, the sum of the parts, v and w).
 // Order 1 000: 12.8 ms by the cluster kernel -> 4.7.
-constexpr int kTdgRowWarps = kTdfWarps - 2;   // the others: R's product, the scalars
+constexpr int kTdgRowWarps = kTdfWarps - 1;   // the other: the scalars
 constexpr int kTdgParts = 4;                  // warps a row at most
 constexpr int kTdgPolls = 1 << 20;            // a barrier's reads before it gives up (about a second)
 
-// 8-byte slots before the resident rows: V[2], W, one row of R, S by parts and a_{i,k+1} of own rows
-__host__ __device__ inline size_t tdg_fixed(int n, int G) {
-    return 4 * (size_t)n + (kTdgParts + 1) * (size_t)((n + G - 1) / G) + kTdfWarps + 16;
+// 8-byte slots before the resident rows (H CTAs with rows): V[2], W, one row of R, S by parts and
+// a_{i,k+1} of own rows
+__host__ __device__ inline size_t tdg_fixed(int n, int H) {
+    return 4 * (size_t)n + (kTdgParts + 1) * (size_t)((n + H - 1) / H) + kTdfWarps + 16;
 }
 __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_grid(const DyJob *jobs, int nlim, int smem_df, double *work,
                                                                  const long long *work_first) {
@@ -727,30 +735,33 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_grid(const DyJob *jo
     __syncthreads();
     const int n = J.nc, D = J.D;
     if (n < kTdgMin || n > nlim) return;   // another kernel's (the whole grid leaves)
-    const int nrm = (n + G - 1) / G, nr = rank < n ? (n - rank + G - 1) / G : 0;   // own rows i = rank + q G
+    const int H = G - D;   // CTAs with rows of the matrix; the others have row rank - H of R
+    const bool own_r = rank >= H;
+    const int nrm = (n + H - 1) / H, nr = !own_r && rank < n ? (n - rank + H - 1) / H : 0;   // own rows i = rank + q H
     extern __shared__ double sm[];
     df *V = reinterpret_cast<df *>(sm);          // [2][n]
     df *w = V + 2 * (size_t)n;                   // [n]
-    df *R = w + n;                               // [n] row rank of R, if rank < D
-    df *rs = R + n;                              // [kTdgParts][nrm] parts of S of own rows
+    double *R = reinterpret_cast<double *>(w + n);   // [n] the own row of R
+    df *rs = reinterpret_cast<df *>(R + n);      // [kTdgParts][nrm] parts of S of own rows
     df *ra = rs + (size_t)kTdgParts * nrm;       // [nrm] a_{i,k+1}
     df *sb = ra + nrm;                           // [kTdfWarps] partials of |x_1:|^2
-    df *rows = reinterpret_cast<df *>(sm) + tdg_fixed(n, G);
-    const int room = max(0, (smem_df - (int)tdg_fixed(n, G)) / n);
+    df *rows = reinterpret_cast<df *>(sm) + tdg_fixed(n, H);
+    const int room = max(0, (smem_df - (int)tdg_fixed(n, H)) / n);
     const int qs = max(0, nr - room);            // own rows q >= qs in shared memory
     double *wk = work + work_first[0];
     df *spill = reinterpret_cast<df *>(wk);
-    auto row = [&](int q) -> df * { return q >= qs ? rows + (size_t)(q - qs) * n : spill + (size_t)(rank + q * G) * n; };
+    auto row = [&](int q) -> df * { return q >= qs ? rows + (size_t)(q - qs) * n : spill + (size_t)(rank + q * H) * n; };
     df *Yx = reinterpret_cast<df *>(wk + tdg_exchange(J.n)), *Bx = Yx + 2 * (size_t)n, *Kx = Bx + 2 * (size_t)n;
     unsigned *count = reinterpret_cast<unsigned *>(wk + tdg_count(J.n));
-    __shared__ df s_sc[2], s_rd, s_c;   // tau, s of the step; R_d . x of the own R row, -tau R_d . v
-    __shared__ df s_k[2];               // -(tau^2 / 2) v^T A v, w_{k+1}
-    const df zero{0.0f, 0.0f}, one{1.0f, 0.0f};
-    const bool own_r = rank < D;
+    __shared__ df s_sc[2];              // h, v_0 of the step
+    __shared__ float s_g;               // and the power of two that scales x
+    __shared__ double s_rd[kTdfWarps], s_c;   // parts of R_d . x of the own R row, -h R_d . v
+    __shared__ df s_k[2];               // -(h^2 / 2) v^T A v, w_{k+1}
+    const df zero{0.0f, 0.0f};
     auto put = [](double *p, df x) { *reinterpret_cast<float2 *>(p) = make_float2(x.h, x.l); };
     auto far = [](const df *p) { const float2 f = __ldcg(reinterpret_cast<const float2 *>(p)); return df{f.x, f.y}; };
     for (int q = warp; q < nr; q += kTdfWarps) {
-        const int i = rank + q * G;
+        const int i = rank + q * H;
         df *a = row(q);
         for (int j = lane; j < n; j += 32) a[j] = df_from_bits(__ldcg(J.A + (j <= i ? (size_t)i * n + j : (size_t)j * n + i)));
     }
@@ -760,7 +771,7 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_grid(const DyJob *jo
         V[j] = xj;
         V[n + j] = zero;
         w[j] = zero;
-        R[j] = (j == rank) ? one : zero;
+        R[j] = (j == rank - H) ? 1.0 : 0.0;
         if (j >= 2) sq0 = dfm::fma(xj, xj, sq0);
     }
     sq0 = dfm::warp_sum(sq0);
@@ -772,50 +783,28 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_grid(const DyJob *jo
         df *x = V + (size_t)cur * n, *vp = V + (size_t)(cur ^ 1) * n;
         df *yk = Yx + (size_t)cur * n, *bk = Bx + (size_t)cur * n, *kb = Kx + (size_t)cur * kTdgMax;
         const int b0 = k + 1;
-        const int q0 = b0 <= rank ? 0 : (b0 - rank + G - 1) / G;   // first own row >= b0
+        const int q0 = b0 <= rank ? 0 : (b0 - rank + H - 1) / H;   // first own row >= b0
         const int na = max(0, nr - q0);
         const int np = 4 * na <= kTdgRowWarps ? 4 : 2 * na <= kTdgRowWarps ? 2 : 1;
         // pass
         if (warp == kTdScal) {
             df s2 = lane < kTdfWarps ? sb[lane] : zero;
             s2 = dfm::warp_sum(s2);
-            const df al = x[b0];
-            df tau = zero, scal = zero, beta = al;
-            if (s2.h != 0.0f || s2.l != 0.0f) {
-                const int ea = (al.h != 0.0f) ? f32_exponent(al.h) : -1000;
-                int e = max(ea, f32_exponent(s2.h) >> 1);
-                e = min(max(e, -126), 126);
-                const float sg = pow2_f32(-e);
-                const df alt{al.h * sg, al.l * sg}, s2t{(s2.h * sg) * sg, (s2.l * sg) * sg};
-                const df x2 = dfm::fma(alt, alt, s2t);   // in [1, 12)
-                const df r = dfm::rsqrt2(x2), nx = dfm::mul(x2, r);
-                const bool ng = signbit(alt.h);
-                const df aa = ng ? dfm::neg(alt) : alt;
-                tau = dfm::fma(aa, r, one);
-                df st = dfm::rcp2(dfm::add(aa, nx));   // 1 / (alpha~ - beta~)
-                if (ng) st = dfm::neg(st);
-                scal = df{st.h * sg, st.l * sg};         // 1 / (alpha - beta)
-                const df bt = ng ? nx : dfm::neg(nx);
-                const float un = pow2_f32(e);
-                beta = df{bt.h * un, bt.l * un};
-            }
+            const Reflector r = reflector(x[b0], s2);
             if (lane == 0) {
-                s_sc[0] = tau;
-                s_sc[1] = scal;
-                if (rank == 0) { put(J.e + k, beta); put(J.tau + k, tau); }
+                s_sc[0] = r.h;
+                s_sc[1] = r.v0;
+                s_g = r.g;
+                if (rank == 0) put(J.e + k, r.beta);
             }
-        } else if (warp == kTdScal - 1) {
-            if (own_r) {   // R_d . x_{1:}
-                df s0 = zero, s1 = zero;
-                int j = b0 + 1 + lane;
-                for (; j + 32 < n; j += 64) { s0 = dfm::fma(R[j], x[j], s0); s1 = dfm::fma(R[j + 32], x[j + 32], s1); }
-                if (j < n) s0 = dfm::fma(R[j], x[j], s0);
-                s0 = dfm::warp_sum(dfm::add(s0, s1));
-                if (lane == 0) s_rd = s0;
-            }
+        } else if (own_r) {   // R_d . x_{1:}
+            double t = 0.0;
+            for (int j = b0 + 1 + tid; j < n; j += 32 * kTdScal) t = fma(R[j], df_value(x[j]), t);
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            if (lane == 0) s_rd[warp] = t;
         } else {
             for (int u = warp; u < na * np; u += kTdgRowWarps) {
-                const int q = q0 + u / np, part = u % np, i0 = rank + q * G;
+                const int q = q0 + u / np, part = u % np, i0 = rank + q * H;
                 df *a0 = row(q);
                 const df v0 = vp[i0], w0 = w[i0];
                 df s0 = zero, s1 = zero;   // two columns at a time
@@ -835,21 +824,22 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_grid(const DyJob *jo
             }
         }
         __syncthreads();
-        const df tau = s_sc[0], s = s_sc[1];
-        const bool nz = (tau.h != 0.0f);
-        if (warp == 0) {   // y of own rows, and their part of v . y
+        const df hs = s_sc[0], v0 = s_sc[1];
+        const float g = s_g;
+        const bool nz = (hs.h != 0.0f);
+        if (warp == 0 && !own_r) {   // y of own rows, and their part of v . y
             df kv = zero;
             for (int q = q0 + lane; q < nr; q += 32) {
-                const int i = rank + q * G;
+                const int i = rank + q * H;
                 df S = rs[q];
                 for (int p = 1; p < np; ++p) S = dfm::add(S, rs[(size_t)p * nrm + q]);
-                const df yi = nz ? dfm::fma(s, S, ra[q]) : zero;
+                const df yi = nz ? dfm::fma(v0, ra[q], scaled(S, g)) : zero;
                 yk[i] = yi;
-                kv = (i == b0) ? dfm::add(kv, yi) : dfm::fma(dfm::mul(s, x[i]), yi, kv);
+                kv = dfm::fma((i == b0) ? v0 : scaled(x[i], g), yi, kv);
             }
             kv = dfm::warp_sum(kv);
             if (lane == 0) kb[rank] = kv;
-        } else if (b0 % G == rank) {   // row k+1
+        } else if (b0 % H == rank) {   // row k+1 (not with an R row's CTA: rank < H)
             const df *a = row(q0);
             for (int j = b0 + tid - 32; j < n; j += kTdfThreads - 32) bk[j] = a[j];
         }
@@ -882,30 +872,32 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_grid(const DyJob *jo
                 ya[h] = far(yk + j);
                 ba[h] = far(bk + j);
             }
-            const df vb = nz ? one : zero;
+            const df vb = nz ? v0 : zero;
             if (warp == 0) {
                 df ka[kTdgMax / 32];
 #pragma unroll
-                for (int h = 0; h < kTdgMax / 32; ++h) ka[h] = lane + 32 * h < G ? far(kb + lane + 32 * h) : zero;
+                for (int h = 0; h < kTdgMax / 32; ++h) ka[h] = lane + 32 * h < H ? far(kb + lane + 32 * h) : zero;
                 const df yb = far(yk + b0);
 #pragma unroll
                 for (int o = kTdgMax / 64; o > 0; o >>= 1)
 #pragma unroll
                     for (int h = 0; h < o; ++h) ka[h] = dfm::add(ka[h], ka[h + o]);
                 const df K = dfm::warp_sum(ka[0]);
-                const df tk = dfm::mul(tau, tau);
-                const df nk = dfm::neg(dfm::mul(df{0.5f * tk.h, 0.5f * tk.l}, K));
-                const df wk1 = dfm::fma(nk, vb, dfm::mul(tau, yb));
+                const df hh = dfm::mul(hs, hs);
+                const df nk = dfm::neg(dfm::mul(df{0.5f * hh.h, 0.5f * hh.l}, K));
+                const df wk1 = dfm::fma(nk, vb, dfm::mul(hs, yb));
                 if (lane == 0) { s_k[0] = nk; s_k[1] = wk1; }
-            } else if (warp == 1 && own_r && lane == 0) {
-                s_c = dfm::neg(dfm::mul(tau, dfm::fma(s, s_rd, R[b0])));
+            } else if (warp == 1 && own_r) {
+                double t = lane < kTdScal ? s_rd[lane] : 0.0;
+                for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+                if (lane == 0) s_c = -df_value(hs) * fma(df_value(v0), R[b0], (double)g * t);
             }
             __syncthreads();   // (R_{b0} changes behind it too)
             const df nK = s_k[0], wb = s_k[1];
             df sq = zero;
             auto one_row = [&](int j, df yj, df bj) {
-                const df vj = !nz ? zero : (j == b0) ? one : dfm::mul(s, x[j]);
-                const df wj = dfm::fma(nK, vj, dfm::mul(tau, yj));
+                const df vj = !nz ? zero : (j == b0) ? v0 : scaled(x[j], g);
+                const df wj = dfm::fma(nK, vj, dfm::mul(hs, yj));
                 const df t = rank2(bj, vj, wb, wj, vb);
                 w[j] = wj;
                 x[j] = vj;
@@ -913,9 +905,9 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_grid(const DyJob *jo
                 if (j > b0 + 1) sq = dfm::fma(t, t, sq);
                 if (rank == 0 && j == b0) put(J.d + b0, t);
                 if (rank == 0 && j == b0 + 1 && k + 3 == n) put(J.e + n - 2, t);
-                if (k + 3 == n && j == n - 1 && (n - 1) % G == rank)   // the last step: the last diagonal entry
+                if (k + 3 == n && j == n - 1 && (n - 1) % H == rank)   // the last step: the last diagonal entry
                     J.d[n - 1] = dfm::to_double(rank2(row(nr - 1)[n - 1], vj, wj, wj, vj));
-                if (own_r) R[j] = dfm::fma(s_c, vj, R[j]);
+                if (own_r) R[j] = fma(s_c, df_value(vj), R[j]);
             };
 #pragma unroll
             for (int h = 0; h < NA; ++h)
@@ -930,10 +922,9 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_grid(const DyJob *jo
         for (int j = tid; j < n; j += kTdfThreads) {
             auto conv = [](double *p) { const float2 f = __ldcg(reinterpret_cast<const float2 *>(p)); *p = dfm::to_double(df{f.x, f.y}); };
             if (j + 1 < n) { conv(J.d + j); conv(J.e + j); } else J.e[j] = 0.0;
-            if (j + 2 < n) conv(J.tau + j); else J.tau[j] = 0.0;
         }
     if (own_r)
-        for (int j = tid; j < n; j += kTdfThreads) J.R[(size_t)rank * n + j] = dfm::to_double(R[j]);
+        for (int j = tid; j < n; j += kTdfThreads) J.R[(size_t)(rank - H) * n + j] = R[j];
 }
 
 // the kernel for a cluster size (1, 2, 4, 8 or 16)
@@ -1279,7 +1270,7 @@ static int grid_ctas() {
 
 // One matrix in the launch, of an order that k_tridiag_grid may take
 static bool tridiag_on_grid(int njobs, int nmax, int nlim) {
-    return njobs == 1 && std::min(nmax, nlim) >= kTdgMin && grid_ctas() > 0;
+    return njobs == 1 && std::min(nmax, nlim) >= kTdgMin && grid_ctas() > 8;
 }
 
 // Kernels launch_dyson starts for matrices of order up to nmax: deflate, assemble, the
