@@ -101,6 +101,110 @@ __device__ __forceinline__ void long_dots(FixedSum (&acc)[4], const int *const (
     }
 }
 
+// Whether one of the n pivots (of D) has couplings that the ones before it span but for the part tol of
+// their square: elimination in the pivots' order of their Gram matrix, from the orbitals' (G, lower
+// triangle).  A warp; H holds n^2 values.
+template <typename T>
+__device__ bool pivots_depend(const T *G, const double *piv, int n, int D, T *H, T tol, int lane) {
+    for (int e = lane; e < n * n; e += 32) {
+        const double *a = piv + e / n * D, *b = piv + e % n * D;
+        T s = 0;
+        for (int c = 0; c < D; ++c) {
+            T t = 0;
+            for (int d = 0; d < D; ++d) t += G[c >= d ? c * (c + 1) / 2 + d : d * (d + 1) / 2 + c] * (T)b[d];
+            s += (T)a[c] * t;
+        }
+        H[e] = s;
+    }
+    __syncwarp();
+    const T own = lane < n ? H[lane * n + lane] : (T)0;
+    for (int q = 0; q < n; ++q) {
+        const T p = H[q * n + q];
+        if (!(p > tol * __shfl_sync(0xffffffffu, own, q))) return true;   // the same in every lane
+        const T inv = (T)1 / p;
+        for (int e = lane; e < n * n; e += 32) {
+            const int a = e / n, b = e % n;
+            if (a > q && b > q) H[e] -= H[a * n + q] * inv * H[q * n + b];
+        }
+        __syncwarp();
+    }
+    return false;
+}
+
+// The CTA's sums of m_a m_b over its poles into G (shared memory), warp after warp.
+template <typename T, typename Coupling>
+__device__ __forceinline__ void long_gram(int S, int D, double *G, Coupling coupling) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    T g[kGramEntries];
+#pragma unroll
+    for (int u = 0; u < kGramEntries; ++u) g[u] = 0;
+    for (int i = tid; i < S; i += kLongThreads) {
+        T m[8];
+#pragma unroll
+        for (int d = 0; d < 8; ++d) m[d] = d < D ? coupling(d, i) : (T)0;
+#pragma unroll
+        for (int a = 0; a < 8; ++a)
+#pragma unroll
+            for (int b = 0; b <= a; ++b)
+                if (a < D) g[a * (a + 1) / 2 + b] += m[a] * m[b];
+    }
+    T own[2] = {0, 0};   // entries lane and lane + 32
+#pragma unroll
+    for (int u = 0; u < kGramEntries; ++u)
+        if (u < D * (D + 1) / 2) {
+            T x = g[u];
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+            if (lane == (u & 31)) own[u >> 5] = x;
+        }
+    for (int q = 0; q < kMaxWarps; ++q) {
+        if (warp == q) {
+            G[lane] = (q ? G[lane] : 0.0) + (double)own[0];
+            if (lane + 32 < kGramEntries) G[lane + 32] = (q ? G[lane + 32] : 0.0) + (double)own[1];
+        }
+        __syncthreads();
+    }
+}
+
+// Whether the chain's pivots depend on one another, from their couplings: FP32 sums tell nearly all sets that
+// do not, FP64 ones the rest.  The whole cluster, with the same answer; sm: 160 doubles.
+__device__ __noinline__ bool couplings_depend(const LzChain &C, int S, int i0, double *sm) {
+    cg::cluster_group cluster = cg::this_cluster();
+    const int CL = (int)cluster.num_blocks(), lane = threadIdx.x & 31, n = min(C.n_used, 9);
+    double *mine = sm, *all = sm + 36, *H = sm + 72;   // (H: 81)
+    int *flag = reinterpret_cast<int *>(sm + 156);
+    const double *cp = C.M + i0;
+    const int own = min(S, C.N - i0);
+    auto coupling = [&](int d, int i) { return i < own ? cp[(size_t)d * C.N + i] : 0.0; };
+    for (int pass = 0; pass < 2; ++pass) {
+        if (pass == 0) long_gram<float>(S, C.D, mine, [&](int d, int i) { return f32_trunc(coupling(d, i)); });
+        else long_gram<double>(S, C.D, mine, coupling);
+        cluster.sync();
+        if (threadIdx.x < 36) {
+            double x = 0.0;
+            for (int r = 0; r < CL; ++r) x += cluster.map_shared_rank(mine, r)[threadIdx.x];
+            all[threadIdx.x] = x;
+        }
+        cluster.sync();   // (peers have read mine)
+        if (threadIdx.x < 32) {
+            bool d;
+            if (pass == 0) {
+                float *G = reinterpret_cast<float *>(mine);
+                for (int u = lane; u < 36; u += 32) G[u] = (float)all[u];
+                __syncwarp();
+                d = pivots_depend<float>(G, C.piv, n, C.D, reinterpret_cast<float *>(H), 1e-4f, lane);
+            } else {
+                d = pivots_depend<double>(all, C.piv, n, C.D, H, 1e-13, lane);
+            }
+            if (lane == 0) *flag = d;
+        }
+        __syncthreads();
+        const bool dep = *flag != 0;
+        __syncthreads();
+        if (!dep) return false;
+    }
+    return true;
+}
+
 }  // namespace
 
 // CTAs a chain where the slices are in shared memory: at one CTA an SM the GPCs hold 15 clusters of
@@ -185,6 +289,12 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
         cluster.sync();   // peers have read s_rng (a CTA that leaves frees its shared memory)
         if (!fixed_range(me) || !fixed_range(mm)) return;
     }
+    const int Qg = C.gE ? C.gInfo[0] : 0;
+    const int dtot = Qg > 0 ? C.gInfo[Qg] : 0;
+    // Pivots that depend on one another (an orbital that couples to nothing among them) end a chain in a
+    // restart vector where no unreached direction is left: k_lanczos's from the start, not after rows of it
+    // here (20 000 poles, the last orbital the first less the second: 6.5 ms; 5.5 by k_lanczos alone).
+    if (dtot == 0 && couplings_depend(C, S, i0, sm)) return;
     int nvec = 0;
     // planes of stored vector t: a at the address, b C.ld behind it
     int *Vg = reinterpret_cast<int *>(C.V) + i0;
@@ -212,8 +322,6 @@ __global__ void __launch_bounds__(kLongThreads, 1) k_lz_long(const LzChain *chai
         *reinterpret_cast<int2 *>(ws + i) = make_int2(x.x, y.x);
         *reinterpret_cast<int2 *>(ws + S + i) = make_int2(x.y, y.y);
     };
-    const int Qg = C.gE ? C.gInfo[0] : 0;
-    const int dtot = Qg > 0 ? C.gInfo[Qg] : 0;
     auto group_of = [&](int d) {
         int lo = 0, hi = Qg - 1;
         while (lo < hi) { const int mid = (lo + hi) >> 1; if (C.gInfo[1 + mid] > d) hi = mid; else lo = mid + 1; }

@@ -204,3 +204,32 @@ def test_elements_of_one_size(bdmod, overlap):
     assert abs(got[1, 1] - g) < tol * 300.0
     assert abs(got[1, 3]) < tol * np.sqrt(N)          # <M_0|u>, nothing
     assert abs(got[1, 4] - np.dot(M[1], u)) < tol * np.sqrt(N)
+
+
+# pivots whose couplings depend on one another: exactly, through a combination, but for 1e-5 of them (the FP64 sums
+# tell), by an orbital that couples to nothing
+@pytest.mark.parametrize("kind", ["twice", "difference", "close", "none"])
+@pytest.mark.parametrize("N", [2500, 20011])
+def test_dependent_pivots(bdmod, N, kind):
+    rng = np.random.default_rng(N)
+    nit = 8
+    E = np.sort(rng.uniform(20.0, 300.0, N))
+    M = rng.standard_normal((3, N))
+    if kind == "twice":
+        M[2] = 2.0 * M[0]
+    elif kind == "difference":
+        M[2] = M[0] - M[1]
+    elif kind == "close":
+        M[2] = M[0] - M[1] + 1e-5 * M[2]
+    else:
+        M[2] = 0.0
+    got = _run(bdmod, E, M, nit)
+    assert got.shape == (3 * nit, 7) and np.isfinite(got).all()
+    n = 3 if kind == "close" else 2              # (the third chain's are restart vectors otherwise)
+    ref = _reference(E, M[:n], nit)
+    r = n * nit
+    # FP64 rounding of E v over the steps, of the couplings' remainder where they are close
+    tol = 1e-11 if kind != "close" else 1e-9
+    assert np.abs(got[:r, 0] - ref[:, 0]).max() < tol * 300.0
+    assert np.abs(got[:r, 2:1 + n] - ref[:, 2:1 + n]).max() < tol * 300.0
+    assert np.abs(got[:r, 4:4 + n] - ref[:, 1 + n:]).max() < tol * np.sqrt(N)
