@@ -1046,12 +1046,17 @@ int ensure_dyson(bd_ctx *ctx, bool lanczos) {
                 g += lz_group_bytes(dir == 0 ? ctx->chans[I].nfw : ctx->chans[I].nbk);
             }
         }
-        int rc;
-        if ((rc = dalloc(ctx, &ctx->d_dygrp, (size_t)g))) return rc;
-        if ((rc = dalloc(ctx, &ctx->d_dycp, (size_t)2 * ns * (size_t)kCpBytes))) return rc;
-        if ((rc = dalloc(ctx, &ctx->d_dychains, (size_t)2 * ns))) return rc;
-        if ((rc = dalloc(ctx, &ctx->d_dyio, (size_t)2 * ns))) return rc;
-        if ((rc = dalloc(ctx, &ctx->d_dyplain, (size_t)(ctx->tot_fw + ctx->tot_mfw + ctx->tot_bk + ctx->tot_mbk)))) return rc;
+        // in one allocation (every part a multiple of 256 bytes, the rows last), so that a failed one leaves nothing
+        auto pad = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+        const size_t cp = (size_t)2 * ns * (size_t)kCpBytes, ch = pad(sizeof(LzChain) * 2 * ns), io = pad(sizeof(PlainIO) * 2 * ns);
+        const size_t rows = sizeof(double) * (size_t)(ctx->tot_fw + ctx->tot_mfw + ctx->tot_bk + ctx->tot_mbk);
+        char *p = nullptr;
+        if (int rc = dalloc(ctx, &p, pad((size_t)g) + cp + ch + io + rows)) return rc;
+        ctx->d_dygrp = p;
+        ctx->d_dycp = p + pad((size_t)g);
+        ctx->d_dychains = reinterpret_cast<LzChain *>(ctx->d_dycp + cp);
+        ctx->d_dyio = reinterpret_cast<PlainIO *>(ctx->d_dycp + cp + ch);
+        ctx->d_dyplain = reinterpret_cast<double *>(ctx->d_dycp + cp + ch + io);
     }
     if (a > ctx->dyA_cap || v > ctx->dyvec_cap || s > ctx->dysol_cap || r > ctx->dyR_cap || w > ctx->dywork_cap) {
         graph_invalidate(ctx);
@@ -2204,7 +2209,12 @@ int bd_lanczos_vectors(bd_ctx *ctx, int ish, int dir, int fp32, double *out, lon
     const char *base = ctx->d_lzV + ctx->lz_v_off[dir][ish];
     CU(cudaStreamSynchronize(ctx->st));
     int handled = 0;
-    double *expanded = nullptr;
+    struct Expanded {   // given back on every way out
+        double *p = nullptr;
+        cudaStream_t st;
+        ~Expanded() { if (p) cudaFreeAsync(p, st); }
+    } expanded;
+    expanded.st = ctx->st;
     if (!fp32 && P.L > 0) {   // a chain reduced in its couplings' space: its vectors over the poles, formed here
         char *cp = ctx->d_lzcp + (size_t)(2 * ish + dir) * kCpBytes;
         CompactInfo info;
@@ -2216,14 +2226,14 @@ int bd_lanczos_vectors(bd_ctx *ctx, int ish, int dir, int fp32, double *out, lon
                 if ((rc = launch_sort(ctx, ish, ish + 1, C.lz_ref))) return rc;
                 C.ref_sorted = C.lz_ref;
             }
-            CU(cudaMallocAsync(&expanded, sizeof(double) * (size_t)P.L * ld, ctx->st));
+            CU(cudaMallocAsync(&expanded.p, sizeof(double) * (size_t)P.L * ld, ctx->st));
             LzChain z{};
             z.N = P.N; z.D = C.D; z.ld = ld; z.V = ctx->d_lzV + ctx->lz_v_off[dir][ish]; z.cp = cp;
             z.M = (dir == 0 ? ctx->d_Mfw_s : ctx->d_Mbk_s) + (dir == 0 ? C.mfw_off : C.mbk_off);
-            CU(launch_lz_expand(z, expanded, ctx->st));
+            CU(launch_lz_expand(z, expanded.p, ctx->st));
             ctx->launches += 1;
             CU(cudaStreamSynchronize(ctx->st));
-            base = reinterpret_cast<const char *>(expanded);
+            base = reinterpret_cast<const char *>(expanded.p);
         }
     }
     // rows of a deflated tail have no stored vector: zero rows
@@ -2250,7 +2260,6 @@ int bd_lanczos_vectors(bd_ctx *ctx, int ish, int dir, int fp32, double *out, lon
         for (int j = 0; j < P.L; ++j)
             for (int i = 0; i < P.N; ++i) out[(size_t)j * P.N + i] = slot[j] < 0 ? 0.0 : tmp[(size_t)slot[j] * ld + i];
     }
-    if (expanded) CU(cudaFreeAsync(expanded, ctx->st));
     return BD_OK;
 }
 
