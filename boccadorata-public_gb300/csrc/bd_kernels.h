@@ -79,8 +79,6 @@ cudaError_t launch_nonfinite(const double *x, long long n, int *bad, cudaStream_
 constexpr int kHeapMax = 49152;  // longest channel put in the reference's heap-sort order
 cudaError_t launch_heap_order(const double *E, const int *d_off, int nseg, int max_len, long long n0, int *perm,
                               cudaStream_t st);
-__global__ void k_chunk_place(const unsigned long long *tk, const int *ti, const int4 *chunks, int nchunks,
-                              long long n, long long base, int *perm);
 __global__ void k_pair_rank(const int *iabJ, const int *icdJ, int n, int norb, const int *orb_sh, const int *ch,
                             const int *ip, const int *seg_str, int nJ, int *prank);
 __global__ void k_pole_index(const int *off, int ns, long long n, int *seg, int *idx);
@@ -104,7 +102,7 @@ cudaError_t launch_plain_rotate(const LzChain *d_chains, const PlainIO *d_ios, i
 void compact_smem_init();
 // FP64 vectors, long chains (k_lanczos_long.cu): chains with done set and at least nmin
 // poles (lz_long_from), before launch_lanczos.  lanczos_long_form: which form of it takes a chain, 0 none
-// (rows beyond shared memory), 1 slices in shared memory, 2 in the chain.s scratch; forms: all of
+// (rows beyond shared memory), 1 slices in shared memory, 2 in the chain's scratch; forms: all of
 // a launch (1 | 2).  Their stored vectors are two planes of integers (k_lanczos_long.cu) per slot.
 int lanczos_long_form(int N, int rmax, int cluster);
 cudaError_t launch_lanczos_long(const LzChain *d_chains, int nchains, int rmax, int nmin, int cluster, double eta, int forms,

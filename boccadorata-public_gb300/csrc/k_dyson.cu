@@ -1231,13 +1231,6 @@ int tridiag_fit_order(int cluster) {
     return lo;
 }
 
-void tridiag_fit_warm() {
-    for (int c = 1; c <= 16; c <<= 1) tridiag_fit_order(c);
-    allow_dynamic_smem((const void *)k_tridiag_small);
-    allow_dynamic_smem((const void *)k_tridiag);
-    for (int c = 1; c <= 16; c <<= 1) allow_dynamic_smem((const void *)tridiag_df_kernel(c));
-}
-
 // Shared memory of k_tridiag_df (8-byte slots, at most kTdfSlots: 224 KB) and the largest
 // order it takes in a launch of orders up to nmax: as far as its vectors fit (the rows may
 // spill), where all of the launch's orders leave k_tridiag room for a partial vector a warp
@@ -1266,6 +1259,15 @@ static int grid_ctas() {
         return std::min(sms, kTdgMax);
     }();
     return g;
+}
+
+void tridiag_fit_warm() {
+    for (int c = 1; c <= 16; c <<= 1) tridiag_fit_order(c);
+    allow_dynamic_smem((const void *)k_tridiag_small);
+    allow_dynamic_smem((const void *)k_tridiag);
+    for (int c = 1; c <= 16; c <<= 1) allow_dynamic_smem((const void *)tridiag_df_kernel(c));
+    allow_dynamic_smem((const void *)k_tridiag_grid);
+    grid_ctas();
 }
 
 // One matrix in the launch, of an order that k_tridiag_grid may take
