@@ -402,7 +402,7 @@ def dressed_run(bd, prob, device, z_cut=1e-3, max_frag=2):
             "mixed_lanczos": {"kernel": "k_lanczos<float> (global slices)", "kernel_ms": l32, "algorithmic_bytes": alg32,
                               "achieved_gbs": alg32 / (l32 / 1e3) / 1e9, "peak_gbs": peak,
                               "frac": alg32 / (l32 / 1e3) / 1e9 / peak, "peak_source": src},
-            "fp64_lanczos": {"kernel": "k_lanczos<double> (global slices)", "kernel_ms": l64, "algorithmic_bytes": alg64,
+            "fp64_lanczos": {"kernel": "k_lz_long (chains it leaves: k_lanczos<double>)", "kernel_ms": l64, "algorithmic_bytes": alg64,
                              "achieved_gbs": alg64 / (l64 / 1e3) / 1e9, "frac": alg64 / (l64 / 1e3) / 1e9 / peak},
             "accuracy": acc}
 

@@ -152,3 +152,35 @@ def test_orders_beyond_2300_in_fp64(bdmod, problems):
     got, ref = got[np.argsort(got[:, 0])], v[:D].T
     x = got[:, 2:] * np.where((got[:, 2:] * ref).sum(1) < 0.0, -1.0, 1.0)[:, None]
     assert np.median(np.abs(x - ref).max(1)) < 6e-15
+
+
+# more orbitals than the model spaces above have, on the cluster kernel and on the whole GPU (a row of Q each)
+@pytest.mark.parametrize("n,nmax,D", [(203, 12, 7), (305, 14, 8), (400, 12, 7), (611, 14, 8)])
+def test_seven_and_eight_orbitals(bdmod, synth, n, nmax, D):
+    ms = synth.make_modspace(nmax, 20.0)
+    prop = synth.make_unperturbed_propagator(ms)
+    none = synth.Interaction(np.zeros(1, np.int32), np.zeros(1, np.int32), np.zeros(1))
+    ctx = bdmod.Context().upload(synth.Problem(ms, prop, none, synth.make_pivots(ms, prop, 1), 0, 1.0), with_pivots=False)
+    assert int(ms.no[0]) == D
+    rng = np.random.default_rng(n)
+    nb = n // 4
+    nf = n - D - nb
+    fw, bk = np.zeros((nf, 2 + D)), np.zeros((nb, 2 + D))
+    fw[:, 0], bk[:, 0] = rng.uniform(20.0, 300.0, nf), -rng.uniform(60.0, 250.0, nb)
+    fw[:, 2:], bk[:, 2:] = rng.standard_normal((nf, D)) * 0.3, rng.standard_normal((nb, D)) * 0.3
+    s1, hf = np.diag(np.linspace(-20.0, 60.0, D)), np.zeros((D, D))
+    r = ctx.dyson_rows(0, 2, fw, bk, sig1b=s1, sighf=hf, efermi=-50.0)
+    ctx.close()
+    A = np.diag(np.concatenate([np.zeros(D), fw[:, 0], bk[:, 0]]))
+    A[:D, :D] = s1
+    A[D:, :D] = np.concatenate([fw[:, 2:], bk[:, 2:]])
+    A[:D, D:] = A[D:, :D].T
+    w, v = np.linalg.eigh(A)
+    got = np.concatenate([r["qp"], r["qh"]])
+    # as test_large_orders_against_lapack
+    np.testing.assert_allclose(np.sort(got[:, 0]), w, rtol=1e-11, atol=1e-11 * np.abs(A).sum(0).max())
+    ref = np.concatenate([w[:, None], (v[:D] ** 2).sum(0)[:, None], v[:D].T], 1)
+    e, z = strong_diffs(ref, got)
+    assert e < 1e-10 and z < 1e-8
+    x = got[:, 2:]
+    assert np.abs(x.T @ x - np.eye(D)).max() < 1e-11

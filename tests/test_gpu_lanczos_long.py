@@ -233,3 +233,26 @@ def test_dependent_pivots(bdmod, N, kind):
     assert np.abs(got[:r, 0] - ref[:, 0]).max() < tol * 300.0
     assert np.abs(got[:r, 2:1 + n] - ref[:, 2:1 + n]).max() < tol * 300.0
     assert np.abs(got[:r, 4:4 + n] - ref[:, 1 + n:]).max() < tol * np.sqrt(N)
+
+
+# many chains in a launch: the longest below the length from which k_lz_long takes them all, and above it
+@pytest.mark.parametrize("nmax,frag,long", [(6, 1, False), (4, 2, True)])
+def test_batches_on_both_sides_of_the_rule(bdmod, problems, nmax, frag, long):
+    p = problems(nmax, 20.0, 1, 12)
+    ctx = bdmod.Context().upload(p)
+    ctx.run_all(lanczos=True)
+    ctx.dressed_propagator(1e-3, frag)
+    n = [max(ctx.count_poles(i)) for i in range(p.ms.nsubsh)]
+    assert p.ms.nsubsh > 15 and max(n) > 2048 and (max(n) >= 8192) == long
+    got = []
+    for mode in (0, 1):   # 1: k_lanczos alone
+        ctx.set_lanczos_slices(mode)
+        ctx.run_all(lanczos=True)
+        got.append([ctx.result(i) for i in range(p.ms.nsubsh)])
+    for a, b in zip(*got):
+        for tag in ("qp", "qh"):
+            assert len(a[tag]) == len(b[tag])
+            e, z = strong_diffs(b[tag], a[tag])
+            assert e < 1e-10 and z < 1e-9
+        np.testing.assert_allclose(a["koltun"], b["koltun"], rtol=1e-10, atol=1e-11)
+    ctx.close()
