@@ -216,17 +216,16 @@ static_assert(kCpDim <= kFixedRun, "a chain's sums are one run");
 // group has left) is left to k_lanczos as a whole.
 //
 // A step is a chain of short phases between barriers, and an FP64 instruction holds an SM
-// sub-partition's FP64 unit for ~64 cycles, so FP64 is kept to what needs it (alpha, g, the
-// recurrence, 1/|w|): the sweep's dot products, |w|^2 and m are fixed-point sums (lz_fixed.cuh),
+// sub-partition's FP64 unit for ~64 cycles, so FP64 is kept to what needs it (w = M p, alpha, g,
+// the recurrence, 1/|w|): the sweep's dot products, |w|^2 and m are fixed-point sums (lz_fixed.cuh),
 // the update is FP32 where the coefficients are rounding-sized (|c| <= 1e-9 |w|: an error below
 // 2^-23 1e-9 |w|) and fixed point otherwise.  Stored vectors lie element by element: in the dot
 // products a lane takes a vector and the warps split the elements, in the update a thread takes
 // an element and the idle ones split the vectors, so neither sums across lanes; one warp takes
 // the decision beside the other warps' sums.
 // Measured (N_max = 10, 100 iterations per pivot): the reduction of all 84 chains takes
-// 0.30 ms against 3.59 ms in the poles' space (N_max = 12: 0.44 against 12.2); about 8 000 cycles
-// a step of a 54-coordinate chain (11 000 with a warp's lanes summing each dot product and the
-// decision after them).
+// 0.29 ms against 3.59 ms in the poles' space (N_max = 12: 0.44 against 12.2); 600 000 cycles for
+// the longest chain, 54 steps in 54 coordinates and its set-up.
 __global__ void __launch_bounds__(kCpThreads) k_lz_compact(const LzChain *chains, int nchains, double eta2) {
     const int cid = blockIdx.x;
     if (cid >= nchains) return;

@@ -93,8 +93,8 @@ __device__ inline void dy_mark_branch_starts(const DyJob &J, int r, int *flag) {
 
 constexpr int kTdgMax = 256;   // CTAs of k_tridiag_grid at most
 // Its smallest order: a column costs it about the same at any order below 700, the cluster kernel's
-// 16 CTAs less up to orders of 350 (a solve of 300: 2.25 against 2.14 ms, 400: 2.90 and 2.99, 500: 3.6
-// and 4.0)
+// 16 CTAs less up to orders of 350 (a solve of 300: 2.22 against 2.12 ms, 350: 2.52 and 2.55, 400: 2.83
+// and 3.00, 500: 3.51 and 4.12)
 constexpr int kTdgMin = 384;
 // the exchange area in a job's work space (5 n^2 doubles, the spilled rows in the first n^2):
 // y[2][n], row k+1 [2][n], parts of v^T A v [2][kTdgMax], the barrier's count (zeroed by
@@ -402,8 +402,9 @@ __global__ void __launch_bounds__(kTdThreads) k_tridiag(const DyJob *jobs, int n
 // Bound by these two cluster barriers and the chains between them (about 4 000 cycles a
 // column) up to orders of a few hundred, by the FP32 pipe (41 instructions an element)
 // beyond.  Against the two passes from L2 with eight warps that this replaced, and k_qrows
-// for R (one CTA, FP64, a pass of its own): order 1 000 alone on 16 CTAs 34.4 + 6.4 -> 12.8 ms,
-// a batch of orders up to 205 on 8 CTAs each 1.99 + 0.96 -> 0.68 ms.
+// for R (one CTA, FP64, a pass of its own): order 1 000 alone on 16 CTAs 34.4 + 6.4 -> 13.0 ms,
+// a batch of orders up to 205 on 8 CTAs each 1.99 + 0.96 -> 0.69 ms (0.68 with R in double-float and v
+// rounded, which took an eigenvector's components 3 to 11 % further off).
 namespace {
 
 // x as hi + lo from its bits: hi the double truncated to FP32, lo the next bits of the
@@ -712,9 +713,9 @@ __global__ void __launch_bounds__(kTdfThreads, 1) k_tridiag_df(const DyJob *jobs
 //   all rows  v, w, R; from row k+1, which is column k+1, that column after this step's update (x
 //             of the next step, d_{k+1} on the diagonal), and the sum of its squares, by every CTA
 //             for itself
-// Bound by the barrier and what surrounds it in a column (order 1 000, 9 000 cycles: the pass beside
-// the scalars' chain 3 000, y 1 000, the barrier 3 200, then L2, the sum of the parts, v and w).
-// Order 1 000: 12.8 ms by the cluster kernel -> 4.7.
+// Bound by the barrier and what surrounds it in a column (order 1 000, 9 900 cycles: of 9 000 in an
+// earlier form the pass beside the scalars' chain was 3 000, y 1 000, the barrier 3 200, then L2, the
+// sum of the parts, v and w).  Order 1 000: 13.0 ms by the cluster kernel -> 4.8.
 constexpr int kTdgRowWarps = kTdfWarps - 1;   // the other: the scalars
 constexpr int kTdgParts = 4;                  // warps a row at most
 constexpr int kTdgPolls = 1 << 20;            // a barrier's reads before it gives up (about a second)

@@ -31,10 +31,10 @@
 // state is read from shared memory where it is used and the loads in flight are unconditional
 // (with 250 bytes a thread spilled the step below took 9.4 ms).
 // Bound by the planes' traffic and the phases around it in batches (12 bytes a stored element
-// and step: 2.1 M poles in 52 chains, 20 iterations a pivot, 18.3 -> 7.7 ms against 3.2 at the
+// and step: 2.1 M poles in 52 chains, 20 iterations a pivot, 18.3 -> 7.6 ms against 3.2 at the
 // copy bandwidth; two thirds of a 41 000-pole chain's step are the sweep's loads, a fifth the
 // FP64 instructions) and by the chain of phases for one chain on its 16 SMs (20 000 poles, 80
-// vectors: the call 5.36 -> 2.26 ms).  FP64 dot products took 17.1 and 4.2 ms, double-float ones
+// vectors: the call 5.36 -> 2.27 ms).  FP64 dot products took 17.1 and 4.2 ms, double-float ones
 // formed from the doubles' bits 12.5 and 3.1 (off by 2e-15 |w| where this is off by 5e-16, as
 // FP64 is).
 #include <algorithm>
